@@ -687,6 +687,7 @@ void matmul_grouped(const Coef &c, const std::vector<GroupedItem> &items, cudaSt
 }
 
 void BseOperator::check_errors(cudaStream_t s) {
+  ws.check();
   if (mixed) mixed->check(s);
 }
 

@@ -281,6 +281,7 @@ struct DenseApply : DeviceOperator {
     if (ham) op->ham_matmul(X, ldx, k, Y, ldy, s); else op->matmul(X, ldx, k, Y, ldy, s);
   }
   void diagonal(double *D, cudaStream_t s) override;
+  void check(cudaStream_t) override { op->ws.check(); }
 };
 
 // Combine kernel for the HamiltonianOperator reshaping trick

@@ -37,6 +37,7 @@ struct bse_handle {
   void check_errors(cudaStream_t s) {
     if (kind == 0) bse->check_errors(s);
     else if (kind == 2) uks->check_errors(s);
+    else dense->ws.check();
   }
 };
 

@@ -266,6 +266,10 @@ struct Ctx {
   cudaStream_t s;
   int64_t n;
   GemmWorkspace ws;
+  // Split-precision solves keep the FMA kernel's order of operations: one bit of a trial vector
+  // can move a bf16 rounding of the next split product, which the returned eigenvectors show at
+  // 1e-10 (2e-10 with digit products here, against 4e-13 in an FP64 solve).
+  int gemm_path = 0;
   DeviceBuffer<double> red_partial, scal, gs_part;
   DeviceBuffer<unsigned> gs_bar;
   DeviceBuffer<int> gs_err;
@@ -295,7 +299,7 @@ struct Ctx {
     g.M = m; g.N = nc; g.K = rows < 0 ? n : rows;
     g.a_colmajor(A, lda, true).b_colmajor(B, ldb, false).c_colmajor(C, ldc);
     g.alpha = alpha; g.beta = beta;
-    dgemm(g, s, &ws);
+    dgemm(g, s, &ws, gemm_path);
   }
   // C (n x nc) = alpha * A (n x k) B (k x nc) + beta C
   void gemm_nn(const double *A, int64_t lda, int64_t k, const double *B, int64_t ldb, int64_t nc,
@@ -304,7 +308,7 @@ struct Ctx {
     g.M = n; g.N = nc; g.K = k;
     g.a_colmajor(A, lda, false).b_colmajor(B, ldb, false).c_colmajor(C, ldc);
     g.alpha = alpha; g.beta = beta;
-    dgemm(g, s, &ws);
+    dgemm(g, s, &ws, gemm_path);
   }
   void copy_cols(const double *src, int64_t lds, double *dst, int64_t ldd, int64_t ncols) {
     if (ncols <= 0) return;
@@ -587,6 +591,7 @@ bool fp64_polish(Ctx &x, TimedApply &apply, const double *Dd, const double *q0, 
     VGB_CUDA(cudaMemcpyAsync(lam.data(), lamd.get(), np * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (!ham) VGB_CUDA(cudaMemcpyAsync(&einfo_h, einfo.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     std::vector<double> resn = to_host(work.get() + np, np);
+    x.ws.check();
     if (einfo_h != 0) fail(BSE_ERR_NUMERICAL, "Small hermitian eigenvalue problem failed.");
     double maxres = 0.0;
     std::vector<int64_t> upd;
@@ -714,6 +719,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
   Ctx x;
   x.s = s;
   x.n = n;
+  x.gemm_path = A.split_precision() ? kFmaSplits : 0;
   DeviceBuffer<double> V(n * capc), AV(n * capc), AAV, D(n), q, res, Ud, tmp, lamd, work, cbuf;
   // the projected matrices stay on the device (ld capc): T = V^T A V and, for HAM, B = V^T A A V
   DeviceBuffer<double> Td(capc * capc), Bd, eigw;
@@ -826,6 +832,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
     VGB_CUDA(cudaMemcpyAsync(lam.data(), lamd.get(), needed * sizeof(double), cudaMemcpyDeviceToHost, s));
     VGB_CUDA(cudaMemcpyAsync(einfo_h, einfo.get(), (ham ? 2 : 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
     VGB_CUDA(cudaStreamSynchronize(s));
+    x.ws.check();
     if (!ham && einfo_h[0] != 0) fail(BSE_ERR_NUMERICAL, "Small hermitian eigenvalue problem failed.");
     if (ham && einfo_h[0] == 4)
       fail(BSE_ERR_NUMERICAL, "Eigenvalue:" + std::to_string(einfo_h[1]) + " is complex but has no partner.");

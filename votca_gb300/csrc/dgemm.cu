@@ -2,6 +2,9 @@
 #include "dgemm.cuh"
 
 #include <mutex>
+#include <vector>
+
+#include "oz_gemm.cuh"
 
 namespace vgb {
 
@@ -206,10 +209,51 @@ int sm_count() {
   return n;
 }
 
+namespace {
+
+// Error slots of the workspaces: ints of one page-locked allocation that is kept for the process,
+// handed out and taken back.
+struct SlotPool {
+  std::mutex mu;
+  std::vector<int *> free;
+} g_slots;
+constexpr int kSlotPage = 1024;
+
+}  // namespace
+
+int *GemmWorkspace::error_slot() {
+  if (slot_) return slot_;
+  std::lock_guard<std::mutex> lk(g_slots.mu);
+  if (g_slots.free.empty()) {
+    int *page = nullptr;
+    VGB_CUDA(cudaHostAlloc((void **)&page, kSlotPage * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    for (int i = 0; i < kSlotPage; ++i) g_slots.free.push_back(page + i);
+  }
+  slot_ = g_slots.free.back();
+  g_slots.free.pop_back();
+  *slot_ = 0;
+  return slot_;
+}
+
+GemmWorkspace::~GemmWorkspace() {
+  if (!slot_) return;
+  std::lock_guard<std::mutex> lk(g_slots.mu);
+  g_slots.free.push_back(slot_);
+}
+
+void GemmWorkspace::check() {
+  if (!slot_) return;
+  const int code = *(volatile int *)slot_;
+  if (code == 0) return;
+  *slot_ = 0;
+  fail(BSE_ERR_TIMEOUT, "tensor-core FP64 GEMM: a bounded pipeline wait gave up (code " + std::to_string(code) + ")");
+}
+
 void dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws, int splitk) {
   VGB_REQUIRE(d.M >= 0 && d.N >= 0 && d.K >= 0, "dgemm: negative size");
   const int64_t nbatch = d.nb1 * d.nb2;
   if (d.M == 0 || d.N == 0 || nbatch == 0) return;
+  if (splitk == 0 && oz_dgemm(d, stream, ws)) return;
   if (d.K == 0) {  // C = beta * C
     const int64_t total = d.M * d.N * nbatch;
     scale_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream>>>(d, nbatch);

@@ -1,0 +1,28 @@
+// FP64 GEMM on the 5th-generation tensor cores: exact products of digit planes.
+//
+// GB300 runs FP64 at 2 FMA per clock and SM (1.2 TFLOP/s), 1600 times slower than its bf16 tensor
+// rate, so an FP64 contraction large enough to fill the chip is cheaper as many exact bf16 products
+// (Ozaki, Ogita, Oishi, Rump, Numer. Algorithms 59 (2012) 95-118; Mukunoki, Ozaki, Ogita, Imamura,
+// ISC 2020).  Every row of either operand is cut, per run of 1024 K elements, into seven balanced
+// base-256 digits (55 bits and sign below the run's largest element) held as bf16 planes; the
+// products of planes a and b with a + b <= 7 (34 of 49) are accumulated in FP32, exactly, and the
+// level sums are added as float pairs and written as FP64 values.  The relative error of a
+// contraction (6e-17 to 2e-16 of its 2-norm over Gaussian, graded and six-decade inputs) is below
+// that of the FMA chain it replaces (2e-16 to 1e-15 on the same inputs), which is why 34 pairs
+// are kept: the 28 pairs with a + b <= 6 lose to the chain on inputs graded over both operands
+// (1.3e-15 and 1.8e-15 against 7.7e-16).
+//
+// Measured on a GB300, FMA kernel against this one (L2 flushed between runs): 4096^3 110 ms and
+// 3.0 ms (46 TFLOP/s of FP64 results), the Hd stage 1 of eight vectors of v64 c512 and 256
+// auxiliary functions 55.3 and 2.2 ms, 1000^3 2.03 and 0.13 ms.
+#pragma once
+
+#include "dgemm.cuh"
+
+namespace vgb {
+
+// Runs d on the tensor cores when it is large enough and of a form they take (see oz_gemm.cu);
+// false: nothing was launched.  Stream-ordered; takes its scratch from ws (grown on demand).
+bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws);
+
+}  // namespace vgb

@@ -157,6 +157,7 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
   VGB_LAUNCH_CHECK();
   VGB_CUDA(cudaMemcpyAsync(eps_host, eps.get(), naux * naux * sizeof(double), cudaMemcpyDeviceToHost, s));
   VGB_CUDA(cudaStreamSynchronize(s));
+  ws.check();
 }
 
 void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_host, int64_t ldi,
@@ -231,6 +232,7 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
   VGB_CUDA(cudaMemcpy2DAsync(inv_host, ldi * sizeof(double), A.get(), n * sizeof(double),
                              n * sizeof(double), n, cudaMemcpyDeviceToHost, s));
   VGB_CUDA(cudaStreamSynchronize(s));
+  ws.check();
 }
 
 void mmn_multiply_right(const bse_mmn_desc &desc, double *const *slices, const double *U_host,
@@ -259,6 +261,7 @@ void mmn_multiply_right(const bse_mmn_desc &desc, double *const *slices, const d
       VGB_CUDA(cudaMemcpyAsync(slices[m0 + i], out.get() + i * per, per * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
     VGB_CUDA(cudaStreamSynchronize(s));
+    ws.check();
   }
 }
 
@@ -292,6 +295,7 @@ void positive_inverse(int64_t n, const double *a_host, int64_t lda, double cutof
   VGB_CUDA(cudaMemcpy2DAsync(inv_host, ldi * sizeof(double), dW.get(), n * sizeof(double), n * sizeof(double), n,
                              cudaMemcpyDeviceToHost, s));
   VGB_CUDA(cudaStreamSynchronize(s));
+  ws.check();
 }
 
 }  // namespace vgb

@@ -42,6 +42,7 @@ void spectral_product(int64_t n, const std::vector<double> &U, const std::vector
   g.C = d_out; g.c_rs = 1; g.c_cs = n;
   dgemm(g, s, &ws);
   VGB_CUDA(cudaStreamSynchronize(s));  // the host staging goes out of scope
+  ws.check();
 }
 
 // f_i = 1/sqrt(lambda_i) for lambda_i >= etol, else 0 (the function is removed)
@@ -121,6 +122,7 @@ void aux_pseudo_inv_sqrt_gwbse(int64_t n, const double *S, int64_t lds, const do
   VGB_CUDA(cudaMemcpy2DAsync(out, ldo * sizeof(double), T.get(), n * sizeof(double), n * sizeof(double), n,
                              cudaMemcpyDeviceToHost, s));
   VGB_CUDA(cudaStreamSynchronize(s));
+  ws.check();
   if (removed) *removed = rem;
 }
 
@@ -167,6 +169,7 @@ void fill_3c_mo(const bse_mmn_desc &desc, double *const *slices, const double *a
       VGB_CUDA(cudaMemcpyAsync(slices[m] + p0 * nt, R.get() + m * cnt * nt, cnt * nt * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
     VGB_CUDA(cudaStreamSynchronize(s));  // A, T and R are reused by the next chunk
+    ws.check();
   }
 }
 
@@ -225,6 +228,7 @@ void transition_dipoles(const double *ao_dip, int64_t nbf, const double *C, int6
     }
     VGB_CUDA(cudaMemcpyAsync(out.data(), R.get(), 3 * nstates * sizeof(double), cudaMemcpyDeviceToHost, s));
     VGB_CUDA(cudaStreamSynchronize(s));
+    ws.check();
   }
   for (int64_t t = 0; t < 3 * nstates; ++t) dip[t] = accumulate ? dip[t] + out[t] : out[t];
 }
