@@ -61,3 +61,11 @@ extern "C" int oz_plan_run(const int64_t *v, const double *A, const double *B, d
   out[6] = q.kb_per; out[7] = q.nkb; out[8] = q.faster;
   return 1;
 }
+
+// the FMA plan: tile, splits, K elements per split, and the fixed split rule
+extern "C" void fma_plan_of(const int64_t *v, int64_t sms, int32_t splitk, int64_t *out) {
+  GemmDesc d;
+  d.M = v[0]; d.N = v[1]; d.K = v[2]; d.nb1 = v[3];
+  const vgb::FmaPlan f = vgb::fma_plan(d, (int)sms, splitk);
+  out[0] = f.tm; out[1] = f.tn; out[2] = f.splits; out[3] = f.kchunk; out[4] = vgb::fma_chain_splits(d, (int)sms);
+}

@@ -1,4 +1,4 @@
-"""The FP64 products that run as exact digit products on the tensor cores (csrc/oz_gemm.cu), through
+"""FP64 products: the FMA kernel's tiles (small operators), and the products that run as exact digit products on the tensor cores (csrc/oz_gemm.cu), through
 the dense operator (C = A X at any size) and the auxiliary-metric product (a batched form).
 
 Bound: an element is rounded to 55 bits below its run's largest element, |dx| <= 2^-55 max|x|, so
@@ -21,6 +21,20 @@ def _bound(A, X):
 
 def _exact(A, X):
     return A.astype(np.longdouble) @ X.astype(np.longdouble)
+
+
+# n and k around the FMA kernel's tiles (16, 32, 64) and its K step (16) and splits; its error is
+# that of a K-term chain, K 2^-53 sum |a||x|
+@pytest.mark.parametrize("n", [1, 15, 17, 33, 48, 65, 100, 129])
+@pytest.mark.parametrize("k", [1, 16, 17, 33, 65])
+def test_fma_tiles(n, k):
+    rng = np.random.default_rng(100 * n + k)
+    A, X = rng.standard_normal((n, n)), rng.standard_normal((n, k))
+    op = bo.DenseGpuOperator(A)
+    Y = op.matmul(X)
+    op.close()
+    err = np.abs(Y - _exact(A, X)).astype(np.float64)
+    assert np.all(err <= n * 2.0**-53 * (np.abs(A) @ np.abs(X)) + 2.0**-52 * np.abs(Y))
 
 
 # n around the tile (128, 64), stage (32), drain (256) and run (1024) sizes

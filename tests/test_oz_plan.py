@@ -67,3 +67,21 @@ def test_plan_keeps_small_products_on_fma(lib):
         assert lib.oz_plan_run(p(v), p(A), p(B), p(C), p(C.copy()), ctypes.c_double(1.0), ctypes.c_double(0.0),
                                ctypes.c_int64(152), ctypes.c_int64(1 << 30), p(counts), p(out))
         assert out[8] == want
+
+
+@pytest.mark.parametrize("M,N,K,nb", [(1, 1, 1, 1), (60, 15, 8192, 1), (8192, 15, 60, 1), (64, 64, 64, 1),
+                                      (65, 17, 300, 7), (900, 900, 64, 1), (30, 30, 100000, 2)])
+def test_fma_plan(lib, M, N, K, nb):
+    """Every K element is in one split; a fixed split keeps the chain the 64 x 64 tiles had."""
+    v = np.array([M, N, K, nb], dtype=np.int64)
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    for splitk in (0, -1, 1, 5):
+        out = np.zeros(5, dtype=np.int64)
+        lib.fma_plan_of(p(v), ctypes.c_int64(152), ctypes.c_int32(splitk), p(out))
+        tm, tn, splits, kc, rule = (int(x) for x in out)
+        assert tm in (16, 32, 64) and tn in (16, 32, 64) and tn <= tm
+        assert kc % 16 == 0 and (splits - 1) * kc < K <= splits * kc
+        if splitk != 0:
+            want = rule if splitk < 0 else splitk
+            chunk = -(-(-(-K // want)) // 16) * 16
+            assert kc == chunk and splits == -(-K // chunk)

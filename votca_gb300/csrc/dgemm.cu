@@ -4,26 +4,32 @@
 #include <mutex>
 #include <vector>
 
+#include "fma_plan.hpp"
 #include "oz_gemm.cuh"
 
 namespace vgb {
 
 namespace {
 
-constexpr int TM = 64;
-constexpr int TN = 64;
-constexpr int TK = 16;
+constexpr int TK = kFmaStep;
 constexpr int THREADS = 256;
 
 struct Grid {
   int64_t mt, nt, nbatch, splits, kchunk;
 };
 
+// TM x TN outputs per 256-thread block, (TM / 16) x (TN / 16) per thread; the next K step's
+// operands are in flight while the current one is multiplied.  The FP64 pipe bounds it: a block
+// of 64 x 64 x 16 products keeps its SM busy for 32768 clocks (17 us), so small products want many
+// small tiles (fma_plan.hpp).  The sum of an output does not depend on the tile: one chain of FMAs
+// in K order per split.
+template <int TM, int TN>
 __global__ void __launch_bounds__(THREADS)
     dgemm_kernel(const GemmDesc d, const Grid g, double *__restrict__ partial, int a_icontig,
                  int b_lcontig) {
-  __shared__ double As[TK][TM + 1];
-  __shared__ double Bs[TK][TN + 1];
+  constexpr int RM = TM / 16, RN = TN / 16;
+  __shared__ double As[2][TK][TM + 1];
+  __shared__ double Bs[2][TK][TN + 1];
 
   // flat block index -> (split, batch, n-tile, m-tile)
   int64_t bid = blockIdx.x;
@@ -44,67 +50,82 @@ __global__ void __launch_bounds__(THREADS)
 
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  double acc[4][4];
+  double acc[RM][RN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+    for (int j = 0; j < RN; ++j) acc[i][j] = 0.0;
 
-  for (int64_t k0 = kbeg; k0 < kend; k0 += TK) {
+  double ra[RM], rb[RN];
+  auto load = [&](int64_t k0) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < RM; ++r) {
       const int e = tid + THREADS * r;
-      int i, l;
-      if (a_icontig) { i = e & (TM - 1); l = e >> 6; } else { l = e & (TK - 1); i = e >> 4; }
+      const int i = a_icontig ? e & (TM - 1) : e >> 4, l = a_icontig ? e / TM : e & (TK - 1);
       const int64_t gi = m0 + i, gl = k0 + l;
-      As[l][i] = (gi < d.M && gl < kend) ? A[gi * d.a_rs + gl * d.a_cs] : 0.0;
-      int n;
-      if (b_lcontig) { l = e & (TK - 1); n = e >> 4; } else { n = e & (TN - 1); l = e >> 6; }
-      const int64_t gn = n0 + n, gl2 = k0 + l;
-      Bs[l][n] = (gn < d.N && gl2 < kend) ? B[gl2 * d.b_rs + gn * d.b_cs] : 0.0;
+      ra[r] = (gi < d.M && gl < kend) ? A[gi * d.a_rs + gl * d.a_cs] : 0.0;
     }
-    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RN; ++r) {
+      const int e = tid + THREADS * r;
+      const int l = b_lcontig ? e & (TK - 1) : e / TN, n = b_lcontig ? e >> 4 : e & (TN - 1);
+      const int64_t gn = n0 + n, gl = k0 + l;
+      rb[r] = (gn < d.N && gl < kend) ? B[gl * d.b_rs + gn * d.b_cs] : 0.0;
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int r = 0; r < RM; ++r) {
+      const int e = tid + THREADS * r;
+      As[buf][a_icontig ? e / TM : e & (TK - 1)][a_icontig ? e & (TM - 1) : e >> 4] = ra[r];
+    }
+#pragma unroll
+    for (int r = 0; r < RN; ++r) {
+      const int e = tid + THREADS * r;
+      Bs[buf][b_lcontig ? e & (TK - 1) : e / TN][b_lcontig ? e >> 4 : e & (TN - 1)] = rb[r];
+    }
+  };
+
+  load(kbeg);
+  store(0);
+  __syncthreads();
+  int buf = 0;
+  for (int64_t k0 = kbeg; k0 < kend; k0 += TK) {
+    const bool more = k0 + TK < kend;
+    if (more) load(k0 + TK);
 #pragma unroll
     for (int l = 0; l < TK; ++l) {
-      double a[4], b[4];
+      double a[RM], b[RN];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[l][ty + 16 * i];
+      for (int i = 0; i < RM; ++i) a[i] = As[buf][l][ty + 16 * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[l][tx + 16 * j];
+      for (int j = 0; j < RN; ++j) b[j] = Bs[buf][l][tx + 16 * j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < RN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
     }
+    if (more) store(buf ^ 1);
     __syncthreads();
+    buf ^= 1;
   }
 
-  if (g.splits == 1) {
-    double *__restrict__ C = d.C + b1 * d.c_b1 + b2 * d.c_b2;
+  double *__restrict__ C = g.splits == 1 ? d.C + b1 * d.c_b1 + b2 * d.c_b2
+                                         : partial + (batch * g.splits + s) * d.M * d.N;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t gi = m0 + ty + 16 * i;
-      if (gi >= d.M) continue;
+  for (int i = 0; i < RM; ++i) {
+    const int64_t gi = m0 + ty + 16 * i;
+    if (gi >= d.M) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int64_t gn = n0 + tx + 16 * j;
-        if (gn >= d.N) continue;
+    for (int j = 0; j < RN; ++j) {
+      const int64_t gn = n0 + tx + 16 * j;
+      if (gn >= d.N) continue;
+      if (g.splits == 1) {
         double *c = C + gi * d.c_rs + gn * d.c_cs;
         const double v = d.alpha * acc[i][j];
         *c = (d.beta == 0.0) ? v : fma(d.beta, *c, v);
-      }
-    }
-  } else {
-    double *__restrict__ P = partial + (batch * g.splits + s) * d.M * d.N;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t gi = m0 + ty + 16 * i;
-      if (gi >= d.M) continue;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int64_t gn = n0 + tx + 16 * j;
-        if (gn >= d.N) continue;
-        P[gi + gn * d.M] = acc[i][j];
+      } else {
+        C[gi + gn * d.M] = acc[i][j];
       }
     }
   }
@@ -121,7 +142,8 @@ __global__ void splitk_reduce_kernel(const GemmDesc d, const Grid g,
     const int64_t i = e % d.M, n = e / d.M;
     const double *p = partial + batch * g.splits * mn + e;
     double acc = 0.0;
-    for (int64_t s = 0; s < g.splits; ++s) acc += p[s * mn];
+#pragma unroll 8
+    for (int64_t s = 0; s < g.splits; ++s) acc += p[s * mn];  // in split order; the loads overlap
     const int64_t b1 = batch / d.nb2, b2 = batch % d.nb2;
     double *c = d.C + b1 * d.c_b1 + b2 * d.c_b2 + i * d.c_rs + n * d.c_cs;
     const double v = d.alpha * acc;
@@ -138,6 +160,40 @@ __global__ void scale_kernel(const GemmDesc d, int64_t nbatch) {
     const int64_t b1 = batch / d.nb2, b2 = batch % d.nb2;
     double *c = d.C + b1 * d.c_b1 + b2 * d.c_b2 + i * d.c_rs + n * d.c_cs;
     *c = (d.beta == 0.0) ? 0.0 : d.beta * *c;
+  }
+}
+
+template <int TM, int TN>
+void launch_tile(const GemmDesc &d, const Grid &g, double *partial, cudaStream_t stream) {
+  const int64_t blocks = g.mt * g.nt * g.nbatch * g.splits;
+  VGB_REQUIRE(blocks < (1LL << 31), "dgemm: grid too large");
+  dgemm_kernel<TM, TN><<<(unsigned)blocks, THREADS, 0, stream>>>(d, g, partial, d.a_rs == 1 ? 1 : 0,
+                                                                  d.b_rs == 1 ? 1 : 0);
+  VGB_LAUNCH_CHECK();
+}
+
+void launch(const GemmDesc &d, const FmaPlan &f, double *partial, cudaStream_t stream) {
+  Grid g;
+  g.mt = ceil_div(d.M, f.tm);
+  g.nt = ceil_div(d.N, f.tn);
+  g.nbatch = d.nb1 * d.nb2;
+  g.splits = f.splits;
+  g.kchunk = f.kchunk;
+  if (f.tm == 64) {
+    if (f.tn == 64) launch_tile<64, 64>(d, g, partial, stream);
+    else if (f.tn == 32) launch_tile<64, 32>(d, g, partial, stream);
+    else launch_tile<64, 16>(d, g, partial, stream);
+  } else if (f.tm == 32) {
+    if (f.tn == 32) launch_tile<32, 32>(d, g, partial, stream);
+    else launch_tile<32, 16>(d, g, partial, stream);
+  } else {
+    launch_tile<16, 16>(d, g, partial, stream);
+  }
+  if (f.splits > 1) {
+    const int64_t total = d.M * d.N * g.nbatch;
+    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0,
+                           stream>>>(d, g, partial);
+    VGB_LAUNCH_CHECK();
   }
 }
 
@@ -260,40 +316,14 @@ void dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws, int splitk
     VGB_LAUNCH_CHECK();
     return;
   }
-  Grid g;
-  g.mt = ceil_div(d.M, TM);
-  g.nt = ceil_div(d.N, TN);
-  g.nbatch = nbatch;
-  const int64_t tiles = g.mt * g.nt * nbatch;
-  int64_t splits = splitk;
-  if (splits <= 0) {
-    const int64_t target = 3LL * sm_count();
-    splits = 1;
-    if (tiles < target && d.K > 4 * TK) {
-      splits = std::min<int64_t>(ceil_div(target, tiles), ceil_div(d.K, 8 * TK));
-      splits = std::max<int64_t>(1, std::min<int64_t>(splits, 256));
-    }
-  }
-  g.kchunk = ceil_div(ceil_div(d.K, splits), TK) * TK;
-  g.splits = ceil_div(d.K, g.kchunk);
+  const FmaPlan f = fma_plan(d, sm_count(), splitk);
   double *partial = nullptr;
-  if (g.splits > 1) {
+  if (f.splits > 1) {
     VGB_REQUIRE(ws != nullptr, "dgemm: split-K needs a workspace");
-    ws->partial.resize((size_t)(nbatch * g.splits * d.M * d.N));
+    ws->partial.resize((size_t)(nbatch * f.splits * d.M * d.N));
     partial = ws->partial.get();
   }
-  const int64_t blocks = tiles * g.splits;
-  VGB_REQUIRE(blocks < (1LL << 31), "dgemm: grid too large");
-  const int a_icontig = (d.a_rs == 1) ? 1 : 0;
-  const int b_lcontig = (d.b_rs == 1) ? 1 : 0;
-  dgemm_kernel<<<(unsigned)blocks, THREADS, 0, stream>>>(d, g, partial, a_icontig, b_lcontig);
-  VGB_LAUNCH_CHECK();
-  if (g.splits > 1) {
-    const int64_t total = d.M * d.N * nbatch;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0,
-                           stream>>>(d, g, partial);
-    VGB_LAUNCH_CHECK();
-  }
+  launch(d, f, partial, stream);
 }
 
 void dgemm_prealloc(const GemmDesc &d, cudaStream_t stream, double *ws, int64_t ws_count) {
@@ -306,32 +336,10 @@ void dgemm_prealloc(const GemmDesc &d, cudaStream_t stream, double *ws, int64_t 
     VGB_LAUNCH_CHECK();
     return;
   }
-  Grid g;
-  g.mt = ceil_div(d.M, TM);
-  g.nt = ceil_div(d.N, TN);
-  g.nbatch = nbatch;
-  const int64_t tiles = g.mt * g.nt * nbatch;
-  int64_t splits = 1;
-  const int64_t target = 3LL * sm_count();
-  if (ws && tiles < target && d.K > 4 * TK) {
-    splits = std::min<int64_t>(ceil_div(target, tiles), ceil_div(d.K, 8 * TK));
-    splits = std::max<int64_t>(1, std::min<int64_t>(splits, 256));
-    const int64_t fit = ws_count / std::max<int64_t>(1, nbatch * d.M * d.N);
-    splits = std::max<int64_t>(1, std::min(splits, fit));
-  }
-  g.kchunk = ceil_div(ceil_div(d.K, splits), TK) * TK;
-  g.splits = ceil_div(d.K, g.kchunk);
-  const int64_t blocks = tiles * g.splits;
-  VGB_REQUIRE(blocks < (1LL << 31), "dgemm: grid too large");
-  dgemm_kernel<<<(unsigned)blocks, THREADS, 0, stream>>>(d, g, g.splits > 1 ? ws : nullptr,
-                                                          (d.a_rs == 1) ? 1 : 0, (d.b_rs == 1) ? 1 : 0);
-  VGB_LAUNCH_CHECK();
-  if (g.splits > 1) {
-    const int64_t total = d.M * d.N * nbatch;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0,
-                           stream>>>(d, g, ws);
-    VGB_LAUNCH_CHECK();
-  }
+  int64_t splits = fma_chain_splits(d, sm_count());
+  if (!ws) splits = 1;
+  else splits = std::max<int64_t>(1, std::min(splits, ws_count / std::max<int64_t>(1, nbatch * d.M * d.N)));
+  launch(d, fma_plan(d, sm_count(), (int)splits), ws, stream);
 }
 
 }  // namespace vgb

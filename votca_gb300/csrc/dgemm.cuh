@@ -1,12 +1,13 @@
 // Strided, two-level-batched FP64 GEMM on CUDA cores with deterministic split-K.
 //
 // GB300 runs FP64 at ~1.2 TFLOP/s (2 DFMA/clk/SM), so every FP64 contraction
-// of this library is DFMA-bound long before it is bandwidth-bound: the kernel
-// needs only enough register blocking (4x4 per thread) and resident warps to
-// keep the DFMA pipe busy, and arbitrary element strides cost nothing that
-// matters.  This lets one kernel serve all FP64 contractions (the Hd/Hd2/Hx
-// stages and the Davidson projections) by describing the operands with
-// strides instead of materialising transposes.
+// of this library is DFMA-bound long before it is bandwidth-bound: large ones run
+// as digit products on the tensor cores (oz_gemm.cuh); for the others the kernel
+// needs only enough blocks and resident warps to keep every SM's DFMA pipe busy
+// (tiles of 64 x 64 down to 16 x 16, fma_plan.hpp), and arbitrary element strides
+// cost nothing that matters.  This lets one interface serve all FP64 contractions
+// (the Hd/Hd2/Hx stages and the Davidson projections) by describing the operands
+// with strides instead of materialising transposes.
 #pragma once
 
 #include "common.cuh"

@@ -7,6 +7,7 @@
 #include <utility>
 #include <vector>
 
+#include "fma_plan.hpp"
 #include "gemm_desc.hpp"
 
 #ifdef __CUDACC__
@@ -123,13 +124,12 @@ inline bool oz_plan(const GemmDesc &d, int sms, int64_t plane_budget, OzPlan &q)
   if (most * plane_row > 4 * plane_budget || most * kOzDigits >= (1LL << 31)) return false;
   // Times of either path in microseconds, from measurements on a GB300: the digit path is two to
   // four launches, 30 bytes of traffic per operand element (read twice, planes written) and 2500
-  // clocks per stage and wave of tiles; the FMA kernel runs whole 64 x 64 tiles at 1.15 TFLOP/s.
+  // clocks per stage and wave of tiles.
   const double elems = (double)(q.M + q.N) * q.nbatch * d.K;
   const double waves = (double)oz_ceil(tiles * q.splits, sms);
   const double t_oz = 14.0 + elems * 30.0 / 3.5e6 + waves * (q.kb_per * 2500.0 + 4000.0) / 1.9e3 +
                       (q.splits > 1 ? 3.0 + 16.0 * q.splits * q.M * q.N * q.nbatch / 4e6 : 0.0);
-  const double t_fma = 5.0 + (double)oz_ceil(d.M, 64) * oz_ceil(d.N, 64) * d.nb1 * d.nb2 * 8192.0 * d.K / 1.15e6;
-  q.faster = t_oz < t_fma;
+  q.faster = t_oz < fma_plan(d, sms, 0).time_us;
   return true;
 }
 
