@@ -25,15 +25,45 @@ __host__ __device__ inline int64_t eig_ld(int64_t m) { return (m % 2 == 0) ? m +
 // and m + 1 cluster starts
 __host__ __device__ inline int64_t eig_vec_doubles(int64_t m) { return 5 * m + 32 + (4 * m + 4) / 2 + 2; }
 
-__device__ double block_sum(double v, double *red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();  // earlier readers of red are done
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  // pairwise in a fixed order (deterministic): three dependent FP64 adds instead of eight
-  static_assert(kEigWarps == 8, "block_sum adds eight warp sums");
-  return ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+// The sum over the block of v, of which only the first nact warps hold nonzeros, in two steps: a
+// butterfly in those warps, then (after the caller's barrier) the warp sums in pairs, in a fixed
+// order.  Idle warps stay off the FP64 pipe: an instruction holds its SM quarter for 64 clocks
+// whatever its active lanes, so eight warps repeating a scalar queue two deep in every quarter.
+__device__ __forceinline__ void sum_warps(double v, double *red, int nact, int64_t n) {
+  const int warp = threadIdx.x >> 5;
+  if (warp < nact) {
+    // the first n lanes hold the values when one warp does: levels that add only zeros are left out
+    for (int o = n > 16 ? 16 : n > 8 ? 8 : n > 4 ? 4 : n > 2 ? 2 : 1; o > 0; o >>= 1)
+      v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[warp] = v;
+  }
 }
+__device__ __forceinline__ double sum_combine(const double *red, int nact) {
+  double a = red[0];
+  if (nact > 1) a += red[1];
+  if (nact > 2) {
+    double b = red[2];
+    if (nact > 3) b += red[3];
+    a += b;
+  }
+  if (nact > 4) {
+    double c = red[4];
+    if (nact > 5) c += red[5];
+    if (nact > 6) {
+      double d = red[6];
+      if (nact > 7) d += red[7];
+      c += d;
+    }
+    a += c;
+  }
+  return a;
+}
+__device__ __forceinline__ int warps_for(int64_t n) { return (int)min((int64_t)kEigWarps, (n + 31) / 32); }
+// integer forms of FP64 tests (no NaN): they do not use the FP64 pipe
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & ~(1ull << 63);
+}
+__device__ __forceinline__ bool negative(double x) { return __double_as_longlong(x) < 0 && abs_bits(x) != 0; }
 
 __device__ double block_max(double v, double *red) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -59,76 +89,121 @@ __device__ int sturm_count(const float *d, const float *e2, int64_t m, float x, 
 }
 
 // LU with partial pivoting of the tridiagonal (d - sigma, e): rows i and i+1 swap when the
-// subdiagonal entry is larger than the pivot; U has two superdiagonals.  r0 holds 1/U_ii.
-__device__ void tri_lu(const double *d, const double *e, int64_t m, double sigma, double tiny,
-                       double *r0, double *u1, double *u2, double *l, double *pv) {
-  double da = d[0] - sigma, db = m > 1 ? e[0] : 0.0;
-  for (int64_t i = 0; i + 1 < m; ++i) {
-    const double c = e[i], an = d[i + 1] - sigma, bn = (i + 2 < m) ? e[i + 1] : 0.0;
-    if (fabs(da) >= fabs(c)) {
-      if (fabs(da) < tiny) da = da < 0.0 ? -tiny : tiny;
-      const double r = 1.0 / da;  // one division per row
-      const double li = c * r;
-      r0[i] = r; l[i] = li; u1[i] = db; u2[i] = 0.0; pv[i] = 0.0;
-      da = an - li * db;
-      db = bn;
-    } else {
-      const double r = 1.0 / c;
-      const double li = da * r;
-      r0[i] = r; l[i] = li; u1[i] = an; u2[i] = bn; pv[i] = 1.0;
-      const double nda = db - li * an;
-      db = -li * bn;
-      da = nda;
-    }
+// subdiagonal entry is larger than the pivot; U has two superdiagonals.  r0 holds 1/U_ii.  Both
+// cases share one division and one update (lanes of a warp take different cases).  ds: the
+// shifted diagonal d - sigma; may be r0 itself (an entry is read before it is written).
+__device__ void tri_lu(const double *ds, const double *__restrict__ e, int m, double tiny,
+                       double *r0, double *__restrict__ u1, double *__restrict__ u2, double *__restrict__ l,
+                       double *__restrict__ pv) {
+  double da = ds[0], db = m > 1 ? e[0] : 0.0;
+  const unsigned long long tb = abs_bits(tiny);
+  double c = db, an = m > 1 ? ds[1] : 0.0;  // row i + 1's entries are loaded a row ahead
+  for (int i = 0; i + 1 < m; ++i) {
+    const double bn = (i + 2 < m) ? e[i + 1] : 0.0, an1 = (i + 2 < m) ? ds[i + 2] : 0.0;
+    const bool keep = abs_bits(da) >= abs_bits(c);
+    if (keep && abs_bits(da) < tb) da = negative(da) ? -tiny : tiny;
+    const double r = 1.0 / (keep ? da : c);  // one division per row
+    const double li = (keep ? c : da) * r;
+    r0[i] = r; l[i] = li;
+    u1[i] = keep ? db : an;
+    u2[i] = keep ? 0.0 : bn;
+    pv[i] = keep ? 0.0 : 1.0;
+    const double x = keep ? an : db, y = keep ? db : an;
+    da = x - li * y;
+    db = keep ? bn : -li * bn;
+    c = bn;
+    an = an1;
   }
-  if (fabs(da) < tiny) da = da < 0.0 ? -tiny : tiny;
+  if (abs_bits(da) < tb) da = negative(da) ? -tiny : tiny;
   r0[m - 1] = 1.0 / da;
 }
 
 // z <- (T - sigma)^-1 z with the factors of tri_lu
-__device__ void tri_solve(int64_t m, const double *r0, const double *u1, const double *u2,
-                          const double *l, const double *pv, double *z, int64_t zs) {
-  for (int64_t i = 0; i + 1 < m; ++i) {
-    double a = z[i * zs], b = z[(i + 1) * zs];
-    if (pv[i] != 0.0) { const double t = a; a = b; b = t; }
-    z[i * zs] = a;
-    z[(i + 1) * zs] = b - l[i] * a;
+__device__ void tri_solve(int m, const double *__restrict__ r0, const double *__restrict__ u1,
+                          const double *__restrict__ u2, const double *__restrict__ l,
+                          const double *__restrict__ pv, double *__restrict__ z) {
+  double a = z[0];
+#pragma unroll 4
+  for (int i = 0; i + 1 < m; ++i) {
+    const double b = z[i + 1];
+    const bool sw = abs_bits(pv[i]) != 0;
+    const double x = sw ? b : a, y = sw ? a : b;
+    z[i] = x;
+    a = y - l[i] * x;
   }
-  for (int64_t i = m - 1; i >= 0; --i) {
-    double s = z[i * zs];
-    if (i + 1 < m) s -= u1[i] * z[(i + 1) * zs];
-    if (i + 2 < m) s -= u2[i] * z[(i + 2) * zs];
-    z[i * zs] = s * r0[i];
+  z[m - 1] = a;
+  double z1 = a * r0[m - 1], z2 = 0.0;  // rows m - 1 and m - 2 have fewer superdiagonals
+  z[m - 1] = z1;
+  if (m > 1) {
+    double s = z[m - 2];
+    s -= u1[m - 2] * z1;
+    z2 = z1;
+    z1 = s * r0[m - 2];
+    z[m - 2] = z1;
+  }
+#pragma unroll 4
+  for (int i = m - 3; i >= 0; --i) {
+    double s = z[i];
+    s -= u1[i] * z1;
+    s -= u2[i] * z2;
+    s *= r0[i];
+    z[i] = s;
+    z2 = z1;
+    z1 = s;
   }
 }
 
 __device__ double vnorm(const double *z, int64_t m) {
   double s = 0.0;
-  for (int64_t i = 0; i < m; ++i) s = fma(z[i], z[i], s);
+#pragma unroll 4
+  for (int i = 0; i < m; ++i) s = fma(z[i], z[i], s);
   return sqrt(s);
 }
 __device__ void vscale(double *z, int64_t m, double f) {
   for (int64_t i = 0; i < m; ++i) z[i] *= f;
 }
-// z^T T z for the tridiagonal (d, e)
-__device__ double tri_rq(const double *d, const double *e, const double *z, int64_t m) {
-  double s = 0.0;
-  for (int64_t i = 0; i < m; ++i) {
+// a fixed, well-spread positive start vector (an integer hash of (i, j) mapped to [0.5, 1.5))
+__device__ double start_value(int64_t i, int64_t j) {
+  uint32_t h = (uint32_t)i * 2654435761u ^ ((uint32_t)j * 40503u + 12345u);
+  h ^= h >> 15;
+  h *= 2246822519u;
+  h ^= h >> 13;
+  return 0.5 + (double)(h >> 8) * (1.0 / 16777216.0);
+}
+__device__ void start_vector(double *z, int64_t m, int64_t j) {
+  for (int64_t i = 0; i < m; ++i) z[i] = start_value(i, j);
+}
+
+// z_c *= f[c - cb] for the vectors of the single clusters c = cb .. of a batch, over the block
+__device__ void scale_singles(double *Z, int64_t ldz, int64_t m, const int *cl, int64_t cb, int64_t ncl,
+                              const double *f) {
+  const int64_t n = min((int64_t)kEigThreads, ncl - cb);
+  for (int64_t t = threadIdx.x; t < m * n; t += kEigThreads) {
+    const int64_t c = cb + t / m;
+    if (cl[c + 1] - cl[c] == 1) Z[t % m + ldz * cl[c]] *= f[c - cb];
+  }
+}
+// d - sigma into the first m of each one's 5 m scratch doubles
+__device__ void shift_singles(const double *d, int64_t m, const int *cl, int64_t cb, int64_t ncl,
+                              const double *sigma, double *scratch) {
+  const int64_t n = min((int64_t)kEigThreads, ncl - cb);
+  for (int64_t t = threadIdx.x; t < m * n; t += kEigThreads) {
+    const int64_t c = cb + t / m, i = t % m;
+    if (cl[c + 1] - cl[c] == 1) scratch[5 * m * cl[c] + i] = d[i] - sigma[c - cb];
+  }
+}
+// y = T z of the same vectors into the last m of each one's 5 m scratch doubles
+__device__ void tri_apply_singles(const double *d, const double *e, const double *Z, int64_t ldz, int64_t m,
+                                  const int *cl, int64_t cb, int64_t ncl, double *scratch) {
+  const int64_t n = min((int64_t)kEigThreads, ncl - cb);
+  for (int64_t t = threadIdx.x; t < m * n; t += kEigThreads) {
+    const int64_t c = cb + t / m, i = t % m;
+    if (cl[c + 1] - cl[c] != 1) continue;
+    const double *z = Z + ldz * cl[c];
     double y = d[i] * z[i];
     if (i > 0) y = fma(e[i - 1], z[i - 1], y);
     if (i + 1 < m) y = fma(e[i], z[i + 1], y);
-    s = fma(z[i], y, s);
-  }
-  return s;
-}
-// a fixed, well-spread positive start vector (an integer hash of (i, j) mapped to [0.5, 1.5))
-__device__ void start_vector(double *z, int64_t m, int64_t j) {
-  for (int64_t i = 0; i < m; ++i) {
-    uint32_t h = (uint32_t)i * 2654435761u ^ ((uint32_t)j * 40503u + 12345u);
-    h ^= h >> 15;
-    h *= 2246822519u;
-    h ^= h >> 13;
-    z[i] = 0.5 + (double)(h >> 8) * (1.0 / 16777216.0);
+    scratch[5 * m * cl[c] + 4 * m + i] = y;
   }
 }
 
@@ -155,6 +230,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   const bool a_sm = off + ld * m <= g.smem_doubles;
   double *A = a_sm ? sm + off : q.work;
   if (a_sm) off += ld * m;
+  double *part4 = off + 4 * m <= g.smem_doubles ? sm + off : q.work + ld * m;  // step 1 only, before Z
   const bool z_sm = off + m * nw <= g.smem_doubles;
   double *Z = z_sm ? sm + off : q.U;
   const int64_t ldz = z_sm ? m : q.ldu;
@@ -171,60 +247,89 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   __syncthreads();
 
   // ---- 1. Householder tridiagonalisation ----
+  // Scalars are computed by warp 0 alone and broadcast; the two divisions of a reflector share an
+  // instruction; the four interleaved chains of a row of A v run in four threads.
+  __shared__ double sc[4], scl[kEigThreads];
   for (int64_t k = 0; k + 2 < m; ++k) {
     const int64_t k1 = k + 1;
+    const int na = warps_for(m - k - 2), nr = warps_for(m - k1);
     double s = 0.0;
     for (int64_t i = k + 2 + tid; i < m; i += kEigThreads) s = fma(A[i + ld * k], A[i + ld * k], s);
-    const double xn2 = block_sum(s, red);
-    const double alpha = A[k1 + ld * k];
-    if (xn2 == 0.0) {
-      if (tid == 0) { tau[k] = 0.0; e[k] = alpha; d[k] = A[k + ld * k]; }
+    sum_warps(s, red, na, m - k - 2);
+    if (na > 1) __syncthreads();
+    else __syncwarp();
+    if (warp == 0) {
+      const double xn2 = sum_combine(red, na), alpha = A[k1 + ld * k];
+      if (xn2 == 0.0) {
+        if (lane == 0) { tau[k] = 0.0; e[k] = alpha; d[k] = A[k + ld * k]; sc[2] = 0.0; }
+      } else {
+        const double beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
+        // tau = (beta - alpha) / beta in lane 0, 1 / (alpha - beta) in lane 1
+        const double diff = lane == 0 ? beta - alpha : alpha - beta;
+        const double v = (lane == 0 ? diff : 1.0) / (lane == 0 ? beta : diff);
+        if (lane < 2) sc[lane] = v;
+        if (lane == 0) { tau[k] = v; e[k] = beta; d[k] = A[k + ld * k]; sc[2] = 1.0; }
+      }
+    }
+    __syncthreads();
+    if (sc[2] == 0.0) {
       __syncthreads();
       continue;
     }
-    const double beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-    const double tk = (beta - alpha) / beta;
-    const double scal = 1.0 / (alpha - beta);
+    const double tk = sc[0], scal = sc[1];
     for (int64_t i = k1 + tid; i < m; i += kEigThreads) {
       const double vi = (i == k1) ? 1.0 : A[i + ld * k] * scal;
       vv[i] = vi;
       if (i > k1) A[i + ld * k] = vi;
     }
-    if (tid == 0) { tau[k] = tk; e[k] = beta; d[k] = A[k + ld * k]; }
     __syncthreads();
-    // p = tau A22 v from the lower triangle; four interleaved partial sums per row (a chain of
-    // dependent FP64 FMAs is the latency of this step)
+    // p = tau A22 v from the lower triangle, as four interleaved partial sums per row
+    {
+      const int u = tid >> 6;  // columns k1 + u, k1 + u + 4, ..
+      for (int64_t i = k1 + (tid & 63); i < m; i += 64) {
+        double acc = 0.0;
+#pragma unroll 4
+        for (int jj = (int)k1 + u; jj < (int)m; jj += 4) {
+          const double a = A[jj <= i ? (int)i + (int)ld * jj : jj + (int)ld * (int)i];
+          acc = fma(a, vv[jj], acc);
+        }
+        part4[u * m + i] = acc;
+      }
+    }
+    __syncthreads();
     double pv_part = 0.0;
     for (int64_t i = k1 + tid; i < m; i += kEigThreads) {
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
-      int64_t j = k1;
-      for (; j + 4 <= m; j += 4) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int64_t jj = j + u;
-          const double a = (jj <= i) ? A[i + ld * jj] : A[jj + ld * i];
-          acc[u] = fma(a, vv[jj], acc[u]);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {  // at most three left
-        const int64_t jj = j + u;
-        if (jj < m) {
-          const double a = (jj <= i) ? A[i + ld * jj] : A[jj + ld * i];
-          acc[u] = fma(a, vv[jj], acc[u]);
-        }
-      }
-      const double p = tk * ((acc[0] + acc[1]) + (acc[2] + acc[3]));
+      const double p = tk * ((part4[i] + part4[m + i]) + (part4[2 * m + i] + part4[3 * m + i]));
       pp[i] = p;
       pv_part = fma(p, vv[i], pv_part);
     }
-    const double K = -0.5 * tk * block_sum(pv_part, red);
+    sum_warps(pv_part, red, nr, m - k1);
+    if (nr > 1) __syncthreads();
+    else __syncwarp();
+    if (warp == 0) {
+      const double K = -0.5 * tk * sum_combine(red, nr);
+      if (lane == 0) sc[3] = K;
+    }
+    __syncthreads();
+    const double K = sc[3];
     for (int64_t i = k1 + tid; i < m; i += kEigThreads) pp[i] = fma(K, vv[i], pp[i]);  // w
     __syncthreads();
-    // A22 -= v w^T + w v^T (lower triangle), one warp per column
-    for (int64_t j = k1 + warp; j < m; j += kEigWarps) {
-      const double vj = vv[j], wj = pp[j];
-      for (int64_t i = j + lane; i < m; i += 32) A[i + ld * j] -= fma(vv[i], wj, pp[i] * vj);
+    // A22 -= v w^T + w v^T, lower triangle: columns a and n - 1 - a make one run of n + 1
+    // elements, so the warps' lanes are full
+    {
+      const int n = (int)(m - k1);
+      const int total = (n + 1) / 2 * (n + 1);
+      for (int t = tid; t < total; t += kEigThreads) {
+        const int a = t / (n + 1), b = t % (n + 1);
+        int j = a, i = a + b;
+        if (b >= n - a) {
+          j = n - 1 - a;
+          i = j + b - (n - a);
+          if (j == a) continue;  // the middle column is its own pair
+        }
+        const int64_t gi = k1 + i, gj = k1 + j;
+        A[gi + ld * gj] -= fma(vv[gi], pp[gj], pp[gi] * vv[gj]);
+      }
     }
     __syncthreads();
   }
@@ -259,14 +364,44 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   e2max = block_max(e2max, red);
   const double nrm = fmax(fmax(fabs(lo), fabs(hi)), 1e-300);
   const float pivmin = (float)(1e-30 * fmax(1.0, e2max));
-  for (int64_t j = tid; j < nw; j += kEigThreads) {
-    float a = (float)(lo - 1e-6 * nrm) - 1e-30f, b = (float)(hi + 1e-6 * nrm) + 1e-30f;
-    for (int it = 0; it < 80; ++it) {
-      if (b - a <= 2.4e-7f * fmaxf(fabsf(a), fabsf(b)) + 4.f * pivmin) break;
-      const float mid = 0.5f * (a + b);
-      if (sturm_count(d32, e2, m, mid, pivmin) > (int)j) b = mid; else a = mid;
+  // Every eigenvalue's bisection runs on a group of 7, 3 or 1 threads: the counts at the mid
+  // points that its next 3, 2 or 1 steps can reach are taken at once, then the steps are walked
+  // (the same intervals as one step at a time).
+  {
+    const int lv = 7 * nw <= kEigThreads ? 3 : 3 * nw <= kEigThreads ? 2 : 1;
+    const int G = (1 << lv) - 1;
+    const int nslot = kEigThreads / G;
+    int *cnt = reinterpret_cast<int *>(scl);  // one per thread
+    for (int64_t j0 = 0; j0 < nw; j0 += nslot) {
+      const int slot = tid / G, node = tid % G + 1;  // heap order: children of x are 2x, 2x + 1
+      const int64_t j = j0 + slot;
+      const bool act = slot < nslot && j < nw;
+      float a = (float)(lo - 1e-6 * nrm) - 1e-30f, b = (float)(hi + 1e-6 * nrm) + 1e-30f;
+      int it = 0;
+      bool done = !act;
+      while (__syncthreads_or(!done)) {
+        if (!done) {
+          float na = a, nb = b, mid = 0.5f * (a + b);
+          int depth = 31 - __clz(node);
+          for (int x = depth - 1; x >= 0; --x) {
+            if ((node >> x) & 1) na = mid; else nb = mid;
+            mid = 0.5f * (na + nb);
+          }
+          cnt[tid] = sturm_count(d32, e2, m, mid, pivmin);
+        }
+        __syncthreads();
+        if (!done) {
+          int x = 1;
+          for (int st = 0; st < lv; ++st) {
+            if (it >= 80 || b - a <= 2.4e-7f * fmaxf(fabsf(a), fabsf(b)) + 4.f * pivmin) { done = true; break; }
+            const float mid = 0.5f * (a + b);
+            if (cnt[slot * G + x - 1] > (int)j) { b = mid; x = 2 * x; } else { a = mid; x = 2 * x + 1; }
+            ++it;
+          }
+        }
+      }
+      if (act && node == 1) lam32[j] = 0.5f * (a + b);
     }
-    lam32[j] = 0.5f * (a + b);
   }
   __syncthreads();
   // clusters of eigenvalues closer than 1e-5 of the spectral radius (cl: starts, then nw): the
@@ -284,18 +419,64 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   __syncthreads();
 
   // ---- 3. eigenvectors of the tridiagonal by inverse iteration (FP64) ----
+  // One thread per cluster runs the serial chains; the elementwise work of the single
+  // eigenvalues (start vectors, scalings, T z) is spread over the block between barriers.
   const double tiny = 2.3e-16 * nrm;
+  {
+    for (int64_t cb = 0; cb < ncl; cb += kEigThreads) {
+      const int64_t c = cb + tid;
+      const bool single = c < ncl && cl[c + 1] - cl[c] == 1;
+      const int64_t j = single ? cl[c] : 0;
+      double *w = scratch + 5 * m * j, *z = Z + ldz * j;
+      double *r0 = w, *u1 = w + m, *u2 = w + 2 * m, *l = w + 3 * m, *pv = w + 4 * m;
+      const int64_t jb0 = cl[cb], jb1 = cl[min((int64_t)ncl, cb + kEigThreads)];  // vectors of this batch
+      const int64_t nel = m * (jb1 - jb0);
+      for (int64_t t = tid; t < nel; t += kEigThreads) Z[t % m + ldz * (jb0 + t / m)] = start_value(t % m, jb0 + t / m);
+      __syncthreads();
+      double sigma = single ? (double)lam32[j] : 0.0;
+      for (int half = 0; half < 2; ++half) {
+        scl[tid] = sigma;
+        __syncthreads();
+        shift_singles(d, m, cl, cb, ncl, scl, scratch);
+        __syncthreads();
+        if (single) tri_lu(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
+        for (int st = 0; st < 2; ++st) {
+          if (single) {
+            tri_solve((int)m, r0, u1, u2, l, pv, z);
+            scl[tid] = 1.0 / vnorm(z, m);
+          } else {
+            scl[tid] = 1.0;
+          }
+          __syncthreads();
+          scale_singles(Z, ldz, m, cl, cb, ncl, scl);
+          __syncthreads();
+        }
+        // T z beside the factors (pv is free), then the Rayleigh quotient
+        tri_apply_singles(d, e, Z, ldz, m, cl, cb, ncl, scratch);
+        __syncthreads();
+        if (single) {
+          double s = 0.0;
+#pragma unroll 4
+          for (int i = 0; i < m; ++i) s = fma(z[i], pv[i], s);
+          sigma = s;
+        }
+      }
+      if (single) q.lam[j] = sigma;
+      __syncthreads();
+    }
+  }
   for (int c = tid; c < ncl; c += kEigThreads) {
     const int64_t j0 = cl[c], j1 = cl[c + 1], s = j1 - j0;
+    if (s == 1) continue;
     double *w = scratch + 5 * m * j0;  // 5 m per member, contiguous over the cluster
     double *r0 = w, *u1 = w + m, *u2 = w + 2 * m, *l = w + 3 * m, *pv = w + 4 * m;
     for (int64_t jj = j0; jj < j1; ++jj) {
       double *z = Z + ldz * jj;
       start_vector(z, m, jj);
-      tri_lu(d, e, m, (double)lam32[jj], tiny, r0, u1, u2, l, pv);
-      const int steps = s == 1 ? 2 : 5;
-      for (int st = 0; st < steps; ++st) {
-        tri_solve(m, r0, u1, u2, l, pv, z, 1);
+      for (int64_t i = 0; i < m; ++i) r0[i] = d[i] - (double)lam32[jj];
+      tri_lu(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
+      for (int st = 0; st < 5; ++st) {
+        tri_solve((int)m, r0, u1, u2, l, pv, z);
         for (int64_t kk = j0; kk < jj; ++kk) {  // earlier members of the cluster
           const double *y = Z + ldz * kk;
           double dot = 0.0;
@@ -304,16 +485,8 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
         }
         vscale(z, m, 1.0 / vnorm(z, m));
       }
-      if (s == 1) {  // Rayleigh quotient iteration: two steps at the FP64 shift
-        tri_lu(d, e, m, tri_rq(d, e, z, m), tiny, r0, u1, u2, l, pv);
-        for (int st = 0; st < 2; ++st) {
-          tri_solve(m, r0, u1, u2, l, pv, z, 1);
-          vscale(z, m, 1.0 / vnorm(z, m));
-        }
-        q.lam[jj] = tri_rq(d, e, z, m);
-      }
     }
-    if (s > 1) {  // Rayleigh-Ritz on the cluster: cyclic Jacobi on C = Z_c^T T Z_c
+    {  // Rayleigh-Ritz on the cluster: cyclic Jacobi on C = Z_c^T T Z_c
       double *C = w, *W = w + s * s, *y = w + 2 * s * s;
       for (int64_t b = 0; b < s; ++b) {
         const double *zb = Z + ldz * (j0 + b);
@@ -418,7 +591,8 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
       }
     }
   } else {
-    __shared__ double part[kEigThreads];
+    double *part = scl;
+    double *fac = vv;  // one factor per vector of a batch (vv and pp are free)
     const int G = (int)std::min<int64_t>(32, std::max<int64_t>(1, kEigThreads / nw));
     const int per_batch = kEigThreads / G;
     const int slot = tid / G, sub = tid % G;
@@ -434,10 +608,14 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
           for (int64_t i = k + 1 + sub; i < m; i += G) s = fma(i == k + 1 ? 1.0 : A[i + ld * k], z[i], s);
         part[tid] = s;
         __syncthreads();
-        if (act) {
+        if (tid < min((int64_t)per_batch, nw - j0)) {  // the partial sums of a vector by one thread: few warps add
           double t = 0.0;
-          for (int p = 0; p < G; ++p) t += part[slot * G + p];
-          const double f = tk * t;
+          for (int p = 0; p < G; ++p) t += part[tid * G + p];
+          fac[tid] = tk * t;
+        }
+        __syncthreads();
+        if (act) {
+          const double f = fac[slot];
           for (int64_t i = k + 1 + sub; i < m; i += G) z[i] = fma(-f, i == k + 1 ? 1.0 : A[i + ld * k], z[i]);
         }
         __syncthreads();  // part is written again for the next reflector
@@ -488,10 +666,12 @@ void sym_eig_device(const SymEigJob *jobs, int64_t njobs, cudaStream_t s) {
       // (the kernel places them in the same order)
       int64_t job_need = eig_vec_doubles(jb.m);
       if (job_need + eig_ld(jb.m) * jb.m <= limit) job_need += eig_ld(jb.m) * jb.m;
+      const int64_t with_part = job_need + 4 * jb.m;  // step 1's partial sums, before the vectors
       if (job_need + jb.m * jb.nw <= limit) {
         job_need += jb.m * jb.nw;
         if (job_need + 5 * jb.m * jb.nw <= limit) job_need += 5 * jb.m * jb.nw;
       }
+      if (with_part <= limit) job_need = std::max(job_need, with_part);
       need = std::max(need, job_need);
     }
     g->smem_doubles = need;
