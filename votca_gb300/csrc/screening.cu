@@ -27,25 +27,35 @@ unsigned g1d(int64_t n) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), 16LL * 152));
 }
 
-// B[(m, c)][P] = M(rpamin+m, lumo+c, P) scaled by -2 chi_{m,c}  (Bw) and unscaled (B)
-__global__ void rpa_weights_kernel(const double *raw, int64_t n_occ_chunk, int64_t m0, int64_t n_unocc,
-                                   int64_t naux, int64_t nsize, int64_t row0,
-                                   const double *energies, int64_t lumo_idx, double wr, double wi,
-                                   double eta, double *B, double *Bw, int64_t ldb) {
-  const int64_t total = n_occ_chunk * n_unocc * naux;
+// -2 chi of the (m, c) pairs: two divisions each, once per pair and not once per (pair, P)
+__global__ void rpa_chi_kernel(const double *energies, int64_t n_occ_chunk, int64_t m0, int64_t n_unocc,
+                               int64_t lumo_idx, double wr, double wi, double eta, double *chi2) {
+  const int64_t total = n_occ_chunk * n_unocc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = t % n_unocc;
-    const int64_t P = (t / n_unocc) % naux;
-    const int64_t mi = t / (n_unocc * naux);
-    const double x = raw[(mi * naux + P) * nsize + row0 + c];
+    const int64_t c = t % n_unocc, mi = t / n_unocc;
     const double dE = energies[lumo_idx + c] - energies[m0 + mi];
     const double dm = wr - dE, dp = wr + dE;
     const double s1 = (wi + eta) * (wi + eta), s2 = (wi - eta) * (wi - eta);
     const double chi = dm / (dm * dm + s1) - dp / (dp * dp + s2);
-    const int64_t row = mi * n_unocc + c;
-    B[row + ldb * P] = x;
-    Bw[row + ldb * P] = -2.0 * chi * x;
+    chi2[t] = -2.0 * chi;
+  }
+}
+
+// B[(m, c)][P] = M(rpamin+m, lumo+c, P), and the same scaled by -2 chi_{m,c} (Bw); one grid row
+// per (m, P), so that no thread divides an index.  Bound: HBM, 24 bytes an element (v32 c256
+// Naux1000: 359 us with the divisions inside, 40 us).
+__global__ void rpa_weights_kernel(const double *raw, int64_t n_unocc, int64_t naux, int64_t nsize, int64_t row0,
+                                   const double *chi2, double *B, double *Bw, int64_t ldb, int64_t rows) {
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {  // r = mi * naux + P
+    const int64_t mi = r / naux, P = r - mi * naux;
+    const double *src = raw + r * nsize + row0, *w = chi2 + mi * n_unocc;
+    double *b = B + mi * n_unocc + ldb * P, *bw = Bw + mi * n_unocc + ldb * P;
+    for (int64_t c = threadIdx.x; c < n_unocc; c += blockDim.x) {
+      const double x = src[c];
+      b[c] = x;
+      bw[c] = w[c] * x;
+    }
   }
 }
 
@@ -55,60 +65,93 @@ __global__ void add_identity_kernel(double *A, int64_t n) {
     A[i + n * i] += 1.0;
 }
 
-// Unblocked Cholesky of the nb x nb diagonal block at A + j (lda), lower triangle;
-// the strict upper triangle of the block is zeroed.  One CTA, block in shared memory.
-__global__ void potrf_block_kernel(double *A, int64_t lda, int nb, int *info, int64_t j0) {
-  __shared__ double a[NB][NB + 1];
-  const int t = threadIdx.x;
-  for (int e = t; e < nb * nb; e += blockDim.x) a[e % nb][e / nb] = A[(e % nb) + lda * (e / nb)];
-  __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    if (t == 0) {
-      const double d = a[k][k];
-      if (!(d > 0.0)) { if (*info == 0) *info = (int)(j0 + k + 1); a[k][k] = 1.0; }
-      else a[k][k] = sqrt(d);
-    }
-    __syncthreads();
-    const double dk = a[k][k];
-    for (int i = k + 1 + t; i < nb; i += blockDim.x) a[i][k] /= dk;
-    __syncthreads();
-    for (int e = t; e < (nb - k - 1) * (nb - k - 1); e += blockDim.x) {
-      const int i = k + 1 + e % (nb - k - 1), jj = k + 1 + e / (nb - k - 1);
-      if (jj <= i) a[i][jj] -= a[i][k] * a[jj][k];
-    }
-    __syncthreads();
-  }
-  for (int e = t; e < nb * nb; e += blockDim.x) {
-    const int i = e % nb, jj = e / nb;
-    A[i + lda * jj] = (jj <= i) ? a[i][jj] : 0.0;
-  }
+// 1 / sqrt(d) for d > 0: an FP32 estimate of the mantissa (exponent split off, any FP64 range) and
+// one step of Householder's third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2 < 2^-20:
+// five FP64 instructions instead of a square root and a division (1265 clocks of the pipe).
+__device__ __forceinline__ double rsqrt64(double d) {
+  const long long b = __double_as_longlong(d);
+  const int ex = (int)((b >> 52) & 0x7FF) - 1023;
+  if (ex == -1023) return 1.0 / sqrt(d);  // subnormal
+  const int h = ex >> 1;                  // d = m 4^h, m in [1, 4)
+  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | ((long long)(1023 + (ex & 1)) << 52));
+  const double y = (double)rsqrtf((float)m);
+  const double e = fma(-(m * y), y, 1.0);
+  const double r = fma(y * e, fma(0.375, e, 0.5), y);
+  return __longlong_as_double(__double_as_longlong(r) - ((long long)h << 52));
 }
 
-// Inverse of the nb x nb lower-triangular block L (lda) into Li (ld nb): column j
-// by forward substitution, one thread per column.
-__global__ void trtri_block_kernel(const double *L, int64_t lda, int nb, double *Li) {
-  __shared__ double l[NB][NB + 1];
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) l[e % nb][e / nb] = L[(e % nb) + lda * (e / nb)];
-  __syncthreads();
-  const int j = threadIdx.x;
-  if (j < nb) {
-    double x[NB];
-    for (int i = 0; i < nb; ++i) {
-      double s = (i == j) ? 1.0 : 0.0;
-      for (int p = j; p < i; ++p) s -= l[i][p] * x[p];
-      x[i] = (i < j) ? 0.0 : s / l[i][i];
-    }
-    for (int i = 0; i < nb; ++i) Li[i + nb * j] = x[i];
+// Cholesky factor L and its inverse of the nb x nb (<= 64) diagonal block at A (lda), one CTA: the
+// factorisation of [A | I] in registers, so that column k of L and row k of L^-1 come out
+// together.  L: lower triangle, zeros above, at Lo (ldl); L^-1 likewise at Li (ldi).
+// An element (i, j) holds A's until step j and L^-1's from then on, and every step is one FMA of
+// column k with row k for the rows below.  Bound: the FP64 pipe (64 clocks of an SM quarter per
+// warp instruction) and the pivot's chain; a warp has 8 rows, the two warps of a quarter rows q
+// and 7 - q of eight, which have 18 instructions a step together whatever q (columns past the
+// diagonal are left out).  64 x 64: 263 us as two kernels with divisions, 100 us from shared
+// memory, 87 us.
+__global__ void __launch_bounds__(256) chol_block_kernel(const double *A, int64_t lda, int nb, double *Lo,
+                                                         int64_t ldl, double *Li, int64_t ldi, int *info,
+                                                         int64_t j0) {
+  __shared__ double colk[NB], rowk[NB], l[NB], rk[NB];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int blk = warp < 4 ? warp : 11 - warp;  // rows 8 blk ..
+  const int i = 8 * blk + (lane & 7), c = lane >> 3;  // columns c, c + 4, ..
+  double v[16];
+#pragma unroll
+  for (int s = 0; s < 16; ++s) {
+    const int j = c + 4 * s;
+    v[s] = j > i ? 0.0 : (i < nb ? A[i + lda * j] : (i == j ? 1.0 : 0.0));
   }
-}
-
-__global__ void set_identity_rows_kernel(double *Y, int64_t n, int64_t i0, int64_t nb) {
-  // Y[i0:i0+nb, :] = E (identity rows), leaves other rows untouched
-  const int64_t total = nb * n;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = t % nb, c = t / nb;
-    Y[(i0 + r) + n * c] = (i0 + r == c) ? 1.0 : 0.0;
+#pragma unroll
+  for (int sk = 0; sk < 16; ++sk) {
+#pragma unroll 1
+    for (int ck = 0; ck < 4; ++ck) {
+      const int k = 4 * sk + ck;
+      if (c == ck && i >= k) colk[i] = v[sk];
+      if (i == k) {
+#pragma unroll
+        for (int s = 0; s <= sk; ++s) rowk[c + 4 * s] = v[s];
+      }
+      __syncthreads();
+      if (warp < 4) {  // one warp per quarter: column k of L (warps 0, 1), row k of L^-1 (warps 2, 3)
+        const double d = colk[k];
+        const long long b = __double_as_longlong(d);  // an FP64 comparison costs what an FMA does
+        const bool ok = b > 0 && b <= 0x7FF0000000000000ll;
+        const double y = ok ? rsqrt64(d) : 1.0;
+        const int e = (warp & 1) * 32 + lane;
+        if (warp < 2) {
+          const double x = e > k ? colk[e] : ok ? d : 1.0;
+          const double lv = x * y;
+          if (e >= k) {
+            if (e > k) { l[e] = lv; rk[e] = lv; }
+            if (e < nb) Lo[e + ldl * k] = lv;
+          } else if (e < nb && k < nb) {
+            Lo[e + ldl * k] = 0.0;
+          }
+          if (e == k && !ok && *info == 0) *info = (int)(j0 + k + 1);
+        } else if (e <= k) {
+          rk[e] = (e < k ? rowk[e] : 1.0) * y;
+        }
+      }
+      __syncthreads();
+      if (i == k) {  // row k of L^-1 is final
+#pragma unroll
+        for (int s = 0; s <= sk; ++s)
+          if (c + 4 * s <= k) v[s] = rk[c + 4 * s];
+      }
+      if (8 * blk + 7 > k) {  // the warp has rows below k
+        const double li = i > k ? l[i] : 0.0;
+        if (c == ck && i > k) v[sk] = 0.0;
+#pragma unroll
+        for (int s = 0; s < 16; ++s)
+          if (s <= 2 * blk + 1) v[s] = fma(-li, rk[c + 4 * s], v[s]);
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < 16; ++s) {
+    const int j = c + 4 * s;
+    if (i < nb && j < nb) Li[i + ldi * j] = j <= i ? v[s] : 0.0;
   }
 }
 
@@ -130,7 +173,7 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
   // occupied levels in chunks so that the pair matrices stay below ~1 GB
   const int64_t per_m = n_unocc * naux;
   const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(n_occ, (64LL << 20) / std::max<int64_t>(per_m, 1)));
-  DeviceBuffer<double> raw(chunk * naux * nsize), B(chunk * per_m), Bw(chunk * per_m);
+  DeviceBuffer<double> raw(chunk * naux * nsize), B(chunk * per_m), Bw(chunk * per_m), chi(chunk * n_unocc);
   GemmWorkspace ws;
   for (int64_t m0 = 0; m0 < n_occ; m0 += chunk) {
     const int64_t cnt = std::min(chunk, n_occ - m0);
@@ -142,9 +185,10 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
     }
     const int64_t rows = cnt * n_unocc;
     // Mmn_[m].bottomRows(n_unocc), as the reference reads it
-    rpa_weights_kernel<<<g1d(rows * naux), 256, 0, s>>>(raw.get(), cnt, m0, n_unocc, naux, nsize,
-                                                        nsize - n_unocc, dE.get(), lumo - rpamin, wr,
-                                                        wi, eta, B.get(), Bw.get(), rows);
+    rpa_chi_kernel<<<g1d(rows), 256, 0, s>>>(dE.get(), cnt, m0, n_unocc, lumo - rpamin, wr, wi, eta, chi.get());
+    VGB_LAUNCH_CHECK();
+    rpa_weights_kernel<<<(unsigned)std::min<int64_t>(cnt * naux, 64LL * sm_count()), 128, 0, s>>>(
+        raw.get(), n_unocc, naux, nsize, nsize - n_unocc, chi.get(), B.get(), Bw.get(), rows, cnt * naux);
     VGB_LAUNCH_CHECK();
     GemmDesc g;  // eps (+)= B^T Bw
     g.M = naux; g.N = naux; g.K = rows;
@@ -163,34 +207,30 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
 void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_host, int64_t ldi,
                       cudaStream_t s) {
   VGB_REQUIRE(n >= 1 && lda >= n && ldi >= n, "cholesky_inverse: bad size");
-  DeviceBuffer<double> A(n * n), Y(n * n), Li(NB * NB), T(NB * n);
+  // L beside A (the panel product then needs no copy), Y = L^-1
+  DeviceBuffer<double> A(n * n), L(n * n), Y(n * n), T((n / 2 + NB) * (n / 2 + NB) + n * NB);
   DeviceBuffer<int> info(1);
   GemmWorkspace ws;
   VGB_CUDA(cudaMemcpy2DAsync(A.get(), n * sizeof(double), a_host, lda * sizeof(double),
                              n * sizeof(double), n, cudaMemcpyHostToDevice, s));
   VGB_CUDA(cudaMemsetAsync(info.get(), 0, sizeof(int), s));
-  // right-looking blocked Cholesky: A = L L^T (lower)
+  VGB_CUDA(cudaMemsetAsync(Y.get(), 0, n * n * sizeof(double), s));
+  // right-looking blocked Cholesky: A = L L^T (lower), the diagonal blocks' inverses into Y
   for (int64_t j = 0; j < n; j += NB) {
     const int nb = (int)std::min<int64_t>(NB, n - j);
-    double *Ajj = A.get() + j + n * j;
-    potrf_block_kernel<<<1, 256, 0, s>>>(Ajj, n, nb, info.get(), j);
+    chol_block_kernel<<<1, 256, 0, s>>>(A.get() + j + n * j, n, nb, L.get() + j + n * j, n,
+                                                 Y.get() + j + n * j, n, info.get(), j);
     VGB_LAUNCH_CHECK();
     const int64_t rest = n - j - nb;
     if (rest > 0) {
-      trtri_block_kernel<<<1, NB, 0, s>>>(Ajj, n, nb, Li.get());
-      VGB_LAUNCH_CHECK();
-      // L21 = A21 L11^-T
-      double *A21 = A.get() + (j + nb) + n * j;
-      GemmDesc t;
+      double *L21 = L.get() + (j + nb) + n * j;
+      GemmDesc t;  // L21 = A21 L11^-T
       t.M = rest; t.N = nb; t.K = nb;
-      t.a_colmajor(A21, n, false).b_colmajor(Li.get(), nb, true).c_colmajor(T.get(), rest);
+      t.a_colmajor(A.get() + (j + nb) + n * j, n, false).b_colmajor(Y.get() + j + n * j, n, true).c_colmajor(L21, n);
       dgemm(t, s, &ws);
-      VGB_CUDA(cudaMemcpy2DAsync(A21, n * sizeof(double), T.get(), rest * sizeof(double),
-                                 rest * sizeof(double), nb, cudaMemcpyDeviceToDevice, s));
-      // A22 -= L21 L21^T
-      GemmDesc u;
+      GemmDesc u;  // A22 -= L21 L21^T
       u.M = rest; u.N = rest; u.K = nb;
-      u.a_colmajor(A21, n, false).b_colmajor(A21, n, true).c_colmajor(A.get() + (j + nb) + n * (j + nb), n);
+      u.a_colmajor(L21, n, false).b_colmajor(L21, n, true).c_colmajor(A.get() + (j + nb) + n * (j + nb), n);
       u.alpha = -1.0; u.beta = 1.0;
       dgemm(u, s, &ws);
     }
@@ -201,28 +241,29 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
   if (hinfo != 0)
     fail(BSE_ERR_NUMERICAL, "cholesky_inverse: matrix is not positive definite (pivot " +
                                 std::to_string(hinfo) + ")");
-  // Y = L^-1 by block forward substitution over block rows: Y_i = L_ii^-1 (E_i - L_i,<i Y_<i)
-  // (upper blocks of L were zeroed, so whole block rows can be used)
-  VGB_CUDA(cudaMemsetAsync(Y.get(), 0, n * n * sizeof(double), s));
-  for (int64_t i = 0; i < n; i += NB) {
-    const int nb = (int)std::min<int64_t>(NB, n - i);
-    set_identity_rows_kernel<<<g1d(nb * n), 256, 0, s>>>(Y.get(), n, i, nb);
-    VGB_LAUNCH_CHECK();
-    if (i > 0) {  // Y_i -= L[i, 0:i] Y[0:i, :]
-      GemmDesc g;
-      g.M = nb; g.N = n; g.K = i;
-      g.a_colmajor(A.get() + i, n, false).b_colmajor(Y.get(), n, false).c_colmajor(Y.get() + i, n);
-      g.alpha = -1.0; g.beta = 1.0;
-      dgemm(g, s, &ws);
+  // Y = L^-1 by doubling: of [L11 0; L21 L22] with the inverses of both diagonal blocks of h rows,
+  // Y21 = -Y22 (L21 Y11), all pairs of a level at once: 2 log2(n / 64) launches of large products
+  // in place of 5 small ones per block row.
+  for (int64_t h = NB; h < n; h *= 2) {
+    const int64_t full = n / (2 * h);  // pairs of two whole blocks
+    const int64_t i0 = full * 2 * h, last = n - i0 - h;  // a last pair whose second block is short
+    for (int r = 0; r < 2; ++r) {
+      const int64_t np = r == 0 ? full : (last > 0 ? 1 : 0), h2 = r == 0 ? h : last, o = r == 0 ? 0 : i0;
+      if (np == 0) continue;
+      const int64_t step = 2 * h * (n + 1);
+      GemmDesc t;  // T = L21 Y11
+      t.M = h2; t.N = h; t.K = h;
+      t.a_colmajor(L.get() + o + h + n * o, n, false).b_colmajor(Y.get() + o + n * o, n, false).c_colmajor(T.get(), h2);
+      t.nb1 = np; t.a_b1 = step; t.b_b1 = step; t.c_b1 = h * h2;
+      dgemm(t, s, &ws);
+      GemmDesc u;  // Y21 = -Y22 T
+      u.M = h2; u.N = h; u.K = h2;
+      u.a_colmajor(Y.get() + (o + h) * (n + 1), n, false).b_colmajor(T.get(), h2, false)
+          .c_colmajor(Y.get() + o + h + n * o, n);
+      u.alpha = -1.0;
+      u.nb1 = np; u.a_b1 = step; u.b_b1 = h * h2; u.c_b1 = step;
+      dgemm(u, s, &ws);
     }
-    trtri_block_kernel<<<1, NB, 0, s>>>(A.get() + i + n * i, n, nb, Li.get());
-    VGB_LAUNCH_CHECK();
-    GemmDesc h;  // Y_i = L_ii^-1 Y_i
-    h.M = nb; h.N = n; h.K = nb;
-    h.a_colmajor(Li.get(), nb, false).b_colmajor(Y.get() + i, n, false).c_colmajor(T.get(), nb);
-    dgemm(h, s, &ws);
-    VGB_CUDA(cudaMemcpy2DAsync(Y.get() + i, n * sizeof(double), T.get(), nb * sizeof(double),
-                               nb * sizeof(double), n, cudaMemcpyDeviceToDevice, s));
   }
   // A^-1 = L^-T L^-1 = Y^T Y
   GemmDesc f;
