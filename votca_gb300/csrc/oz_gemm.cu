@@ -24,10 +24,16 @@ constexpr int LB = 4;         // stages between drains of levels 4 .. 7: 7 pairs
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
 constexpr int STAGE_BYTES = S * (A_BYTES + B_BYTES);  // 86016
 constexpr int STAGES = 2;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+// output offsets and scale exponents of a tile's rows and columns, two tiles deep
+struct TileTab {
+  int64_t row[BM], col[BN];  // row: -1 beyond the matrix
+  int ea[BM], eb[BN];
+};
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 2 * (int)sizeof(TileTab);
 constexpr int kEpi = 16;                     // epilogue warps: four per TMEM lane quarter
 constexpr int EC = BN / 4;                   // columns of an epilogue thread
-constexpr int kGemmThreads = 64 + 32 * kEpi; // warp 0: TMA, warp 1: MMA, rest: epilogue
+constexpr int kTab = 2;                       // warps that prepare a tile's output addresses
+constexpr int kGemmThreads = 64 + 32 * (kEpi + kTab);  // warp 0: TMA, warp 1: MMA, epilogue, tables
 constexpr int BITS = 8 * S - 1;              // digit window: |x| < 2^e -> |m| <= 2^BITS
 constexpr int BIAS = 50;                     // operand digits carry 2^(BIAS - row exponent)
 constexpr int ZERO_RUN = -100000;            // exponent of a run of zeros
@@ -41,194 +47,208 @@ struct Operand {
   int64_t r0 = 0, rows = 0, K = 0, Kp = 0, ks = 1;
   uint16_t *planes = nullptr;  // [t][rows][Kp]
   int *erow = nullptr;         // exponent of the row's largest element (per row)
-  int *erun = nullptr;         // per (row, run), only when there is more than one run
+  int *erun = nullptr;         // per (row, run), only for rows of several segments
   int nruns = 1;
 };
 
 // ---------------- digits ----------------
 
-// Digits of four consecutive K elements, packed per plane.  x = sum_t d_t 2^(e - 7 - 8 t), the
-// value m = round(x 2^(BITS - e)) in 64-bit integers (the FP64 pipe is the slow one here) and its
-// balanced bytes: adding 128 to every byte but the top one makes each byte d + 128.  The bf16
-// value d 2^(rel + BIAS - 7 - 8 t) comes from one FFMA on 2^23 + byte.
-__device__ __forceinline__ void digits4(const double (&x)[4], int e, const float (&sc)[S], uint2 (&out)[S]) {
-  uint32_t lo[4], hi[4];
-  int top[4];
-  constexpr long long bias = 0x0000808080808080ll;
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x[v]);
-    const int ef = (int)((b >> 52) & 0x7FF);
-    const int sh = e - (ef - 1022);  // 0 .. : |x| < 2^(ef - 1022) <= 2^e
-    unsigned long long m = ((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << (BITS - 53);
-    m = (ef == 0 || sh > BITS + 1) ? 0ull : (sh > 0 ? (m + (1ull << (sh - 1))) >> sh : m);
-    const long long u = ((b >> 63) ? -(long long)m : (long long)m) + bias;
-    lo[v] = (uint32_t)u;
-    hi[v] = (uint32_t)((unsigned long long)u >> 32);
-    top[v] = (int)(u >> 48);  // -128 .. 128
-  }
+// Digits of two consecutive K elements, one packed word per plane.  x = +-sum_t d_t 2^(e - 7 - 8 t):
+// the value m = round(|x| 2^(BITS - e)) in 64-bit integers and its balanced bytes (adding 128 to
+// every byte but the top one makes each byte d + 128); the bf16 value d sc_t comes from one FFMA
+// on 2^23 + byte, the sign from one XOR per pair.  Zeros, subnormals and runs of zeros
+// (e = ZERO_RUN) shift out to 0.
+__device__ __forceinline__ void digits2(unsigned long long x0, unsigned long long x1, int e, const float (&sc)[S],
+                                        const float (&cc)[S], uint32_t (&out)[S]) {
+  // (m << 1) + 1 + 2 bias before the last shift: rounding and bias in one addition
+  constexpr unsigned long long rb = 2 * 0x0000808080808080ull + 1;
+  auto fixed = [&](unsigned long long x) {
+    const uint32_t h = (uint32_t)(x >> 32), l = (uint32_t)x;
+    // mantissa 2^10 (63 bits) shifted right by (e - exponent) + 62 - BITS: 2 m with one guard bit
+    const unsigned long long M = ((unsigned long long)((h & 0xFFFFFu) | 0x100000u) << 32 | l) << 10;
+    const uint32_t sh = (uint32_t)(e + 1022 + 62 - BITS) - ((h >> 20) & 0x7FFu);
+    unsigned long long t;
+    asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(M), "r"(sh));  // amounts beyond 63 give 0
+    return (t + rb) >> 1;
+  };
+  const unsigned long long u0 = fixed(x0), u1 = fixed(x1);
+  const uint32_t lo0 = (uint32_t)u0, hi0 = (uint32_t)(u0 >> 32), lo1 = (uint32_t)u1, hi1 = (uint32_t)(u1 >> 32);
+  const uint32_t sg = __byte_perm((uint32_t)(x0 >> 32), (uint32_t)(x1 >> 32), 0x7632) & 0x80008000u;
 #pragma unroll
   for (int t = 0; t < S; ++t) {
-    float f[4];
-    const float c = -8388736.0f * sc[t];  // -(2^23 + 128) scale
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      uint32_t w;
-      if (t == 0) w = 0x4B000000u + (uint32_t)(top[v] + 128);
-      else if (t <= 2) w = __byte_perm(hi[v], 0x4B000000u, t == 1 ? 0x7651 : 0x7650);
-      else w = __byte_perm(lo[v], 0x4B000000u, t == 3 ? 0x7653 : t == 4 ? 0x7652 : t == 5 ? 0x7651 : 0x7650);
-      f[v] = fmaf(__uint_as_float(w), sc[t], c);
+    uint32_t w0, w1;
+    if (t == 0) {
+      w0 = 0x4B000080u + (hi0 >> 16);  // the top digit is not biased: 0 .. 128
+      w1 = 0x4B000080u + (hi1 >> 16);
+    } else {
+      const int sel = t == 1 || t == 5 ? 0x7651 : t == 2 || t == 6 ? 0x7650 : t == 3 ? 0x7653 : 0x7652;
+      w0 = __byte_perm(t <= 2 ? hi0 : lo0, 0x4B000000u, sel);
+      w1 = __byte_perm(t <= 2 ? hi1 : lo1, 0x4B000000u, sel);
     }
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out[t].x) : "f"(f[1]), "f"(f[0]));
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out[t].y) : "f"(f[3]), "f"(f[2]));
+    const float f0 = fmaf(__uint_as_float(w0), sc[t], cc[t]), f1 = fmaf(__uint_as_float(w1), sc[t], cc[t]);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(out[t]) : "f"(f1), "f"(f0));
+    out[t] ^= sg;
   }
 }
 
-// One block per (32 rows, run).  phase 1: run and row exponents only (more than one run per row);
-// phase 2: digits from stored exponents; phase 3: both (a row is one run: its elements are read
-// twice, the second time through L2).  Reads are coalesced along K (ks == 1) or along the rows
-// (through a shared-memory transpose); the planes are written along K.
-// Bound: HBM (8 bytes read, 14 written per element) when large; about 40 integer and FP32
-// instructions per element keep the issue slots under that.
-constexpr int SROWS = 32, SK = 64, SLD = SK + 2;
-__global__ void __launch_bounds__(256) oz_slice_kernel(const __grid_constant__ Operand oa,
-                                                       const __grid_constant__ Operand ob, int64_t units_a,
-                                                       int64_t units, int phase, int *flag) {
-  __shared__ __align__(16) double tile[SROWS][SLD];
-  __shared__ unsigned long long red[8][SROWS];
-  __shared__ int s_e[SROWS], s_rel[SROWS];
+// Eight consecutive K elements into the planes (16 bytes each).
+__device__ __forceinline__ void store8(const unsigned long long *x, int e, const float (&sc)[S], const float (&cc)[S],
+                                       uint16_t *out, int64_t plane) {
+  uint32_t d[4][S];
+#pragma unroll
+  for (int v = 0; v < 4; ++v) digits2(x[2 * v], x[2 * v + 1], e, sc, cc, d[v]);
+#pragma unroll
+  for (int t = 0; t < S; ++t, out += plane)
+    *reinterpret_cast<uint4 *>(out) = make_uint4(d[0][t], d[1][t], d[2][t], d[3][t]);
+}
+
+// Scales of a row's digits, sc[t] = 2^(rel + BIAS - 7 - 8 t), and cc[t] = -(2^23 + 128) sc[t]; runs
+// far below their row (rel < -169) vanish.
+__device__ __forceinline__ void digit_scales(int rel, float (&sc)[S], float (&cc)[S]) {
+  const int pe = 127 + rel + BIAS - 7;
+  sc[0] = pe >= 1 ? __int_as_float(pe << 23) : 0.f;
+#pragma unroll
+  for (int t = 1; t < S; ++t) sc[t] = sc[t - 1] * 0.00390625f;
+#pragma unroll
+  for (int t = 0; t < S; ++t) cc[t] = -8388736.0f * sc[t];
+}
+
+// Rows of one block's unit (256 threads, segments of 256 K elements): 32, and more where the rows
+// are shorter.
+constexpr int SEG = 256;
+__host__ __device__ __forceinline__ int slice_rows(int64_t Kp) {
+  return Kp <= 32 ? 256 : Kp <= 64 ? 128 : Kp <= 128 ? 64 : 32;
+}
+
+// Digit planes of slice_rows rows and a segment of K per block.  phase 3 (rows of one segment): the
+// row maxima, then the digits; longer rows: phase 1 takes the run and row exponents, phase 2 the
+// digits.  Every element is loaded once per phase.  The digits are made by a warp (part) per row,
+// eight elements per lane, so that the planes are written in whole lines; operands contiguous
+// along K are read that way, others (contiguous along the rows) with a lane per row, 32 elements
+// of it in flight, and turned in shared memory.  Bound: HBM (8 bytes read, 14 written per element)
+// when large.  66000 x 220 contiguous along the rows: 125 us in strips of 64 elements with 130
+// instructions per element, 143 us with a lane per row to the end (16-byte stores to 32 lines),
+// 70 us.
+constexpr int SLICE_SMEM = 256 * (32 + 2) * 8;  // the largest tile: rows x (elements + 2)
+__global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant__ Operand oa,
+                                                          const __grid_constant__ Operand ob, int units_a, int units,
+                                                          int phase, int *flag) {
+  extern __shared__ __align__(16) unsigned long long tile[];
+  __shared__ unsigned long long red[256];
+  __shared__ int s_e[256];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int64_t u0 = blockIdx.x; u0 < units; u0 += gridDim.x) {
+  constexpr unsigned long long kAbs = ~(1ull << 63);  // |x| as integers: of a double it is an FP64 instruction
+  for (int u0 = blockIdx.x; u0 < units; u0 += gridDim.x) {  // 32-bit divisions: 64-bit ones use the FP64 pipe
     const bool is_a = u0 < units_a;
     const Operand &o = is_a ? oa : ob;
-    const int64_t u = is_a ? u0 : u0 - units_a;
-    const int64_t rb = u / o.nruns * SROWS, run = u % o.nruns;
-    const int64_t k0 = run * RUN, k1 = min(o.K, k0 + RUN), kp1 = min(o.Kp, k0 + RUN);
-    const bool kc = o.ks == 1;
-    const int nrow = (int)min((int64_t)SROWS, o.rows - rb);
-    __syncthreads();  // the previous unit's shared values are read
-    if (phase & 1) {
-      if (kc) {
-        for (int q = 0; q < 4; ++q) {
-          const int row = warp * 4 + q;
-          unsigned long long mx = 0;
-          if (row < nrow) {
-            const double *src = o.p + o.map.at(o.r0 + rb + row);
-#pragma unroll 4
-            for (int64_t k = k0 + lane; k < k1; k += 32) {
-              const unsigned long long a = (unsigned long long)__double_as_longlong(__ldg(src + k)) & ~(1ull << 63);
-              mx = a > mx ? a : mx;
-            }
-          }
-#pragma unroll
-          for (int w = 16; w; w >>= 1) {
-            const unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, w);
-            mx = y > mx ? y : mx;
-          }
-          if (lane == 0) red[0][row] = mx;
-        }
-        __syncthreads();
+    const int u = is_a ? u0 : u0 - units_a;
+    const int nseg = ((int)o.Kp + SEG - 1) / SEG, urows = slice_rows(o.Kp);
+    const int64_t rb = (int64_t)(u / nseg) * urows;
+    const int nrow = (int)min((int64_t)urows, o.rows - rb);
+    const int seg = u % nseg, run = seg / (RUN / SEG);
+    const int64_t k0 = (int64_t)seg * SEG;
+    const int kn = (int)min((int64_t)SEG, o.K - k0), kp = (int)min((int64_t)SEG, o.Kp - k0);  // and with padding
+    const int64_t plane = o.rows * o.Kp;
+    const unsigned long long *base = reinterpret_cast<const unsigned long long *>(o.p);
+    const int nwk = 256 / urows, ldt = 32 * nwk + 2;  // warps along K (32 elements each), row stride of the tile
+    auto exponent = [&](unsigned long long mx) {  // mx < 2^e
+      const int e = mx == 0 ? ZERO_RUN : (int)(mx >> 52) - 1022;
+      // infinities, NaNs and the ends of the exponent range: the whole product by FMA
+      if (mx != 0 && (e > E_MAX || e < -E_MAX)) atomicMax(flag, 1);
+      return e;
+    };
+    auto record = [&](int64_t row, int e) {
+      if (phase == 1) {
+        atomicMax(o.erun + row * o.nruns + run, e);
+        atomicMax(o.erow + row, e);
       } else {
-        unsigned long long mx = 0;
-        if (lane < nrow) {
-          const double *src = o.p + o.map.at(o.r0 + rb + lane);
-#pragma unroll 4
-          for (int64_t k = k0 + warp; k < k1; k += 8) {
-            const unsigned long long a =
-                (unsigned long long)__double_as_longlong(__ldg(src + k * o.ks)) & ~(1ull << 63);
-            mx = a > mx ? a : mx;
-          }
-        }
-        red[warp][lane] = mx;
-        __syncthreads();
-        if (warp == 0) {
-#pragma unroll
-          for (int w = 1; w < 8; ++w) mx = red[w][lane] > mx ? red[w][lane] : mx;
-          red[0][lane] = mx;
-        }
-        __syncthreads();
+        o.erow[row] = e;
       }
-      if (tid < SROWS) {
-        const unsigned long long mx = red[0][tid];
-        const int e = mx == 0 ? ZERO_RUN : (int)(mx >> 52) - 1022;  // mx < 2^e
-        // infinities, NaNs and the ends of the exponent range: the whole product by FMA
-        if (mx != 0 && (e > E_MAX || e < -E_MAX)) atomicMax(flag, 1);
-        s_e[tid] = e;
-        s_rel[tid] = 0;
-        if (tid < nrow) {
-          if (phase == 1) {
-            o.erun[(rb + tid) * o.nruns + run] = e;
-            atomicMax(o.erow + rb + tid, e);
-          } else {
-            o.erow[rb + tid] = e;
-          }
-        }
+    };
+    const bool turned = o.ks != 1;
+    if (turned) {  // lanes along the rows: loads, maxima, tile
+      const int r = (warp / nwk) * 32 + lane, k = (warp % nwk) * 32;
+      const bool in = r < nrow && k < kp;
+      unsigned long long x[32];
+      const unsigned long long *src = base + o.map.at(o.r0 + rb + (in ? r : 0)) + (k0 + k) * o.ks;
+#pragma unroll
+      for (int v = 0; v < 32; ++v, src += o.ks) x[v] = in && k + v < kn ? __ldg(src) : 0ull;
+      __syncthreads();  // the previous unit's shared values are read
+      if (phase & 1) {
+        unsigned long long mx = 0;
+#pragma unroll
+        for (int v = 0; v < 32; ++v) mx = (x[v] & kAbs) > mx ? (x[v] & kAbs) : mx;
+        red[tid] = mx;
+      }
+      if (phase != 1) {
+#pragma unroll
+        for (int v = 0; v < 32; ++v) tile[r * ldt + k + v] = x[v];
+      }
+      __syncthreads();
+      if ((phase & 1) && warp % nwk == 0 && r < nrow) {
+        unsigned long long mx = red[tid];
+        for (int w = 1; w < nwk; ++w) mx = red[tid + 32 * w] > mx ? red[tid + 32 * w] : mx;
+        const int e = exponent(mx);
+        s_e[r] = e;
+        record(rb + r, e);
       }
       if (phase == 1) continue;
-    } else {
-      if (tid < nrow) {
-        const int e = o.erun[(rb + tid) * o.nruns + run];
-        s_e[tid] = e;
-        s_rel[tid] = e - o.erow[rb + tid];
-      }
+      if (phase == 3) __syncthreads();
     }
-    __syncthreads();
-    // digits: a thread takes four consecutive K elements of two rows of every 64-wide strip
-    float sc[2][S];
-    int ee[2];
-    const double *src[2];
-    const int kq = (tid & 15) * 4;
+    // digits: lanes of one row, eight elements each
+    const int lpr = kp <= 32 ? 4 : kp <= 64 ? 8 : kp <= 128 ? 16 : 32, rpw = 32 / lpr;
+    const int k = 8 * (lane & (lpr - 1));
+    for (int q = 0; q < urows / 8; q += rpw) {
+      const int r = warp * (urows / 8) + q + lane / lpr;
+      const int64_t row = rb + r;
+      const bool in = r < nrow && k < kp;
+      unsigned long long x[8];
+      if (turned) {
+        const unsigned long long *src = tile + (in ? r * ldt + k : 0);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int row = (tid >> 4) + 16 * i;
-      ee[i] = row < nrow ? s_e[row] : ZERO_RUN;
-      const int rel = row < nrow && ee[i] != ZERO_RUN ? s_rel[row] : 0;
-      src[i] = o.p + (row < nrow ? o.map.at(o.r0 + rb + row) : 0);
-#pragma unroll
-      for (int t = 0; t < S; ++t) {  // 2^(rel + BIAS - 7 - 8 t); below the FP32 range: 0
-        const int pe = 127 + rel + BIAS - 7 - 8 * t;
-        sc[i][t] = pe >= 1 ? __int_as_float(pe << 23) : 0.f;
-      }
-    }
-    for (int64_t kt = k0; kt < kp1; kt += SK) {
-      if (!kc) {
-        __syncthreads();
-        const double *sr = o.p + (lane < nrow ? o.map.at(o.r0 + rb + lane) : 0);
-#pragma unroll
-        for (int j = 0; j < SK / 8; ++j) {
-          const int64_t k = kt + warp + 8 * j;
-          tile[lane][warp + 8 * j] = (lane < nrow && k < k1) ? __ldg(sr + k * o.ks) : 0.0;
+        for (int v = 0; v < 8; v += 2) {
+          const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(src + v);
+          x[v] = a.x;
+          x[v + 1] = a.y;
         }
-        __syncthreads();
-      }
-      if (kt + kq >= kp1) continue;
+      } else {
+        const unsigned long long *src = base + (in ? o.map.at(o.r0 + row) + k0 + k : 0);
+        if (in && ((uintptr_t)src & 15) == 0 && k + 8 <= kn) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int row = (tid >> 4) + 16 * i;
-        if (row >= nrow) continue;
-        double x[4];
-        const int64_t k = kt + kq;
-        if (kc) {
-          const double *q = src[i] + k;
-          if (k + 4 <= k1 && ((uintptr_t)q & 15) == 0) {
-            const double2 a = __ldg(reinterpret_cast<const double2 *>(q));
-            const double2 b = __ldg(reinterpret_cast<const double2 *>(q) + 1);
-            x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-          } else {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) x[v] = k + v < k1 ? __ldg(q + v) : 0.0;
+          for (int v = 0; v < 8; v += 2) {
+            const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(src + v));
+            x[v] = a.x;
+            x[v + 1] = a.y;
           }
         } else {
-          const double2 a = *reinterpret_cast<const double2 *>(&tile[row][kq]);
-          const double2 b = *reinterpret_cast<const double2 *>(&tile[row][kq + 2]);
-          x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-        }
-        uint2 d[S];
-        digits4(x, ee[i], sc[i], d);
-        uint16_t *out = o.planes + (rb + row) * o.Kp + k;
-        const int64_t plane = o.rows * o.Kp;
 #pragma unroll
-        for (int t = 0; t < S; ++t) *reinterpret_cast<uint2 *>(out + t * plane) = d[t];
+          for (int v = 0; v < 8; ++v) x[v] = in && k + v < kn ? __ldg(src + v) : 0ull;
+        }
+      }
+      int e = 0, rel = 0;
+      if (phase == 2) {
+        if (in) {
+          e = o.erun[row * o.nruns + run];
+          rel = e == ZERO_RUN ? 0 : e - o.erow[row];
+        }
+      } else if (turned) {
+        if (in) e = s_e[r];
+      } else {
+        unsigned long long mx = 0;
+#pragma unroll
+        for (int v = 0; v < 8; ++v) mx = (x[v] & kAbs) > mx ? (x[v] & kAbs) : mx;
+        for (int w = lpr / 2; w; w >>= 1) {
+          const unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, w);
+          mx = y > mx ? y : mx;
+        }
+        e = mx == 0 ? ZERO_RUN : (int)(mx >> 52) - 1022;
+        if (k == 0 && in) record(row, exponent(mx));
+        if (phase == 1) continue;
+      }
+      if (in) {
+        float sc[S], cc[S];
+        digit_scales(rel, sc, cc);
+        store8(x, e, sc, cc, o.planes + row * o.Kp + k0 + k, plane);
       }
     }
   }
@@ -243,7 +263,7 @@ struct GemmArgs {
   int a_plane, b_plane;      // operand rows between planes
   int nkb, kb_per, splits;   // K stages, stages per split (a multiple of HB)
   int64_t m_first, b_first;  // first C row and batch of this launch (chunks)
-  int64_t mt, nt, ntiles;
+  int mt, nt, ntiles;
   const int *erow_a, *erow_b, *flag;
   Operand A, B;              // sources, for the FMA path
   OzMap crow, ccol, cbatch;  // C offsets of tile rows, columns and batches
@@ -251,26 +271,28 @@ struct GemmArgs {
   double *C;
   double alpha, beta;
   int alpha_exp, alpha_pow2; // alpha = +-2^alpha_exp
+  int accumulate;            // beta != 0 (an FP64 comparison costs what an FMA does)
+  int plain;                 // neither alpha (a power of two) nor beta costs FP64 work per element
   int *err;
 };
 
 struct Tile {
-  int64_t m, n, b;
-  int s;
+  int m, n, b, s;
 };
 // M tiles in panels of 16, so that the tiles in flight share their A and B planes in L2
-__device__ __forceinline__ Tile tile_of(const GemmArgs &p, int64_t t) {
+__device__ __forceinline__ Tile tile_of(const GemmArgs &p, int tile) {
   Tile c;
-  const int64_t per = p.mt * p.nt * p.splits;
-  c.b = t / per;
+  uint32_t t = (uint32_t)tile;
+  const uint32_t per = (uint32_t)(p.mt * p.nt * p.splits);
+  c.b = (int)(t / per);
   t -= c.b * per;
-  const int64_t pw = 16 * p.nt * p.splits, pan = t / pw;
+  const uint32_t pw = 16u * (uint32_t)(p.nt * p.splits), pan = t / pw;
   t -= pan * pw;
-  const int64_t g = min((int64_t)16, p.mt - pan * 16);
-  c.m = pan * 16 + t % g;
+  const uint32_t g = min(16u, (uint32_t)p.mt - pan * 16u);
+  c.m = (int)(pan * 16 + t % g);
   t /= g;
-  c.n = t % p.nt;
-  c.s = (int)(t / p.nt);
+  c.n = (int)(t % (uint32_t)p.nt);
+  c.s = (int)(t / (uint32_t)p.nt);
   return c;
 }
 
@@ -280,60 +302,62 @@ __device__ __forceinline__ void two_sum(float &h, float &l, float x) {
   h = s;
 }
 
-__device__ __forceinline__ void add_level(float (&h)[EC], float (&l)[EC], const uint32_t (&r)[EC]) {
+// the 16 columns of a thread at TMEM address t, eight at a time, into the pair sums (h, l) or l
+__device__ __forceinline__ void add_level(float (&h)[EC], float (&l)[EC], uint32_t t) {
 #pragma unroll
-  for (int j = 0; j < EC; ++j) two_sum(h[j], l[j], __uint_as_float(r[j]));
+  for (int j0 = 0; j0 < EC; j0 += 8) {
+    uint32_t r[8];
+    tmem_ld8(t + j0, r);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) two_sum(h[j0 + j], l[j0 + j], __uint_as_float(r[j]));
+  }
 }
-__device__ __forceinline__ void add_low(float (&l)[EC], const uint32_t (&r)[EC]) {
+__device__ __forceinline__ void add_low(float (&l)[EC], uint32_t t) {
 #pragma unroll
-  for (int j = 0; j < EC; ++j) l[j] += __uint_as_float(r[j]);
+  for (int j0 = 0; j0 < EC; j0 += 8) {
+    uint32_t r[8];
+    tmem_ld8(t + j0, r);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) l[j0 + j] += __uint_as_float(r[j]);
+  }
 }
 
-__device__ __forceinline__ long long mant24(float f) {
-  const uint32_t b = __float_as_uint(f);
-  const int m = (b & 0x7F800000u) ? (int)((b & 0x7FFFFFu) | 0x800000u) : 0;
-  return (b >> 31) ? -m : m;
+// The float with bits b as a fixed point: mantissa 2^36 shifted down by top - its exponent (a zero
+// has no exponent to speak of and shifts out)
+__device__ __forceinline__ long long place(uint32_t b, int top) {
+  const int sg = (int)b >> 31;
+  const int m = ((int)((b & 0x7FFFFFu) | 0x800000u) ^ sg) - sg;
+  long long r;
+  // shifts beyond 63 give the sign
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"((long long)((unsigned long long)(uint32_t)(m << 4) << 32)),
+      "r"((uint32_t)(top - (int)((b >> 23) & 0xFF))));
+  return r;
 }
 
-// (h1 + l1 + h2 + l2) 2^e rounded to FP64, in integers (an FP64 instruction costs 16 clocks of a
-// warp here): the sum as three non-overlapping floats, a 61-bit fixed point, a rounded mantissa.
+// (h1 + l1 + h2 + l2) 2^e rounded to FP64: l1 + h2 + l2 as a float pair, the three floats in one
+// 62-bit fixed point, one conversion, the exponent in integers.  Every FP64 instruction of an
+// element (also one behind a false predicate) is 64 clocks of an SM quarter, 4096 a tile: with a
+// comparison, a scaling and an update compiled in for all, the last step was a third of the
+// kernel on 66000 x 450 x 220 (440 us, 345 without them).
 __device__ __forceinline__ double assemble(float h1, float l1, float h2, float l2, int e, bool neg) {
-  float z = 0.f, c = l1, x = h1, y = 0.f, w = 0.f;
+  float c = l1, z = 0.f;
   two_sum(c, z, h2);
   z += l2;
-  two_sum(x, y, c);   // x + y = h1 + c
-  two_sum(y, w, z);   // y + w = y + z
-  float t = 0.f;
-  two_sum(x, t, y);   // renormalise: x leads, t + w trail
-  float t2 = 0.f;
-  two_sum(t, t2, w);
-  const uint32_t bx = __float_as_uint(x);
-  const int ex = (int)((bx >> 23) & 0xFF);
-  if (ex == 0) return neg ? -0.0 : 0.0;
-  long long T = mant24(x) << 36;  // unit 2^(ex - 186)
-  const int s1 = 36 - (ex - (int)((__float_as_uint(t) >> 23) & 0xFF));
-  const long long m1 = mant24(t);
-  T += s1 >= 0 ? m1 << s1 : (s1 > -32 ? m1 >> -s1 : 0);
-  const int s2 = 36 - (ex - (int)((__float_as_uint(t2) >> 23) & 0xFF));
-  const long long m2 = mant24(t2);
-  T += s2 >= 0 ? m2 << s2 : (s2 > -32 ? m2 >> -s2 : 0);
-  unsigned long long u = (unsigned long long)(T < 0 ? -T : T);
-  const int lz = __clzll((long long)u);
-  u <<= lz;
-  const unsigned long long v = u + 0x3FFull + ((u >> 11) & 1ull);  // round to nearest even
-  const int be = ex - 123 - lz + e + 1023 + (v < u ? 1 : 0);
-  const bool sg = (T < 0) != neg;
-  if (be >= 1 && be <= 2046) {
-    const unsigned long long bits = ((unsigned long long)sg << 63) | ((unsigned long long)be << 52) |
-                                    ((v >> 11) & 0xFFFFFFFFFFFFFull);
-    return __longlong_as_double((long long)bits);
-  }
-  const double r = scalbn((double)(u >> 11), ex - 186 - lz + 11 + e);  // over- or underflow
-  return sg ? -r : r;
+  const uint32_t b0 = __float_as_uint(h1), b1 = __float_as_uint(c), b2 = __float_as_uint(z);
+  const int top = max((int)((b0 >> 23) & 0xFF), max((int)((b1 >> 23) & 0xFF), (int)((b2 >> 23) & 0xFF)));
+  const double v = __ll2double_rn(place(b0, top) + place(b1, top) + place(b2, top));
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  const int sg = neg ? (int)0x80000000 : 0;
+  if (top == 0 || hi == 0) return __hiloint2double(sg, 0);  // zero
+  const int k = e + top - 186;  // 2^36 and the float's 2^(top - 150)
+  const int be = ((hi >> 20) & 0x7FF) + k;
+  if (be >= 1 && be <= 2046) return __hiloint2double((hi + (k << 20)) ^ sg, lo);
+  const double r = scalbn(v, k);  // over- or underflow
+  return neg ? -r : r;
 }
 
 __device__ __forceinline__ void store_c(const GemmArgs &p, double *c, double v) {
-  *c = p.beta == 0.0 ? v : fma(p.beta, *c, v);
+  *c = p.accumulate ? fma(p.beta, *c, v) : v;
 }
 
 // The tile by FP64 FMA, for operands with infinities, NaNs or exponents at the ends of the range:
@@ -348,7 +372,7 @@ __device__ __noinline__ void fma_tile(const GemmArgs &p, const Tile &tc, double 
   const int64_t cb = p.cbatch.at(p.b_first + tc.b) + tc.s * p.c_split;
   const bool ak = p.A.ks == 1, bk = p.B.ks == 1;
   for (int h = 0; h < 2; ++h) {
-    const int64_t m0 = tc.m * BM + 64 * h, n0 = tc.n * BN;
+    const int64_t m0 = (int64_t)tc.m * BM + 64 * h, n0 = (int64_t)tc.n * BN;
     if (m0 >= p.M) break;
     __syncthreads();
     if (tid < 64) {
@@ -412,7 +436,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   if (*p.flag > 0) {  // uniform over the grid: set by the slicer, an earlier launch
-    for (int64_t R = blockIdx.x; R < p.ntiles; R += gridDim.x)
+    for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x)
       fma_tile(p, tile_of(p, R), reinterpret_cast<double *>(smem));
     return;
   }
@@ -420,8 +444,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
   uint64_t *empty = full + STAGES;
   uint64_t *accf = empty + STAGES;  // [0]: H complete, [1]: L complete
   uint64_t *acce = accf + 2;        // drained
-  uint32_t *tmem_slot = (uint32_t *)(acce + 2);
+  uint64_t *tabf = acce + 2;        // table of a tile ready / read, two deep
+  uint64_t *tabe = tabf + 2;
+  uint32_t *tmem_slot = (uint32_t *)(tabe + 2);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  TileTab *tabs = reinterpret_cast<TileTab *>(smem + STAGES * STAGE_BYTES + 256);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
@@ -431,6 +458,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
     for (int i = 0; i < 2; ++i) {
       mbar_init(&accf[i], 1);
       mbar_init(&acce[i], kEpi);
+      mbar_init(&tabf[i], 32 * kTab);
+      mbar_init(&tabe[i], kEpi);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -449,9 +478,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      for (int64_t R = blockIdx.x; R < p.ntiles; R += gridDim.x) {
+      for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x) {
         const Tile tc = tile_of(p, R);
-        const int ya = (int)(tc.b * p.M + tc.m * BM), yb = (int)(tc.b * p.N + tc.n * BN);
+        const int ya = (int)(tc.b * p.M) + tc.m * BM, yb = (int)(tc.b * p.N) + tc.n * BN;
         const int kb0 = tc.s * p.kb_per, kb1 = min(p.nkb, kb0 + p.kb_per);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 11)) goto tma_done;
@@ -474,7 +503,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0, eh = 0, el = 0;
-      for (int64_t R = blockIdx.x; R < p.ntiles; R += gridDim.x) {
+      for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x) {
         const Tile tc = tile_of(p, R);
         const int kb0 = tc.s * p.kb_per, n = min(p.nkb, kb0 + p.kb_per) - kb0;
         for (int i = 0; i < n; ++i) {
@@ -522,30 +551,49 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
       }
     mma_done:;
     }
+  } else if (warp >= 2 + kEpi) {
+    // ---- output offsets and exponents of every tile, ahead of its epilogue ----
+    const int i = threadIdx.x - 64 - 32 * kEpi;  // 0 .. 63
+    static_assert(32 * kTab == BN && 2 * BN == BM, "two rows and one column per table thread");
+    int it = 0;
+    for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x, ++it) {
+      const Tile tc = tile_of(p, R);
+      TileTab &tb = tabs[it & 1];
+      if (!mbar_wait(&tabe[it & 1], ((it >> 1) & 1) ^ 1, abort_flag, p.err, 18)) break;
+      const int64_t cb = p.cbatch.at(p.b_first + tc.b) + tc.s * p.c_split;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int64_t row = (int64_t)tc.m * BM + i + 64 * h;
+        const bool in = row < p.M;
+        tb.row[i + 64 * h] = in ? cb + p.crow.at(p.m_first + row) : -1;
+        tb.ea[i + 64 * h] = in ? max(p.erow_a[tc.b * p.M + row], -5000) - 2 * BIAS + p.alpha_exp : 0;
+      }
+      const int64_t col = (int64_t)tc.n * BN + i;
+      const bool in = col < p.N;
+      tb.col[i] = in ? p.ccol.at(col) : -1;
+      tb.eb[i] = in ? max(p.erow_b[tc.b * p.N + col], -5000) : 0;
+      mbar_arrive(&tabf[it & 1]);
+    }
   } else {
     const int q = warp % 4, part = (warp - 2) / 4;
     const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * EC);
+    const bool neg = p.alpha_pow2 < 0;
+    int it = 0;
     uint32_t ph = 0, pl = 0;
     float h1[EC], l1[EC], h2[EC], l2[EC];  // levels 0..2 as one pair, 3..7 as the other
-    for (int64_t R = blockIdx.x; R < p.ntiles; R += gridDim.x) {
-      const Tile tc = tile_of(p, R);
-      const int kb0 = tc.s * p.kb_per, n = min(p.nkb, kb0 + p.kb_per) - kb0;
+    for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x, ++it) {
+      const int kb0 = tile_of(p, R).s * p.kb_per, n = min(p.nkb, kb0 + p.kb_per) - kb0;
 #pragma unroll
       for (int j = 0; j < EC; ++j) h1[j] = l1[j] = h2[j] = l2[j] = 0.f;
       for (int i = 0; i < n; ++i) {
-        uint32_t r[EC];
         if ((i + 1) % HB == 0 || i + 1 == n) {
           if (!mbar_wait(&accf[0], ph, abort_flag, p.err, 14)) goto epi_done;
           ph ^= 1;
           fence_after();
-          tmem_ld16(tl, r);
-          add_level(h1, l1, r);
-          tmem_ld16(tl + 64, r);
-          add_level(h1, l1, r);
-          tmem_ld16(tl + 128, r);
-          add_level(h1, l1, r);
-          tmem_ld16(tl + 192, r);
-          add_level(h2, l2, r);
+          add_level(h1, l1, tl);
+          add_level(h1, l1, tl + 64);
+          add_level(h1, l1, tl + 128);
+          add_level(h2, l2, tl + 192);
           fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acce[0]);
@@ -554,41 +602,51 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
           if (!mbar_wait(&accf[1], pl, abort_flag, p.err, 17)) goto epi_done;
           pl ^= 1;
           fence_after();
-          tmem_ld16(tl + 448, r);
-          add_low(l2, r);
-          tmem_ld16(tl + 384, r);
-          add_low(l2, r);
-          tmem_ld16(tl + 320, r);
-          add_low(l2, r);
-          tmem_ld16(tl + 256, r);
-          add_level(h2, l2, r);
+          add_low(l2, tl + 448);
+          add_low(l2, tl + 384);
+          add_low(l2, tl + 320);
+          add_level(h2, l2, tl + 256);
           fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acce[1]);
         }
       }
-      const int64_t row = tc.m * BM + q * 32 + lane;
-      if (row < p.M) {
-        const int64_t cb = p.cbatch.at(p.b_first + tc.b) + tc.s * p.c_split;
-        double *crow = p.C + cb + p.crow.at(p.m_first + row);
-        const int ea = max(p.erow_a[tc.b * p.M + row], -5000) - 2 * BIAS + p.alpha_exp;
-        const bool neg = p.alpha_pow2 < 0;
-        const int64_t n0 = tc.n * BN + part * EC;
-        int64_t q0 = n0 % p.ccol.n0, q1 = (n0 / p.ccol.n0) % p.ccol.n1, q2 = n0 / p.ccol.n0 / p.ccol.n1;
+      if (!mbar_wait(&tabf[it & 1], (it >> 1) & 1, abort_flag, p.err, 19)) goto epi_done;
+      const TileTab &tb = tabs[it & 1];
+      const int64_t ro = tb.row[q * 32 + lane];
+      if (ro >= 0) {
+        double *crow = p.C + ro;
+        const int ea = tb.ea[q * 32 + lane];
+        if (p.plain) {
 #pragma unroll
-        for (int j = 0; j < EC; ++j) {
-          if (n0 + j < p.N) {
-            const int e = ea + max(__ldg(p.erow_b + tc.b * p.N + n0 + j), -5000);
-            double v = assemble(h1[j], l1[j], h2[j], l2[j], e, neg);
-            if (p.alpha_pow2 == 0) v *= p.alpha;
-            store_c(p, crow + q2 * p.ccol.s2 + q1 * p.ccol.s1 + q0 * p.ccol.s0, v);
+          for (int j = 0; j < EC; ++j) {
+            const int64_t co = tb.col[part * EC + j];
+            if (co >= 0) crow[co] = assemble(h1[j], l1[j], h2[j], l2[j], ea + tb.eb[part * EC + j], neg);
           }
-          if (++q0 == p.ccol.n0) {
-            q0 = 0;
-            if (++q1 == p.ccol.n1) { q1 = 0; ++q2; }
+        } else {
+#pragma unroll
+          for (int j0 = 0; j0 < EC; j0 += 4) {  // four columns at a time: their loads overlap
+            double old[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int64_t co = tb.col[part * EC + j0 + v];
+              old[v] = co >= 0 && p.accumulate ? crow[co] : 0.0;
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int j = j0 + v;
+              const int64_t co = tb.col[part * EC + j];
+              if (co >= 0) {
+                double x = assemble(h1[j], l1[j], h2[j], l2[j], ea + tb.eb[part * EC + j], neg);
+                if (p.alpha_pow2 == 0) x *= p.alpha;
+                crow[co] = p.accumulate ? fma(p.beta, old[v], x) : x;
+              }
+            }
           }
         }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tabe[it & 1]);
     }
   epi_done:;
   }
@@ -619,7 +677,7 @@ __global__ void oz_reduce_kernel(const double *__restrict__ part, int64_t M, int
 
 // ---------------- host ----------------
 
-constexpr int64_t kPlaneBudget = 1LL << 30;  // bytes of digit planes per operand and launch
+constexpr int64_t kPlaneBudget = 3LL << 29;  // bytes of digit planes per operand and launch
 
 }  // namespace
 
@@ -627,11 +685,13 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   OzPlan q;
   if (!ws || !oz_plan(d, sm_count(), kPlaneBudget, q) || !q.faster) return false;
   const int nruns = (int)ceil_div(q.Kp, RUN);
+  const int64_t nseg = ceil_div(q.Kp, SEG);
+  const bool two = nseg > 1;  // exponents before digits
   const int64_t rows_a = q.m_chunk * q.tb_chunk, rows_b = q.N * q.tb_chunk;
   const int64_t ni = 64 + rows_a + rows_b;  // [flag | row exponents of A | of B], then run exponents
   double *partial = nullptr;
   try {
-    ws->oz_int.resize((size_t)(ni + (nruns > 1 ? (rows_a + rows_b) * nruns : 0)));
+    ws->oz_int.resize((size_t)(ni + (two ? (rows_a + rows_b) * nruns : 0)));
     ws->oz_a.resize((size_t)(rows_a * q.Kp * S));
     ws->oz_b.resize((size_t)(rows_b * q.Kp * S));
     if (q.splits > 1) {
@@ -646,6 +706,7 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   static std::once_flag attr;
   std::call_once(attr, [] {
     VGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    VGB_CUDA(cudaFuncSetAttribute(oz_slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SLICE_SMEM));
   });
   GemmArgs p;
   Operand A, B;
@@ -680,29 +741,37 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
     p.alpha = d.alpha; p.beta = d.beta;
     p.crow = q.crow; p.ccol = q.ccol; p.cbatch = q.cbatch;
   }
+  p.accumulate = p.beta != 0.0 ? 1 : 0;
   int ae = 0;
   const double am = std::frexp(p.alpha, &ae);
   p.alpha_pow2 = am == 0.5 ? 1 : am == -0.5 ? -1 : 0;
   p.alpha_exp = p.alpha_pow2 ? ae - 1 : 0;
+  p.plain = p.alpha_pow2 && !p.accumulate ? 1 : 0;
   // exponents start below any value (0x80808080), the flag at "not set"
-  VGB_CUDA(cudaMemsetAsync(ip, 0x80, (size_t)ni * sizeof(int), stream));
+  const int64_t nrun_ints = two ? (rows_a + rows_b) * nruns : 0;
+  VGB_CUDA(cudaMemsetAsync(ip, 0x80, (size_t)(ni + nrun_ints) * sizeof(int), stream));
   for (int64_t t0 = 0; t0 < q.nbatch; t0 += q.tb_chunk)
     for (int64_t m0 = 0; m0 < q.M; m0 += q.m_chunk) {
       const int64_t tn = std::min(q.tb_chunk, q.nbatch - t0), mn = std::min(q.m_chunk, q.M - m0);
       const bool new_b = m0 == 0;
       A.r0 = t0 * q.M + m0; A.rows = tn * mn;  // row chunks only without batches
       B.r0 = t0 * q.N; B.rows = tn * q.N;
-      if (t0 + m0 > 0 && nruns > 1) {
+      if (t0 + m0 > 0 && two) {
         VGB_CUDA(cudaMemsetAsync(A.erow, 0x80, (size_t)A.rows * sizeof(int), stream));
-        if (new_b) VGB_CUDA(cudaMemsetAsync(B.erow, 0x80, (size_t)B.rows * sizeof(int), stream));
+        VGB_CUDA(cudaMemsetAsync(A.erun, 0x80, (size_t)(A.rows * nruns) * sizeof(int), stream));
+        if (new_b) {
+          VGB_CUDA(cudaMemsetAsync(B.erow, 0x80, (size_t)B.rows * sizeof(int), stream));
+          VGB_CUDA(cudaMemsetAsync(B.erun, 0x80, (size_t)(B.rows * nruns) * sizeof(int), stream));
+        }
       }
-      const int64_t ua = ceil_div(A.rows, SROWS) * nruns, ub = new_b ? ceil_div(B.rows, SROWS) * nruns : 0;
+      const int64_t ua = ceil_div(A.rows, slice_rows(q.Kp)) * nseg;
+      const int64_t ub = new_b ? ceil_div(B.rows, slice_rows(q.Kp)) * nseg : 0;
       const unsigned sg = (unsigned)std::min<int64_t>(ua + ub, 64LL * sm_count());
-      if (nruns > 1) {
-        oz_slice_kernel<<<sg, 256, 0, stream>>>(A, B, ua, ua + ub, 1, ip);
+      if (two) {
+        oz_slice_kernel<<<sg, 256, SLICE_SMEM, stream>>>(A, B, (int)ua, (int)(ua + ub), 1, ip);
         VGB_LAUNCH_CHECK();
       }
-      oz_slice_kernel<<<sg, 256, 0, stream>>>(A, B, ua, ua + ub, nruns > 1 ? 2 : 3, ip);
+      oz_slice_kernel<<<sg, 256, SLICE_SMEM, stream>>>(A, B, (int)ua, (int)(ua + ub), two ? 2 : 3, ip);
       VGB_LAUNCH_CHECK();
       encode_kmajor(&p.map_a, A.planes, S * A.rows, q.Kp, q.Kp, BM, BK);
       encode_kmajor(&p.map_b, B.planes, S * B.rows, q.Kp, q.Kp, BN, BK);
@@ -714,12 +783,12 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
       p.b_plane = (int)B.rows;
       p.erow_a = A.erow;
       p.erow_b = B.erow;
-      p.mt = ceil_div(p.M, BM);
-      p.nt = ceil_div(p.N, BN);
-      p.ntiles = p.mt * p.nt * tn * q.splits;
+      p.mt = (int)ceil_div(p.M, BM);
+      p.nt = (int)ceil_div(p.N, BN);
+      p.ntiles = (int)(p.mt * p.nt * tn * q.splits);
       p.m_first = m0;
       p.b_first = t0;
-      oz_gemm_kernel<<<(unsigned)std::min<int64_t>(p.ntiles, sm_count()), kGemmThreads, SMEM_BYTES, stream>>>(p);
+      oz_gemm_kernel<<<(unsigned)std::min(p.ntiles, sm_count()), kGemmThreads, SMEM_BYTES, stream>>>(p);
       VGB_LAUNCH_CHECK();
     }
   if (q.splits > 1) {

@@ -27,10 +27,17 @@ constexpr int64_t kOzOne = 1LL << 62;  // a map of one level
 // Index r = (q2 * n1 + q1) * n0 + q0 at q2 s2 + q1 s1 + q0 s0.
 struct OzMap {
   int64_t n0 = 1, n1 = 1, s0 = 0, s1 = 0, s2 = 0;
+  // 32-bit divisions where the index fits (64-bit ones convert through the FP64 pipe)
   VGB_HD int64_t at(int64_t r) const {
-    const int64_t q0 = r % n0;
-    r /= n0;
-    return (r / n1) * s2 + (r % n1) * s1 + q0 * s0;
+    if (r < n0) return r * s0;
+    if (r >> 32) {
+      const int64_t q0 = r % n0, q = r / n0;
+      return (q / n1) * s2 + (q % n1) * s1 + q0 * s0;
+    }
+    const uint32_t x = (uint32_t)r, d = (uint32_t)n0, q = x / d, q0 = x - q * d;  // n0 <= r
+    if (q < n1) return (int64_t)q * s1 + (int64_t)q0 * s0;
+    const uint32_t e = (uint32_t)n1, q2 = q / e;
+    return (int64_t)q2 * s2 + (int64_t)(q - q2 * e) * s1 + (int64_t)q0 * s0;
   }
 };
 
@@ -106,29 +113,43 @@ inline bool oz_plan(const GemmDesc &d, int sms, int64_t plane_budget, OzPlan &q)
   q.Kp = oz_ceil(d.K, kOzStageK) * kOzStageK;
   if (q.Kp >= (1LL << 31) || q.M >= (1LL << 27) || q.N >= (1LL << 27)) return false;
   const int64_t tiles = oz_ceil(q.M, kOzTileM) * oz_ceil(q.N, kOzTileN) * q.nbatch;
+  if (tiles >= (1LL << 24)) return false;  // tile indices (times at most 152 splits) in 32 bits
   q.nkb = (int)(q.Kp / kOzStageK);
-  // K splits: one wave of the SMs; a split is a whole number of drain intervals
-  q.splits = 1;
-  if (tiles < sms) q.splits = (int)std::max<int64_t>(1, std::min<int64_t>(sms / tiles, q.nkb / kOzDrain));
-  q.kb_per = q.splits == 1 ? q.nkb : (int)(oz_ceil(oz_ceil(q.nkb, q.splits), kOzDrain) * kOzDrain);
-  q.splits = (int)oz_ceil(q.nkb, q.kb_per);
-  // chunks: whole batches, or rows of A, within the budget of planes
+  // chunks: equal shares of the batches, or of the row tiles of A, within the budget of planes
   const int64_t plane_row = (int64_t)kOzDigits * q.Kp * 2;
   q.m_chunk = q.M;
   q.tb_chunk = q.nbatch;
-  if (q.nbatch > 1)
-    q.tb_chunk = std::max<int64_t>(1, std::min<int64_t>(q.nbatch, plane_budget / (plane_row * std::max(q.M, q.N))));
-  else if (q.M * plane_row > plane_budget)
-    q.m_chunk = std::min(q.M, std::max<int64_t>(kOzTileM, plane_budget / plane_row / kOzTileM * kOzTileM));
+  if (q.nbatch > 1) {
+    const int64_t fit = std::max<int64_t>(1, plane_budget / (plane_row * std::max(q.M, q.N)));
+    q.tb_chunk = oz_ceil(q.nbatch, oz_ceil(q.nbatch, fit));
+  } else if (q.M * plane_row > plane_budget) {
+    const int64_t mt = oz_ceil(q.M, kOzTileM), fit = std::max<int64_t>(1, plane_budget / plane_row / kOzTileM);
+    q.m_chunk = std::min(q.M, oz_ceil(mt, oz_ceil(mt, fit)) * kOzTileM);
+  }
   const int64_t most = std::max(q.m_chunk, q.N) * q.tb_chunk;
   if (most * plane_row > 4 * plane_budget || most * kOzDigits >= (1LL << 31)) return false;
-  // Times of either path in microseconds, from measurements on a GB300: the digit path is two to
-  // four launches, 30 bytes of traffic per operand element (read twice, planes written) and 2500
-  // clocks per stage and wave of tiles.
+  if ((most / 16 + 2) * (q.Kp / 256 + 1) >= (1LL << 31)) return false;  // units of the slicer
+  // K splits (whole drain intervals): the fewest waves of work items over the SMs, against the FP64
+  // partials they write.  Times in microseconds, from measurements on a GB300: 2400 clocks per
+  // stage, 6000 per item.
+  const int64_t nchunks = q.nbatch > 1 ? oz_ceil(q.nbatch, q.tb_chunk) : oz_ceil(q.M, q.m_chunk);
+  const int64_t ctiles = oz_ceil(q.m_chunk, kOzTileM) * oz_ceil(q.N, kOzTileN) * q.tb_chunk;
+  double t_gemm = 1e300;
+  for (int s = 1; s <= std::max(1, std::min(64, q.nkb / kOzDrain)); ++s) {
+    const int per = s == 1 ? q.nkb : (int)(oz_ceil(oz_ceil(q.nkb, s), kOzDrain) * kOzDrain);
+    const int sp = (int)oz_ceil(q.nkb, per);
+    const double t = nchunks * (double)oz_ceil(ctiles * sp, sms) * (per * 2400.0 + 6000.0) / 1.9e3 +
+                     (sp > 1 ? 5.0 + 16.0 * sp * q.M * q.N * q.nbatch / 4e6 : 0.0);
+    if (t < 0.98 * t_gemm) {
+      t_gemm = t;
+      q.splits = sp;
+      q.kb_per = per;
+    }
+    if (ctiles * sp >= 8LL * sms) break;
+  }
+  // the slicer: 5e-6 us per element (read once or twice, planes written), and the launches
   const double elems = (double)(q.M + q.N) * q.nbatch * d.K;
-  const double waves = (double)oz_ceil(tiles * q.splits, sms);
-  const double t_oz = 14.0 + elems * 30.0 / 3.5e6 + waves * (q.kb_per * 2500.0 + 4000.0) / 1.9e3 +
-                      (q.splits > 1 ? 3.0 + 16.0 * q.splits * q.M * q.N * q.nbatch / 4e6 : 0.0);
+  const double t_oz = nchunks * (q.Kp > 256 ? 20.0 : 15.0) + elems * 5.2e-6 + t_gemm;
   q.faster = t_oz < fma_plan(d, sms, 0).time_us;
   return true;
 }
