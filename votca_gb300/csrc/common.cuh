@@ -46,7 +46,7 @@ struct AllocStreamScope {
 };
 void *device_alloc(size_t bytes, cudaStream_t &used);
 void device_free(void *p, cudaStream_t used);
-void trim_pool();  // return unused stream-ordered blocks to the driver
+void trim_pool(size_t keep = 0);  // return unused stream-ordered blocks to the driver, down to keep bytes
 
 // Owning device buffer.
 template <typename T>

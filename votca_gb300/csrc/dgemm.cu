@@ -228,7 +228,13 @@ void *device_alloc(size_t bytes, cudaStream_t &used) {
     keep_pool_blocks();
     VGB_CUDA(cudaMallocAsync(&p, bytes, used));
   } else {
-    VGB_CUDA(cudaMalloc(&p, bytes));
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {  // the pool's unused blocks may be what is missing
+      cudaGetLastError();
+      trim_pool();
+      e = cudaMalloc(&p, bytes);
+    }
+    VGB_CUDA(e);
   }
   return p;
 }
@@ -248,11 +254,11 @@ void device_free(void *p, cudaStream_t used) {
   }
 }
 
-void trim_pool() {
+void trim_pool(size_t keep) {
   int dev = 0;
   cudaMemPool_t pool;
   if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
-    cudaMemPoolTrimTo(pool, 0);
+    cudaMemPoolTrimTo(pool, keep);
 }
 
 int sm_count() {
