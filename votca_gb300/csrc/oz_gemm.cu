@@ -307,7 +307,7 @@ __device__ __forceinline__ void add_level(float (&h)[EC], float (&l)[EC], uint32
 #pragma unroll
   for (int j0 = 0; j0 < EC; j0 += 8) {
     uint32_t r[8];
-    tmem_ld8(t + j0, r);
+    tmem_ld(t + j0, r);
 #pragma unroll
     for (int j = 0; j < 8; ++j) two_sum(h[j0 + j], l[j0 + j], __uint_as_float(r[j]));
   }
@@ -316,7 +316,7 @@ __device__ __forceinline__ void add_low(float (&l)[EC], uint32_t t) {
 #pragma unroll
   for (int j0 = 0; j0 < EC; j0 += 8) {
     uint32_t r[8];
-    tmem_ld8(t + j0, r);
+    tmem_ld(t + j0, r);
 #pragma unroll
     for (int j = 0; j < 8; ++j) l[j0 + j] += __uint_as_float(r[j]);
   }

@@ -13,8 +13,6 @@ namespace vgb {
 namespace {
 
 constexpr int BM = 128;
-constexpr int kEpiWarps = 8;   // two warps per TMEM lane quarter, each drains half the columns
-constexpr int kThreads = 64 + 32 * kEpiWarps;  // warp 0: TMA, warp 1: MMA + TMEM owner, rest: epilogue
 constexpr int kSmemRing = 196608;                     // bytes of operand ring per CTA
 
 // BK = bf16 elements of K per stage row: 64 -> 128-byte rows (SWIZZLE_128B),
@@ -31,6 +29,13 @@ struct Cfg {
   static constexpr int UNIT = 256 / BN < kMaxDigits ? 256 / BN : kMaxDigits;  // B planes per unit
   static constexpr int STAGE_BYTES = SLICE ? A_BYTES + UNIT * B_BYTES : 2 * A_BYTES + 2 * B_BYTES;
   static constexpr int STAGES = kSmemRing / STAGE_BYTES > 8 ? 8 : kSmemRing / STAGE_BYTES;
+  // Epilogue warps: two per TMEM lane quarter, each drains half the columns.  Slice mode: four, for
+  // the seven additions per element and digit pair bound the kernel (640 x 262144 outputs at
+  // K 256: 1.86 ms with two warps and one column per instruction, 1.51 ms).
+  static constexpr int EPI = SLICE ? 16 : 8;
+  static constexpr int THREADS = 64 + 32 * EPI;  // warp 0: TMA, warp 1: MMA + TMEM owner, rest: epilogue
+  // columns of the float-pair sums of an epilogue thread
+  static constexpr int KCOLS = SLICE ? BN / 4 : BN <= 64 ? 32 : 1;
   // accumulator buffers in TMEM: four for the narrow tiles (short K splits: the epilogue of a
   // split may lag the MMAs of the next three), two for the wide ones; slice mode: two unit
   // buffers of 256 columns
@@ -53,34 +58,49 @@ struct KParams {
   // (a, q, b) for A plane a, run q, B plane b < nsl - a (pairs up to digit level nsl - 1)
   int nsl, cpr, rpg;
   int64_t a_plane, b_plane;  // slice mode: operand rows between consecutive digit planes
-  int64_t mt, nt, ntiles;
+  int64_t mt, nt, ntiles, nitems;
   TcEpilogue epi;
   int *err;
 };
+
+// Quotient and remainder of indices, in 32 bits where they fit: a 64-bit division converts through
+// the FP64 pipe, where an instruction holds its SM quarter for 64 clocks.
+struct QuotRem {
+  int64_t q, r;
+};
+__device__ __forceinline__ QuotRem quot_rem(int64_t a, int64_t b) {
+  if (((uint64_t)(a | b) >> 32) == 0) {
+    const uint32_t x = (uint32_t)a, d = (uint32_t)b, q = x / d;
+    return {(int64_t)q, (int64_t)(x - q * d)};
+  }
+  return {a / b, a % b};
+}
 
 struct TileCoord {
   int64_t m, n, s, b;
 };
 __device__ __forceinline__ TileCoord decode(const KParams &p, int64_t t) {
   TileCoord c;
+  QuotRem x;
   if (p.kacc) {  // the K splits of a (tile, group) item are consecutive jobs of one CTA
-    const int64_t u = t % p.spg;
-    t /= p.spg;
-    const int64_t groups = p.ksplit / p.spg;
-    c.s = (t % groups) * p.spg + u;
-    t /= groups;
-    c.m = t % p.mt;
-    t /= p.mt;
-    c.n = t % p.nt;
-    c.b = t / p.nt;
+    x = quot_rem(t, p.spg);
+    const int64_t u = x.r;
+    x = quot_rem(x.q, (uint32_t)p.ksplit / (uint32_t)p.spg);
+    c.s = x.r * p.spg + u;
+    x = quot_rem(x.q, p.mt);
+    c.m = x.r;
+    x = quot_rem(x.q, p.nt);
+    c.n = x.r;
+    c.b = x.q;
     return c;
   }
-  c.m = t % p.mt;
-  t /= p.mt;
-  c.n = t % p.nt;
-  t /= p.nt;
-  c.s = t % p.ksplit;
-  c.b = t / p.ksplit;
+  x = quot_rem(t, p.mt);
+  c.m = x.r;
+  x = quot_rem(x.q, p.nt);
+  c.n = x.r;
+  x = quot_rem(x.q, p.ksplit);
+  c.s = x.r;
+  c.b = x.q;
   return c;
 }
 
@@ -101,36 +121,60 @@ __device__ __forceinline__ void epi_store(const TcEpilogue &e, int64_t off, floa
   }
 }
 
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n"
+      " mov.b64 {%0, %1}, x;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.f32x2 x, x, y;\n"
+      " mov.b64 {%0, %1}, x;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
 // The K splits' FP32 sums of a tile are added as an unevaluated pair of floats (Knuth's TwoSum,
 // error-free; about 48 significant bits) in kh[j] + kl[j]: no FP64 instruction per split (the
 // FP64 pipe of GB300 runs at 2 operations per clock and SM).  In slice mode every split sum is
 // exact, so the result is the exact sum of the splits to that precision.
-__device__ __forceinline__ void pair_add(float (&kh)[32], float (&kl)[32], const uint32_t (&r)[32], bool first) {
+template <int W>
+__device__ __forceinline__ void pair_add(float (&kh)[W], float (&kl)[W], const uint32_t (&r)[W], bool first) {
   if (first) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
+    for (int j = 0; j < W; ++j) {
       kh[j] = __uint_as_float(r[j]);
       kl[j] = 0.f;
     }
     return;
   }
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    const float x = __uint_as_float(r[j]), hi = kh[j];
-    const float sum = hi + x;
-    const float bb = sum - hi;
-    kl[j] += (hi - (sum - bb)) + (x - bb);
-    kh[j] = sum;
+  for (int j = 0; j < W; j += 2) {  // two columns per instruction
+    const float2 x = make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+    const float2 hi = make_float2(kh[j], kh[j + 1]);
+    const float2 sum = add2(hi, x);
+    const float2 bb = sub2(sum, hi);
+    const float2 lo = add2(make_float2(kl[j], kl[j + 1]), add2(sub2(hi, sub2(sum, bb)), sub2(x, bb)));
+    kh[j] = sum.x;
+    kh[j + 1] = sum.y;
+    kl[j] = lo.x;
+    kl[j + 1] = lo.y;
   }
 }
 
-// Writes a thread's 32 float-pair sums (columns n0 ..) of row base rbase through the epilogue map.
-__device__ __forceinline__ void pair_write(const float (&kh)[32], const float (&kl)[32], const TcEpilogue &e,
+// Writes a thread's float-pair sums (columns n0 ..) of row base rbase through the epilogue map.
+template <int W>
+__device__ __forceinline__ void pair_write(const float (&kh)[W], const float (&kl)[W], const TcEpilogue &e,
                                            int64_t N, int64_t n0,
                                            int64_t rbase) {
-  int64_t n = n0, nq = n / e.cd, nr = n % e.cd;
+  const QuotRem nx = quot_rem(n0, e.cd);
+  int64_t n = n0, nq = nx.q, nr = nx.r;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < W; ++j) {
     if (n < N && nr < e.clim) {
       const int64_t off = rbase + nq * e.co1 + nr * e.co2;
       const float hi = kh[j], lo = kl[j];
@@ -156,7 +200,7 @@ __device__ __forceinline__ void pair_write(const float (&kh)[32], const float (&
 // accumulation (kacc), the ksplit consecutive jobs of one output tile; items are strided over
 // the CTAs and a CTA runs the jobs of its item in order.
 __host__ __device__ __forceinline__ int64_t item_count(const KParams &p) {
-  return p.kacc ? p.ntiles / p.spg : p.ntiles;
+  return p.kacc ? p.nitems : p.ntiles;
 }
 __device__ __forceinline__ int64_t item_len(const KParams &p) { return p.kacc ? p.spg : 1; }
 
@@ -210,7 +254,7 @@ struct GroupSrc {
 static_assert(sizeof(GroupSrc) <= 32000, "grouped GEMM parameters exceed the kernel parameter space");
 
 template <int BN, int BK, class Src, bool SLICE = false>
-__global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_constant__ Src src) {
+__global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel(const __grid_constant__ Src src) {
   using C = Cfg<BN, BK, SLICE>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -229,7 +273,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     }
     for (int i = 0; i < C::NBUF; ++i) {
       mbar_init(&accf[i], 1);
-      mbar_init(&acce[i], kEpiWarps);  // one arrive per epilogue warp
+      mbar_init(&acce[i], C::EPI);  // one arrive per epilogue warp
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -268,7 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
           // the item's split group g: runs [q0, q0 + rpg); units (a, run, b0) in order, each K
           // block of a unit one stage with A plane a and B planes b0 .. b0 + nb - 1
           const int kchunks = (int)(p.K / BK);
-          const int q0 = (int)(tc.s / p.spg) * p.rpg;
+          const int q0 = ((int)tc.s / p.spg) * p.rpg;
           for (int a = 0; a < p.nsl; ++a)
             for (int qr = q0; qr < q0 + p.rpg; ++qr)
               for (int b0 = 0; b0 < p.nsl - a; b0 += C::UNIT) {
@@ -330,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
           // units (a, run, b0) in the producer's order: one accumulator buffer per unit, nb
           // adjacent accumulators of BN columns filled by one MMA of width nb * BN per K step
           const int kchunks = (int)(p.K / BK);
-          const int q0 = (int)(tc.s / p.spg) * p.rpg;
+          const int q0 = ((int)tc.s / p.spg) * p.rpg;
           for (int a = 0; a < p.nsl; ++a)
             for (int qr = q0; qr < q0 + p.rpg; ++qr)
               for (int b0 = 0; b0 < p.nsl - a; b0 += C::UNIT) {
@@ -395,16 +439,14 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     }
   } else {
     // ---------------- epilogue warps ----------------
-    // A warp may only read the TMEM lane quarter 32 * (warp % 4); the two warps
-    // of each quarter split the tile's columns.
+    // A warp may only read the TMEM lane quarter 32 * (warp % 4); the warps of each quarter split
+    // the tile's columns.
     const int q = warp % 4;
-    const int half = (warp - 2) / 4;
-    constexpr int COLS = BN >= 64 ? BN / 2 : BN;
-    const int cbeg = (BN >= 64 || half == 0) ? half * COLS : BN;
-    const int cend = (BN >= 64 || half == 0) ? cbeg + COLS : BN;
-    // float-pair sums over the K splits of a tile (kacc; BN <= 64: at most 32 columns per thread)
-    constexpr int KACC = BN <= 64 ? 32 : 1;
-    float kh[KACC], kl[KACC];
+    const int part = (warp - 2) / 4;
+    constexpr int COLS = SLICE ? BN / 4 : BN >= 64 ? BN / 2 : BN;
+    const int cbeg = min(part * COLS, BN);
+    const int cend = min(cbeg + COLS, BN);
+    float kh[C::KCOLS], kl[C::KCOLS];  // float-pair sums over the K splits of a tile (kacc, slices)
     int buf = 0;
     uint32_t aphase = 0;
     int hint = 0;
@@ -417,13 +459,14 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       // the jobs of an item share the tile and the split group: row terms once per item
       TileCoord tc = decode(p, li * len);
       const int64_t i = tc.m * BM + q * 32 + lane;
-      const bool row_ok = i < p.M && (i % e.rd) < e.rlim;
+      const QuotRem ix = quot_rem(i, e.rd);
+      const bool row_ok = i < p.M && ix.r < e.rlim;
       // partial offset: the K split (F32 partials) or the split group (kacc groups)
-      const int64_t rbase = (i / e.rd) * e.ro1 + (i % e.rd) * e.ro2 + tc.b * e.bo +
-                            (p.kacc ? (tc.s / p.spg) * e.so : tc.s * e.so);
+      const int64_t rbase = ix.q * e.ro1 + ix.r * e.ro2 + tc.b * e.bo +
+                            (p.kacc ? ((int)tc.s / p.spg) * e.so : tc.s * e.so);
       if constexpr (SLICE) {
         // the units of the item in the MMA's order; each buffer holds nb adjacent accumulators
-        const int q0 = (int)(tc.s / p.spg) * p.rpg;
+        const int q0 = ((int)tc.s / p.spg) * p.rpg;
         bool first = true;
         for (int a = 0; a < p.nsl; ++a)
           for (int qr = q0; qr < q0 + p.rpg; ++qr)
@@ -431,31 +474,29 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
               const int nb = min(C::UNIT, p.nsl - a - b0);
               if (!mbar_wait(&accf[buf], aphase, abort_flag, err, 4)) goto epi_done;
               fence_after();
-              if (cbeg < cend) {
-                for (int j = 0; j < nb; ++j) {
-                  uint32_t r[32];
-                  tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + j * BN + cbeg), r);
-                  pair_add(kh, kl, r, first);
-                  first = false;
-                }
+              for (int j = 0; j < nb; ++j) {
+                uint32_t r[C::KCOLS];
+                tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + j * BN + cbeg), r);
+                pair_add(kh, kl, r, first);
+                first = false;
               }
               fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive(&acce[buf]);
               if (++buf == C::NBUF) { buf = 0; aphase ^= 1; }
             }
-        if (row_ok && cbeg < cend) pair_write(kh, kl, e, p.N, tc.n * BN + cbeg, rbase);
+        if (row_ok) pair_write(kh, kl, e, p.N, tc.n * BN + cbeg, rbase);
         continue;
       }
       for (int64_t u = 0; u < len; ++u, ++tc.s) {
       if (!mbar_wait(&accf[buf], aphase, abort_flag, err, 4)) goto epi_done;
       fence_after();
-      if constexpr (BN <= 64) {
+      if constexpr (BN <= 64 && !SLICE) {
         if (p.kacc) {
           // this thread's 32 columns (cbeg == cend for the idle half of a BN = 32 tile)
           if (cbeg < cend) {
             uint32_t r[32];
-            tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + cbeg), r);
+            tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + cbeg), r);
             const int64_t sg = u;  // position inside the split group (an item is one group)
             pair_add(kh, kl, r, sg == 0);
             if (row_ok && sg == p.spg - 1) pair_write(kh, kl, e, p.N, tc.n * BN + cbeg, rbase);  // split order
@@ -470,10 +511,11 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
 #pragma unroll 1
       for (int c0 = cbeg; c0 < cend; c0 += 32) {
         uint32_t r[32];
-        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + c0), r);
+        tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + c0), r);
         if (!row_ok) continue;
         const int64_t n0 = tc.n * BN + c0;
-        const int64_t nq0 = n0 / e.cd, nr0 = n0 % e.cd;
+        const QuotRem nx = quot_rem(n0, e.cd);
+        const int64_t nq0 = nx.q, nr0 = nx.r;
         if (nr0 + 32 <= e.cd && n0 + 32 <= p.N && nr0 + 32 <= e.clim) {
           // fast path: the 32 columns are one arithmetic run of offsets
           const int64_t base = rbase + nq0 * e.co1 + nr0 * e.co2;
@@ -537,8 +579,10 @@ __device__ __forceinline__ void split_range(const double *__restrict__ x, int64_
                                             int64_t step) {
   const int64_t total = rows * cols;
   for (int64_t t = t0; t < total; t += step) {
-    const int64_t r = t / cols, c = t % cols;
-    const int64_t rq = r / m.rdiv, rr = r % m.rdiv;
+    const QuotRem tx = quot_rem(t, cols);
+    const int64_t r = tx.q, c = tx.r;
+    const QuotRem rx = quot_rem(r, m.rdiv);
+    const int64_t rq = rx.q, rr = rx.r;
     if (rr >= m.rlim) continue;
     const double v = x[rq * m.rs1 + rr * m.rs2 + c * m.cs];
     const __nv_bfloat16 h = __double2bfloat16(v);
@@ -576,8 +620,9 @@ __device__ __forceinline__ void reduce_range(const float *__restrict__ part, int
                                              int ksplit, const TcEpilogue &e, int64_t t0, int64_t step) {
   const int64_t total = M * N;
   for (int64_t t = t0; t < total; t += step) {
-    const int64_t i = t / N, n = t % N;
-    if ((i % e.rd) >= e.rlim || (n % e.cd) >= e.clim) continue;
+    const QuotRem tx = quot_rem(t, N);
+    const QuotRem ix = quot_rem(tx.q, e.rd), nx = quot_rem(tx.r, e.cd);
+    if (ix.r >= e.rlim || nx.r >= e.clim) continue;
     double acc = 0.0;
     // the same summation order as a plain loop; the unroll lets the independent loads of
     // eight partials be in flight together (the loop is latency-bound otherwise)
@@ -585,7 +630,7 @@ __device__ __forceinline__ void reduce_range(const float *__restrict__ part, int
     for (int s = 0; s < ksplit; ++s) acc += (double)part[s * total + t];
     // the partial sums are added in FP64; the final value enters the epilogue
     // as FP64 for AXPBY (no extra rounding) and as FP32 for the bf16 split
-    const int64_t off = (i / e.rd) * e.ro1 + (i % e.rd) * e.ro2 + (n / e.cd) * e.co1 + (n % e.cd) * e.co2;
+    const int64_t off = ix.q * e.ro1 + ix.r * e.ro2 + nx.q * e.co1 + nx.r * e.co2;
     if (e.kind == TcEpilogue::AXPBY_F64) {
       double *y = e.out_f64 + off;
       const double r = e.alpha * acc;
@@ -618,17 +663,16 @@ __device__ __forceinline__ long long fixed_point(unsigned long long bits, int e,
   return (bits >> 63) ? -m : m;
 }
 
-// The same fixed point for a float given by its bits.
+// The same fixed point for a float given by its bits: value = mant 2^(ef - 150), m = mant
+// 2^(ef - 150 + B - e).  The mantissa is shifted to 2 m with one guard bit (right by at least
+// 26 - B + 12 >= 1 for B <= 35; amounts beyond 63 give 0), then rounded half up.
 __device__ __forceinline__ long long fixed_point_f32(unsigned bits, int e, int B) {
   const int ef = (int)((bits >> 23) & 0xFF);
-  if (ef == 0) return 0;
-  const long long mant = (long long)((bits & 0x7FFFFFu) | 0x800000u);
-  // value = mant 2^(ef - 150), m = mant 2^(ef - 150 + B - e)
-  const int sh = 150 + e - ef - B;
-  long long m;
-  if (sh <= 0) m = mant << (-sh);  // |value| < 2^(e + 1): at most 2^(B + 1)
-  else m = sh < 40 ? (mant + (1LL << (sh - 1))) >> sh : 0;
-  return (bits >> 31) ? -m : m;
+  const unsigned mant = ef ? (bits & 0x7FFFFFu) | 0x800000u : 0u;
+  unsigned long long t;
+  asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"((unsigned long long)mant << 13), "r"((unsigned)(162 + e - ef - B)));
+  const long long m = (long long)((t + 1) >> 1);
+  return (int)bits < 0 ? -m : m;
 }
 
 // Input element access of the slicer: FP64 values, or float pairs (hi, lo) with value hi + lo.
@@ -717,8 +761,8 @@ __global__ void slice_kernel(const In in, int64_t rows, int64_t cols, const Spli
   const int64_t units = rows * nchunks;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps) {
-    const int64_t r = u / nchunks, q = u % nchunks;
-    const int64_t rq = r / m.rdiv, rr = r % m.rdiv;
+    const QuotRem ux = quot_rem(u, nchunks), rx = quot_rem(ux.q, m.rdiv);
+    const int64_t r = ux.q, q = ux.r, rq = rx.q, rr = rx.r;
     if (rr >= m.rlim) continue;  // uniform over the warp
     const int64_t base = rq * m.rs1 + rr * m.rs2;
     const int64_t c0 = q * chunk, c1 = min(cols, c0 + chunk);
@@ -802,7 +846,10 @@ __global__ void slice_kernel(const In in, int64_t rows, int64_t cols, const Spli
 // holds its (up to) 8 groups of 4 consecutive elements of the run in registers, so every load
 // of the run is in flight at once and the input is read from memory once (the two-pass kernel
 // above re-reads the run for its digits and keeps one load per lane in flight).  The digits and
-// their bf16 bits are those of slice_kernel, element for element.
+// their bf16 bits are those of slice_kernel, element for element: digit t is round(m / 2^s_t) less
+// 2^7 round(m / 2^s_(t-1)), in 32 bits from m >> 6, and becomes a float by one addition and one
+// multiplication (64-bit digits and integer conversions: 868 us for the 5120 x 32768 float
+// pairs of a 3.0 GB pass, 668 us).
 constexpr int kRunGroups = 8;  // 8 groups x 4 elements x 32 lanes = 1024 columns per run
 template <class In, int NSL>
 __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t rows, int64_t cols, const SplitMap m,
@@ -813,8 +860,8 @@ __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t row
   const int64_t units = rows * nchunks;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps) {
-    const int64_t r = u / nchunks, q = u % nchunks;
-    const int64_t rq = r / m.rdiv, rr = r % m.rdiv;
+    const QuotRem ux = quot_rem(u, nchunks), rx = quot_rem(ux.q, m.rdiv);
+    const int64_t r = ux.q, q = ux.r, rq = rx.q, rr = rx.r;
     if (rr >= m.rlim) continue;  // uniform over the warp
     const int64_t base = rq * m.rs1 + rr * m.rs2;
     const int64_t c0 = q * chunk, c1 = min(cols, c0 + chunk);
@@ -844,40 +891,51 @@ __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t row
       mx = y > mx ? y : mx;
     }
     const int e = In::exponent(mx);
+    float sc[NSL];  // digit scales; those below the FP32 normal range flush to 0, as digit_bits
+#pragma unroll
+    for (int sl = 0; sl < NSL; ++sl) {
+      const int pe = e - 7 * (sl + 1) + 127;
+      sc[sl] = pe >= 1 && pe <= 254 ? __int_as_float(pe << 23) : 0.f;
+    }
     uint16_t *orow = out + r * ldo;
 #pragma unroll
     for (int g = 0; g < kRunGroups; ++g) {
       const int64_t c = c0 + 128 * g + 4 * lane;
       if (c >= c1) continue;
-      unsigned long long packed[NSL];
+      uint32_t packed[NSL][2];
 #pragma unroll
-      for (int sl = 0; sl < NSL; ++sl) packed[sl] = 0;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
+      for (int v = 0; v < 4; v += 2) {
         // zero-filled words past the run's end slice to zero digits and are not stored
-        long long rem = mx != 0 ? In::fixed_word(w[g][v], e, 7 * NSL) : 0;
+        float f[2][NSL];
 #pragma unroll
-        for (int sl = 0; sl < NSL; ++sl) {
-          const int shift = 7 * (NSL - 1 - sl);
-          long long d = rem;
-          if (shift > 0) {
-            d = (rem + (1LL << (shift - 1))) >> shift;  // round half up, as digits()
-            rem -= d << shift;
+        for (int h = 0; h < 2; ++h) {
+          const long long m = In::fixed_word(w[g][v + h], e, 7 * NSL);
+          const int u = (int)(m >> 6);
+          int above = 0;  // m rounded (half up) to the digits before this one
+#pragma unroll
+          for (int sl = 0; sl < NSL; ++sl) {
+            const int shift = 7 * (NSL - 1 - sl);
+            const int cur = shift > 0 ? (u + (1 << (shift - 7 & 31))) >> (shift - 6 & 31) : (int)m;
+            // the digit (|d| <= 128) as a float: 1.5 2^23 + d, less 1.5 2^23
+            f[h][sl] = (__int_as_float(0x4B400000 + cur - (above << 7)) - 12582912.f) * sc[sl];
+            above = cur;
           }
-          packed[sl] |= (unsigned long long)digit_bits(d, e, sl + 1) << (16 * v);
         }
+#pragma unroll
+        for (int sl = 0; sl < NSL; ++sl)
+          asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed[sl][v / 2]) : "f"(f[1][sl]), "f"(f[0][sl]));
       }
       if (c + 4 <= c1) {
 #pragma unroll
         for (int sl = 0; sl < NSL; ++sl)
-          *reinterpret_cast<unsigned long long *>(orow + sl * plane + c) = packed[sl];
+          *reinterpret_cast<uint2 *>(orow + sl * plane + c) = make_uint2(packed[sl][0], packed[sl][1]);
       } else {
         const int nv = (int)(c1 - c);
 #pragma unroll
         for (int sl = 0; sl < NSL; ++sl)
 #pragma unroll
           for (int v = 0; v < 3; ++v)
-            if (v < nv) orow[sl * plane + c + v] = (uint16_t)(packed[sl] >> (16 * v));
+            if (v < nv) orow[sl * plane + c + v] = (uint16_t)(packed[sl][v / 2] >> (16 * (v & 1)));
       }
     }
   }
@@ -887,11 +945,12 @@ __global__ void reduce_f64_kernel(const double *__restrict__ part, int64_t M, in
                                   const TcEpilogue e) {
   const int64_t total = M * N;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % M, n = t / M;
-    if ((i % e.rd) >= e.rlim || (n % e.cd) >= e.clim) continue;
+    const QuotRem tx = quot_rem(t, M);
+    const QuotRem ix = quot_rem(tx.r, e.rd), nx = quot_rem(tx.q, e.cd);
+    if (ix.r >= e.rlim || nx.r >= e.clim) continue;
     double acc = 0.0;
     for (int g = 0; g < G; ++g) acc += part[g * total + t];
-    double *y = e.out_f64 + (i / e.rd) * e.ro1 + (i % e.rd) * e.ro2 + (n / e.cd) * e.co1 + (n % e.cd) * e.co2;
+    double *y = e.out_f64 + ix.q * e.ro1 + ix.r * e.ro2 + nx.q * e.co1 + nx.r * e.co2;
     const double r = e.alpha * acc;
     *y = (e.beta == 0.0) ? r : fma(e.beta, *y, r);
   }
@@ -912,7 +971,7 @@ void launch_src(const Src &src, int64_t ntiles, cudaStream_t s) {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   });
   const int64_t grid = std::min<int64_t>(ntiles, sm_count());
-  tc_gemm_kernel<BN, BK, Src, SLICE><<<(unsigned)grid, kThreads, C::SMEM, s>>>(src);
+  tc_gemm_kernel<BN, BK, Src, SLICE><<<(unsigned)grid, C::THREADS, C::SMEM, s>>>(src);
   VGB_LAUNCH_CHECK();
 }
 
@@ -1028,6 +1087,7 @@ KParams make_params(const TcMat &A, const TcMat &B, const TcShape &sh, const TcE
   p.mt = ceil_div(sh.M, BM);
   p.nt = ceil_div(sh.N, bn);
   p.ntiles = p.mt * p.nt * p.ksplit * sh.nbatch;
+  p.nitems = p.ntiles / p.spg;
   p.epi = epi;
   p.err = err;
   return p;
