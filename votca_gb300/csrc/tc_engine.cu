@@ -25,6 +25,7 @@
 #include <tuple>
 #include <mutex>
 
+#include "slice_gemm.cuh"
 #include "tc_gemm.cuh"
 
 #include <cuda_bf16.h>
@@ -393,51 +394,6 @@ void MixedEngine::apply(BseOperator &op, const Coef &c, const double *X, int64_t
   }
 }
 
-namespace {
-
-// All pairs (a, b) of digit planes with a + b < nsl: the products kept by the Ozaki scheme (the
-// dropped levels are below 2^(-7 nsl) of the row and column scales).
-void set_pairs(TcShape &sh, int nsl) { sh.nslices = nsl; }
-
-// One slice-mode product: C (M x N) = sum over pairs of A planes (rows a_plane apart, K-major,
-// row stride K) times B planes, through the final FP64 epilogue fe.  When the tiles alone do
-// not fill the SMs, the K splits of a tile are shared by several CTAs whose FP64 partials are
-// added by a reduction launch.
-// chain: the run of one digit scale along K in both operands (a multiple of 64 dividing K).
-void sliced_gemm(const TcMat &A, int64_t a_plane, const TcMat &B, int64_t b_plane, int64_t M, int64_t N,
-                 int64_t K, int64_t chain, int nsl, int bn, const TcEpilogue &fe, DeviceBuffer<double> &gpart,
-                 int *err, cudaStream_t s) {
-  TcShape sh;
-  sh.M = M; sh.N = N; sh.K = K;
-  set_pairs(sh, nsl);
-  sh.a_plane = a_plane;
-  sh.b_plane = b_plane;
-  sh.chain = chain;
-  sh.kacc = true;
-  const int64_t tiles = ceil_div(M, 128) * ceil_div(N, bn);
-  const int64_t runs = ceil_div(K / 64, sh.chain / 64);
-  int groups = 1;  // float-pair outputs are written by the CTA that owns the tile
-  for (int g = 2; g <= 64 && fe.kind == TcEpilogue::AXPBY_F64; ++g)
-    if (runs % g == 0 && tiles * g <= sm_count()) groups = g;
-  if (groups == 1) {
-    tc_gemm(A, B, sh, fe, bn, err, s);
-    return;
-  }
-  sh.kgroups = groups;
-  gpart.resize((size_t)groups * M * N);
-  TcEpilogue pe;  // FP64 partials, column-major per group
-  pe.kind = TcEpilogue::AXPBY_F64;
-  pe.rd = M; pe.ro2 = 1; pe.rlim = M;
-  pe.cd = N; pe.co2 = M; pe.clim = N;
-  pe.so = M * N;
-  pe.out_f64 = gpart.get();
-  pe.alpha = 1.0; pe.beta = 0.0;
-  tc_gemm(A, B, sh, pe, bn, err, s);
-  reduce_f64_groups(gpart.get(), M, N, groups, fe, s);
-}
-
-}  // namespace
-
 void MixedEngine::apply_sliced(BseOperator &op, const Coef &c, const double *X, int64_t ldx, int64_t k,
                                double *Y, int64_t ldy, bool accumulate, cudaStream_t s) {
   Impl &m = *impl_;
@@ -491,38 +447,35 @@ void MixedEngine::apply_sliced(BseOperator &op, const Coef &c, const double *X, 
   }
   op.timer.end(STAGE_TC_SPLIT, s);
   const uint16_t *px = m.pX.get();
-  const int64_t xrows = nsl * k * vt;  // rows of the X planes as one matrix ([(j, v)] view)
 
   if (hx) {
     op.timer.begin(STAGE_TC_HX, s);
-    const TcMat &Ab = m.mat(m.pBvc2.get(), m.pBvc2.get(), nsl * naux, m.dimP, 128, 64);
+    const SliceMat Ab{m.pBvc2.get(), m.dimP, naux, 0};
     m.fZ.resize(k * m.Kn);
     for (int64_t j0 = 0; j0 < k; j0 += 64) {  // Z[j][P] = sum_I' Bvc[P][I'] X_j[I']
       const int64_t kc = std::min<int64_t>(64, k - j0);
-      const int bn = kc > 32 ? 64 : 32;
-      TcMat Bx = make_tc_mat(px + j0 * m.dimP, px + j0 * m.dimP, nsl * k - j0, m.dimP, m.dimP, bn, 64);
+      const SliceMat Bx{px + j0 * m.dimP, m.dimP, k, j0};
       TcEpilogue e;
       e.kind = TcEpilogue::AXPBY_F64;
       e.rd = naux; e.ro2 = 1; e.rlim = naux;
       e.cd = kc; e.co2 = m.Kn; e.clim = kc;
       e.out_f64 = m.fZ.get() + j0 * m.Kn; e.alpha = 1.0; e.beta = 0.0;
-      sliced_gemm(Ab, naux, Bx, k, naux, kc, m.dimP, chc, nsl, bn, e, m.gpart, err, s);
+      slice_gemm(Ab, Bx, naux, kc, m.dimP, chc, nsl, e, m.gpart, err, s);
     }
     m.pZ.ensure(k, m.Kn, nsl, s);
     SplitMap z;
     z.rdiv = 1; z.rs1 = m.Kn; z.rs2 = 0; z.cs = 1; z.rlim = 1;
     slice_f64(m.fZ.get(), k, naux, z, nsl, chn, m.pZ.get(), m.Kn, m.pZ.plane(), s);
-    const TcMat &At = m.mat(m.pBvcT.get(), m.pBvcT.get(), nsl * m.dimP, m.Kn, 128, 64);
+    const SliceMat At{m.pBvcT.get(), m.Kn, m.dimP, 0};
     for (int64_t j0 = 0; j0 < k; j0 += 64) {  // Y(I, j) (+)= cx sum_P BvcT[I'][P] Z[j][P]
       const int64_t kc = std::min<int64_t>(64, k - j0);
-      const int bn = kc > 32 ? 64 : 32;
-      TcMat Bz = make_tc_mat(m.pZ.get() + j0 * m.Kn, m.pZ.get() + j0 * m.Kn, nsl * k - j0, m.Kn, m.Kn, bn, 64);
+      const SliceMat Bz{m.pZ.get() + j0 * m.Kn, m.Kn, k, j0};
       TcEpilogue e;
       e.kind = TcEpilogue::AXPBY_F64;
       e.rd = m.Kc; e.ro1 = ct; e.ro2 = 1; e.rlim = ct;
       e.cd = kc; e.co2 = ldy; e.clim = kc;
       e.out_f64 = Y + j0 * ldy; e.alpha = c.cx; e.beta = acc ? 1.0 : 0.0;
-      sliced_gemm(At, m.dimP, Bz, k, m.dimP, kc, m.Kn, chn, nsl, bn, e, m.gpart, err, s);
+      slice_gemm(At, Bz, m.dimP, kc, m.Kn, chn, nsl, e, m.gpart, err, s);
     }
     acc = true;
     op.timer.end(STAGE_TC_HX, s);
@@ -542,7 +495,7 @@ void MixedEngine::apply_sliced(BseOperator &op, const Coef &c, const double *X, 
     for (int64_t j0 = 0; j0 < k; j0 += jc) {
       const int64_t kc = std::min(jc, k - j0);
       op.timer.begin(is_hd ? STAGE_TC_HD : STAGE_TC_HD2, s);
-      TcMat Ax = make_tc_mat(px + j0 * vt * m.Kc, px + j0 * vt * m.Kc, xrows - j0 * vt, m.Kc, m.Kc, 128, 64);
+      const SliceMat Ax{px + j0 * vt * m.Kc, m.Kc, k * vt, j0 * vt};
       TcEpilogue e;  // stage 1 into the intermediate [(j, row)][(P, v)], FP64 sums as float pairs
       e.kind = TcEpilogue::PAIR_F32;
       e.rd = vt; e.ro2 = 1; e.rlim = vt;
@@ -550,11 +503,11 @@ void MixedEngine::apply_sliced(BseOperator &op, const Coef &c, const double *X, 
       e.cd = is_hd ? ct : vt; e.co1 = vt; e.co2 = m.Kg; e.clim = e.cd;
       e.out_f32 = reinterpret_cast<float *>(m.fT.get());
       if (is_hd) {  // S[(j, c1)][(P, v)] = sum_c X_j(v, c) M(c1, c, P)
-        const TcMat &Bm = m.mat(m.pMcc.get(), m.pMcc.get(), nsl * naux * ct, m.Kc, 64, 64);
-        sliced_gemm(Ax, k * vt, Bm, naux * ct, kc * vt, naux * ct, m.Kc, chc, nsl, 64, e, m.gpart, err, s);
+        const SliceMat Bm{m.pMcc.get(), m.Kc, naux * ct, 0};
+        slice_gemm(Ax, Bm, kc * vt, naux * ct, m.Kc, chc, nsl, e, m.gpart, err, s);
       } else {      // U[(j, v1)][(P, v)] = sum_c X_j(v, c) M(v1, c, P)
-        const TcMat &Bm = m.mat(m.pBvc2.get(), m.pBvc2.get(), nsl * naux * vt, m.Kc, 64, 64);
-        sliced_gemm(Ax, k * vt, Bm, naux * vt, kc * vt, naux * vt, m.Kc, chc, nsl, 64, e, m.gpart, err, s);
+        const SliceMat Bm{m.pBvc2.get(), m.Kc, naux * vt, 0};
+        slice_gemm(Ax, Bm, kc * vt, naux * vt, m.Kc, chc, nsl, e, m.gpart, err, s);
       }
       op.timer.end(is_hd ? STAGE_TC_HD : STAGE_TC_HD2, s);
       op.timer.begin(STAGE_TC_SPLIT, s);
@@ -565,37 +518,33 @@ void MixedEngine::apply_sliced(BseOperator &op, const Coef &c, const double *X, 
       op.timer.end(STAGE_TC_SPLIT, s);
       op.timer.begin(is_hd ? STAGE_TC_HD_B : STAGE_TC_HD2_B, s);
       if (is_hd) {  // Y_j(c1, v1) += alpha sum_{(P,v)} S[(j, c1)][(P,v)] G[v1][(P,v)]
-        TcMat As = make_tc_mat(m.pT.get(), m.pT.get(), nsl * tplane, m.Kg, m.Kg, 128, 64);
+        const SliceMat As{m.pT.get(), m.Kg, tplane, 0};
         for (int64_t n0 = 0; n0 < vt; n0 += 64) {
           const int64_t nn = std::min<int64_t>(64, vt - n0);
-          const int bn = nn > 32 ? 64 : 32;
-          TcMat Bg = make_tc_mat(m.pG2.get() + n0 * m.Kg, m.pG2.get() + n0 * m.Kg, nsl * vt - n0, m.Kg, m.Kg,
-                                 bn, 64);
+          const SliceMat Bg{m.pG2.get() + n0 * m.Kg, m.Kg, vt, n0};
           TcEpilogue r;
           r.kind = TcEpilogue::AXPBY_F64;
           r.rd = ct; r.ro1 = ldy; r.ro2 = 1; r.rlim = ct;
           r.cd = nn; r.co2 = ct; r.clim = nn;
           r.out_f64 = Y + j0 * ldy + n0 * ct; r.alpha = alpha; r.beta = acc ? 1.0 : 0.0;
-          sliced_gemm(As, tplane, Bg, vt, kc * ct, nn, m.Kg, chg, nsl, bn, r, m.gpart, err, s);
+          slice_gemm(As, Bg, kc * ct, nn, m.Kg, chg, nsl, r, m.gpart, err, s);
         }
       } else {      // Y_j(c1, v1) += alpha sum_{(P,v)} McvT[c1][(P,v)] U[(j, v1)][(P,v)]
-        const TcMat &Am = m.mat(m.pMcvT.get(), m.pMcvT.get(), nsl * ct, m.Kg, 128, 64);
+        const SliceMat Am{m.pMcvT.get(), m.Kg, ct, 0};
         // column blocks of whole vectors (vt <= 64) or of 64 v1 of one vector
         const int64_t nv = vt <= 64 ? std::max<int64_t>(1, 64 / vt) : 1;
         for (int64_t j = 0; j < kc; j += nv) {
           const int64_t vj = std::min(nv, kc - j);
           for (int64_t v0 = 0; v0 < vt; v0 += 64) {
             const int64_t nn = vt <= 64 ? vj * vt : std::min<int64_t>(64, vt - v0);
-            const int bn = nn > 32 ? 64 : 32;
             const int64_t r0 = j * vt + v0;  // first intermediate row of the block
-            TcMat Bu = make_tc_mat(m.pT.get() + r0 * m.Kg, m.pT.get() + r0 * m.Kg, nsl * tplane - r0, m.Kg, m.Kg,
-                                   bn, 64);
+            const SliceMat Bu{m.pT.get() + r0 * m.Kg, m.Kg, tplane, r0};
             TcEpilogue r;
             r.kind = TcEpilogue::AXPBY_F64;
             r.rd = ct; r.ro2 = 1; r.rlim = ct;
             r.cd = vt <= 64 ? vt : nn; r.co1 = ldy; r.co2 = ct; r.clim = r.cd;
             r.out_f64 = Y + (j0 + j) * ldy + v0 * ct; r.alpha = alpha; r.beta = acc ? 1.0 : 0.0;
-            sliced_gemm(Am, ct, Bu, tplane, ct, nn, m.Kg, chg, nsl, bn, r, m.gpart, err, s);
+            slice_gemm(Am, Bu, ct, nn, m.Kg, chg, nsl, r, m.gpart, err, s);
             if (vt <= 64) break;
           }
         }
@@ -635,10 +584,8 @@ void MixedEngine::gemm_sliced(BseOperator &op, const double *A, const SplitMap &
   }
   m.pA.ensure(M, Kp, nsl, s);
   slice_f64(A, M, K, am, nsl, chain, m.pA.get(), Kp, m.pA.plane(), s);
-  const int bn = N > 32 ? 64 : 32;
-  TcMat Am = make_tc_mat(m.pA.get(), m.pA.get(), nsl * M, Kp, Kp, 128, 64);
-  TcMat Bm = make_tc_mat(bp, bp, nsl * bplane, Kp, Kp, bn, 64);
-  sliced_gemm(Am, M, Bm, bplane, M, N, Kp, chain, nsl, bn, e, m.gpart, m.err.get(), s);
+  slice_gemm(SliceMat{m.pA.get(), Kp, M, 0}, SliceMat{bp, Kp, bplane, 0}, M, N, Kp, chain, nsl, e, m.gpart,
+             m.err.get(), s);
 }
 
 namespace {

@@ -1,5 +1,7 @@
 // tcgen05 BF16x3 GEMM (see tc_gemm.cuh).
 #include "tc_gemm.cuh"
+
+#include "tc_epilogue.cuh"
 #include "tc_ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -13,35 +15,22 @@ namespace vgb {
 namespace {
 
 constexpr int BM = 128;
+constexpr int kEpiWarps = 8;   // two warps per TMEM lane quarter, each drains half the columns
+constexpr int kThreads = 64 + 32 * kEpiWarps;  // warp 0: TMA, warp 1: MMA + TMEM owner, rest: epilogue
 constexpr int kSmemRing = 196608;                     // bytes of operand ring per CTA
 
 // BK = bf16 elements of K per stage row: 64 -> 128-byte rows (SWIZZLE_128B),
 // 32 -> 64-byte rows (SWIZZLE_64B, half the stage size, twice the stages).
-// SLICE: the slice-mode kernel (Ozaki digit planes).  A unit is one A plane a and up to UNIT
-// B planes b0 .. b0 + nb - 1 (pairs of one digit level or less): a stage holds the unit's planes
-// of one K block, and one MMA of width nb * BN multiplies the A plane by the stacked B planes
-// into nb adjacent accumulators (A is read once per K step for nb pairs).
-constexpr int kMaxDigits = 5;
-template <int BN, int BK, bool SLICE = false>
+template <int BN, int BK>
 struct Cfg {
   static constexpr int A_BYTES = BM * BK * 2;            // one of hi / lo (one plane)
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int UNIT = 256 / BN < kMaxDigits ? 256 / BN : kMaxDigits;  // B planes per unit
-  static constexpr int STAGE_BYTES = SLICE ? A_BYTES + UNIT * B_BYTES : 2 * A_BYTES + 2 * B_BYTES;
+  static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
   static constexpr int STAGES = kSmemRing / STAGE_BYTES > 8 ? 8 : kSmemRing / STAGE_BYTES;
-  // Epilogue warps: two per TMEM lane quarter, each drains half the columns.  Slice mode: four, for
-  // the seven additions per element and digit pair bound the kernel (640 x 262144 outputs at
-  // K 256: 1.86 ms with two warps and one column per instruction, 1.51 ms).
-  static constexpr int EPI = SLICE ? 16 : 8;
-  static constexpr int THREADS = 64 + 32 * EPI;  // warp 0: TMA, warp 1: MMA + TMEM owner, rest: epilogue
-  // columns of the float-pair sums of an epilogue thread
-  static constexpr int KCOLS = SLICE ? BN / 4 : BN <= 64 ? 32 : 1;
   // accumulator buffers in TMEM: four for the narrow tiles (short K splits: the epilogue of a
-  // split may lag the MMAs of the next three), two for the wide ones; slice mode: two unit
-  // buffers of 256 columns
-  static constexpr int NBUF = SLICE ? 2 : (BN <= 64 ? 4 : 2);
-  static constexpr int BUFW = SLICE ? 256 : BN;  // TMEM columns per buffer
-  static constexpr int TMEM_COLS = NBUF * BUFW < 32 ? 32 : NBUF * BUFW;
+  // split may lag the MMAs of the next three), two for the wide ones
+  static constexpr int NBUF = BN <= 64 ? 4 : 2;
+  static constexpr int TMEM_COLS = NBUF * BN < 32 ? 32 : NBUF * BN;
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr uint32_t SBO = BK == 64 ? 1024 : 512;     // 8 rows of one swizzle atom
   static constexpr uint64_t LAYOUT = BK == 64 ? 2 : 4;       // SWIZZLE_128B / SWIZZLE_64B
@@ -49,32 +38,14 @@ struct Cfg {
 
 struct KParams {
   int64_t M, N, K;
-  int products;  // 3: hi.hi + hi.lo + lo.hi;  4: + lo.lo;  1: slice mode (hi maps only)
+  int products;  // 3: hi.hi + hi.lo + lo.hi;  4: + lo.lo
   int64_t nbatch, a_brows, b_brows;
   int ksplit, kc_per;
-  int kacc;  // 1: one CTA runs K splits of a tile and sums them in FP64 registers
-  int spg;   // kacc: consecutive splits per work item (ksplit / spg groups per tile)
-  // slice mode: digit planes per operand, K runs, runs per split group; the splits of a group are
-  // (a, q, b) for A plane a, run q, B plane b < nsl - a (pairs up to digit level nsl - 1)
-  int nsl, cpr, rpg;
-  int64_t a_plane, b_plane;  // slice mode: operand rows between consecutive digit planes
+  int kacc;  // 1: one CTA runs the K splits of a tile and sums them as float pairs
   int64_t mt, nt, ntiles, nitems;
   TcEpilogue epi;
   int *err;
 };
-
-// Quotient and remainder of indices, in 32 bits where they fit: a 64-bit division converts through
-// the FP64 pipe, where an instruction holds its SM quarter for 64 clocks.
-struct QuotRem {
-  int64_t q, r;
-};
-__device__ __forceinline__ QuotRem quot_rem(int64_t a, int64_t b) {
-  if (((uint64_t)(a | b) >> 32) == 0) {
-    const uint32_t x = (uint32_t)a, d = (uint32_t)b, q = x / d;
-    return {(int64_t)q, (int64_t)(x - q * d)};
-  }
-  return {a / b, a % b};
-}
 
 struct TileCoord {
   int64_t m, n, s, b;
@@ -82,11 +53,9 @@ struct TileCoord {
 __device__ __forceinline__ TileCoord decode(const KParams &p, int64_t t) {
   TileCoord c;
   QuotRem x;
-  if (p.kacc) {  // the K splits of a (tile, group) item are consecutive jobs of one CTA
-    x = quot_rem(t, p.spg);
-    const int64_t u = x.r;
-    x = quot_rem(x.q, (uint32_t)p.ksplit / (uint32_t)p.spg);
-    c.s = x.r * p.spg + u;
+  if (p.kacc) {  // the K splits of a tile are consecutive jobs of one CTA
+    x = quot_rem(t, p.ksplit);
+    c.s = x.r;
     x = quot_rem(x.q, p.mt);
     c.m = x.r;
     x = quot_rem(x.q, p.nt);
@@ -104,105 +73,13 @@ __device__ __forceinline__ TileCoord decode(const KParams &p, int64_t t) {
   return c;
 }
 
-// v - float(hi) is exact in FP32 (hi is v rounded to 8 significant bits), so
-// the split costs no FP64 work in the epilogue.
-__device__ __forceinline__ void epi_store(const TcEpilogue &e, int64_t off, float v) {
-  if (e.kind == TcEpilogue::SPLIT_BF16) {
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    const __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-    e.out_hi[off] = __bfloat16_as_ushort(h);
-    e.out_lo[off] = __bfloat16_as_ushort(l);
-  } else if (e.kind == TcEpilogue::STORE_F32) {
-    e.out_f32[off] = v;
-  } else {
-    double *y = e.out_f64 + off;
-    const double r = e.alpha * (double)v;
-    *y = (e.beta == 0.0) ? r : fma(e.beta, *y, r);
-  }
-}
-
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n"
-      " mov.b64 {%0, %1}, x;\n}\n"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.f32x2 x, x, y;\n"
-      " mov.b64 {%0, %1}, x;\n}\n"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-
-// The K splits' FP32 sums of a tile are added as an unevaluated pair of floats (Knuth's TwoSum,
-// error-free; about 48 significant bits) in kh[j] + kl[j]: no FP64 instruction per split (the
-// FP64 pipe of GB300 runs at 2 operations per clock and SM).  In slice mode every split sum is
-// exact, so the result is the exact sum of the splits to that precision.
-template <int W>
-__device__ __forceinline__ void pair_add(float (&kh)[W], float (&kl)[W], const uint32_t (&r)[W], bool first) {
-  if (first) {
-#pragma unroll
-    for (int j = 0; j < W; ++j) {
-      kh[j] = __uint_as_float(r[j]);
-      kl[j] = 0.f;
-    }
-    return;
-  }
-#pragma unroll
-  for (int j = 0; j < W; j += 2) {  // two columns per instruction
-    const float2 x = make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-    const float2 hi = make_float2(kh[j], kh[j + 1]);
-    const float2 sum = add2(hi, x);
-    const float2 bb = sub2(sum, hi);
-    const float2 lo = add2(make_float2(kl[j], kl[j + 1]), add2(sub2(hi, sub2(sum, bb)), sub2(x, bb)));
-    kh[j] = sum.x;
-    kh[j + 1] = sum.y;
-    kl[j] = lo.x;
-    kl[j + 1] = lo.y;
-  }
-}
-
-// Writes a thread's float-pair sums (columns n0 ..) of row base rbase through the epilogue map.
-template <int W>
-__device__ __forceinline__ void pair_write(const float (&kh)[W], const float (&kl)[W], const TcEpilogue &e,
-                                           int64_t N, int64_t n0,
-                                           int64_t rbase) {
-  const QuotRem nx = quot_rem(n0, e.cd);
-  int64_t n = n0, nq = nx.q, nr = nx.r;
-#pragma unroll
-  for (int j = 0; j < W; ++j) {
-    if (n < N && nr < e.clim) {
-      const int64_t off = rbase + nq * e.co1 + nr * e.co2;
-      const float hi = kh[j], lo = kl[j];
-      if (e.kind == TcEpilogue::PAIR_F32) {
-        reinterpret_cast<float2 *>(e.out_f32)[off] = make_float2(hi, lo);
-      } else {
-        const double val = (double)hi + (double)lo;
-        if (e.kind == TcEpilogue::AXPBY_F64) {
-          double *y = e.out_f64 + off;
-          const double rv = e.alpha * val;
-          *y = (e.beta == 0.0) ? rv : fma(e.beta, *y, rv);
-        } else {
-          epi_store(e, off, (float)val);
-        }
-      }
-    }
-    ++n;
-    if (++nr == e.cd) { nr = 0; ++nq; }
-  }
-}
-
 // Work items of the persistent kernel: an item is one tile job, or, for a problem with in-CTA K
 // accumulation (kacc), the ksplit consecutive jobs of one output tile; items are strided over
 // the CTAs and a CTA runs the jobs of its item in order.
 __host__ __device__ __forceinline__ int64_t item_count(const KParams &p) {
   return p.kacc ? p.nitems : p.ntiles;
 }
-__device__ __forceinline__ int64_t item_len(const KParams &p) { return p.kacc ? p.spg : 1; }
+__device__ __forceinline__ int64_t item_len(const KParams &p) { return p.kacc ? p.ksplit : 1; }
 
 // K blocks [kb, ke) of split s.
 struct KRange {
@@ -253,9 +130,9 @@ struct GroupSrc {
 };
 static_assert(sizeof(GroupSrc) <= 32000, "grouped GEMM parameters exceed the kernel parameter space");
 
-template <int BN, int BK, class Src, bool SLICE = false>
-__global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel(const __grid_constant__ Src src) {
-  using C = Cfg<BN, BK, SLICE>;
+template <int BN, int BK, class Src>
+__global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_constant__ Src src) {
+  using C = Cfg<BN, BK>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t *full = (uint64_t *)(smem + C::STAGES * C::STAGE_BYTES);
@@ -273,7 +150,7 @@ __global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel
     }
     for (int i = 0; i < C::NBUF; ++i) {
       mbar_init(&accf[i], 1);
-      mbar_init(&acce[i], C::EPI);  // one arrive per epilogue warp
+      mbar_init(&acce[i], kEpiWarps);  // one arrive per epilogue warp  // one arrive per epilogue warp
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -308,40 +185,17 @@ __global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel
         TileCoord tc = decode(p, li * len);
         const int ya = (int)(tc.b * p.a_brows + tc.m * BM);
         const int yb = (int)(tc.b * p.b_brows + tc.n * BN);
-        if constexpr (SLICE) {
-          // the item's split group g: runs [q0, q0 + rpg); units (a, run, b0) in order, each K
-          // block of a unit one stage with A plane a and B planes b0 .. b0 + nb - 1
-          const int kchunks = (int)(p.K / BK);
-          const int q0 = ((int)tc.s / p.spg) * p.rpg;
-          for (int a = 0; a < p.nsl; ++a)
-            for (int qr = q0; qr < q0 + p.rpg; ++qr)
-              for (int b0 = 0; b0 < p.nsl - a; b0 += C::UNIT) {
-                const int nb = min(C::UNIT, p.nsl - a - b0);
-                const int kb = qr * p.kc_per, ke = min(kchunks, kb + p.kc_per);
-                for (int kc = kb; kc < ke; ++kc) {
-                  if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, err, 1)) goto producer_done;
-                  uint8_t *st = smem + stage * C::STAGE_BYTES;
-                  mbar_expect_tx(&full[stage], (uint32_t)(C::A_BYTES + nb * C::B_BYTES));
-                  tma_load_2d(smem_u32(st), mAhi, &full[stage], kc * BK, ya + a * (int)p.a_plane);
-                  for (int b = 0; b < nb; ++b)
-                    tma_load_2d(smem_u32(st + C::A_BYTES + b * C::B_BYTES), mBhi, &full[stage], kc * BK,
-                                yb + (b0 + b) * (int)p.b_plane);
-                  if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-                }
-              }
-        } else {
-          for (int64_t u = 0; u < len; ++u, ++tc.s) {
-            const KRange kr = k_range<BK>(p, tc.s);
-            for (int kc = kr.kb; kc < kr.ke; ++kc) {
-              if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, err, 1)) goto producer_done;
-              uint8_t *st = smem + stage * C::STAGE_BYTES;
-              mbar_expect_tx(&full[stage], (uint32_t)C::STAGE_BYTES);
-              tma_load_2d(smem_u32(st), mAhi, &full[stage], kc * BK, ya);
-              tma_load_2d(smem_u32(st + C::A_BYTES), mAlo, &full[stage], kc * BK, ya);
-              tma_load_2d(smem_u32(st + 2 * C::A_BYTES), mBhi, &full[stage], kc * BK, yb);
-              tma_load_2d(smem_u32(st + 2 * C::A_BYTES + C::B_BYTES), mBlo, &full[stage], kc * BK, yb);
-              if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-            }
+        for (int64_t u = 0; u < len; ++u, ++tc.s) {
+          const KRange kr = k_range<BK>(p, tc.s);
+          for (int kc = kr.kb; kc < kr.ke; ++kc) {
+            if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, err, 1)) goto producer_done;
+            uint8_t *st = smem + stage * C::STAGE_BYTES;
+            mbar_expect_tx(&full[stage], (uint32_t)C::STAGE_BYTES);
+            tma_load_2d(smem_u32(st), mAhi, &full[stage], kc * BK, ya);
+            tma_load_2d(smem_u32(st + C::A_BYTES), mAlo, &full[stage], kc * BK, ya);
+            tma_load_2d(smem_u32(st + 2 * C::A_BYTES), mBhi, &full[stage], kc * BK, yb);
+            tma_load_2d(smem_u32(st + 2 * C::A_BYTES + C::B_BYTES), mBlo, &full[stage], kc * BK, yb);
+            if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
           }
         }
       }
@@ -370,39 +224,6 @@ __global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel
         const int64_t len = item_len(p);
         // the jobs of an item share the tile; only the K split advances (decode once per item)
         TileCoord tc = decode(p, li * len);
-        if constexpr (SLICE) {
-          // units (a, run, b0) in the producer's order: one accumulator buffer per unit, nb
-          // adjacent accumulators of BN columns filled by one MMA of width nb * BN per K step
-          const int kchunks = (int)(p.K / BK);
-          const int q0 = ((int)tc.s / p.spg) * p.rpg;
-          for (int a = 0; a < p.nsl; ++a)
-            for (int qr = q0; qr < q0 + p.rpg; ++qr)
-              for (int b0 = 0; b0 < p.nsl - a; b0 += C::UNIT) {
-                const int nb = min(C::UNIT, p.nsl - a - b0);
-                const int kb = qr * p.kc_per, ke = min(kchunks, kb + p.kc_per);
-                const uint32_t idesc_u = (idesc & ~(0x3Fu << 17)) | ((uint32_t)((nb * BN) >> 3) << 17);
-                if (!mbar_wait(&acce[buf], aphase ^ 1, abort_flag, err, 2)) goto mma_done;
-                fence_after();
-                const uint32_t dtu = tmem_base + (uint32_t)(buf * C::BUFW);
-                for (int kc = kb; kc < ke; ++kc) {
-                  if (!mbar_wait(&full[stage], phase, abort_flag, err, 3)) goto mma_done;
-                  fence_after();
-                  const uint32_t st = smem_u32(smem + stage * C::STAGE_BYTES);
-                  // descriptors are linear in the address (bits 0-13 hold addr >> 4): + 2 per
-                  // 16-element K step; the B planes of the unit are one stacked operand
-                  const uint64_t da = sdesc(st, C::SBO, C::LAYOUT);
-                  const uint64_t db = sdesc(st + C::A_BYTES, C::SBO, C::LAYOUT);
-                  mma_bf16(dtu, da, db, idesc_u, kc > kb ? 1u : 0u);
-#pragma unroll
-                  for (int kk = 1; kk < BK / 16; ++kk) mma_bf16(dtu, da + 2 * kk, db + 2 * kk, idesc_u, 1u);
-                  mma_commit(&empty[stage]);
-                  if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-                }
-                mma_commit(&accf[buf]);
-                if (++buf == C::NBUF) { buf = 0; aphase ^= 1; }
-              }
-          continue;
-        }
         for (int64_t u = 0; u < len; ++u, ++tc.s) {
           const KRange kr = k_range<BK>(p, tc.s);
           const int kb = kr.kb, ke = kr.ke;
@@ -443,10 +264,12 @@ __global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel
     // the tile's columns.
     const int q = warp % 4;
     const int part = (warp - 2) / 4;
-    constexpr int COLS = SLICE ? BN / 4 : BN >= 64 ? BN / 2 : BN;
+    constexpr int COLS = BN >= 64 ? BN / 2 : BN;
     const int cbeg = min(part * COLS, BN);
     const int cend = min(cbeg + COLS, BN);
-    float kh[C::KCOLS], kl[C::KCOLS];  // float-pair sums over the K splits of a tile (kacc, slices)
+    // float-pair sums over the K splits of a tile (kacc; BN <= 64: at most 32 columns per thread)
+    constexpr int KACC = BN <= 64 ? 32 : 1;
+    float kh[KACC], kl[KACC];
     int buf = 0;
     uint32_t aphase = 0;
     int hint = 0;
@@ -456,50 +279,24 @@ __global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel
       const KParams p = src.params(src.locate(R, li, hint));
       const TcEpilogue &e = p.epi;
       const int64_t len = item_len(p);
-      // the jobs of an item share the tile and the split group: row terms once per item
+      // the jobs of an item share the tile: row terms once per item
       TileCoord tc = decode(p, li * len);
       const int64_t i = tc.m * BM + q * 32 + lane;
       const QuotRem ix = quot_rem(i, e.rd);
       const bool row_ok = i < p.M && ix.r < e.rlim;
-      // partial offset: the K split (F32 partials) or the split group (kacc groups)
-      const int64_t rbase = ix.q * e.ro1 + ix.r * e.ro2 + tc.b * e.bo +
-                            (p.kacc ? ((int)tc.s / p.spg) * e.so : tc.s * e.so);
-      if constexpr (SLICE) {
-        // the units of the item in the MMA's order; each buffer holds nb adjacent accumulators
-        const int q0 = ((int)tc.s / p.spg) * p.rpg;
-        bool first = true;
-        for (int a = 0; a < p.nsl; ++a)
-          for (int qr = q0; qr < q0 + p.rpg; ++qr)
-            for (int b0 = 0; b0 < p.nsl - a; b0 += C::UNIT) {
-              const int nb = min(C::UNIT, p.nsl - a - b0);
-              if (!mbar_wait(&accf[buf], aphase, abort_flag, err, 4)) goto epi_done;
-              fence_after();
-              for (int j = 0; j < nb; ++j) {
-                uint32_t r[C::KCOLS];
-                tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + j * BN + cbeg), r);
-                pair_add(kh, kl, r, first);
-                first = false;
-              }
-              fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&acce[buf]);
-              if (++buf == C::NBUF) { buf = 0; aphase ^= 1; }
-            }
-        if (row_ok) pair_write(kh, kl, e, p.N, tc.n * BN + cbeg, rbase);
-        continue;
-      }
+      // partial offset: the K split (F32 partials); none with kacc
+      const int64_t rbase = ix.q * e.ro1 + ix.r * e.ro2 + tc.b * e.bo + (p.kacc ? 0 : tc.s * e.so);
       for (int64_t u = 0; u < len; ++u, ++tc.s) {
       if (!mbar_wait(&accf[buf], aphase, abort_flag, err, 4)) goto epi_done;
       fence_after();
-      if constexpr (BN <= 64 && !SLICE) {
+      if constexpr (BN <= 64) {
         if (p.kacc) {
           // this thread's 32 columns (cbeg == cend for the idle half of a BN = 32 tile)
           if (cbeg < cend) {
             uint32_t r[32];
-            tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + cbeg), r);
-            const int64_t sg = u;  // position inside the split group (an item is one group)
-            pair_add(kh, kl, r, sg == 0);
-            if (row_ok && sg == p.spg - 1) pair_write(kh, kl, e, p.N, tc.n * BN + cbeg, rbase);  // split order
+            tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + cbeg), r);
+            pair_add(kh, kl, r, u == 0);
+            if (row_ok && u == len - 1) pair_write(kh, kl, e, p.N, tc.n * BN + cbeg, rbase);  // split order
           }
           fence_before();
           __syncwarp();
@@ -511,7 +308,7 @@ __global__ void __launch_bounds__(Cfg<BN, BK, SLICE>::THREADS, 1) tc_gemm_kernel
 #pragma unroll 1
       for (int c0 = cbeg; c0 < cend; c0 += 32) {
         uint32_t r[32];
-        tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::BUFW + c0), r);
+        tmem_ld(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + c0), r);
         if (!row_ok) continue;
         const int64_t n0 = tc.n * BN + c0;
         const QuotRem nx = quot_rem(n0, e.cd);
@@ -646,6 +443,8 @@ __global__ void reduce_partials_kernel(const float *__restrict__ part, int64_t M
   reduce_range(part, M, N, ksplit, e, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
                (int64_t)gridDim.x * blockDim.x);
 }
+
+constexpr int kMaxDigits = 5;
 
 // One warp per (row, run of chunk columns): the run's maximum, then its digits, all in integer
 // arithmetic on the FP64 bit patterns (the FP64 pipe of GB300 is slow; these are INT32/INT64
@@ -848,8 +647,7 @@ __global__ void slice_kernel(const In in, int64_t rows, int64_t cols, const Spli
 // above re-reads the run for its digits and keeps one load per lane in flight).  The digits and
 // their bf16 bits are those of slice_kernel, element for element: digit t is round(m / 2^s_t) less
 // 2^7 round(m / 2^s_(t-1)), in 32 bits from m >> 6, and becomes a float by one addition and one
-// multiplication (64-bit digits and integer conversions: 868 us for the 5120 x 32768 float
-// pairs of a 3.0 GB pass, 668 us).
+// multiplication.
 constexpr int kRunGroups = 8;  // 8 groups x 4 elements x 32 lanes = 1024 columns per run
 template <class In, int NSL>
 __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t rows, int64_t cols, const SplitMap m,
@@ -941,18 +739,95 @@ __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t row
   }
 }
 
-__global__ void reduce_f64_kernel(const double *__restrict__ part, int64_t M, int64_t N, int G,
-                                  const TcEpilogue e) {
-  const int64_t total = M * N;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const QuotRem tx = quot_rem(t, M);
-    const QuotRem ix = quot_rem(tx.r, e.rd), nx = quot_rem(tx.q, e.cd);
-    if (ix.r >= e.rlim || nx.r >= e.clim) continue;
-    double acc = 0.0;
-    for (int g = 0; g < G; ++g) acc += part[g * total + t];
-    double *y = e.out_f64 + ix.q * e.ro1 + ix.r * e.ro2 + nx.q * e.co1 + nx.r * e.co2;
-    const double r = e.alpha * acc;
-    *y = (e.beta == 0.0) ? r : fma(e.beta, *y, r);
+// Digits of float pairs (values hi + lo) for runs of at most 128 NG columns and five digits: a lane
+// holds its NG groups of 4 consecutive elements of the run in registers, so every load of the run
+// is in flight at once and the input is read once.  The digits come from additions (Ozaki et al.'s
+// extraction: adding and taking back 1.5 2^23 units of a digit rounds to it): digit t of r in
+// units of 2^(1 - 7 t) for r = value 2^(1 - e), e the exponent of the run's largest value, three
+// from hi and two more after adding lo; two elements per instruction.  Bound: HBM (8 bytes read,
+// 10 written per element).  5120 x 32768 pairs in runs of 1024: 868 us with 64-bit integer digits,
+// 668 us with 32-bit ones, 428 us; 9000 x 40000 in runs of 320: 2090 us with the registers of 1024
+// columns, 946 us.
+template <int NG>
+__global__ void __launch_bounds__(256) slice_pairs_kernel(const float *__restrict__ x2, int64_t rows, int64_t cols,
+                                                          const SplitMap m, int64_t chunk, uint16_t *__restrict__ out,
+                                                          int64_t ldo, int64_t plane) {
+  constexpr int S = kMaxDigits;
+  const int lane = threadIdx.x & 31;
+  const int64_t nchunks = (cols + chunk - 1) / chunk;
+  const int64_t units = rows * nchunks;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps) {
+    const QuotRem ux = quot_rem(u, nchunks), rx = quot_rem(ux.q, m.rdiv);
+    if (rx.r >= m.rlim) continue;  // uniform over the warp
+    const float4 *src = reinterpret_cast<const float4 *>(x2) + (rx.q * m.rs1 + rx.r * m.rs2) / 2;
+    const int64_t c0 = ux.r * chunk, c1 = min(cols, c0 + chunk);
+    float2 h[NG][2], l[NG][2];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      const int64_t c = c0 + 128 * g + 4 * lane;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+      if (c + 4 <= c1) {
+        a = __ldg(src + c / 2);
+        b = __ldg(src + c / 2 + 1);
+      } else if (c < c1) {
+        const float2 *p = reinterpret_cast<const float2 *>(src) + c;
+        const float2 y0 = __ldg(p);
+        a.x = y0.x; a.y = y0.y;
+        if (c + 1 < c1) { const float2 y = __ldg(p + 1); a.z = y.x; a.w = y.y; }
+        if (c + 2 < c1) { const float2 y = __ldg(p + 2); b.x = y.x; b.y = y.y; }
+      }
+      h[g][0] = make_float2(a.x, a.z); l[g][0] = make_float2(a.y, a.w);
+      h[g][1] = make_float2(b.x, b.z); l[g][1] = make_float2(b.y, b.w);
+    }
+    unsigned mx = 0;
+#pragma unroll
+    for (int g = 0; g < NG; ++g)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        // normalised pairs (TwoSum): |lo| <= 2^-24 |hi|
+        const float2 s = add2(h[g][v], l[g][v]), bb = sub2(s, h[g][v]);
+        l[g][v] = add2(sub2(h[g][v], sub2(s, bb)), sub2(l[g][v], bb));
+        h[g][v] = s;
+        mx = max(mx, max(__float_as_uint(s.x) & 0x7FFFFFFFu, __float_as_uint(s.y) & 0x7FFFFFFFu));
+      }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    const int e = min(max((int)(mx >> 23), 1) - 126, 127);  // mx < 2^e; infinities and NaN stay what they are
+    const float down = __int_as_float((127 + 1 - e) << 23), up = mx ? __int_as_float((127 + e - 1) << 23) : 0.f;
+    const float2 dn2 = make_float2(down, down), up2 = make_float2(up, up);
+    uint16_t *orow = out + ux.q * ldo;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      const int64_t c = c0 + 128 * g + 4 * lane;
+      if (c >= c1) continue;
+      uint32_t packed[S][2];
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        float2 r = mul2(h[g][v], dn2);
+#pragma unroll
+        for (int t = 1; t <= S; ++t) {
+          if (t == 4) r = add2(r, mul2(l[g][v], dn2));
+          const float mg = 12582912.f / (float)(1ull << (7 * t - 1));  // 1.5 2^23 units of 2^(1 - 7 t)
+          const float2 mg2 = make_float2(mg, mg);
+          const float2 d = sub2(add2(r, mg2), mg2);
+          r = sub2(r, d);
+          const float2 f = mul2(d, up2);
+          asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed[t - 1][v]) : "f"(f.y), "f"(f.x));
+        }
+      }
+      if (c + 4 <= c1) {
+#pragma unroll
+        for (int t = 0; t < S; ++t)
+          *reinterpret_cast<uint2 *>(orow + t * plane + c) = make_uint2(packed[t][0], packed[t][1]);
+      } else {
+        const int nv = (int)(c1 - c);
+#pragma unroll
+        for (int t = 0; t < S; ++t)
+#pragma unroll
+          for (int v = 0; v < 3; ++v)
+            if (v < nv) orow[t * plane + c + v] = (uint16_t)(packed[t][v / 2] >> (16 * (v & 1)));
+      }
+    }
   }
 }
 
@@ -962,16 +837,16 @@ __global__ void reduce_group_kernel(const __grid_constant__ ReduceGroup g) {
                (int64_t)gridDim.x * blockDim.x);
 }
 
-template <int BN, int BK, class Src, bool SLICE = false>
+template <int BN, int BK, class Src>
 void launch_src(const Src &src, int64_t ntiles, cudaStream_t s) {
-  using C = Cfg<BN, BK, SLICE>;
+  using C = Cfg<BN, BK>;
   static std::once_flag attr;
   std::call_once(attr, [] {
-    VGB_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<BN, BK, Src, SLICE>,
+    VGB_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<BN, BK, Src>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   });
   const int64_t grid = std::min<int64_t>(ntiles, sm_count());
-  tc_gemm_kernel<BN, BK, Src, SLICE><<<(unsigned)grid, C::THREADS, C::SMEM, s>>>(src);
+  tc_gemm_kernel<BN, BK, Src><<<(unsigned)grid, kThreads, C::SMEM, s>>>(src);
   VGB_LAUNCH_CHECK();
 }
 
@@ -1025,16 +900,6 @@ KParams make_params(const TcMat &A, const TcMat &B, const TcShape &sh, const TcE
   VGB_REQUIRE(A.bk == B.bk, "tc_gemm: operands staged with different K boxes");
   const int BK = A.bk;
   VGB_REQUIRE(sh.K % BK == 0 && A.K >= sh.K && B.K >= sh.K, "tc_gemm: K not padded");
-  int64_t a_extra = 0, b_extra = 0;  // slice mode: rows of the highest digit plane addressed
-  if (sh.nslices > 0) {
-    VGB_REQUIRE(sh.nslices <= kMaxDigits && sh.chain >= BK && sh.chain % BK == 0 && sh.nbatch == 1 &&
-                    BK == 64 && bn <= 64,
-                "tc_gemm: bad slice-mode shape");
-    VGB_REQUIRE(sh.a_plane >= sh.M && sh.b_plane >= sh.N, "tc_gemm: slice planes smaller than the problem");
-    VGB_REQUIRE((int64_t)sh.nslices * std::max(sh.a_plane, sh.b_plane) < (1LL << 31), "tc_gemm: planes too large");
-    a_extra = (sh.nslices - 1) * sh.a_plane;
-    b_extra = (sh.nslices - 1) * sh.b_plane;
-  }
   VGB_REQUIRE(epi.rd >= 1 && epi.cd >= 1, "tc_gemm: bad epilogue map");
   KParams p;
   p.ntiles = 0;
@@ -1042,52 +907,29 @@ KParams make_params(const TcMat &A, const TcMat &B, const TcShape &sh, const TcE
   if (sh.M <= 0 || sh.N <= 0 || sh.nbatch <= 0) return p;
   // rows addressed by the last batch must exist in the operands (TMA fills beyond with zeros,
   // but row coordinates must stay within the int32 range of the descriptor)
-  VGB_REQUIRE((sh.nbatch - 1) * sh.a_batch_rows + a_extra + sh.M <= A.rows + BM, "tc_gemm: A rows");
-  VGB_REQUIRE((sh.nbatch - 1) * sh.b_batch_rows + b_extra + sh.N <= B.rows + bn, "tc_gemm: B rows");
+  VGB_REQUIRE((sh.nbatch - 1) * sh.a_batch_rows + sh.M <= A.rows + BM, "tc_gemm: A rows");
+  VGB_REQUIRE((sh.nbatch - 1) * sh.b_batch_rows + sh.N <= B.rows + bn, "tc_gemm: B rows");
   VGB_REQUIRE(A.rows < (1LL << 31) && B.rows < (1LL << 31), "tc_gemm: too many rows");
   p.M = sh.M; p.N = sh.N; p.K = sh.K;
-  p.products = sh.nslices > 0 ? 1 : (sh.products == 4 ? 4 : 3);
-  p.nsl = sh.nslices > 0 ? sh.nslices : 0;
-  p.a_plane = sh.a_plane;
-  p.b_plane = sh.b_plane;
+  p.products = sh.products == 4 ? 4 : 3;
   p.nbatch = sh.nbatch;
   p.a_brows = sh.a_batch_rows;
   p.b_brows = sh.b_batch_rows;
   const int kchunks = (int)(sh.K / BK);
   VGB_REQUIRE(kchunks >= 1, "tc_gemm: K must be positive");
-  const int npairs = p.nsl * (p.nsl + 1) / 2;
-  int groups = 1;
-  if (p.nsl) {  // every split: one digit pair on one run of at most chain K elements
-    p.kc_per = (int)std::min<int64_t>(kchunks, sh.chain / BK);
-    p.cpr = (int)ceil_div(kchunks, p.kc_per);
-    p.ksplit = npairs * p.cpr;
-    p.kacc = 1;
-    groups = std::max(1, sh.kgroups);
-    VGB_REQUIRE(p.cpr % groups == 0, "tc_gemm: split groups must divide the K runs");
-    p.rpg = p.cpr / groups;
-  } else {
-    int ks = std::max(1, std::min(sh.ksplit, kchunks));
-    p.kc_per = (int)ceil_div(kchunks, ks);
-    p.ksplit = (int)ceil_div(kchunks, p.kc_per);
-    p.cpr = p.ksplit;
-    p.rpg = 0;
-    p.kacc = (sh.kacc && p.ksplit > 1) ? 1 : 0;
-    groups = p.kacc ? std::max(1, sh.kgroups) : 1;
-    VGB_REQUIRE(p.ksplit % groups == 0, "tc_gemm: split groups must divide the K splits");
-  }
-  VGB_REQUIRE(groups == 1 || (epi.kind == TcEpilogue::AXPBY_F64 && epi.beta == 0.0),
-              "tc_gemm: split groups write FP64 partials");
-  p.spg = p.ksplit / groups;
+  const int ks = std::max(1, std::min(sh.ksplit, kchunks));
+  p.kc_per = (int)ceil_div(kchunks, ks);
+  p.ksplit = (int)ceil_div(kchunks, p.kc_per);
+  p.kacc = (sh.kacc && p.ksplit > 1) ? 1 : 0;
+  VGB_REQUIRE(epi.kind != TcEpilogue::PAIR_F32, "tc_gemm: float-pair output is for slice products");
   VGB_REQUIRE(!p.kacc || (bn <= 64 && epi.kind != TcEpilogue::STORE_F32),
               "tc_gemm: in-CTA K accumulation needs BN <= 64 and a final (split or FP64) epilogue");
-  VGB_REQUIRE(epi.kind != TcEpilogue::PAIR_F32 || (p.kacc && p.nsl > 0 && (int64_t)bn <= 64),
-              "tc_gemm: float-pair output needs slice mode with in-CTA K accumulation");
   VGB_REQUIRE(p.ksplit == 1 || p.kacc || epi.kind == TcEpilogue::STORE_F32,
               "tc_gemm: K split needs F32 partials or in-CTA accumulation");
   p.mt = ceil_div(sh.M, BM);
   p.nt = ceil_div(sh.N, bn);
   p.ntiles = p.mt * p.nt * p.ksplit * sh.nbatch;
-  p.nitems = p.ntiles / p.spg;
+  p.nitems = p.ntiles / p.ksplit;
   p.epi = epi;
   p.err = err;
   return p;
@@ -1105,12 +947,7 @@ int tc_gemm(const TcMat &A, const TcMat &B, const TcShape &sh, const TcEpilogue 
   src.maps[2] = B.map_hi;
   src.maps[3] = B.map_lo;
   src.p = p;
-  if (p.nsl) {  // slice mode (validated: K box 64, BN <= 64)
-    if (bn == 32) launch_src<32, 64, SingleSrc, true>(src, item_count(p), s);
-    else launch_src<64, 64, SingleSrc, true>(src, item_count(p), s);
-  } else {
-    launch_any(bn, A.bk, src, item_count(p), s);
-  }
+  launch_any(bn, A.bk, src, item_count(p), s);
   return p.ksplit;
 }
 
@@ -1159,7 +996,6 @@ void tc_gemm_grouped(const std::vector<const TcProblem *> &probs, int bn, int *e
     int64_t total = 0;
     for (; i < probs.size() && src->n < gmax; ++i) {
       const TcProblem &q = *probs[i];
-      VGB_REQUIRE(q.shape.nslices == 0, "tc_gemm_grouped: slice mode runs through tc_gemm");
       const KParams p = make_params(q.A, q.B, q.shape, q.epi, bn, err);
       if (ksplit_out) ksplit_out[i] = p.ksplit;
       if (p.ntiles == 0) continue;
@@ -1273,20 +1109,23 @@ void slice_pairs(const float *x2, int64_t rows, int64_t cols, const SplitMap &m,
   const PairIn in{reinterpret_cast<const unsigned long long *>(x2)};
   if (m.cs == 1 && chunk % 4 == 0 && m.rs1 % 4 == 0 && m.rs2 % 4 == 0 && ldo % 4 == 0 && plane % 4 == 0 &&
       ((uintptr_t)x2 & 31) == 0 && ((uintptr_t)out & 7) == 0) {
-    if (nslices == 5) slice_run_kernel<PairIn, 5><<<blocks, 256, 0, s>>>(in, rows, cols, m, chunk, out, ldo, plane);
-    else slice_kernel<PairIn, 4, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    if (nslices == 5) {
+      const int ng = (int)ceil_div(std::min(chunk, cols), 128);
+#define VGB_SLICE(NG) slice_pairs_kernel<NG><<<blocks, 256, 0, s>>>(x2, rows, cols, m, chunk, out, ldo, plane)
+      switch (ng) {
+        case 1: VGB_SLICE(1); break;
+        case 2: VGB_SLICE(2); break;
+        case 3: VGB_SLICE(3); break;
+        case 4: VGB_SLICE(4); break;
+        case 5: VGB_SLICE(5); break;
+        case 6: VGB_SLICE(6); break;
+        default: VGB_SLICE(8); break;
+      }
+#undef VGB_SLICE
+    } else slice_kernel<PairIn, 4, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
   } else {
     slice_kernel<PairIn, 1, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
   }
-  VGB_LAUNCH_CHECK();
-}
-
-void reduce_f64_groups(const double *part, int64_t M, int64_t N, int ngroups, const TcEpilogue &epi,
-                       cudaStream_t s) {
-  if (M <= 0 || N <= 0) return;
-  VGB_REQUIRE(epi.kind == TcEpilogue::AXPBY_F64 && ngroups >= 1 && epi.rd >= 1 && epi.cd >= 1,
-              "reduce_f64_groups: bad epilogue");
-  reduce_f64_kernel<<<grid_1d(M * N), 256, 0, s>>>(part, M, N, ngroups, epi);
   VGB_LAUNCH_CHECK();
 }
 

@@ -37,7 +37,7 @@ TcMat make_tc_mat(const uint16_t *hi, const uint16_t *lo, int64_t rows, int64_t 
 //   (i / rd) * ro1 + (i % rd) * ro2 + (n / cd) * co1 + (n % cd) * co2 + b * bo + s * so
 // and is written only when i < M, n < N, (i % rd) < rlim, (n % cd) < clim.
 struct TcEpilogue {
-  // PAIR_F32 (slice mode with kacc only): the FP64 sum as an unevaluated pair of floats
+  // PAIR_F32 (slice products only): the sum as an unevaluated pair of floats
   // (hi, lo), stored as a float2 at out_f32 + 2 * offset
   enum Kind { SPLIT_BF16 = 0, STORE_F32 = 1, AXPBY_F64 = 2, PAIR_F32 = 3 };
   int kind = AXPBY_F64;
@@ -59,21 +59,6 @@ struct TcShape {
   // with ksplit > 1 and BN <= 64: one CTA runs all splits of a tile and sums them in FP64
   // registers (in split order) before the epilogue map; no partials, no reduction launch
   bool kacc = false;
-  // kacc: the splits of a tile shared out to kgroups CTAs (kgroups divides the split count);
-  // group g writes its FP64 sum through the epilogue map at offset g * epi.so (beta = 0), and
-  // reduce_f64_groups adds the groups
-  int kgroups = 1;
-  // slice mode (nslices > 0, nbatch 1, K box 64, BN <= 64): the operands hold nslices bf16 digit
-  // planes stacked by rows (digit t of operand row r is row t * plane + r, see slice_f64); the
-  // product is the sum of A plane a times B plane b over all a + b < nslices, one bf16 MMA per K
-  // step.  Every K split covers one digit pair on one run of at most `chain` K elements (the run
-  // of one digit scale), its FP32 accumulator is exact, and the splits are summed on the CTA.
-  // A pipeline stage holds A plane a and B planes 0 .. nslices - 1 - a of one K block, whose
-  // products go to separate accumulators (one A load for up to nslices pairs).  kgroups must
-  // divide the number of runs.
-  int nslices = 0;
-  int64_t a_plane = 0, b_plane = 0;
-  int64_t chain = 1024;
 };
 
 // Launch the persistent GEMM; bn in {32, 64, 128, 256}.  err: device int set
@@ -124,11 +109,6 @@ void slice_f64(const double *x, int64_t rows, int64_t cols, const SplitMap &m, i
 // the map addresses float2 elements.
 void slice_pairs(const float *x2, int64_t rows, int64_t cols, const SplitMap &m, int nslices, int64_t chunk,
                  uint16_t *out, int64_t ldo, int64_t plane, cudaStream_t s);
-
-// Y = epi(sum over g < ngroups of part[g * M * N + n * M + i]) for the M x N partials of a
-// kgroups product (column-major per group), summed in FP64 in group order; epi: AXPBY_F64.
-void reduce_f64_groups(const double *part, int64_t M, int64_t N, int ngroups, const TcEpilogue &epi,
-                       cudaStream_t s);
 
 // Many independent splits / reductions in one launch per 96 jobs (one grid row per job).
 struct SplitJob {
