@@ -68,50 +68,70 @@ struct TnJob {
   int64_t lda, ldb, n, m, p;
   double *part;  // [chunk][m * p]
 };
-__global__ void __launch_bounds__(kThreads, 4) tn_partial_kernel(const __grid_constant__ Group<TnJob> g) {
-  const TnJob q = g.j[blockIdx.y];
-  const int64_t r0 = (int64_t)blockIdx.x * kTnRows;
-  if (r0 >= q.n) return;
-  const int64_t r1 = min(q.n, r0 + kTnRows);
-  __shared__ double sm[kTileLd * kTnCols];
-  const int cols = (int)(q.m + q.p);
-  const int64_t mp = q.m * q.p;
-  // Fewer outputs than threads (m p <= 128): the rows of a tile are split over S lanes of one
-  // warp per output, so that every warp of the block issues FP64 FMAs (GB300 has about 2 FP64
-  // FMA lanes per clock and SM: a block whose outputs fit in two warps would use half of them).
-  int S = 1;
-  while (S < 32 && mp * 2 * S <= kThreads) S *= 2;
+// The outputs of a chunk are shared out to parts CTAs (blockIdx.x = chunk * parts + part), as
+// every output is one chain of FMAs: a chunk with 200 outputs keeps two warps of every SM quarter
+// on 512 FMAs of 64 clocks each, while a batch of 24 molecules has about 120 chunks for 152
+// SMs.  The next tile's elements are in flight while this one is multiplied.  24 molecules of v
+// 4..32, c 32..256, 7 new columns: 65 us a launch, 35 us.
+// NL: elements of a tile per thread (8 columns each); NO: outputs per thread.
+template <int NL, int NO>
+__device__ __forceinline__ void tn_chunk(const TnJob &q, double *sm, int chunk, int part, int per, int S) {
+  const int64_t r0 = (int64_t)chunk * kTnRows;
+  const int nrows = (int)min((int64_t)kTnRows, q.n - r0);
+  const int m = (int)q.m, cols = (int)(q.m + q.p), mp = (int)(q.m * q.p);
   const int sub = threadIdx.x & (S - 1);
-  const int64_t os = threadIdx.x / S;  // the output of this thread when S > 1
-  double acc[kTnOut];
+  const int o0 = part * per, o1 = min(mp, o0 + per);
+  // the parts of a chunk put their outputs on different warps, so that CTAs sharing an SM load
+  // all its quarters
+  const int rot = part * (per * S / 32) & (kThreads / 32 - 1);
+  const int t = ((int)threadIdx.x + kThreads - 32 * rot) & (kThreads - 1);
+  const double *pa[NO], *pb[NO];  // the outputs' columns in the tile
+  double acc[NO];
 #pragma unroll
-  for (int k = 0; k < kTnOut; ++k) acc[k] = 0.0;
-  for (int64_t rt = r0; rt < r1; rt += kTile) {
-    const int rows = (int)min((int64_t)kTile, r1 - rt);
-    for (int e = threadIdx.x; e < kTile * cols; e += kThreads) {
-      const int col = e / kTile, r = e % kTile;
-      double v = 0.0;
-      if (r < rows) v = col < q.m ? q.A[rt + r + col * q.lda] : q.B[rt + r + (col - q.m) * q.ldb];
-      sm[col * kTileLd + r] = v;
-    }
+  for (int k = 0; k < NO; ++k) {
+    const int o = o0 + t / S + k * (kThreads / S);
+    const int c = o / m;
+    pa[k] = o < o1 ? sm + (o - c * m) * kTileLd : nullptr;
+    pb[k] = sm + (m + c) * kTileLd;
+    acc[k] = 0.0;
+  }
+  const int lr = threadIdx.x & (kTile - 1), lc = threadIdx.x / kTile;
+  constexpr int kStep = kThreads / kTile;
+  const double *src[NL];
+  double nx[NL];
+#pragma unroll
+  for (int e = 0; e < NL; ++e) {
+    const int col = lc + e * kStep;
+    src[e] = (col < m ? q.A + col * q.lda : q.B + (min(col, cols - 1) - m) * q.ldb) + r0 + lr;
+  }
+  auto load = [&](int rt) {
+#pragma unroll
+    for (int e = 0; e < NL; ++e) nx[e] = rt + lr < nrows ? src[e][rt] : 0.0;
+  };
+  load(0);
+  for (int rt = 0; rt < nrows; rt += kTile) {
+    const int rows = min(kTile, nrows - rt);
+#pragma unroll
+    for (int e = 0; e < NL; ++e) sm[(lc + e * kStep) * kTileLd + lr] = nx[e];
     __syncthreads();
-    if (S > 1) {
-      if (os < mp) {
-        const double *a = sm + (os % q.m) * kTileLd, *b = sm + (q.m + os / q.m) * kTileLd;
-        double s = acc[0];
-        for (int r = sub; r < rows; r += S) s = fma(a[r], b[r], s);
-        acc[0] = s;
-      }
-    } else {
+    if (rt + kTile < nrows) load(rt + kTile);
 #pragma unroll
-      for (int k = 0; k < kTnOut; ++k) {
-        const int64_t o = threadIdx.x + (int64_t)k * kThreads;
-        if (o < mp) {
-          const double *a = sm + (o % q.m) * kTileLd, *b = sm + (q.m + o / q.m) * kTileLd;
-          double s = acc[k];
-          for (int r = 0; r < rows; ++r) s = fma(a[r], b[r], s);
-          acc[k] = s;
+    for (int k = 0; k < NO; ++k) {
+      if (pa[k]) {
+        double s = acc[k];
+        int r = sub;
+        for (; r + 7 * S < rows; r += 8 * S) {  // eight loads of each operand in flight
+          double x[8], y[8];
+#pragma unroll
+          for (int v = 0; v < 8; ++v) {
+            x[v] = pa[k][r + v * S];
+            y[v] = pb[k][r + v * S];
+          }
+#pragma unroll
+          for (int v = 0; v < 8; ++v) s = fma(x[v], y[v], s);
         }
+        for (; r < rows; r += S) s = fma(pa[k][r], pb[k][r], s);
+        acc[k] = s;
       }
     }
     __syncthreads();
@@ -119,14 +139,30 @@ __global__ void __launch_bounds__(kThreads, 4) tn_partial_kernel(const __grid_co
   if (S > 1) {  // the S lanes of an output are consecutive lanes of one warp (S divides 32)
     double v = acc[0];
     for (int off = S / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (sub == 0 && os < mp) q.part[blockIdx.x * mp + os] = v;
-    return;
+    acc[0] = v;
   }
 #pragma unroll
-  for (int k = 0; k < kTnOut; ++k) {
-    const int64_t o = threadIdx.x + (int64_t)k * kThreads;
-    if (o < mp) q.part[blockIdx.x * mp + o] = acc[k];
-  }
+  for (int k = 0; k < NO; ++k)
+    if (pa[k] && sub == 0) q.part[(int64_t)chunk * mp + o0 + t / S + k * (kThreads / S)] = acc[k];
+}
+__global__ void __launch_bounds__(kThreads, 2) tn_partial_kernel(const __grid_constant__ Group<TnJob> g, int parts) {
+  const TnJob q = g.j[blockIdx.y];
+  const int chunk = (int)blockIdx.x / parts, part = (int)blockIdx.x - chunk * parts;
+  if ((int64_t)chunk * kTnRows >= q.n) return;
+  __shared__ double sm[kTileLd * kTnCols];
+  const int cols = (int)(q.m + q.p), mp = (int)(q.m * q.p);
+  // Fewer outputs than threads (m p <= 128): the rows of a tile are split over S lanes of one
+  // warp per output, so that every warp of the block issues FP64 FMAs (GB300 has about 2 FP64
+  // FMA lanes per clock and SM: a block whose outputs fit in two warps would use half of them).
+  int S = 1;
+  while (S < 32 && mp * 2 * S <= kThreads) S *= 2;
+  const int per = (((mp * S + parts - 1) / parts + 31) / 32) * 32 / S;  // this CTA's outputs: whole warps
+  if (part * per >= mp) return;
+  if (per * S > kThreads) tn_chunk<kTnCols / 8, kTnOut>(q, sm, chunk, part, per, S);
+  else if (cols <= 16) tn_chunk<2, 1>(q, sm, chunk, part, per, S);
+  else if (cols <= 32) tn_chunk<4, 1>(q, sm, chunk, part, per, S);
+  else if (cols <= 64) tn_chunk<8, 1>(q, sm, chunk, part, per, S);
+  else tn_chunk<kTnCols / 8, 1>(q, sm, chunk, part, per, S);
 }
 struct TnReduceJob {
   const double *part;
@@ -141,7 +177,8 @@ __global__ void tn_reduce_kernel(const __grid_constant__ Group<TnReduceJob> g) {
        o += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int64_t c = 0; c < q.chunks; ++c) s += q.part[c * mp + o];
-    q.C[(o % q.m) + (o / q.m) * q.ldc] = s;
+    const uint32_t c = (uint32_t)o / (uint32_t)q.m;
+    q.C[((uint32_t)o - c * (uint32_t)q.m) + c * q.ldc] = s;
   }
 }
 
@@ -154,21 +191,18 @@ struct NnJob {
   double alpha, beta;
 };
 template <int PC>
-__global__ void __launch_bounds__(kThreads) nn_kernel(const __grid_constant__ Group<NnJob> g) {
-  const NnJob q = g.j[blockIdx.y];
-  __shared__ double us[kNnSmem / sizeof(double)];
-  for (int64_t e = threadIdx.x; e < q.m * q.p; e += kThreads)
-    us[e] = q.U[(e % q.m) + (e / q.m) * q.ldu];
-  __syncthreads();
-  for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < q.n;
-       r += (int64_t)gridDim.x * kThreads) {
+__device__ __forceinline__ void nn_rows(const NnJob &q, const double *us) {
+  for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < q.n; r += (int64_t)gridDim.x * kThreads) {
     double acc[PC];
 #pragma unroll
     for (int j = 0; j < PC; ++j) acc[j] = 0.0;
-    for (int64_t l = 0; l < q.m; ++l) {
-      const double a = q.A[r + l * q.lda];
+    const int m = (int)q.m;
+    const double *a = q.A + r;
+#pragma unroll 4
+    for (int l = 0; l < m; ++l) {
+      const double x = a[l * q.lda];
 #pragma unroll
-      for (int j = 0; j < PC; ++j) acc[j] = fma(a, us[l + q.m * j], acc[j]);
+      for (int j = 0; j < PC; ++j) acc[j] = fma(x, us[l + m * j], acc[j]);
     }
 #pragma unroll
     for (int j = 0; j < PC; ++j) {
@@ -177,43 +211,80 @@ __global__ void __launch_bounds__(kThreads) nn_kernel(const __grid_constant__ Gr
     }
   }
 }
+// One launch for the jobs of every column count: three launches of a third of the SMs' work each
+// took 54 us per product of 24 molecules, 25 us here.
+__global__ void __launch_bounds__(kThreads) nn_kernel(const __grid_constant__ Group<NnJob> g) {
+  const NnJob q = g.j[blockIdx.y];
+  __shared__ double us[kNnSmem / sizeof(double)];
+  const int m = (int)q.m, p = (int)q.p;
+  if (blockIdx.x * (int64_t)kThreads >= q.n) return;
+  for (int e = threadIdx.x; e < m * p; e += kThreads) {
+    const int c = e / m;
+    us[e] = q.U[(e - c * m) + c * q.ldu];
+  }
+  __syncthreads();
+  switch (p) {
+    case 1: nn_rows<1>(q, us); break;
+    case 2: nn_rows<2>(q, us); break;
+    case 4: nn_rows<4>(q, us); break;
+    case 8: nn_rows<8>(q, us); break;
+    default: nn_rows<16>(q, us); break;
+  }
+}
 
-// ---- column norms (or dots with B) over n rows, one block per column ----
+// ---- column norms (or dots with B) over n rows, one block per column, with the elementwise work
+// before and after them (a launch of its own for each is 5 us) ----
 struct NormJob {
   const double *A, *B;  // B null: norms
   int64_t lda, ldb, n, p;
   double *out;
-  double *inv = nullptr;  // norms only: also 1 / norm where norm > 0, else 0
+  // the column first: A -= lam * sub (residuals)
+  double *a_out = nullptr;  // A, where it is written
+  const double *sub = nullptr, *lam = nullptr;
+  int64_t ldsub = 0;
+  bool scale = false;  // and last: A *= 1 / norm (a zero column stays, as with Eigen's normalize)
 };
 __global__ void norm_kernel(const __grid_constant__ Group<NormJob> g) {
   const NormJob q = g.j[blockIdx.y];
   const int64_t c = blockIdx.x;
   if (c >= q.p) return;
   const double *a = q.A + c * q.lda, *b = q.B ? q.B + c * q.ldb : a;
+  double *w = q.a_out + c * q.lda;
+  if (q.sub) {  // every thread reads back only what it wrote
+    const double lam = q.lam[c], *u = q.sub + c * q.ldsub;
+#pragma unroll 4
+    for (int64_t r = threadIdx.x; r < q.n; r += kThreads) w[r] -= lam * u[r];
+  }
   double s = 0.0;
+#pragma unroll 8
   for (int64_t r = threadIdx.x; r < q.n; r += kThreads) s = fma(a[r], b[r], s);
   __shared__ double red[kThreads];
   red[threadIdx.x] = s;
   __syncthreads();
-  for (int w = kThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+  for (int h = kThreads / 2; h > 0; h >>= 1) {
+    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
     __syncthreads();
   }
   if (threadIdx.x == 0) {
     const double r = q.B ? red[0] : sqrt(red[0]);
     q.out[c] = r;
-    // the FP64 division runs once per column here instead of once per element of a scaling
-    if (q.inv) q.inv[c] = r > 0.0 ? 1.0 / r : 0.0;
+    if (q.scale) red[1] = r > 0.0 ? 1.0 / r : 0.0;
+  }
+  if (!q.scale) return;
+  __syncthreads();
+  const double iv = red[1];
+  if (iv > 0.0) {
+#pragma unroll 4
+    for (int64_t r = threadIdx.x; r < q.n; r += kThreads) w[r] *= iv;
   }
 }
 
 // ---- elementwise column work ----
 struct ColJob {
-  int kind;  // 0: A *= 1 / norm (v holds the reciprocal norms, 0 for a zero column);
-             // 1: A -= lam * B (residual); 2: copy B -> A;
+  int kind;  // 2: copy B -> A;
              // 3: DPR A[:, kk] = -B[:, cols[kk]] / (D - lam[kk]), non-finite -> 0
   double *A;
-  const double *B, *D, *v;  // v: norms or lambdas
+  const double *B, *D, *v;  // v: lambdas
   const double *cols;       // DPR: root index of each new column (exact small integers)
   int64_t lda, ldb, n, p;
 };
@@ -222,14 +293,10 @@ __global__ void col_kernel(const __grid_constant__ Group<ColJob> g) {
   const int64_t total = q.n * q.p;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % q.n, j = t / q.n;
+    // 32-bit where it fits: a 64-bit division converts through the FP64 pipe
+    const int64_t j = total >> 32 ? t / q.n : (int64_t)((uint32_t)t / (uint32_t)q.n), i = t - j * q.n;
     double *a = q.A + i + j * q.lda;
-    if (q.kind == 0) {
-      const double iv = q.v[j];
-      if (iv > 0.0) *a *= iv;  // Eigen's normalize leaves a zero column unchanged
-    } else if (q.kind == 1) {
-      *a -= q.v[j] * q.B[i + j * q.ldb];
-    } else if (q.kind == 2) {
+    if (q.kind == 2) {
       *a = q.B[i + j * q.ldb];
     } else {
       double v = -q.B[i + (int64_t)q.cols[j] * q.ldb] / (q.D[i] - q.v[j]);
@@ -257,7 +324,75 @@ struct GsJob {
 // the rows of a column is a few dependent loads per thread.
 constexpr int kGsCluster = 4;
 constexpr int kGsThreads = 128;
-__global__ void __cluster_dims__(kGsCluster, 1, 1) __launch_bounds__(kGsThreads, 8)
+
+// This warp's sums of LC columns of M times q over the rows of the CTA, in red.  A predicated FMA
+// costs the FP64 pipe as much as an active one (64 clocks of an SM quarter), so the count is a
+// constant.  The reduction folds the LC sums together, exchanging half of them at each distance: 9
+// additions for 8 sums instead of 40, the same pairs of lanes added in each.
+template <int LC>
+__device__ __forceinline__ void gs_dots(const double *__restrict__ M, const double *qj, int64_t n, int64_t r0,
+                                        int64_t r1, double *red) {
+  double acc[8];
+#pragma unroll
+  for (int l = 0; l < 8; ++l) acc[l] = 0.0;
+#pragma unroll 4
+  for (int64_t i = r0 + threadIdx.x; i < r1; i += kGsThreads) {
+    const double x = qj[i];
+#pragma unroll
+    for (int l = 0; l < LC; ++l) acc[l] = fma(M[l * n + i], x, acc[l]);
+  }
+  const int lane = threadIdx.x & 31;
+  int w = LC;              // sums held per lane
+  int owner = 0, cnt = LC;  // the first of them, and how many are real
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const int half = (w + 1) / 2;
+    if (w > 1) {  // lanes with bit o keep the upper part
+      const bool up = lane & o;
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        if (l >= half) break;
+        const bool two = half + l < w;
+        const double mine = up ? (two ? acc[half + l] : 0.0) : acc[l];
+        const double give = up ? acc[l] : (two ? acc[half + l] : 0.0);
+        acc[l] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+      owner += up ? half : 0;
+      cnt = up ? cnt - half : min(cnt, half);
+      w = half;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    }
+  }
+  if (cnt > 0) red[owner] = acc[0];  // lanes with the same owner hold the same sum
+}
+
+// NR rows of q less their part in the range columns of M, and the squares of the result.
+template <int NR>
+__device__ __forceinline__ void gs_update(const double *__restrict__ M, const double *h, int range, int64_t n,
+                                          double *qi, int64_t i, double &nacc) {
+  double s[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) s[r] = 0.0;
+  const double *m = M + i;
+#pragma unroll 2
+  for (int l = 0; l < range; ++l, m += n)
+#pragma unroll
+    for (int r = 0; r < NR; ++r) s[r] = fma(m[r * kGsThreads], h[l], s[r]);
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const double v = qi[r * kGsThreads] - s[r];
+    qi[r * kGsThreads] = v;
+    nacc = fma(v, v, nacc);
+  }
+}
+
+// STAGED: the CTA's rows of the new columns stay in shared memory (the passes over them are then
+// chains of 30-clock instead of 700-clock loads).  24 molecules of v 4..32, c 32..256, 7 new
+// columns: 168 us from memory with eight predicated columns per pass, 85 us with counted ones,
+// 68 us staged.
+template <bool STAGED>
+__global__ void __cluster_dims__(kGsCluster, 1, 1) __launch_bounds__(kGsThreads, STAGED ? 1 : 8)
     gs_kernel(const __grid_constant__ Group<GsJob> g) {
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank();
@@ -270,31 +405,34 @@ __global__ void __cluster_dims__(kGsCluster, 1, 1) __launch_bounds__(kGsThreads,
   __shared__ double part[2][kReg];  // this CTA's published partial sums
   __shared__ double nrm;
   const int64_t per = (q.n + kGsCluster - 1) / kGsCluster;
-  const int64_t r0 = min(q.n, (int64_t)rank * per), r1 = min(q.n, r0 + per);
-  const double *M = q.Q + q.nstart * q.n;
+  const int64_t f0 = min(q.n, (int64_t)rank * per), f1 = min(q.n, f0 + per);
+  extern __shared__ double staged[];
+  const int64_t r0 = 0, r1 = f1 - f0, ld = STAGED ? per : q.n;  // rows of this CTA
+  double *Mw = STAGED ? staged : q.Q + q.nstart * q.n + f0;
+  if constexpr (STAGED) {
+    for (int64_t j = q.nstart; j < q.ncols; ++j)
+#pragma unroll 4
+      for (int64_t i = threadIdx.x; i < r1; i += kGsThreads) staged[(j - q.nstart) * per + i] = q.Q[j * q.n + f0 + i];
+  }
+  const double *M = Mw;
   int buf = 0;
-  for (int64_t j = q.nstart + 1; j < q.ncols; ++j) {
+  for (int64_t j = q.nstart + 1; j < q.ncols; ++j) {  // every thread works on its own rows throughout
     const int64_t range = j - q.nstart;
-    double *qj = q.Q + j * q.n;
+    double *qj = Mw + range * ld;
     // h = M[:, :range]^T q_j: every thread sums its rows for kReg columns at once (the
     // loads are independent, so they overlap), then one reduction per kReg columns
     for (int64_t l0 = 0; l0 < range; l0 += kReg) {
       const int lc = (int)min((int64_t)kReg, range - l0);
-      double acc[kReg];
-#pragma unroll
-      for (int l = 0; l < kReg; ++l) acc[l] = 0.0;
-#pragma unroll 4
-      for (int64_t i = r0 + threadIdx.x; i < r1; i += kGsThreads) {
-        const double x = qj[i];
-#pragma unroll
-        for (int l = 0; l < kReg; ++l)
-          if (l < lc) acc[l] = fma(M[(l0 + l) * q.n + i], x, acc[l]);
-      }
-#pragma unroll
-      for (int l = 0; l < kReg; ++l) {
-        double v = acc[l];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[warp][l] = v;
+      const double *Ml = M + l0 * ld;
+      switch (lc) {
+        case 1: gs_dots<1>(Ml, qj, ld, r0, r1, red[warp]); break;
+        case 2: gs_dots<2>(Ml, qj, ld, r0, r1, red[warp]); break;
+        case 3: gs_dots<3>(Ml, qj, ld, r0, r1, red[warp]); break;
+        case 4: gs_dots<4>(Ml, qj, ld, r0, r1, red[warp]); break;
+        case 5: gs_dots<5>(Ml, qj, ld, r0, r1, red[warp]); break;
+        case 6: gs_dots<6>(Ml, qj, ld, r0, r1, red[warp]); break;
+        case 7: gs_dots<7>(Ml, qj, ld, r0, r1, red[warp]); break;
+        default: gs_dots<8>(Ml, qj, ld, r0, r1, red[warp]); break;
       }
       __syncthreads();
       if (threadIdx.x < lc) {
@@ -312,13 +450,13 @@ __global__ void __cluster_dims__(kGsCluster, 1, 1) __launch_bounds__(kGsThreads,
       __syncthreads();
     }
     double nacc = 0.0;
-#pragma unroll 4
-    for (int64_t i = r0 + threadIdx.x; i < r1; i += kGsThreads) {
-      double s = 0.0;
-      for (int64_t l = 0; l < range; ++l) s = fma(M[l * q.n + i], h[l], s);
-      const double v = qj[i] - s;
-      qj[i] = v;
-      nacc = fma(v, v, nacc);
+    // four rows at a time: their loads and FMA chains overlap
+    for (int64_t i0 = r0 + threadIdx.x; i0 < r1; i0 += 4 * kGsThreads) {
+      const int nr = (int)min((int64_t)4, (r1 - i0 + kGsThreads - 1) / kGsThreads);
+      if (nr == 4) gs_update<4>(M, h, (int)range, ld, qj + i0, i0, nacc);
+      else if (nr == 3) gs_update<3>(M, h, (int)range, ld, qj + i0, i0, nacc);
+      else if (nr == 2) gs_update<2>(M, h, (int)range, ld, qj + i0, i0, nacc);
+      else gs_update<1>(M, h, (int)range, ld, qj + i0, i0, nacc);
     }
     for (int o = 16; o > 0; o >>= 1) nacc += __shfl_down_sync(0xffffffffu, nacc, o);
     if (lane == 0) red[warp][0] = nacc;
@@ -342,6 +480,10 @@ __global__ void __cluster_dims__(kGsCluster, 1, 1) __launch_bounds__(kGsThreads,
     if (iv > 0.0) {  // Eigen's normalize leaves a zero column unchanged
 #pragma unroll 4
       for (int64_t i = r0 + threadIdx.x; i < r1; i += kGsThreads) qj[i] *= iv;
+    }
+    if constexpr (STAGED) {
+#pragma unroll 4
+      for (int64_t i = threadIdx.x; i < r1; i += kGsThreads) q.Q[j * q.n + f0 + i] = qj[i];
     }
     __syncthreads();
   }
@@ -376,26 +518,26 @@ __global__ void mirror_kernel(const __grid_constant__ Group<MirrorJob> g) {
   const int64_t total = q.c0 * q.nc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = t % q.c0, c = t / q.c0;
+    const int64_t c = (int64_t)((uint32_t)t / (uint32_t)q.c0), r = t - c * q.c0;  // far below 2^32 elements
     q.T[(q.c0 + c) + q.ldt * r] = q.T[r + q.ldt * (q.c0 + c)];
   }
 }
 
-template <class Job, class Kernel>
+template <class Job, class Kernel, class... Args>
 void launch_jobs(const std::vector<Job> &jobs, Kernel kernel, unsigned bx, bool grid_x_is_job,
-                 cudaStream_t s, int threads = kThreads) {
+                 cudaStream_t s, int threads = kThreads, Args... args) {
   std::unique_ptr<Group<Job>> g(new Group<Job>());
   for (size_t i = 0; i < jobs.size();) {
     g->n = 0;
     for (; i < jobs.size() && g->n < kJobs; ++i) g->j[g->n++] = jobs[i];
     // grid_x_is_job: bx consecutive CTAs (a cluster) per job along x
     const dim3 grid = grid_x_is_job ? dim3((unsigned)g->n * bx) : dim3(bx, (unsigned)g->n);
-    kernel<<<grid, threads, 0, s>>>(*g);
+    kernel<<<grid, threads, 0, s>>>(*g, args...);
     VGB_LAUNCH_CHECK();
   }
 }
 
-unsigned rows_blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kThreads), 16)); }
+unsigned rows_blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kThreads), 64)); }
 
 struct Mol {
   BseOperator *op = nullptr;
@@ -409,7 +551,7 @@ struct Mol {
   std::vector<int64_t> upd;
   std::vector<double> upd_lam;
   // device (views into the pool)
-  double *V, *AV, *D, *q, *res, *Ud, *lamd, *cbuf, *norms0, *norms, *inorms, *h, *part, *Td, *eigw;
+  double *V, *AV, *D, *q, *res, *Ud, *lamd, *cbuf, *norms0, *norms, *h, *part, *Td, *eigw;
   int *flag, *einfo;
   // packed host transfer offsets (doubles): off_in = [U (capc x needmax) | lambdas (needmax) |
   // correction columns (capc) | their lambdas (capc)] in din/hin; off_out in hout (diagonal);
@@ -450,9 +592,14 @@ void run_tn(const std::vector<TnReq> &reqs, cudaStream_t s) {
       red.push_back(t);
     }
   }
-  int64_t maxchunks = 1;
-  for (const TnJob &j : jobs) maxchunks = std::max(maxchunks, ceil_div(j.n, (int64_t)kTnRows));
-  launch_jobs(jobs, tn_partial_kernel, (unsigned)maxchunks, false, s);
+  int64_t maxchunks = 1, total = 0;
+  for (const TnJob &j : jobs) {
+    maxchunks = std::max(maxchunks, ceil_div(j.n, (int64_t)kTnRows));
+    total += ceil_div(j.n, (int64_t)kTnRows);
+  }
+  // about four CTAs per SM
+  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(4, 4LL * sm_count() / std::max<int64_t>(1, total)));
+  launch_jobs(jobs, tn_partial_kernel, (unsigned)(maxchunks * parts), false, s, kThreads, parts);
   launch_jobs(red, tn_reduce_kernel, 4, false, s);
 }
 
@@ -478,11 +625,9 @@ void run_nn(const std::vector<NnJob> &jobs, cudaStream_t s) {
     }
     mx = std::max(mx, j.n);
   }
-  launch_jobs(bucket[0], nn_kernel<1>, rows_blocks(mx), false, s);
-  launch_jobs(bucket[1], nn_kernel<2>, rows_blocks(mx), false, s);
-  launch_jobs(bucket[2], nn_kernel<4>, rows_blocks(mx), false, s);
-  launch_jobs(bucket[3], nn_kernel<8>, rows_blocks(mx), false, s);
-  launch_jobs(bucket[4], nn_kernel<16>, rows_blocks(mx), false, s);
+  std::vector<NnJob> all;  // the widest, longest blocks first
+  for (int b = 4; b >= 0; --b) all.insert(all.end(), bucket[b].begin(), bucket[b].end());
+  launch_jobs(all, nn_kernel, rows_blocks(mx), false, s);
 }
 
 void run_norms(const std::vector<NormJob> &jobs, cudaStream_t s) {
@@ -495,6 +640,30 @@ void run_cols(const std::vector<ColJob> &jobs, cudaStream_t s) {
   int64_t mx = 1;
   for (const ColJob &j : jobs) mx = std::max(mx, j.n * j.p);
   launch_jobs(jobs, col_kernel, rows_blocks(mx), false, s);
+}
+
+// Staged where the columns of every molecule fit and the clusters leave the SMs room for them (more
+// CTAs than that share an SM's FP64 pipe, which hides the loads).
+constexpr int kGsStaged = 200 * 1024;
+void run_gs(const std::vector<GsJob> &jobs, cudaStream_t s) {
+  int64_t bytes = 0;
+  for (const GsJob &j : jobs)
+    bytes = std::max<int64_t>(bytes, ceil_div(j.n, (int64_t)kGsCluster) * (j.ncols - j.nstart) * (int64_t)sizeof(double));
+  if (bytes > kGsStaged || (int64_t)jobs.size() * kGsCluster * (bytes + 4096) > (int64_t)sm_count() * kGsStaged) {
+    launch_jobs(jobs, gs_kernel<false>, kGsCluster, true, s, kGsThreads);
+    return;
+  }
+  static std::once_flag attr;
+  std::call_once(attr, [] {
+    VGB_CUDA(cudaFuncSetAttribute(gs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGsStaged));
+  });
+  std::unique_ptr<Group<GsJob>> g(new Group<GsJob>());
+  for (size_t i = 0; i < jobs.size();) {
+    g->n = 0;
+    for (; i < jobs.size() && g->n < kJobs; ++i) g->j[g->n++] = jobs[i];
+    gs_kernel<true><<<(unsigned)g->n * kGsCluster, kGsThreads, (size_t)bytes, s>>>(*g);
+    VGB_LAUNCH_CHECK();
+  }
 }
 
 // Parallel loop over molecules on host threads: a pool of workers kept for the process (starting
@@ -642,7 +811,7 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
     M.needmax = std::min(M.capc, std::max(M.restart_size, M.size_update));
     M.chunks = ceil_div(M.n, (int64_t)kTnRows);
     M.evals.assign(neigen, 0.0);
-    pool_doubles += 2 * M.n * M.capc + 2 * M.n * M.needmax + 4 * M.capc + M.capc * M.capc +
+    pool_doubles += 2 * M.n * M.capc + 2 * M.n * M.needmax + 3 * M.capc + M.capc * M.capc +
                     M.chunks * M.capc * M.capc + 64;
     // projected matrix, Ritz coefficients and values, eigensolver scratch (device)
     pool_doubles += M.capc * M.capc + M.capc * M.needmax + M.needmax + sym_eig_work_doubles(M.capc, M.needmax) + 64;
@@ -668,7 +837,6 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
       M.res = take(M.n * M.needmax);
       M.norms0 = take(M.capc);
       M.norms = take(M.capc);
-      M.inorms = take(M.capc);
       M.h = take(M.capc + M.capc * M.capc);
       M.part = take(M.chunks * M.capc * M.capc);
       p += 64;
@@ -836,7 +1004,6 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
     // ---- Ritz vectors q = V U, residuals res = AV U - q Lambda, their norms ----
     {
       std::vector<NnJob> nn;
-      std::vector<ColJob> cj;
       std::vector<NormJob> nj;
       std::vector<ColJob> lc;
       const int64_t packed =
@@ -847,13 +1014,10 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
         const int64_t pr = std::min(M->needed, M->size_update);
         nn.push_back({M->V, M->Ud, M->n, M->m, M->n, M->m, pr, M->q, M->n, 1.0, 0.0});
         nn.push_back({M->AV, M->Ud, M->n, M->m, M->n, M->m, pr, M->res, M->n, 1.0, 0.0});
-        ColJob c;
-        c.kind = 1; c.A = M->res; c.B = M->q; c.D = nullptr; c.v = M->lamd; c.cols = nullptr;
-        c.lda = M->n; c.ldb = M->n; c.n = M->n; c.p = pr;
-        cj.push_back(c);
         NormJob w;
         w.A = M->res; w.B = nullptr; w.lda = M->n; w.ldb = M->n; w.n = M->n;
-        w.p = std::min(M->needed, M->size_update); w.out = M->cbuf;
+        w.p = pr; w.out = M->cbuf;
+        w.a_out = M->res; w.sub = M->q; w.ldsub = M->n; w.lam = M->lamd;
         nj.push_back(w);
         ColJob l;  // the Ritz values travel behind the norms
         l.kind = 2; l.A = M->cbuf + pr; l.B = M->lamd; l.D = nullptr; l.v = nullptr; l.cols = nullptr;
@@ -861,7 +1025,6 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
         lc.push_back(l);
       }
       run_nn(nn, s);
-      run_cols(cj, s);
       run_norms(nj, s);
       run_cols(lc, s);
       VGB_CUDA(cudaMemcpyAsync(hpack, dpack.get(), packed * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -919,7 +1082,6 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
     {
       std::vector<ColJob> cj;
       std::vector<NormJob> nj;
-      std::vector<ColJob> sc;
       for (Mol *M : ext) {
         ColJob c;
         c.kind = 3; c.A = M->V + M->ncols * M->n; c.B = M->res; c.D = M->D;
@@ -928,16 +1090,11 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
         cj.push_back(c);
         NormJob w;
         w.A = c.A; w.B = nullptr; w.lda = M->n; w.ldb = M->n; w.n = M->n; w.p = M->nupdate; w.out = M->norms;
-        w.inv = M->inorms;
+        w.a_out = c.A; w.scale = true;
         nj.push_back(w);
-        ColJob z;
-        z.kind = 0; z.A = c.A; z.B = nullptr; z.D = nullptr; z.v = M->inorms; z.cols = nullptr;
-        z.lda = M->n; z.ldb = M->n; z.n = M->n; z.p = M->nupdate;
-        sc.push_back(z);
       }
       run_cols(cj, s);
       run_norms(nj, s);
-      run_cols(sc, s);
     }
     mark(5);
     // ---- gramschmidt on the new columns (two passes) ----
@@ -954,7 +1111,6 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
         std::vector<TnReq> tn;
         std::vector<NnJob> nn;
         std::vector<NormJob> nj;
-        std::vector<ColJob> sc;
         std::vector<GsJob> gs;
         for (Mol *M : ext) {
           double *Vn = M->V + M->ncols * M->n;
@@ -962,12 +1118,8 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
           nn.push_back({M->V, M->h, M->n, M->ncols, M->n, M->ncols, M->nupdate, Vn, M->n, -1.0, 1.0});
           NormJob w;
           w.A = Vn; w.B = nullptr; w.lda = M->n; w.ldb = M->n; w.n = M->n; w.p = M->nupdate; w.out = M->norms;
-          w.inv = M->inorms;
+          w.a_out = Vn; w.scale = true;
           nj.push_back(w);
-          ColJob z;
-          z.kind = 0; z.A = Vn; z.B = nullptr; z.D = nullptr; z.v = M->inorms; z.cols = nullptr;
-          z.lda = M->n; z.ldb = M->n; z.n = M->n; z.p = M->nupdate;
-          sc.push_back(z);
           if (M->nupdate > 1) {
             VGB_REQUIRE(M->nupdate <= 256, "batched Davidson: too many new columns");
             GsJob gj;
@@ -979,8 +1131,7 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
         run_tn(tn, s);
         run_nn(nn, s);
         run_norms(nj, s);
-        run_cols(sc, s);
-        launch_jobs(gs, gs_kernel, kGsCluster, true, s, kGsThreads);
+        run_gs(gs, s);
       }
       for (Mol *M : ext) M->ncols += M->nupdate;
     }
