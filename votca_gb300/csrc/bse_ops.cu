@@ -35,9 +35,8 @@ __global__ void scatter_kernel(const ScatterArgs a) {
   const int64_t total = a.m_count * a.naux * nwin;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t nl = t % nwin;
-    const int64_t P = (t / nwin) % a.naux;
-    const int64_t mi = t / (nwin * a.naux);
+    const QuotRem nx = quot_rem(t, nwin), px = quot_rem(nx.q, a.naux);
+    const int64_t nl = nx.r, P = px.r, mi = px.q;
     const int64_t ml = a.m_first + mi;
     const int64_t row = nl < a.vt ? a.n_v0 + nl : a.n_c0 + (nl - a.vt);
     const double val = a.raw[(mi * a.naux + P) * a.nsize + row];
@@ -70,7 +69,8 @@ __global__ void dvv_from_gvv_kernel(const double *Gvv, int64_t naux, int64_t vt,
   const int64_t total = naux * vt;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t v = t % vt, P = t / vt;
+    const QuotRem x = quot_rem(t, vt);
+    const int64_t v = x.r, P = x.q;
     dvv[P * vt + v] = Gvv[(v * naux + P) * vt + v];
   }
 }
@@ -82,8 +82,8 @@ __global__ void hqp_diag_kernel(double cqp, const double *__restrict__ Hcc,
   const int64_t dim = vt * ct, total = dim * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t I = t % dim, j = t / dim;
-    const int64_t v = I / ct, c = I % ct;
+    const QuotRem tx = quot_rem(t, dim), ix = quot_rem(tx.r, ct);
+    const int64_t I = tx.r, j = tx.q, v = ix.q, c = ix.r;
     const double e = Hcc[c + ct * c] - Hvv[v + vt * v];
     const double val = cqp * e * X[I + ldx * j];
     double *y = Y + I + ldy * j;
@@ -114,8 +114,8 @@ __global__ void hqp_diag_group_kernel(const __grid_constant__ HqpGroup g) {
   const int64_t dim = q.vt * q.ct, total = dim * q.k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t I = t % dim, j = t / dim;
-    const int64_t v = I / q.ct, c = I % q.ct;
+    const QuotRem tx = quot_rem(t, dim), ix = quot_rem(tx.r, q.ct);
+    const int64_t I = tx.r, j = tx.q, v = ix.q, c = ix.r;
     const double e = q.diag ? q.diag[I] : q.cqp * (q.Hcc[c + q.ct * c] - q.Hvv[v + q.vt * v]);
     const double val = e * q.X[I + q.ldx * j];
     double *y = q.Y + I + q.ldy * j;
@@ -126,8 +126,10 @@ __global__ void hqp_diag_group_kernel(const __grid_constant__ HqpGroup g) {
 __global__ void zero_cols_kernel(double *Y, int64_t ldy, int64_t rows, int64_t k) {
   const int64_t total = rows * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x)
-    Y[(t % rows) + ldy * (t / rows)] = 0.0;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const QuotRem x = quot_rem(t, rows);
+    Y[x.r + ldy * x.q] = 0.0;
+  }
 }
 
 struct DiagArgs {
@@ -156,7 +158,8 @@ __device__ __forceinline__ double strided_dot(const double *x, int64_t sx, const
 // BSE_OPERATOR::diagonal (bse_operator.cc:133-175), one thread per pair.
 __device__ __forceinline__ void diagonal_range(const DiagArgs &a, int64_t I0, int64_t step) {
   for (int64_t I = I0; I < a.dim; I += step) {
-    const int64_t v = I / a.ct, c = I % a.ct;
+    const QuotRem ix = quot_rem(I, a.ct);
+    const int64_t v = ix.q, c = ix.r;
     double entry = 0.0;
     if (a.cx != 0.0) entry += a.cx * strided_dot(a.Bvc + I, a.dim, a.Bvc + I, a.dim, a.naux);
     if (a.cqp != 0.0) entry += a.cqp * (a.Hcc[c + a.ct * c] - a.Hvv[v + a.vt * v]);
@@ -178,7 +181,8 @@ __global__ void __launch_bounds__(32 * kDiagSlices) diagonal_kernel(const DiagAr
     const int64_t I = I0 + lane;
     double sx0 = 0.0, sx1 = 0.0, sd0 = 0.0, sd1 = 0.0, s20 = 0.0, s21 = 0.0;
     if (I < a.dim) {
-      const int64_t v = I / a.ct, c = I % a.ct;
+      const QuotRem ix = quot_rem(I, a.ct);
+      const int64_t v = ix.q, c = ix.r;
       int64_t P = w;
       for (; P + kDiagSlices < a.naux; P += 2 * kDiagSlices) {
         const int64_t P1 = P + kDiagSlices;
@@ -211,7 +215,8 @@ __global__ void __launch_bounds__(32 * kDiagSlices) diagonal_kernel(const DiagAr
       double entry = 0.0;
 #pragma unroll
       for (int q = 0; q < kDiagSlices; ++q) entry += part[q][lane];
-      const int64_t v = I / a.ct, c = I % a.ct;
+      const QuotRem ix = quot_rem(I, a.ct);
+      const int64_t v = ix.q, c = ix.r;
       if (a.cqp != 0.0) entry += a.cqp * (a.Hcc[c + a.ct * c] - a.Hvv[v + a.vt * v]);
       a.D[I] = entry;
     }
@@ -236,7 +241,8 @@ __global__ void ham_combine_kernel(const double *__restrict__ TA, const double *
   const int64_t total = dim * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t q = t % dim, j = t / dim;
+    const QuotRem x = quot_rem(t, dim);
+    const int64_t q = x.r, j = x.q;
     const double a_top = TA[(2 * j) * dim + q], a_bot = TA[(2 * j + 1) * dim + q];
     const double b_top = TB[(2 * j) * dim + q], b_bot = TB[(2 * j + 1) * dim + q];
     Y[q + ldy * j] = a_top + b_bot;
@@ -256,8 +262,10 @@ __global__ void copy_cols_kernel(const double *X, int64_t ldx, int64_t rows, int
                                  int64_t ldy) {
   const int64_t total = rows * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x)
-    Y[(t % rows) + ldy * (t / rows)] = X[(t % rows) + ldx * (t / rows)];
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const QuotRem x = quot_rem(t, rows);
+    Y[x.r + ldy * x.q] = X[x.r + ldx * x.q];
+  }
 }
 
 unsigned grid_for(int64_t n, int threads = 256) {

@@ -118,4 +118,19 @@ void aux_pseudo_inv_sqrt(int64_t n, const double *V, int64_t ldv, double etol, d
 void aux_pseudo_inv_sqrt_gwbse(int64_t n, const double *S, int64_t lds, const double *V, int64_t ldv,
                                double etol, double *out, int64_t ldo, int64_t *removed, cudaStream_t s);
 
+#ifdef __CUDACC__
+// Quotient and remainder of indices, in 32 bits where they fit: a 64-bit division converts through
+// the FP64 pipe, where an instruction holds its SM quarter for 64 clocks.
+struct QuotRem {
+  int64_t q, r;
+};
+__device__ __forceinline__ QuotRem quot_rem(int64_t a, int64_t b) {
+  if (((uint64_t)(a | b) >> 32) == 0) {
+    const uint32_t x = (uint32_t)a, d = (uint32_t)b, q = x / d;
+    return {(int64_t)q, (int64_t)(x - q * d)};
+  }
+  return {a / b, a % b};
+}
+#endif
+
 }  // namespace vgb

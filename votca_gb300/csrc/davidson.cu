@@ -31,10 +31,12 @@ unsigned blocks_for(int64_t n, int threads = 256) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, threads), 16LL * 152));
 }
 
-// partial[c * kRedChunks + b] = sum over chunk b of A[:, c] * B[:, c]
-__global__ void coldot_partial_kernel(const double *__restrict__ A, int64_t lda,
-                                      const double *__restrict__ B, int64_t ldb, int64_t n,
-                                      double *__restrict__ partial) {
+// out[c] = sum of A[:, c] * B[:, c] (its root with take_sqrt): the sums of kRedChunks chunks of rows,
+// one per block, are added in chunk order by the column's last block.  arrived[c] counts the
+// column's blocks and is back at zero afterwards.
+__global__ void coldot_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ B, int64_t ldb,
+                              int64_t n, double *__restrict__ partial, unsigned *arrived, int take_sqrt,
+                              double *__restrict__ out) {
   const int64_t c = blockIdx.y;
   const int64_t chunk = ceil_div(n, kRedChunks);
   const int64_t r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
@@ -42,22 +44,30 @@ __global__ void coldot_partial_kernel(const double *__restrict__ A, int64_t lda,
   double s = 0.0;
   for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) s = fma(a[r], b[r], s);
   __shared__ double red[256];
+  __shared__ bool last;
   red[threadIdx.x] = s;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[c * kRedChunks + blockIdx.x] = red[0];
-}
-
-__global__ void coldot_final_kernel(const double *__restrict__ partial, int64_t ncols, int take_sqrt,
-                                    double *__restrict__ out) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncols;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < kRedChunks; ++b) s += partial[c * kRedChunks + b];
-    out[c] = take_sqrt ? sqrt(s) : s;
+  if (threadIdx.x == 0) {
+    __stcg(partial + c * kRedChunks + blockIdx.x, red[0]);
+    __threadfence();
+    last = atomicInc(arrived + c, kRedChunks - 1) == kRedChunks - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x < kRedChunks) {
+    __threadfence();
+    red[threadIdx.x] = __ldcg(partial + c * kRedChunks + threadIdx.x);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < kRedChunks; ++k) t += red[k];
+    out[c] = take_sqrt ? sqrt(t) : t;
   }
 }
 
@@ -73,7 +83,7 @@ __global__ void residual_kernel(double *__restrict__ res, const double *__restri
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = t / n;
+    const int64_t j = quot_rem(t, n).q;
     res[t] -= lam[j] * q[t];
   }
 }
@@ -88,7 +98,8 @@ __global__ void dpr_kernel(double *__restrict__ out, int64_t ldo, const double *
   const int64_t total = n * count;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % n, kk = t / n;
+    const QuotRem x = quot_rem(t, n);
+    const int64_t i = x.r, kk = x.q;
     const int64_t j = cols[kk];
     const double den = D[i] - lams[kk];
     double v = -res[j * n + i] / den;
@@ -106,7 +117,8 @@ __global__ void olsen_finish_kernel(double *__restrict__ out, int64_t ldo,
   const int64_t total = n * count;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % n, kk = t / n;
+    const QuotRem x = quot_rem(t, n);
+    const int64_t i = x.r, kk = x.q;
     const double eps = (-num[kk]) / (-den[kk]);
     double v = out[kk * ldo + i] + eps * q[cols[kk] * n + i];
     if (!isfinite(v)) v = 0.0;
@@ -120,7 +132,8 @@ __global__ void scale_columns_kernel(double *A, int64_t lda, int64_t n, int64_t 
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % n, c = t / n;
+    const QuotRem x = quot_rem(t, n);
+    const int64_t i = x.r, c = x.q;
     const double nv = norm[c];
     if (nv > 0.0) A[c * lda + i] /= nv;
   }
@@ -131,7 +144,8 @@ __global__ void copy_block_kernel(const double *src, int64_t lds, double *dst, i
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % n, c = t / n;
+    const QuotRem x = quot_rem(t, n);
+    const int64_t i = x.r, c = x.q;
     dst[c * ldd + i] = src[c * lds + i];
   }
 }
@@ -142,7 +156,8 @@ __global__ void mirror_block_kernel(double *T, int64_t ldt, int64_t c0, int64_t 
   const int64_t total = c0 * nc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = t % c0, c = t / c0;
+    const QuotRem x = quot_rem(t, c0);
+    const int64_t r = x.r, c = x.q;
     T[(c0 + c) + ldt * r] = T[r + ldt * (c0 + c)];
   }
 }
@@ -271,7 +286,7 @@ struct Ctx {
   // 1e-10 (2e-10 with digit products here, against 4e-13 in an FP64 solve).
   int gemm_path = 0;
   DeviceBuffer<double> red_partial, scal, gs_part;
-  DeviceBuffer<unsigned> gs_bar;
+  DeviceBuffer<unsigned> gs_bar, red_arrived;
   DeviceBuffer<int> gs_err;
 
   // out[c] = ||A[:, c]|| (or dot(A[:, c], B[:, c]) when B given), device
@@ -279,12 +294,13 @@ struct Ctx {
                double *out, bool sqrt_) {
     if (ncols <= 0) return;
     red_partial.resize(ncols * kRedChunks);
+    if ((int64_t)red_arrived.count < ncols) {
+      red_arrived.resize(ncols);
+      VGB_CUDA(cudaMemsetAsync(red_arrived.get(), 0, ncols * sizeof(unsigned), s));
+    }
     dim3 grid(kRedChunks, (unsigned)ncols);
-    coldot_partial_kernel<<<grid, 256, 0, s>>>(A, lda, B ? B : A, B ? ldb : lda, n,
-                                               red_partial.get());
-    VGB_LAUNCH_CHECK();
-    coldot_final_kernel<<<blocks_for(ncols, 128), 128, 0, s>>>(red_partial.get(), ncols,
-                                                               sqrt_ ? 1 : 0, out);
+    coldot_kernel<<<grid, 256, 0, s>>>(A, lda, B ? B : A, B ? ldb : lda, n, red_partial.get(), red_arrived.get(),
+                                       sqrt_ ? 1 : 0, out);
     VGB_LAUNCH_CHECK();
   }
   void scale_cols(double *A, int64_t lda, int64_t ncols, const double *norms) {

@@ -32,14 +32,15 @@ __global__ void __launch_bounds__(THREADS)
   __shared__ double Bs[2][TK][TN + 1];
 
   // flat block index -> (split, batch, n-tile, m-tile)
-  int64_t bid = blockIdx.x;
-  const int64_t mtile = bid % g.mt;
-  bid /= g.mt;
-  const int64_t ntile = bid % g.nt;
-  bid /= g.nt;
-  const int64_t s = bid % g.splits;
-  const int64_t batch = bid / g.splits;
-  const int64_t b1 = batch / d.nb2, b2 = batch % d.nb2;
+  const int64_t bid = blockIdx.x;
+  QuotRem x = quot_rem(bid, g.mt);
+  const int64_t mtile = x.r;
+  x = quot_rem(x.q, g.nt);
+  const int64_t ntile = x.r;
+  x = quot_rem(x.q, g.splits);
+  const int64_t s = x.r, batch = x.q;
+  x = quot_rem(batch, d.nb2);
+  const int64_t b1 = x.q, b2 = x.r;
 
   const double *__restrict__ A = d.A + b1 * d.a_b1 + b2 * d.a_b2;
   const double *__restrict__ B = d.B + b1 * d.b_b1 + b2 * d.b_b2;
@@ -138,13 +139,14 @@ __global__ void splitk_reduce_kernel(const GemmDesc d, const Grid g,
   const int64_t total = mn * g.nbatch;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t batch = t / mn, e = t % mn;
-    const int64_t i = e % d.M, n = e / d.M;
-    const double *p = partial + batch * g.splits * mn + e;
+    const QuotRem tx = quot_rem(t, mn), ex = quot_rem(tx.r, d.M);
+    const int64_t batch = tx.q, i = ex.r, n = ex.q;
+    const double *p = partial + batch * g.splits * mn + tx.r;
     double acc = 0.0;
 #pragma unroll 8
     for (int64_t s = 0; s < g.splits; ++s) acc += p[s * mn];  // in split order; the loads overlap
-    const int64_t b1 = batch / d.nb2, b2 = batch % d.nb2;
+    const QuotRem bx = quot_rem(batch, d.nb2);
+    const int64_t b1 = bx.q, b2 = bx.r;
     double *c = d.C + b1 * d.c_b1 + b2 * d.c_b2 + i * d.c_rs + n * d.c_cs;
     const double v = d.alpha * acc;
     *c = (d.beta == 0.0) ? v : fma(d.beta, *c, v);
@@ -155,9 +157,10 @@ __global__ void scale_kernel(const GemmDesc d, int64_t nbatch) {
   const int64_t mn = d.M * d.N, total = mn * nbatch;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t batch = t / mn, e = t % mn;
-    const int64_t i = e % d.M, n = e / d.M;
-    const int64_t b1 = batch / d.nb2, b2 = batch % d.nb2;
+    const QuotRem tx = quot_rem(t, mn), ex = quot_rem(tx.r, d.M);
+    const int64_t batch = tx.q, i = ex.r, n = ex.q;
+    const QuotRem bx = quot_rem(batch, d.nb2);
+    const int64_t b1 = bx.q, b2 = bx.r;
     double *c = d.C + b1 * d.c_b1 + b2 * d.c_b2 + i * d.c_rs + n * d.c_cs;
     *c = (d.beta == 0.0) ? 0.0 : d.beta * *c;
   }

@@ -664,12 +664,13 @@ __global__ void oz_reduce_kernel(const double *__restrict__ part, int64_t M, int
                                  double alpha, double beta) {
   const int64_t mn = M * N, total = mn * nbt;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = t / mn, e = t % mn;
+    const QuotRem tx = quot_rem(t, mn), ex = quot_rem(tx.r, M);
+    const int64_t b = tx.q, e = tx.r;
     const double *q = part + b * splits * mn + e;
     double acc = 0.0;
 #pragma unroll 4
     for (int s = 0; s < splits; ++s) acc += q[s * mn];
-    double *c = C + cbatch.at(b) + crow.at(e % M) + ccol.at(e / M);
+    double *c = C + cbatch.at(b) + crow.at(ex.r) + ccol.at(ex.q);
     const double v = alpha * acc;
     *c = beta == 0.0 ? v : fma(beta, *c, v);
   }

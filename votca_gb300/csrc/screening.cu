@@ -33,7 +33,8 @@ __global__ void rpa_chi_kernel(const double *energies, int64_t n_occ_chunk, int6
   const int64_t total = n_occ_chunk * n_unocc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = t % n_unocc, mi = t / n_unocc;
+    const QuotRem x = quot_rem(t, n_unocc);
+    const int64_t c = x.r, mi = x.q;
     const double dE = energies[lumo_idx + c] - energies[m0 + mi];
     const double dm = wr - dE, dp = wr + dE;
     const double s1 = (wi + eta) * (wi + eta), s2 = (wi - eta) * (wi - eta);
@@ -48,7 +49,8 @@ __global__ void rpa_chi_kernel(const double *energies, int64_t n_occ_chunk, int6
 __global__ void rpa_weights_kernel(const double *raw, int64_t n_unocc, int64_t naux, int64_t nsize, int64_t row0,
                                    const double *chi2, double *B, double *Bw, int64_t ldb, int64_t rows) {
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {  // r = mi * naux + P
-    const int64_t mi = r / naux, P = r - mi * naux;
+    const QuotRem x = quot_rem(r, naux);
+    const int64_t mi = x.q, P = x.r;
     const double *src = raw + r * nsize + row0, *w = chi2 + mi * n_unocc;
     double *b = B + mi * n_unocc + ldb * P, *bw = Bw + mi * n_unocc + ldb * P;
     for (int64_t c = threadIdx.x; c < n_unocc; c += blockDim.x) {

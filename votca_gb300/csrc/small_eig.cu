@@ -179,8 +179,9 @@ __device__ void scale_singles(double *Z, int64_t ldz, int64_t m, const int *cl, 
                               const double *f) {
   const int64_t n = min((int64_t)kEigThreads, ncl - cb);
   for (int64_t t = threadIdx.x; t < m * n; t += kEigThreads) {
-    const int64_t c = cb + t / m;
-    if (cl[c + 1] - cl[c] == 1) Z[t % m + ldz * cl[c]] *= f[c - cb];
+    const QuotRem x = quot_rem(t, m);
+    const int64_t c = cb + x.q;
+    if (cl[c + 1] - cl[c] == 1) Z[x.r + ldz * cl[c]] *= f[c - cb];
   }
 }
 // d - sigma into the first m of each one's 5 m scratch doubles
@@ -188,7 +189,8 @@ __device__ void shift_singles(const double *d, int64_t m, const int *cl, int64_t
                               const double *sigma, double *scratch) {
   const int64_t n = min((int64_t)kEigThreads, ncl - cb);
   for (int64_t t = threadIdx.x; t < m * n; t += kEigThreads) {
-    const int64_t c = cb + t / m, i = t % m;
+    const QuotRem x = quot_rem(t, m);
+    const int64_t c = cb + x.q, i = x.r;
     if (cl[c + 1] - cl[c] == 1) scratch[5 * m * cl[c] + i] = d[i] - sigma[c - cb];
   }
 }
@@ -197,7 +199,8 @@ __device__ void tri_apply_singles(const double *d, const double *e, const double
                                   const int *cl, int64_t cb, int64_t ncl, double *scratch) {
   const int64_t n = min((int64_t)kEigThreads, ncl - cb);
   for (int64_t t = threadIdx.x; t < m * n; t += kEigThreads) {
-    const int64_t c = cb + t / m, i = t % m;
+    const QuotRem x = quot_rem(t, m);
+    const int64_t c = cb + x.q, i = x.r;
     if (cl[c + 1] - cl[c] != 1) continue;
     const double *z = Z + ldz * cl[c];
     double y = d[i] * z[i];
@@ -241,7 +244,8 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   if (tid == 0 && q.clocks) q.clocks[0] = clock64();
   // ---- load the lower triangle ----
   for (int64_t t = tid; t < m * m; t += kEigThreads) {
-    const int64_t j = t / m, i = t % m;
+    const QuotRem x = quot_rem(t, m);
+    const int64_t j = x.q, i = x.r;
     if (i >= j) A[i + ld * j] = q.T[i + q.ldt * j];
   }
   __syncthreads();
@@ -431,7 +435,10 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
       double *r0 = w, *u1 = w + m, *u2 = w + 2 * m, *l = w + 3 * m, *pv = w + 4 * m;
       const int64_t jb0 = cl[cb], jb1 = cl[min((int64_t)ncl, cb + kEigThreads)];  // vectors of this batch
       const int64_t nel = m * (jb1 - jb0);
-      for (int64_t t = tid; t < nel; t += kEigThreads) Z[t % m + ldz * (jb0 + t / m)] = start_value(t % m, jb0 + t / m);
+      for (int64_t t = tid; t < nel; t += kEigThreads) {
+        const QuotRem x = quot_rem(t, m);
+        Z[x.r + ldz * (jb0 + x.q)] = start_value(x.r, jb0 + x.q);
+      }
       __syncthreads();
       double sigma = single ? (double)lam32[j] : 0.0;
       for (int half = 0; half < 2; ++half) {
@@ -593,7 +600,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   } else {
     double *part = scl;
     double *fac = vv;  // one factor per vector of a batch (vv and pp are free)
-    const int G = (int)std::min<int64_t>(32, std::max<int64_t>(1, kEigThreads / nw));
+    const int G = min(32, max(1, kEigThreads / (int)nw));
     const int per_batch = kEigThreads / G;
     const int slot = tid / G, sub = tid % G;
     for (int64_t j0 = 0; j0 < nw; j0 += per_batch) {
@@ -624,7 +631,10 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   }
   __syncthreads();
   if (z_sm)
-    for (int64_t t = tid; t < m * nw; t += kEigThreads) q.U[(t % m) + q.ldu * (t / m)] = Z[t];
+    for (int64_t t = tid; t < m * nw; t += kEigThreads) {
+      const QuotRem x = quot_rem(t, m);
+      q.U[x.r + q.ldu * x.q] = Z[t];
+    }
   if (tid == 0 && q.clocks) q.clocks[4] = clock64();
   if (tid == 0 && q.info) *q.info = 0;
 }

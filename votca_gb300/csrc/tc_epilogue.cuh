@@ -7,19 +7,6 @@
 
 namespace vgb {
 
-// Quotient and remainder of indices, in 32 bits where they fit: a 64-bit division converts through
-// the FP64 pipe, where an instruction holds its SM quarter for 64 clocks.
-struct QuotRem {
-  int64_t q, r;
-};
-__device__ __forceinline__ QuotRem quot_rem(int64_t a, int64_t b) {
-  if (((uint64_t)(a | b) >> 32) == 0) {
-    const uint32_t x = (uint32_t)a, d = (uint32_t)b, q = x / d;
-    return {(int64_t)q, (int64_t)(x - q * d)};
-  }
-  return {a / b, a % b};
-}
-
 // v - float(hi) is exact in FP32 (hi is v rounded to 8 significant bits), so
 // the split costs no FP64 work in the epilogue.
 __device__ __forceinline__ void epi_store(const TcEpilogue &e, int64_t off, float v) {
