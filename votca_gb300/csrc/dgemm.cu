@@ -18,15 +18,26 @@ struct Grid {
   int64_t mt, nt, nbatch, splits, kchunk;
 };
 
+// C = alpha * sum_s p[s mn] + beta * C of one element, in split order (deterministic).
+__device__ __forceinline__ void add_splits(const GemmDesc &d, int64_t b1, int64_t b2, int64_t i, int64_t n,
+                                           const double *p, int64_t mn, int64_t splits) {
+  double acc = 0.0;
+#pragma unroll 8
+  for (int64_t s = 0; s < splits; ++s) acc += __ldcg(p + s * mn);  // the loads overlap
+  double *c = d.C + b1 * d.c_b1 + b2 * d.c_b2 + i * d.c_rs + n * d.c_cs;
+  const double v = d.alpha * acc;
+  *c = (d.beta == 0.0) ? v : fma(d.beta, *c, v);
+}
+
 // TM x TN outputs per 256-thread block, (TM / 16) x (TN / 16) per thread; the next K step's
 // operands are in flight while the current one is multiplied.  The FP64 pipe bounds it: a block
 // of 64 x 64 x 16 products keeps its SM busy for 32768 clocks (17 us), so small products want many
 // small tiles (fma_plan.hpp).  The sum of an output does not depend on the tile: one chain of FMAs
-// in K order per split.
+// in K order per split.  The splits of a 16 x 16 tile are added by the block that finishes last
+// (arrived: one counter per tile, back at zero afterwards) instead of by a launch of 4 us.
 template <int TM, int TN>
 __global__ void __launch_bounds__(THREADS)
-    dgemm_kernel(const GemmDesc d, const Grid g, double *__restrict__ partial, int a_icontig,
-                 int b_lcontig) {
+    dgemm_kernel(const GemmDesc d, const Grid g, double *partial, unsigned *arrived, int a_icontig, int b_lcontig) {
   constexpr int RM = TM / 16, RN = TN / 16;
   __shared__ double As[2][TK][TM + 1];
   __shared__ double Bs[2][TK][TN + 1];
@@ -111,7 +122,7 @@ __global__ void __launch_bounds__(THREADS)
     buf ^= 1;
   }
 
-  double *__restrict__ C = g.splits == 1 ? d.C + b1 * d.c_b1 + b2 * d.c_b2
+  double *C = g.splits == 1 ? d.C + b1 * d.c_b1 + b2 * d.c_b2
                                          : partial + (batch * g.splits + s) * d.M * d.N;
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
@@ -130,26 +141,30 @@ __global__ void __launch_bounds__(THREADS)
       }
     }
   }
+  if constexpr (TM * TN > THREADS) return;
+  if (g.splits == 1 || !arrived) return;
+  // the tile's last block adds its splits
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0)
+    last = atomicInc(arrived + (batch * g.nt + ntile) * g.mt + mtile, (unsigned)g.splits - 1) == (unsigned)g.splits - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int64_t mn = d.M * d.N;
+  const int64_t gi = m0 + tid % TM, gn = n0 + tid / TM;  // lanes along the columns of the partials
+  if (gi < d.M && gn < d.N) add_splits(d, b1, b2, gi, gn, partial + batch * g.splits * mn + gi + gn * d.M, mn, g.splits);
 }
 
-// C = alpha * sum_s partial[s] + beta * C, in a fixed order (deterministic).
-__global__ void splitk_reduce_kernel(const GemmDesc d, const Grid g,
-                                     const double *__restrict__ partial) {
+// The same for all outputs in a launch of its own, for callers without counters.
+__global__ void splitk_reduce_kernel(const GemmDesc d, const Grid g, const double *partial) {
   const int64_t mn = d.M * d.N;
   const int64_t total = mn * g.nbatch;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const QuotRem tx = quot_rem(t, mn), ex = quot_rem(tx.r, d.M);
-    const int64_t batch = tx.q, i = ex.r, n = ex.q;
-    const double *p = partial + batch * g.splits * mn + tx.r;
-    double acc = 0.0;
-#pragma unroll 8
-    for (int64_t s = 0; s < g.splits; ++s) acc += p[s * mn];  // in split order; the loads overlap
-    const QuotRem bx = quot_rem(batch, d.nb2);
-    const int64_t b1 = bx.q, b2 = bx.r;
-    double *c = d.C + b1 * d.c_b1 + b2 * d.c_b2 + i * d.c_rs + n * d.c_cs;
-    const double v = d.alpha * acc;
-    *c = (d.beta == 0.0) ? v : fma(d.beta, *c, v);
+    const QuotRem tx = quot_rem(t, mn), ex = quot_rem(tx.r, d.M), bx = quot_rem(tx.q, d.nb2);
+    add_splits(d, bx.q, bx.r, ex.r, ex.q, partial + tx.q * g.splits * mn + tx.r, mn, g.splits);
   }
 }
 
@@ -167,32 +182,43 @@ __global__ void scale_kernel(const GemmDesc d, int64_t nbatch) {
 }
 
 template <int TM, int TN>
-void launch_tile(const GemmDesc &d, const Grid &g, double *partial, cudaStream_t stream) {
+void launch_tile(const GemmDesc &d, const Grid &g, double *partial, unsigned *arrived, cudaStream_t stream) {
   const int64_t blocks = g.mt * g.nt * g.nbatch * g.splits;
   VGB_REQUIRE(blocks < (1LL << 31), "dgemm: grid too large");
-  dgemm_kernel<TM, TN><<<(unsigned)blocks, THREADS, 0, stream>>>(d, g, partial, d.a_rs == 1 ? 1 : 0,
-                                                                  d.b_rs == 1 ? 1 : 0);
+  dgemm_kernel<TM, TN><<<(unsigned)blocks, THREADS, 0, stream>>>(d, g, partial, arrived,
+                                                                  d.a_rs == 1 ? 1 : 0, d.b_rs == 1 ? 1 : 0);
   VGB_LAUNCH_CHECK();
 }
 
-void launch(const GemmDesc &d, const FmaPlan &f, double *partial, cudaStream_t stream) {
+void launch(const GemmDesc &d, const FmaPlan &f, double *partial, GemmWorkspace *ws, cudaStream_t stream) {
   Grid g;
   g.mt = ceil_div(d.M, f.tm);
   g.nt = ceil_div(d.N, f.tn);
   g.nbatch = d.nb1 * d.nb2;
   g.splits = f.splits;
   g.kchunk = f.kchunk;
-  if (f.tm == 64) {
-    if (f.tn == 64) launch_tile<64, 64>(d, g, partial, stream);
-    else if (f.tn == 32) launch_tile<64, 32>(d, g, partial, stream);
-    else launch_tile<64, 16>(d, g, partial, stream);
-  } else if (f.tm == 32) {
-    if (f.tn == 32) launch_tile<32, 32>(d, g, partial, stream);
-    else launch_tile<32, 16>(d, g, partial, stream);
-  } else {
-    launch_tile<16, 16>(d, g, partial, stream);
+  unsigned *arrived = nullptr;
+  // only the smallest tiles, one output per thread: with two, over 150 splits, the last blocks took
+  // 23 us longer, the launch 13 us
+  if (ws && f.splits > 1 && f.tm == 16) {
+    const int64_t tiles = g.mt * g.nt * g.nbatch;
+    if ((int64_t)ws->arrived.count < tiles) {
+      ws->arrived.resize((size_t)tiles);
+      VGB_CUDA(cudaMemsetAsync(ws->arrived.get(), 0, tiles * sizeof(unsigned), stream));
+    }
+    arrived = ws->arrived.get();
   }
-  if (f.splits > 1) {
+  if (f.tm == 64) {
+    if (f.tn == 64) launch_tile<64, 64>(d, g, partial, arrived, stream);
+    else if (f.tn == 32) launch_tile<64, 32>(d, g, partial, arrived, stream);
+    else launch_tile<64, 16>(d, g, partial, arrived, stream);
+  } else if (f.tm == 32) {
+    if (f.tn == 32) launch_tile<32, 32>(d, g, partial, arrived, stream);
+    else launch_tile<32, 16>(d, g, partial, arrived, stream);
+  } else {
+    launch_tile<16, 16>(d, g, partial, arrived, stream);
+  }
+  if (f.splits > 1 && !arrived) {
     const int64_t total = d.M * d.N * g.nbatch;
     splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0,
                            stream>>>(d, g, partial);
@@ -332,7 +358,7 @@ void dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws, int splitk
     ws->partial.resize((size_t)(nbatch * f.splits * d.M * d.N));
     partial = ws->partial.get();
   }
-  launch(d, f, partial, stream);
+  launch(d, f, partial, ws, stream);
 }
 
 void dgemm_prealloc(const GemmDesc &d, cudaStream_t stream, double *ws, int64_t ws_count) {
@@ -348,7 +374,7 @@ void dgemm_prealloc(const GemmDesc &d, cudaStream_t stream, double *ws, int64_t 
   int64_t splits = fma_chain_splits(d, sm_count());
   if (!ws) splits = 1;
   else splits = std::max<int64_t>(1, std::min(splits, ws_count / std::max<int64_t>(1, nbatch * d.M * d.N)));
-  launch(d, fma_plan(d, sm_count(), (int)splits), ws, stream);
+  launch(d, fma_plan(d, sm_count(), (int)splits), ws, nullptr, stream);
 }
 
 }  // namespace vgb

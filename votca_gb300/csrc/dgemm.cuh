@@ -21,6 +21,7 @@ struct GemmWorkspace {
   DeviceBuffer<double> partial;
   DeviceBuffer<uint16_t> oz_a, oz_b;
   DeviceBuffer<int> oz_int;
+  DeviceBuffer<unsigned> arrived;  // finished splits per tile, zero between products
   GemmWorkspace() = default;
   GemmWorkspace(const GemmWorkspace &) = delete;
   GemmWorkspace &operator=(const GemmWorkspace &) = delete;
