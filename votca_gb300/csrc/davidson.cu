@@ -824,6 +824,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
       GenEigJob job;
       job.T = Td.get(); job.B = Bd.get(); job.ldt = ldT; job.m = m; job.nw = needed;
       job.U = Ud.get(); job.ldu = m; job.lam = lamd.get(); job.work = eigw.get(); job.info = einfo.get();
+      job.fast = x.gemm_path == 0;
       gen_eig_device(&job, 1, s);
     }
     mark(1);

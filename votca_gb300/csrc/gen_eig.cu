@@ -86,14 +86,58 @@ __device__ double wsum(double v) {
 constexpr int kQrThreads = 128;
 __device__ __forceinline__ void qr_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kQrThreads) : "memory"); }
 
+// The float nearest below a double in FP32's range and back, in integers (a conversion is an FP64
+// instruction).
+__device__ __forceinline__ float to_float(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  return __uint_as_float((h & 0x80000000u) | (((h & 0x7FFFFFFFu) - (896u << 20)) << 3) | (l >> 29));
+}
+__device__ __forceinline__ double to_double(float x) {  // normal x
+  const unsigned b = __float_as_uint(x);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+// 1 / sqrt(x) for x within [1, 64) from the FP32 estimate f, and 1 / x: one step of third order
+// (Householder's iteration, e < 2^-20: y (1 + e/2 + 3 e^2 / 8) and y (1 + e + e^2)), six and three FP64
+// instructions for a square root of 700 and a division of 565 clocks.
+__device__ __forceinline__ double fast_rsqrt(double x, float f) {
+  const double y = to_double(f);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double fast_rcp(double x, float f) {
+  const double y = to_double(f);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double with_sign(double a, double b) {  // |a| with b's sign bit
+  return __hiloint2double((__double2hiint(a) & 0x7FFFFFFF) | (__double2hiint(b) & (int)0x80000000), __double2loint(a));
+}
+__device__ __forceinline__ int max_exponent(double p, double q, double r) {
+  return max((__double2hiint(p) >> 20) & 0x7FF, max((__double2hiint(q) >> 20) & 0x7FF, (__double2hiint(r) >> 20) & 0x7FF));
+}
+// x 2^-sh for a normal result (else 0), in integers
+__device__ __forceinline__ double scale_down(double x, int sh) {
+  const int h = __double2hiint(x), e = ((h >> 20) & 0x7FF) - sh;
+  return e > 0 ? __hiloint2double(h - (sh << 20), __double2loint(x)) : 0.0;
+}
+__device__ __forceinline__ double scale_up(double x, int sh) {
+  const int h = __double2hiint(x), e = ((h >> 20) & 0x7FF) + sh;
+  return e > 0 && e < 0x7FF ? __hiloint2double(h + (sh << 20), __double2loint(x)) : scalbn(x, sh);
+}
+
 // Francis double-shift QR iteration on the upper Hessenberg a (n x n, leading dimension ld),
 // eigenvalues only, by the first four warps.  Returns false when an eigenvalue needs more than 60
 // steps.  An FP64 instruction holds its SM quarter for 64 clocks whatever its active lanes, a
 // division 565 and a square root 700, so the scalar recurrence (which every warp runs, one per
 // quarter) is what it costs: independent divisions run as one instruction in different lanes,
 // and the scans for a small subdiagonal and for the start of the bulge test 32 rows at once
-// (one row after another they cost as much as the bulge itself).
-__device__ bool hqr_block(double *a_, int ld, int n, double *wr, double *wi) {
+// (one row after another they cost as much as the bulge itself).  FAST: the reflectors are scaled by
+// a power of two instead of their 1-norm and built with fast_rsqrt and fast_rcp, with differences in
+// the last bits (split-precision solves keep the divisions: their iterations amplify one bit).  m 44
+// with 10 vectors: 4.4 ms with divisions, 3.2 ms; a bulge step is 2.8k clocks of dependent FP64
+// instructions (75 each), half of them the reflector.
+template <bool FAST>
+__device__ __forceinline__ bool hqr_block(double *a_, int ld, int n, double *wr, double *wi) {
   const int tid = threadIdx.x, lane = tid & 31;
   auto A = [&](int r, int c) -> double & { return a_[r + ld * c]; };
   double an = 0.0;
@@ -175,10 +219,17 @@ __device__ bool hqr_block(double *a_, int ld, int n, double *wr, double *wi) {
               p = (r * s0 - w) / A(mm + 1, mm) + A(mm, mm + 1);
               q = A(mm + 1, mm + 1) - z - r - s0;
               r = A(mm + 2, mm + 1);
-              const double s = fabs(p) + fabs(q) + fabs(r);
-              p /= s;
-              q /= s;
-              r /= s;
+              if constexpr (FAST) {
+                const int ex = max_exponent(p, q, r), sh = ex == 0 || ex == 0x7FF ? 0 : ex - 1023;
+                p = scale_down(p, sh);
+                q = scale_down(q, sh);
+                r = scale_down(r, sh);
+              } else {
+                const double s = fabs(p) + fabs(q) + fabs(r);
+                p /= s;
+                q /= s;
+                r /= s;
+              }
               stop = mm == l;
               if (!stop) {
                 const double u = fabs(A(mm, mm - 1)) * (fabs(q) + fabs(r));
@@ -202,7 +253,72 @@ __device__ bool hqr_block(double *a_, int ld, int n, double *wr, double *wi) {
             if (i != m + 2) A(i, i - 3) = 0.0;
           }
           qr_sync();
-          for (int k = m; k <= nn - 1; ++k) {
+          if constexpr (FAST) {
+            for (int k = m; k <= nn - 1; ++k) {
+              if (k != m) {
+                p = A(k, k - 1);
+                q = A(k + 1, k - 1);
+                r = k != nn - 1 ? A(k + 2, k - 1) : 0.0;
+              }
+              const int ex = max_exponent(p, q, r);
+              if (ex == 0) continue;  // zero
+              const int sh = ex == 0x7FF ? 0 : ex - 1023;  // the largest to [1, 2); infinities and NaN stay
+              p = scale_down(p, sh);
+              q = scale_down(q, sh);
+              r = scale_down(r, sh);
+              const double n2 = fma(p, p, fma(q, q, r * r));
+              // the FP32 estimates of 1 / sqrt(n2) and of 1 / (|p| + s), the second while the first is refined
+              const float n2f = to_float(n2);
+              float fs, fp;
+              asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(fs) : "f"(n2f));
+              const double pa = with_sign(p, 1.0);
+              const float pf = __double2hiint(pa) >= 0x3C000000 ? to_float(pa) : 0.f;
+              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(fp) : "f"(fmaf(n2f, fs, pf)));
+              const double rs0 = fast_rsqrt(n2, fs);
+              const double s = with_sign(n2 * rs0, p), rs = with_sign(rs0, p);
+              p += s;
+              const double rp = with_sign(fast_rcp(with_sign(p, 1.0), fp), p);
+              {  // p / s, q / s, r / s, q / p, r / p in lanes 0 .. 4
+                const double num = lane == 0 ? p : (lane == 1 || lane == 3) ? q : r;
+                const double d = num * (lane < 3 ? rs : rp);
+                x = __shfl_sync(0xffffffffu, d, 0);
+                y = __shfl_sync(0xffffffffu, d, 1);
+                z = __shfl_sync(0xffffffffu, d, 2);
+                q = __shfl_sync(0xffffffffu, d, 3);
+                r = __shfl_sync(0xffffffffu, d, 4);
+              }
+              const bool three = k != nn - 1;
+              for (int j = k + tid; j <= nn; j += kQrThreads) {
+                double *a = &A(k, j);
+                const double a0 = a[0], a1 = a[1], a2 = three ? a[2] : 0.0;
+                double pp = fma(q, a1, a0);
+                if (three) {
+                  pp = fma(r, a2, pp);
+                  a[2] = fma(-pp, z, a2);
+                }
+                a[1] = fma(-pp, y, a1);
+                a[0] = fma(-pp, x, a0);
+              }
+              qr_sync();
+              if (tid == 0) {  // every warp has read A(k, k - 1)
+                if (k != m) A(k, k - 1) = scale_up(-s, sh);
+                else if (l != m) A(k, k - 1) = -A(k, k - 1);
+              }
+              const int mmin = nn < k + 3 ? nn : k + 3;
+              for (int i = l + tid; i <= mmin; i += kQrThreads) {
+                double *a = &A(i, k);
+                const double a0 = a[0], a1 = a[ld], a2 = three ? a[2 * ld] : 0.0;
+                double pp = fma(y, a1, x * a0);
+                if (three) {
+                  pp = fma(z, a2, pp);
+                  a[2 * ld] = fma(-pp, r, a2);
+                }
+                a[ld] = fma(-pp, q, a1);
+                a[0] = a0 - pp;
+              }
+              qr_sync();
+            }
+          } else for (int k = m; k <= nn - 1; ++k) {
             if (k != m) {
               p = A(k, k - 1);
               q = A(k + 1, k - 1);
@@ -364,8 +480,10 @@ __host__ __device__ inline int64_t gen_small_doubles(int64_t m, int64_t nw) { re
 inline int64_t gen_smem_doubles(int64_t m, int64_t nw, int64_t limit) {
   int64_t need = 0;
   if (need + gen_small_doubles(m, nw) <= limit) need += gen_small_doubles(m, nw);
-  for (int i = 0; i < 3; ++i)
-    if (need + m * m <= limit) need += m * m;
+  for (int i = 0; i < 3; ++i) {
+    const int64_t n = i == 1 ? (m | 1) * m : m * m;
+    if (need + n <= limit) need += n;
+  }
   if (need + nw * m * m <= limit) need += nw * m * m;
   return need;
 }
@@ -567,8 +685,9 @@ __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_const
   }
   const int m = (int)q.m, nw = (int)q.nw;
   const int64_t mm = (int64_t)m * m;
+  const int hl = m | 1;  // odd: a row of the QR copy touches every bank
   extern __shared__ double sm[];
-  // global scratch: LU, C, Vh, 5 m small, then per selected vector 2 m^2 + 5 m, then m^2
+  // global scratch: LU, C, Vh, 5 m small, then per selected vector 2 m^2 + 5 m, then m (m + 1)
   double *gLU = q.work, *gC = gLU + mm, *gVh = gC + mm, *gsmall = gVh + mm, *vec = gsmall + 5 * (int64_t)m;
   int64_t off = 0;
   auto place = [&](int64_t n, double *glob) {
@@ -579,12 +698,12 @@ __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_const
   };
   double *small = place(gen_small_doubles(m, nw), (double *)nullptr);
   double *C = place(mm, gC);
-  double *LU = place(mm, gLU);  // then the QR copy
+  double *LU = place((int64_t)hl * m, gLU);  // then the QR copy
   double *Vh = place(mm, gVh);
   double *Uf = place((int64_t)nw * mm, vec);
   double *Hq = LU == gLU ? vec + nw * (2 * mm + 5 * (int64_t)m) : LU;
   double *piv = small ? small : gsmall, *wr = piv + m, *wi = wr + m, *colv = wi + m;
-  int *selv = small ? reinterpret_cast<int *>(small + 4 * m + 4 * (int64_t)m * nw) : reinterpret_cast<int *>(vec + nw * (2 * mm + 5 * (int64_t)m) + mm);
+  int *selv = small ? reinterpret_cast<int *>(small + 4 * m + 4 * (int64_t)m * nw) : reinterpret_cast<int *>(vec + nw * (2 * mm + 5 * (int64_t)m) + (int64_t)hl * m);
   if (tid == 0) flag = 0;
   // ---- load ----
   double bm = 0.0;
@@ -740,10 +859,16 @@ __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_const
     __syncthreads();
   }
   // ---- 3. eigenvalues: QR iteration on a copy of H, by the first four warps ----
-  for (int t = tid; t < mm; t += kGenThreads) Hq[t] = C[t];
+  for (int t = tid; t < mm; t += kGenThreads) {
+    const int c = t / m;
+    Hq[t - c * m + hl * c] = C[t];
+  }
   __syncthreads();
   if (tid < kQrThreads) {
-    const bool ok = hqr_block(Hq, m, m, wr, wi);
+    bool ok;
+    if (q.fast && Hq == LU) ok = hqr_block<true>(sm + (Hq - sm), hl, m, wr, wi);  // shared loads, not generic ones
+    else if (q.fast) ok = hqr_block<true>(Hq, hl, m, wr, wi);
+    else ok = hqr_block<false>(Hq, hl, m, wr, wi);
     if (!ok && tid == 0) flag = 3;
   }
   __syncthreads();
@@ -1010,7 +1135,7 @@ void pencil_finish_device(const double *W, int64_t m, const double *nu, const do
   VGB_LAUNCH_CHECK();
 }
 
-int64_t gen_eig_work_doubles(int64_t m, int64_t nw) { return 3 * m * m + 5 * m + nw * (2 * m * m + 5 * m) + m * m + 2 * nw + 64; }
+int64_t gen_eig_work_doubles(int64_t m, int64_t nw) { return 3 * m * m + 5 * m + nw * (2 * m * m + 5 * m) + m * (m + 1) + 2 * nw + 64; }
 
 void gen_eig_device(const GenEigJob *jobs, int64_t njobs, cudaStream_t s) {
   if (njobs <= 0) return;
