@@ -44,6 +44,7 @@ unsigned gfor(int64_t n) {
 
 __global__ void scale_cols_by_kernel(double *Z, int64_t ld, int64_t rows, int64_t ncols,
                                      const double *g) {
+  pdl_wait();
   const int64_t total = rows * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x)
@@ -53,6 +54,7 @@ __global__ void scale_cols_by_kernel(double *Z, int64_t ld, int64_t rows, int64_
 // gH: (vt+ct)^2 column-major window gradient of Hqp
 __global__ void hqp_grad_kernel(const double *X, int64_t ldx, int64_t nr, const double *g,
                                 int64_t vt, int64_t ct, double cqp, double *gH) {
+  pdl_wait();
   const int64_t n = vt + ct, total = n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -83,6 +85,7 @@ __global__ void hqp_grad_kernel(const double *X, int64_t ldx, int64_t nr, const 
 // gw[P] = alpha * sum_{vv'} Q[P][v][v'] Mvv[P][v][v']
 __global__ void dot_per_batch_kernel(const double *Q, const double *M, int64_t nb, int64_t len,
                                      double alpha, double *out) {
+  pdl_wait();
   for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
     double s = 0.0;
     for (int64_t i = threadIdx.x; i < len; i += blockDim.x) s += Q[b * len + i] * M[b * len + i];
@@ -101,6 +104,7 @@ __global__ void dot_per_batch_kernel(const double *Q, const double *M, int64_t n
 // out[P][...] (+)= alpha * w[P] * Q[P][...]
 __global__ void scale_batches_kernel(const double *Q, const double *w, int64_t nb, int64_t len,
                                      double alpha, double *out, int accumulate) {
+  pdl_wait();
   const int64_t total = nb * len;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x)
@@ -115,6 +119,7 @@ struct ScatterGradArgs {
   double *out;
 };
 __global__ void scatter_grad_kernel(const ScatterGradArgs a) {
+  pdl_wait();
   const int64_t total = a.cnt * a.naux * a.nsize;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -147,8 +152,7 @@ void scatter_mmn_gradient(const BseOperator &op, const double *gMvc, const doubl
     a.m_v0 = op.m_v0; a.m_c0 = op.m_c0; a.n_v0 = op.n_v0; a.n_c0 = op.n_c0;
     a.out = buf.get();
     const int64_t total = a.cnt * slice;
-    scatter_grad_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 16LL * 152)),
-                          256, 0, s>>>(a);
+    launch_pdl(scatter_grad_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 16LL * 152)), 256, 0, s, a);
     VGB_LAUNCH_CHECK();
     VGB_CUDA(cudaMemcpyAsync(host_out + m0 * slice, buf.get(), total * sizeof(double),
                              cudaMemcpyDeviceToHost, s));
@@ -174,7 +178,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
   VGB_CUDA(cudaMemcpyAsync(g.get(), g_host, nr * sizeof(double), cudaMemcpyHostToDevice, s));
   const std::vector<double> gh(g_host, g_host + nr);
   if (gH && c.cqp != 0) {
-    hqp_grad_kernel<<<gfor((vt + ct) * (vt + ct)), 256, 0, s>>>(X, ldx, nr, g.get(), vt, ct, c.cqp, gH);
+    launch_pdl(hqp_grad_kernel, gfor((vt + ct) * (vt + ct)), 256, 0, s, X, ldx, nr, g.get(), vt, ct, c.cqp, gH);
     VGB_LAUNCH_CHECK();
   }
   if (gMvc && c.cx != 0) {
@@ -185,7 +189,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
     z.B = X; z.b_rs = 1; z.b_cs = ldx;
     z.C = Zb.get(); z.c_rs = 1; z.c_cs = naux;
     dgemm(z, s, &ws);
-    scale_cols_by_kernel<<<gfor(naux * nr), 256, 0, s>>>(Zb.get(), naux, naux, nr, g.get());
+    launch_pdl(scale_cols_by_kernel, gfor(naux * nr), 256, 0, s, Zb.get(), naux, naux, nr, g.get());
     VGB_LAUNCH_CHECK();
     GemmDesc o;  // gMvc[P][I] += 2 cx sum_k Zg[P][k] X[I][k]
     o.M = naux; o.N = dim; o.K = nr;
@@ -239,7 +243,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
     }
     if (gMvv) {
       if (!dense_screening) {
-        scale_batches_kernel<<<gfor(naux * vt * vt), 256, 0, s>>>(Q.get(), Wscr.get(), naux, vt * vt, -cd, gMvv,
+        launch_pdl(scale_batches_kernel, gfor(naux * vt * vt), 256, 0, s, Q.get(), Wscr.get(), naux, vt * vt, -cd, gMvv,
                                                                    1);
         VGB_LAUNCH_CHECK();
       } else {
@@ -254,7 +258,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
     }
     if (gW) {
       if (!dense_screening) {
-        dot_per_batch_kernel<<<(unsigned)std::min<int64_t>(naux, 4096), 256, 0, s>>>(Q.get(), Mvv.get(), naux,
+        launch_pdl(dot_per_batch_kernel, (unsigned)std::min<int64_t>(naux, 4096), 256, 0, s, Q.get(), Mvv.get(), naux,
                                                                                   vt * vt, -cd, gW);
         VGB_LAUNCH_CHECK();
       } else {
@@ -283,7 +287,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
           dgemm(t, s, &ws);
         }
         copy_cols(X + k0 * ldx, ldx, dim, kc, Xg.get(), dim, s);  // Xg[(k, v)][c] = g_k X_k(v, c)
-        scale_cols_by_kernel<<<gfor(dim * kc), 256, 0, s>>>(Xg.get(), dim, dim, kc, g.get() + k0);
+        launch_pdl(scale_cols_by_kernel, gfor(dim * kc), 256, 0, s, Xg.get(), dim, dim, kc, g.get() + k0);
         VGB_LAUNCH_CHECK();
         SplitMap tm;  // rows (P, c'), columns (k, v)
         tm.rdiv = 1; tm.rs1 = Kt; tm.rs2 = 0; tm.cs = 1; tm.rlim = 1;
@@ -358,7 +362,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
         a.nb1 = naux;
         dgemm(a, s, &ws);
         if (!dense_screening) {
-          dot_per_batch_kernel<<<(unsigned)std::min<int64_t>(naux, 4096), 256, 0, s>>>(T2.get(), T3.get(), naux,
+          launch_pdl(dot_per_batch_kernel, (unsigned)std::min<int64_t>(naux, 4096), 256, 0, s, T2.get(), T3.get(), naux,
                                                                                     vv, alpha, gW);
           VGB_LAUNCH_CHECK();
         } else {
@@ -375,7 +379,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
       if (gMcv) {
         const double *Zw = T2.get();  // sum_Q W_QP Za^Q
         if (!dense_screening) {
-          scale_batches_kernel<<<gfor(naux * vv), 256, 0, s>>>(T2.get(), Wscr.get(), naux, vv, 1.0, T1.get(), 0);
+          launch_pdl(scale_batches_kernel, gfor(naux * vv), 256, 0, s, T2.get(), Wscr.get(), naux, vv, 1.0, T1.get(), 0);
           VGB_LAUNCH_CHECK();
           Zw = T1.get();
         } else {

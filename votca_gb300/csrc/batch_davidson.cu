@@ -146,6 +146,7 @@ __device__ __forceinline__ void tn_chunk(const TnJob &q, double *sm, int chunk, 
     if (pa[k] && sub == 0) q.part[(int64_t)chunk * mp + o0 + t / S + k * (kThreads / S)] = acc[k];
 }
 __global__ void __launch_bounds__(kThreads, 2) tn_partial_kernel(const __grid_constant__ Group<TnJob> g, int parts) {
+  pdl_wait();
   const TnJob q = g.j[blockIdx.y];
   const int chunk = (int)blockIdx.x / parts, part = (int)blockIdx.x - chunk * parts;
   if ((int64_t)chunk * kTnRows >= q.n) return;
@@ -171,6 +172,7 @@ struct TnReduceJob {
   int64_t ldc;
 };
 __global__ void tn_reduce_kernel(const __grid_constant__ Group<TnReduceJob> g) {
+  pdl_wait();
   const TnReduceJob q = g.j[blockIdx.y];
   const int64_t mp = q.m * q.p;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < mp;
@@ -214,6 +216,7 @@ __device__ __forceinline__ void nn_rows(const NnJob &q, const double *us) {
 // One launch for the jobs of every column count: three launches of a third of the SMs' work each
 // took 54 us per product of 24 molecules, 25 us here.
 __global__ void __launch_bounds__(kThreads) nn_kernel(const __grid_constant__ Group<NnJob> g) {
+  pdl_wait();
   const NnJob q = g.j[blockIdx.y];
   __shared__ double us[kNnSmem / sizeof(double)];
   const int m = (int)q.m, p = (int)q.p;
@@ -245,6 +248,7 @@ struct NormJob {
   bool scale = false;  // and last: A *= 1 / norm (a zero column stays, as with Eigen's normalize)
 };
 __global__ void norm_kernel(const __grid_constant__ Group<NormJob> g) {
+  pdl_wait();
   const NormJob q = g.j[blockIdx.y];
   const int64_t c = blockIdx.x;
   if (c >= q.p) return;
@@ -289,6 +293,7 @@ struct ColJob {
   int64_t lda, ldb, n, p;
 };
 __global__ void col_kernel(const __grid_constant__ Group<ColJob> g) {
+  pdl_wait();
   const ColJob q = g.j[blockIdx.y];
   const int64_t total = q.n * q.p;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -394,6 +399,7 @@ __device__ __forceinline__ void gs_update(const double *__restrict__ M, const do
 template <bool STAGED>
 __global__ void __cluster_dims__(kGsCluster, 1, 1) __launch_bounds__(kGsThreads, STAGED ? 1 : 8)
     gs_kernel(const __grid_constant__ Group<GsJob> g) {
+  pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank();
   const GsJob q = g.j[blockIdx.x / kGsCluster];
@@ -498,6 +504,7 @@ struct UnitJob {
   int64_t count;
 };
 __global__ void unit_kernel(const __grid_constant__ Group<UnitJob> g) {
+  pdl_wait();
   const UnitJob q = g.j[blockIdx.y];
   for (int64_t j = threadIdx.x; j < q.count; j += blockDim.x) q.V[(int64_t)q.rows[j] + q.ldv * j] = 1.0;
 }
@@ -514,6 +521,7 @@ struct MirrorJob {
   int64_t ldt, c0, nc;
 };
 __global__ void mirror_kernel(const __grid_constant__ Group<MirrorJob> g) {
+  pdl_wait();
   const MirrorJob q = g.j[blockIdx.y];
   const int64_t total = q.c0 * q.nc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -532,7 +540,7 @@ void launch_jobs(const std::vector<Job> &jobs, Kernel kernel, unsigned bx, bool 
     for (; i < jobs.size() && g->n < kJobs; ++i) g->j[g->n++] = jobs[i];
     // grid_x_is_job: bx consecutive CTAs (a cluster) per job along x
     const dim3 grid = grid_x_is_job ? dim3((unsigned)g->n * bx) : dim3(bx, (unsigned)g->n);
-    kernel<<<grid, threads, 0, s>>>(*g, args...);
+    launch_pdl(kernel, grid, threads, 0, s, *g, args...);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -661,7 +669,7 @@ void run_gs(const std::vector<GsJob> &jobs, cudaStream_t s) {
   for (size_t i = 0; i < jobs.size();) {
     g->n = 0;
     for (; i < jobs.size() && g->n < kJobs; ++i) g->j[g->n++] = jobs[i];
-    gs_kernel<true><<<(unsigned)g->n * kGsCluster, kGsThreads, (size_t)bytes, s>>>(*g);
+    launch_pdl(gs_kernel<true>, (unsigned)g->n * kGsCluster, kGsThreads, (size_t)bytes, s, *g);
     VGB_LAUNCH_CHECK();
   }
 }

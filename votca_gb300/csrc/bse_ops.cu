@@ -31,6 +31,7 @@ struct ScatterArgs {
 };
 
 __global__ void scatter_kernel(const ScatterArgs a) {
+  pdl_wait();
   const int64_t nwin = a.vt + a.ct;
   const int64_t total = a.m_count * a.naux * nwin;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -66,6 +67,7 @@ __global__ void scatter_kernel(const ScatterArgs a) {
 }
 
 __global__ void dvv_from_gvv_kernel(const double *Gvv, int64_t naux, int64_t vt, double *dvv) {
+  pdl_wait();
   const int64_t total = naux * vt;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -79,6 +81,7 @@ __global__ void hqp_diag_kernel(double cqp, const double *__restrict__ Hcc,
                                 const double *__restrict__ Hvv, int64_t vt, int64_t ct,
                                 const double *__restrict__ X, int64_t ldx, int64_t k,
                                 double *__restrict__ Y, int64_t ldy, int accumulate) {
+  pdl_wait();
   const int64_t dim = vt * ct, total = dim * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -110,6 +113,7 @@ struct HqpGroup {
 static_assert(sizeof(HqpGroup) <= 32000, "Hqp job list too large");
 
 __global__ void hqp_diag_group_kernel(const __grid_constant__ HqpGroup g) {
+  pdl_wait();
   const HqpJob q = g.j[blockIdx.y];
   const int64_t dim = q.vt * q.ct, total = dim * q.k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -124,6 +128,7 @@ __global__ void hqp_diag_group_kernel(const __grid_constant__ HqpGroup g) {
 }
 
 __global__ void zero_cols_kernel(double *Y, int64_t ldy, int64_t rows, int64_t k) {
+  pdl_wait();
   const int64_t total = rows * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -175,6 +180,7 @@ __device__ __forceinline__ void diagonal_range(const DiagArgs &a, int64_t I0, in
 // SM to keep the FP64 pipe and the memory system busy.
 constexpr int kDiagSlices = 8;
 __global__ void __launch_bounds__(32 * kDiagSlices) diagonal_kernel(const DiagArgs a) {
+  pdl_wait();
   __shared__ double part[kDiagSlices][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int64_t I0 = blockIdx.x * 32LL; I0 < a.dim; I0 += (int64_t)gridDim.x * 32) {
@@ -232,12 +238,14 @@ struct DiagGroup {
 static_assert(sizeof(DiagGroup) <= 32000, "diagonal job list too large");
 
 __global__ void diagonal_group_kernel(const __grid_constant__ DiagGroup g) {
+  pdl_wait();
   const DiagArgs a = g.j[blockIdx.y];
   diagonal_range(a, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 __global__ void ham_combine_kernel(const double *__restrict__ TA, const double *__restrict__ TB,
                                    int64_t dim, int64_t k, double *__restrict__ Y, int64_t ldy) {
+  pdl_wait();
   const int64_t total = dim * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -251,6 +259,7 @@ __global__ void ham_combine_kernel(const double *__restrict__ TA, const double *
 }
 
 __global__ void ham_diag_kernel(const double *D, int64_t dim, double *D2) {
+  pdl_wait();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < dim;
        t += (int64_t)gridDim.x * blockDim.x) {
     D2[t] = D[t];
@@ -260,6 +269,7 @@ __global__ void ham_diag_kernel(const double *D, int64_t dim, double *D2) {
 
 __global__ void copy_cols_kernel(const double *X, int64_t ldx, int64_t rows, int64_t k, double *Y,
                                  int64_t ldy) {
+  pdl_wait();
   const int64_t total = rows * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -276,18 +286,18 @@ unsigned grid_for(int64_t n, int threads = 256) {
 
 void ham_combine(const double *TA, const double *TB, int64_t dim, int64_t k, double *Y,
                  int64_t ldy, cudaStream_t s) {
-  ham_combine_kernel<<<grid_for(dim * k), 256, 0, s>>>(TA, TB, dim, k, Y, ldy);
+  launch_pdl(ham_combine_kernel, grid_for(dim * k), 256, 0, s, TA, TB, dim, k, Y, ldy);
   VGB_LAUNCH_CHECK();
 }
 
 void ham_diag(const double *D, int64_t dim, double *D2, cudaStream_t s) {
-  ham_diag_kernel<<<grid_for(dim), 256, 0, s>>>(D, dim, D2);
+  launch_pdl(ham_diag_kernel, grid_for(dim), 256, 0, s, D, dim, D2);
   VGB_LAUNCH_CHECK();
 }
 
 void copy_cols(const double *X, int64_t ldx, int64_t rows, int64_t k, double *Y, int64_t ldy,
                cudaStream_t s) {
-  copy_cols_kernel<<<grid_for(rows * k), 256, 0, s>>>(X, ldx, rows, k, Y, ldy);
+  launch_pdl(copy_cols_kernel, grid_for(rows * k), 256, 0, s, X, ldx, rows, k, Y, ldy);
   VGB_LAUNCH_CHECK();
 }
 
@@ -442,7 +452,7 @@ void BseOperator::stage(const bse_mmn_desc &desc, const double *const *slices, c
     a.Mcv = Mcv.get();
     a.Mcv0 = Mcv0.get();
     a.dcc = dcc.get();
-    scatter_kernel<<<grid_for(cnt * naux * nwin), 256, 0, s>>>(a);
+    launch_pdl(scatter_kernel, grid_for(cnt * naux * nwin), 256, 0, s, a);
     VGB_LAUNCH_CHECK();
     VGB_CUDA(cudaStreamSynchronize(s));  // raw is reused by the next chunk
   }
@@ -474,7 +484,7 @@ void BseOperator::stage(const bse_mmn_desc &desc, const double *const *slices, c
     }
     VGB_CUDA(cudaStreamSynchronize(s));
   }
-  dvv_from_gvv_kernel<<<grid_for(naux * vt), 256, 0, s>>>(Gvv.get(), naux, vt, dvv.get());
+  launch_pdl(dvv_from_gvv_kernel, grid_for(naux * vt), 256, 0, s, Gvv.get(), naux, vt, dvv.get());
   VGB_LAUNCH_CHECK();
   VGB_CUDA(cudaStreamSynchronize(s));
   stage_unscreened_vv(desc, slices, opt, s);
@@ -512,7 +522,7 @@ void BseOperator::apply_hqp(double cqp, const double *X, int64_t ldx, int64_t k,
   timer.begin(STAGE_HQP, s);
   struct End { StageTimer &t; cudaStream_t s; ~End() { t.end(STAGE_HQP, s); } } end_{timer, s};
   if (hqp_diagonal) {
-    hqp_diag_kernel<<<grid_for(dim * k), 256, 0, s>>>(cqp, Hcc.get(), Hvv.get(), vt, ct, X, ldx, k,
+    launch_pdl(hqp_diag_kernel, grid_for(dim * k), 256, 0, s, cqp, Hcc.get(), Hvv.get(), vt, ct, X, ldx, k,
                                                       Y, ldy, accumulate ? 1 : 0);
     VGB_LAUNCH_CHECK();
     return;
@@ -639,7 +649,7 @@ void BseOperator::matmul(const Coef &c, const double *X, int64_t ldx, int64_t k,
   if (c.cd != 0) { apply_hd_fp64(-(double)c.cd, X, ldx, k, Y, ldy, acc, s); acc = true; }
   if (c.cd2 != 0) { apply_hd2_fp64(-(double)c.cd2, X, ldx, k, Y, ldy, acc, s); acc = true; }
   if (!acc) {
-    zero_cols_kernel<<<grid_for(dim * k), 256, 0, s>>>(Y, ldy, dim, k);
+    launch_pdl(zero_cols_kernel, grid_for(dim * k), 256, 0, s, Y, ldy, dim, k);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -687,7 +697,7 @@ void matmul_grouped(const Coef &c, const std::vector<GroupedItem> &items, cudaSt
       mx = std::max(mx, hq[i].vt * hq[i].ct * hq[i].k);
     }
     const unsigned bx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(mx, 256), 64));
-    hqp_diag_group_kernel<<<dim3(bx, (unsigned)g->n), 256, 0, s>>>(*g);
+    launch_pdl(hqp_diag_group_kernel, dim3(bx, (unsigned)g->n), 256, 0, s, *g);
     VGB_LAUNCH_CHECK();
   }
   MixedEngine::apply_grouped(c, mixed_items, c.cqp != 0, s, scratch);
@@ -706,7 +716,7 @@ void BseOperator::diagonal(const Coef &c, double *D, cudaStream_t s) {
   a.vt = vt; a.ct = ct; a.naux = naux; a.dim = dim;
   a.Bvc = Bvc.get(); a.Mcv = Mcv.get(); a.dcc = dcc.get(); a.dvv = dvv.get();
   a.Hcc = Hcc.get(); a.Hvv = Hvv.get(); a.D = D;
-  diagonal_kernel<<<(unsigned)std::min<int64_t>(ceil_div(dim, 32), 64LL * sm_count()), 32 * kDiagSlices, 0, s>>>(a);
+  launch_pdl(diagonal_kernel, (unsigned)std::min<int64_t>(ceil_div(dim, 32), 64LL * sm_count()), 32 * kDiagSlices, 0, s, a);
   VGB_LAUNCH_CHECK();
 }
 
@@ -727,7 +737,7 @@ void diagonal_grouped(const Coef &c, const std::vector<BseOperator *> &ops,
       a.Hcc = op.Hcc.get(); a.Hvv = op.Hvv.get(); a.D = D[i];
       mx = std::max(mx, op.dim);
     }
-    diagonal_group_kernel<<<dim3((unsigned)ceil_div(mx, 128), (unsigned)g->n), 128, 0, s>>>(*g);
+    launch_pdl(diagonal_group_kernel, dim3((unsigned)ceil_div(mx, 128), (unsigned)g->n), 128, 0, s, *g);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -784,13 +794,14 @@ void DenseOperator::matmul(const double *X, int64_t ldx, int64_t k, double *Y, i
 }
 
 __global__ void dense_diag_kernel(const double *A, int64_t n, double *D) {
+  pdl_wait();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x)
     D[t] = A[t + n * t];
 }
 
 void DenseOperator::diagonal(double *D, cudaStream_t s) {
-  dense_diag_kernel<<<grid_for(n), 256, 0, s>>>(A.get(), n, D);
+  launch_pdl(dense_diag_kernel, grid_for(n), 256, 0, s, A.get(), n, D);
   VGB_LAUNCH_CHECK();
 }
 

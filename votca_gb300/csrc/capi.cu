@@ -106,6 +106,7 @@ namespace {
 // P = X + Y, M = X - Y (dim x nr, leading dimensions ldx and dim)
 __global__ void plus_minus_kernel(const double *X, const double *Y, int64_t ldx, int64_t dim, int64_t nr,
                                   double *P, double *M) {
+  vgb::pdl_wait();
   const int64_t total = dim * nr;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -132,8 +133,7 @@ void eig_gradient_blocks(vgb::BseOperator &op, const vgb::Coef &a, const vgb::Co
     half[nr + k] = -0.5 * g[k];
   }
   vgb::DeviceBuffer<double> PM(2 * op.dim * nr);
-  plus_minus_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(vgb::ceil_div(op.dim * nr, 256), 2432)),
-                      256, 0, s>>>(X, Y, ldx, op.dim, nr, PM.get(), PM.get() + op.dim * nr);
+  vgb::launch_pdl(plus_minus_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(vgb::ceil_div(op.dim * nr, 256), 2432)), 256, 0, s, X, Y, ldx, op.dim, nr, PM.get(), PM.get() + op.dim * nr);
   VGB_LAUNCH_CHECK();
   op.quad_gradient(*b, PM.get(), op.dim, 2 * nr, half.data(), gvc, gcv, gvv, gcc, gh, gw, true, s);
 }

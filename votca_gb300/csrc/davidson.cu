@@ -37,6 +37,7 @@ unsigned blocks_for(int64_t n, int threads = 256) {
 __global__ void coldot_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ B, int64_t ldb,
                               int64_t n, double *__restrict__ partial, unsigned *arrived, int take_sqrt,
                               double *__restrict__ out) {
+  pdl_wait();
   const int64_t c = blockIdx.y;
   const int64_t chunk = ceil_div(n, kRedChunks);
   const int64_t r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
@@ -72,6 +73,7 @@ __global__ void coldot_kernel(const double *__restrict__ A, int64_t lda, const d
 }
 
 __global__ void set_unit_columns_kernel(double *V, int64_t ldv, const int64_t *rows, int64_t count) {
+  pdl_wait();
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < count;
        j += (int64_t)gridDim.x * blockDim.x)
     V[rows[j] + ldv * j] = 1.0;
@@ -80,6 +82,7 @@ __global__ void set_unit_columns_kernel(double *V, int64_t ldv, const int64_t *r
 // res[:, j] -= lam[j] * q[:, j]
 __global__ void residual_kernel(double *__restrict__ res, const double *__restrict__ q, int64_t n,
                                 int64_t ncols, const double *__restrict__ lam) {
+  pdl_wait();
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -95,6 +98,7 @@ __global__ void dpr_kernel(double *__restrict__ out, int64_t ldo, const double *
                            const double *__restrict__ q, int64_t n, const double *__restrict__ D,
                            const int64_t *__restrict__ cols, const double *__restrict__ lams,
                            int64_t count, int clean, double *__restrict__ dq) {
+  pdl_wait();
   const int64_t total = n * count;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -114,6 +118,7 @@ __global__ void olsen_finish_kernel(double *__restrict__ out, int64_t ldo,
                                     const double *__restrict__ q, int64_t n,
                                     const int64_t *__restrict__ cols, const double *__restrict__ num,
                                     const double *__restrict__ den, int64_t count) {
+  pdl_wait();
   const int64_t total = n * count;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -129,6 +134,7 @@ __global__ void olsen_finish_kernel(double *__restrict__ out, int64_t ldo,
 // A[:, c] /= norm[c] where norm[c] > 0 (Eigen's normalize leaves zero columns alone)
 __global__ void scale_columns_kernel(double *A, int64_t lda, int64_t n, int64_t ncols,
                                      const double *__restrict__ norm) {
+  pdl_wait();
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -141,6 +147,7 @@ __global__ void scale_columns_kernel(double *A, int64_t lda, int64_t n, int64_t 
 
 __global__ void copy_block_kernel(const double *src, int64_t lds, double *dst, int64_t ldd,
                                   int64_t n, int64_t ncols) {
+  pdl_wait();
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -153,6 +160,7 @@ __global__ void copy_block_kernel(const double *src, int64_t lds, double *dst, i
 // T[c0 + c, r] = T[r, c0 + c] for r < c0, c < nc: the lower block of the projected matrix from
 // the columns just computed (updateProjection's bottomLeftCorner = topRightCorner^T)
 __global__ void mirror_block_kernel(double *T, int64_t ldt, int64_t c0, int64_t nc) {
+  pdl_wait();
   const int64_t total = c0 * nc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -299,13 +307,13 @@ struct Ctx {
       VGB_CUDA(cudaMemsetAsync(red_arrived.get(), 0, ncols * sizeof(unsigned), s));
     }
     dim3 grid(kRedChunks, (unsigned)ncols);
-    coldot_kernel<<<grid, 256, 0, s>>>(A, lda, B ? B : A, B ? ldb : lda, n, red_partial.get(), red_arrived.get(),
+    launch_pdl(coldot_kernel, grid, 256, 0, s, A, lda, B ? B : A, B ? ldb : lda, n, red_partial.get(), red_arrived.get(),
                                        sqrt_ ? 1 : 0, out);
     VGB_LAUNCH_CHECK();
   }
   void scale_cols(double *A, int64_t lda, int64_t ncols, const double *norms) {
     if (ncols <= 0) return;
-    scale_columns_kernel<<<blocks_for(n * ncols), 256, 0, s>>>(A, lda, n, ncols, norms);
+    launch_pdl(scale_columns_kernel, blocks_for(n * ncols), 256, 0, s, A, lda, n, ncols, norms);
     VGB_LAUNCH_CHECK();
   }
   // C (m x nc, ldc) = alpha * A[:, a0:a0+m]^T B[:, b0:b0+nc] + beta C
@@ -328,7 +336,7 @@ struct Ctx {
   }
   void copy_cols(const double *src, int64_t lds, double *dst, int64_t ldd, int64_t ncols) {
     if (ncols <= 0) return;
-    copy_block_kernel<<<blocks_for(n * ncols), 256, 0, s>>>(src, lds, dst, ldd, n, ncols);
+    launch_pdl(copy_block_kernel, blocks_for(n * ncols), 256, 0, s, src, lds, dst, ldd, n, ncols);
     VGB_LAUNCH_CHECK();
   }
 };
@@ -341,6 +349,7 @@ struct Ctx {
 constexpr int kCholQrMax = 64;
 __global__ void __launch_bounds__(256) cholqr_kernel(const double *G, int nb, double *Rinv, const double *norms0,
                                                      int chk, int *ok, int *flag) {
+  pdl_wait();
   __shared__ double a[kCholQrMax * kCholQrMax];
   __shared__ int bad;
   const int tid = threadIdx.x;
@@ -413,7 +422,7 @@ void gramschmidt(Ctx &x, double *Q, int64_t nstart, int64_t ncols, DeviceBuffer<
       double *G = x.gs_part.get(), *Ri = G + nupdate * nupdate, *T = Ri + nupdate * nupdate;
       x.gs_err.resize(2);
       x.gemm_tn(Q + nstart * n, n, nupdate, Q + nstart * n, n, nupdate, G, nupdate, 1.0, 0.0);
-      cholqr_kernel<<<1, 256, 0, x.s>>>(G, (int)nupdate, Ri, norms0, pass == 1 ? 1 : 0, x.gs_err.get() + 1,
+      launch_pdl(cholqr_kernel, 1, 256, 0, x.s, G, (int)nupdate, Ri, norms0, pass == 1 ? 1 : 0, x.gs_err.get() + 1,
                                         flag.get());
       VGB_LAUNCH_CHECK();
       int ok = 0;
@@ -549,7 +558,7 @@ bool fp64_polish(Ctx &x, TimedApply &apply, const double *Dd, const double *q0, 
       projJ(V.get() + old * n, nv, AV.get() + old * n, nv, Td.get() + old + cap * old, cap);
       projJ(V.get(), m, V.get() + old * n, nv, Jd.get() + cap * old, cap);
       if (old > 0) {
-        mirror_block_kernel<<<blocks_for(old * nv), 256, 0, s>>>(Jd.get(), cap, old, nv);
+        launch_pdl(mirror_block_kernel, blocks_for(old * nv), 256, 0, s, Jd.get(), cap, old, nv);
         VGB_LAUNCH_CHECK();
       }
     }
@@ -594,7 +603,7 @@ bool fp64_polish(Ctx &x, TimedApply &apply, const double *Dd, const double *q0, 
     // ---- Ritz vectors and residuals: q = V U, res = A V U - q lambda (normalised) ----
     x.gemm_nn(V.get(), n, m, Ud.get(), m, np, q.get(), n, 1.0, 0.0);
     x.gemm_nn(AV.get(), n, m, Ud.get(), m, np, res.get(), n, 1.0, 0.0);
-    residual_kernel<<<blocks_for(n * np), 256, 0, s>>>(res.get(), q.get(), n, np, lamd.get());
+    launch_pdl(residual_kernel, blocks_for(n * np), 256, 0, s, res.get(), q.get(), n, np, lamd.get());
     VGB_LAUNCH_CHECK();
     work.resize(2 * np + 8);
     if (ham) {
@@ -653,7 +662,7 @@ bool fp64_polish(Ctx &x, TimedApply &apply, const double *Dd, const double *q0, 
     VGB_CUDA(cudaMemcpyAsync(lamu, upd_lam.data(), nupdate * sizeof(double), cudaMemcpyHostToDevice, s));
     double *Vnew = V.get() + m * n;
     const bool olsen = correction == 1;
-    dpr_kernel<<<blocks_for(n * nupdate), 256, 0, s>>>(Vnew, n, res.get(), q.get(), n, Dd, colsd.get(), lamu,
+    launch_pdl(dpr_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, res.get(), q.get(), n, Dd, colsd.get(), lamu,
                                                       nupdate, olsen ? 0 : 1, olsen ? dq : nullptr);
     VGB_LAUNCH_CHECK();
     if (olsen) {
@@ -661,7 +670,7 @@ bool fp64_polish(Ctx &x, TimedApply &apply, const double *Dd, const double *q0, 
         x.coldots(q.get() + upd[kk] * n, n, Vnew + kk * n, n, 1, numd + kk, false);
         x.coldots(q.get() + upd[kk] * n, n, dq + kk * n, n, 1, dend + kk, false);
       }
-      olsen_finish_kernel<<<blocks_for(n * nupdate), 256, 0, s>>>(Vnew, n, q.get(), n, colsd.get(), numd, dend,
+      launch_pdl(olsen_finish_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, q.get(), n, colsd.get(), numd, dend,
                                                                  nupdate);
       VGB_LAUNCH_CHECK();
     }
@@ -770,7 +779,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
     std::vector<int64_t> rows(idx.begin() + ind0, idx.begin() + ind0 + ncols);
     colsd.resize(std::max<int64_t>(ncols, 64));
     VGB_CUDA(cudaMemcpyAsync(colsd.get(), rows.data(), ncols * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    set_unit_columns_kernel<<<blocks_for(ncols), 256, 0, s>>>(V.get(), n, colsd.get(), ncols);
+    launch_pdl(set_unit_columns_kernel, blocks_for(ncols), 256, 0, s, V.get(), n, colsd.get(), ncols);
     VGB_LAUNCH_CHECK();
   }
 
@@ -791,7 +800,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
         // T[:, old:ncols] = V^T AV_new, T[old:ncols, :old] its transpose, in HBM
         x.gemm_tn(V.get(), n, ncols, AV.get() + old * n, n, nvec, Td.get() + ldT * old, ldT, 1.0, 0.0);
         if (old > 0) {
-          mirror_block_kernel<<<blocks_for(old * nvec), 256, 0, s>>>(Td.get(), ldT, old, nvec);
+          launch_pdl(mirror_block_kernel, blocks_for(old * nvec), 256, 0, s, Td.get(), ldT, old, nvec);
           VGB_LAUNCH_CHECK();
         }
       } else {
@@ -833,7 +842,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
     res.resize(n * needed);
     x.gemm_nn(V.get(), n, m, Ud.get(), m, needed, q.get(), n, 1.0, 0.0);
     x.gemm_nn(AV.get(), n, m, Ud.get(), m, needed, res.get(), n, 1.0, 0.0);
-    residual_kernel<<<blocks_for(n * needed), 256, 0, s>>>(res.get(), q.get(), n, needed, lamd.get());
+    launch_pdl(residual_kernel, blocks_for(n * needed), 256, 0, s, res.get(), q.get(), n, needed, lamd.get());
     VGB_LAUNCH_CHECK();
 
     mark(2);
@@ -920,7 +929,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
     VGB_CUDA(cudaMemcpyAsync(lamu, upd_lam.data(), nupdate * sizeof(double), cudaMemcpyHostToDevice, s));
     double *Vnew = V.get() + ncols * n;
     const bool olsen = opt.correction == 1;
-    dpr_kernel<<<blocks_for(n * nupdate), 256, 0, s>>>(Vnew, n, res.get(), q.get(), n, D.get(),
+    launch_pdl(dpr_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, res.get(), q.get(), n, D.get(),
                                                       colsd.get(), lamu, nupdate, olsen ? 0 : 1,
                                                       olsen ? dq : nullptr);
     VGB_LAUNCH_CHECK();
@@ -930,7 +939,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
         x.coldots(q.get() + upd[kk] * n, n, Vnew + kk * n, n, 1, numd + kk, false);
         x.coldots(q.get() + upd[kk] * n, n, dq + kk * n, n, 1, dend + kk, false);
       }
-      olsen_finish_kernel<<<blocks_for(n * nupdate), 256, 0, s>>>(Vnew, n, q.get(), n, colsd.get(),
+      launch_pdl(olsen_finish_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, q.get(), n, colsd.get(),
                                                                  numd, dend, nupdate);
       VGB_LAUNCH_CHECK();
     }

@@ -38,6 +38,7 @@ __device__ __forceinline__ void add_splits(const GemmDesc &d, int64_t b1, int64_
 template <int TM, int TN>
 __global__ void __launch_bounds__(THREADS)
     dgemm_kernel(const GemmDesc d, const Grid g, double *partial, unsigned *arrived, int a_icontig, int b_lcontig) {
+  pdl_wait();
   constexpr int RM = TM / 16, RN = TN / 16;
   __shared__ double As[2][TK][TM + 1];
   __shared__ double Bs[2][TK][TN + 1];
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(THREADS)
 
 // The same for all outputs in a launch of its own, for callers without counters.
 __global__ void splitk_reduce_kernel(const GemmDesc d, const Grid g, const double *partial) {
+  pdl_wait();
   const int64_t mn = d.M * d.N;
   const int64_t total = mn * g.nbatch;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -169,6 +171,7 @@ __global__ void splitk_reduce_kernel(const GemmDesc d, const Grid g, const doubl
 }
 
 __global__ void scale_kernel(const GemmDesc d, int64_t nbatch) {
+  pdl_wait();
   const int64_t mn = d.M * d.N, total = mn * nbatch;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -185,7 +188,7 @@ template <int TM, int TN>
 void launch_tile(const GemmDesc &d, const Grid &g, double *partial, unsigned *arrived, cudaStream_t stream) {
   const int64_t blocks = g.mt * g.nt * g.nbatch * g.splits;
   VGB_REQUIRE(blocks < (1LL << 31), "dgemm: grid too large");
-  dgemm_kernel<TM, TN><<<(unsigned)blocks, THREADS, 0, stream>>>(d, g, partial, arrived,
+  launch_pdl(dgemm_kernel<TM, TN>, (unsigned)blocks, THREADS, 0, stream, d, g, partial, arrived,
                                                                   d.a_rs == 1 ? 1 : 0, d.b_rs == 1 ? 1 : 0);
   VGB_LAUNCH_CHECK();
 }
@@ -220,8 +223,7 @@ void launch(const GemmDesc &d, const FmaPlan &f, double *partial, GemmWorkspace 
   }
   if (f.splits > 1 && !arrived) {
     const int64_t total = d.M * d.N * g.nbatch;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0,
-                           stream>>>(d, g, partial);
+    launch_pdl(splitk_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0, stream, d, g, partial);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -347,7 +349,7 @@ void dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws, int splitk
   if (splitk == 0 && oz_dgemm(d, stream, ws)) return;
   if (d.K == 0) {  // C = beta * C
     const int64_t total = d.M * d.N * nbatch;
-    scale_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream>>>(d, nbatch);
+    launch_pdl(scale_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream, d, nbatch);
     VGB_LAUNCH_CHECK();
     return;
   }
@@ -367,7 +369,7 @@ void dgemm_prealloc(const GemmDesc &d, cudaStream_t stream, double *ws, int64_t 
   if (d.M == 0 || d.N == 0 || nbatch == 0) return;
   if (d.K == 0) {
     const int64_t total = d.M * d.N * nbatch;
-    scale_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream>>>(d, nbatch);
+    launch_pdl(scale_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream, d, nbatch);
     VGB_LAUNCH_CHECK();
     return;
   }

@@ -674,6 +674,7 @@ __device__ void real_vectors(const GenEigJob &q, const double *C, const double *
 }
 
 __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_constant__ GenEigGroup g) {
+  pdl_wait();
   const GenEigJob q = g.j[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __shared__ double red[32];
@@ -1020,6 +1021,7 @@ __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_const
 // O = an orthonormal basis of the columns of U (m x r): modified Gram-Schmidt twice, one CTA.
 __global__ void __launch_bounds__(kGenThreads) orthonormalise_kernel(const double *U, int64_t ldu, int64_t m,
                                                                     int64_t r, double *O, int64_t ldo) {
+  pdl_wait();
   __shared__ double red[32];
   for (int64_t t = threadIdx.x; t < m * r; t += kGenThreads) O[(t % m) + ldo * (t / m)] = U[(t % m) + ldu * (t / m)];
   __syncthreads();
@@ -1049,6 +1051,7 @@ __global__ void __launch_bounds__(kGenThreads) orthonormalise_kernel(const doubl
 // status = 1 when S is not positive definite, else 0.
 __global__ void __launch_bounds__(kGenThreads) pencil_reduce_kernel(const double *S, const double *J, int64_t ld,
                                                                    int64_t m, double *W, int *status) {
+  pdl_wait();
   __shared__ int bad;
   double *L = W, *Y = W + m * m, *Mn = W + 2 * m * m;
   if (threadIdx.x == 0) bad = 0;
@@ -1106,6 +1109,7 @@ __global__ void __launch_bounds__(kGenThreads) pencil_reduce_kernel(const double
 // the mu are positive.
 __global__ void pencil_finish_kernel(const double *W, int64_t m, const double *nu, const double *Z, int64_t np,
                                      double *U, double *lam, int *status) {
+  pdl_wait();
   const double *L = W;
   for (int64_t j = threadIdx.x; j < np; j += blockDim.x) {
     if (!(nu[j] < 0.0)) *status = 2;
@@ -1125,13 +1129,13 @@ __global__ void pencil_finish_kernel(const double *W, int64_t m, const double *n
 void pencil_reduce_device(const double *S, const double *J, int64_t ld, int64_t m, double *W, int *status,
                           cudaStream_t s) {
   VGB_REQUIRE(m >= 1 && ld >= m, "pencil_reduce: invalid sizes");
-  pencil_reduce_kernel<<<1, kGenThreads, 0, s>>>(S, J, ld, m, W, status);
+  launch_pdl(pencil_reduce_kernel, 1, kGenThreads, 0, s, S, J, ld, m, W, status);
   VGB_LAUNCH_CHECK();
 }
 
 void pencil_finish_device(const double *W, int64_t m, const double *nu, const double *Z, int64_t np, double *U,
                           double *lam, int *status, cudaStream_t s) {
-  pencil_finish_kernel<<<1, 128, 0, s>>>(W, m, nu, Z, np, U, lam, status);
+  launch_pdl(pencil_finish_kernel, 1, 128, 0, s, W, m, nu, Z, np, U, lam, status);
   VGB_LAUNCH_CHECK();
 }
 
@@ -1169,7 +1173,7 @@ void gen_eig_device(const GenEigJob *jobs, int64_t njobs, cudaStream_t s) {
       need = std::max(need, gen_smem_doubles(jb.m, jb.nw, limit));
     }
     g->smem_doubles = need;
-    gen_eig_kernel<<<g->n, kGenThreads, need * sizeof(double), s>>>(*g);
+    launch_pdl(gen_eig_kernel, g->n, kGenThreads, need * sizeof(double), s, *g);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -1177,7 +1181,7 @@ void gen_eig_device(const GenEigJob *jobs, int64_t njobs, cudaStream_t s) {
 void orthonormalise_device(const double *U, int64_t ldu, int64_t m, int64_t r, double *O, int64_t ldo,
                            cudaStream_t s) {
   VGB_REQUIRE(m >= 1 && r >= 1 && r <= m && ldu >= m && ldo >= m, "orthonormalise: invalid sizes");
-  orthonormalise_kernel<<<1, kGenThreads, 0, s>>>(U, ldu, m, r, O, ldo);
+  launch_pdl(orthonormalise_kernel, 1, kGenThreads, 0, s, U, ldu, m, r, O, ldo);
   VGB_LAUNCH_CHECK();
 }
 

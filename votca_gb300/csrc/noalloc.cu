@@ -60,6 +60,7 @@ __global__ void na_hqp_diag_kernel(double cqp, const double *__restrict__ Hcc,
                                    const double *__restrict__ Hvv, int64_t vt, int64_t ct,
                                    const double *__restrict__ X, int64_t ldx, int64_t k,
                                    double *__restrict__ Y, int64_t ldy) {
+  pdl_wait();
   const int64_t dim = vt * ct, total = dim * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -70,6 +71,7 @@ __global__ void na_hqp_diag_kernel(double cqp, const double *__restrict__ Hcc,
 }
 
 __global__ void na_zero_kernel(double *Y, int64_t ldy, int64_t rows, int64_t k) {
+  pdl_wait();
   const int64_t total = rows * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x)
@@ -110,7 +112,7 @@ void matmul_noalloc(BseOperator &op, const Coef &c, const double *X, int64_t ldx
   bool acc = false;
   if (c.cqp != 0) {
     if (op.hqp_diagonal) {
-      na_hqp_diag_kernel<<<na_grid(dim * k), 256, 0, s>>>(c.cqp, op.Hcc.get(), op.Hvv.get(), vt, ct,
+      launch_pdl(na_hqp_diag_kernel, na_grid(dim * k), 256, 0, s, c.cqp, op.Hcc.get(), op.Hvv.get(), vt, ct,
                                                            X, ldx, k, Y, ldy);
       VGB_LAUNCH_CHECK();
     } else {
@@ -193,7 +195,7 @@ void matmul_noalloc(BseOperator &op, const Coef &c, const double *X, int64_t ldx
     acc = true;
   }
   if (!acc) {
-    na_zero_kernel<<<na_grid(dim * k), 256, 0, s>>>(Y, ldy, dim, k);
+    launch_pdl(na_zero_kernel, na_grid(dim * k), 256, 0, s, Y, ldy, dim, k);
     VGB_LAUNCH_CHECK();
   }
 }

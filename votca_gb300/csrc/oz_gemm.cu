@@ -133,6 +133,7 @@ constexpr int SLICE_SMEM = 256 * (32 + 2) * 8;  // the largest tile: rows x (ele
 __global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant__ Operand oa,
                                                           const __grid_constant__ Operand ob, int units_a, int units,
                                                           int phase, int *flag) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned long long tile[];
   __shared__ unsigned long long red[256];
   __shared__ int s_e[256];
@@ -433,6 +434,7 @@ __device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uin
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_constant__ GemmArgs p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   if (*p.flag > 0) {  // uniform over the grid: set by the slicer, an earlier launch
@@ -662,6 +664,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
 __global__ void oz_reduce_kernel(const double *__restrict__ part, int64_t M, int64_t N, int64_t nbt, int splits,
                                  const OzMap crow, const OzMap ccol, const OzMap cbatch, double *__restrict__ C,
                                  double alpha, double beta) {
+  pdl_wait();
   const int64_t mn = M * N, total = mn * nbt;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const QuotRem tx = quot_rem(t, mn), ex = quot_rem(tx.r, M);
@@ -769,10 +772,10 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
       const int64_t ub = new_b ? ceil_div(B.rows, slice_rows(q.Kp)) * nseg : 0;
       const unsigned sg = (unsigned)std::min<int64_t>(ua + ub, 64LL * sm_count());
       if (two) {
-        oz_slice_kernel<<<sg, 256, SLICE_SMEM, stream>>>(A, B, (int)ua, (int)(ua + ub), 1, ip);
+        launch_pdl(oz_slice_kernel, sg, 256, SLICE_SMEM, stream, A, B, (int)ua, (int)(ua + ub), 1, ip);
         VGB_LAUNCH_CHECK();
       }
-      oz_slice_kernel<<<sg, 256, SLICE_SMEM, stream>>>(A, B, (int)ua, (int)(ua + ub), two ? 2 : 3, ip);
+      launch_pdl(oz_slice_kernel, sg, 256, SLICE_SMEM, stream, A, B, (int)ua, (int)(ua + ub), two ? 2 : 3, ip);
       VGB_LAUNCH_CHECK();
       encode_kmajor(&p.map_a, A.planes, S * A.rows, q.Kp, q.Kp, BM, BK);
       encode_kmajor(&p.map_b, B.planes, S * B.rows, q.Kp, q.Kp, BN, BK);
@@ -789,13 +792,12 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
       p.ntiles = (int)(p.mt * p.nt * tn * q.splits);
       p.m_first = m0;
       p.b_first = t0;
-      oz_gemm_kernel<<<(unsigned)std::min(p.ntiles, sm_count()), kGemmThreads, SMEM_BYTES, stream>>>(p);
+      launch_pdl(oz_gemm_kernel, (unsigned)std::min(p.ntiles, sm_count()), kGemmThreads, SMEM_BYTES, stream, p);
       VGB_LAUNCH_CHECK();
     }
   if (q.splits > 1) {
     const int64_t total = q.nbatch * q.M * q.N;
-    oz_reduce_kernel<<<(unsigned)std::min<int64_t>(ceil_div(total, 256), 8LL * sm_count()), 256, 0, stream>>>(
-        partial, q.M, q.N, q.nbatch, q.splits, q.crow, q.ccol, q.cbatch, d.C, d.alpha, d.beta);
+    launch_pdl(oz_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 8LL * sm_count()), 256, 0, stream, partial, q.M, q.N, q.nbatch, q.splits, q.crow, q.ccol, q.cbatch, d.C, d.alpha, d.beta);
     VGB_LAUNCH_CHECK();
   }
   return true;

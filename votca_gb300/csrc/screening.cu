@@ -30,6 +30,7 @@ unsigned g1d(int64_t n) {
 // -2 chi of the (m, c) pairs: two divisions each, once per pair and not once per (pair, P)
 __global__ void rpa_chi_kernel(const double *energies, int64_t n_occ_chunk, int64_t m0, int64_t n_unocc,
                                int64_t lumo_idx, double wr, double wi, double eta, double *chi2) {
+  pdl_wait();
   const int64_t total = n_occ_chunk * n_unocc;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -48,6 +49,7 @@ __global__ void rpa_chi_kernel(const double *energies, int64_t n_occ_chunk, int6
 // Naux1000: 359 us with the divisions inside, 40 us).
 __global__ void rpa_weights_kernel(const double *raw, int64_t n_unocc, int64_t naux, int64_t nsize, int64_t row0,
                                    const double *chi2, double *B, double *Bw, int64_t ldb, int64_t rows) {
+  pdl_wait();
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {  // r = mi * naux + P
     const QuotRem x = quot_rem(r, naux);
     const int64_t mi = x.q, P = x.r;
@@ -62,6 +64,7 @@ __global__ void rpa_weights_kernel(const double *raw, int64_t n_unocc, int64_t n
 }
 
 __global__ void add_identity_kernel(double *A, int64_t n) {
+  pdl_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     A[i + n * i] += 1.0;
@@ -94,6 +97,7 @@ __device__ __forceinline__ double rsqrt64(double d) {
 __global__ void __launch_bounds__(256) chol_block_kernel(const double *A, int64_t lda, int nb, double *Lo,
                                                          int64_t ldl, double *Li, int64_t ldi, int *info,
                                                          int64_t j0) {
+  pdl_wait();
   __shared__ double colk[NB], rowk[NB], l[NB], rk[NB];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int blk = warp < 4 ? warp : 11 - warp;  // rows 8 blk ..
@@ -187,10 +191,9 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
     }
     const int64_t rows = cnt * n_unocc;
     // Mmn_[m].bottomRows(n_unocc), as the reference reads it
-    rpa_chi_kernel<<<g1d(rows), 256, 0, s>>>(dE.get(), cnt, m0, n_unocc, lumo - rpamin, wr, wi, eta, chi.get());
+    launch_pdl(rpa_chi_kernel, g1d(rows), 256, 0, s, dE.get(), cnt, m0, n_unocc, lumo - rpamin, wr, wi, eta, chi.get());
     VGB_LAUNCH_CHECK();
-    rpa_weights_kernel<<<(unsigned)std::min<int64_t>(cnt * naux, 64LL * sm_count()), 128, 0, s>>>(
-        raw.get(), n_unocc, naux, nsize, nsize - n_unocc, chi.get(), B.get(), Bw.get(), rows, cnt * naux);
+    launch_pdl(rpa_weights_kernel, (unsigned)std::min<int64_t>(cnt * naux, 64LL * sm_count()), 128, 0, s, raw.get(), n_unocc, naux, nsize, nsize - n_unocc, chi.get(), B.get(), Bw.get(), rows, cnt * naux);
     VGB_LAUNCH_CHECK();
     GemmDesc g;  // eps (+)= B^T Bw
     g.M = naux; g.N = naux; g.K = rows;
@@ -199,7 +202,7 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
     dgemm(g, s, &ws);
     VGB_CUDA(cudaStreamSynchronize(s));
   }
-  add_identity_kernel<<<g1d(naux), 256, 0, s>>>(eps.get(), naux);
+  launch_pdl(add_identity_kernel, g1d(naux), 256, 0, s, eps.get(), naux);
   VGB_LAUNCH_CHECK();
   VGB_CUDA(cudaMemcpyAsync(eps_host, eps.get(), naux * naux * sizeof(double), cudaMemcpyDeviceToHost, s));
   VGB_CUDA(cudaStreamSynchronize(s));
@@ -220,7 +223,7 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
   // right-looking blocked Cholesky: A = L L^T (lower), the diagonal blocks' inverses into Y
   for (int64_t j = 0; j < n; j += NB) {
     const int nb = (int)std::min<int64_t>(NB, n - j);
-    chol_block_kernel<<<1, 256, 0, s>>>(A.get() + j + n * j, n, nb, L.get() + j + n * j, n,
+    launch_pdl(chol_block_kernel, 1, 256, 0, s, A.get() + j + n * j, n, nb, L.get() + j + n * j, n,
                                                  Y.get() + j + n * j, n, info.get(), j);
     VGB_LAUNCH_CHECK();
     const int64_t rest = n - j - nb;

@@ -117,6 +117,7 @@ __device__ __forceinline__ void add_levels(int n, float (&kh)[W], float (&kl)[W]
 // here; 5120 x 32 x 32768 460 us, 255 us here (of which 100 us for K runs shared out by waves).
 template <int BN, int S>
 __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __grid_constant__ Args p) {
+  pdl_wait();
   using C = Cfg<BN, S>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
 // Y = epi(sum over the groups' float pairs), part[g][n][i]: a float-pair sum in group order.
 __global__ void reduce_pairs_kernel(const float2 *__restrict__ part, int64_t M, int64_t N, int groups,
                                     const TcEpilogue e) {
+  pdl_wait();
   const int64_t total = M * N;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const QuotRem tx = quot_rem(t, M);
@@ -291,7 +293,7 @@ void launch(const Args &p, cudaStream_t s) {
   std::call_once(attr, [] {
     VGB_CUDA(cudaFuncSetAttribute(slice_gemm_kernel<BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   });
-  slice_gemm_kernel<BN, S><<<(unsigned)std::min(p.nitems, sm_count()), kGemmThreads, C::SMEM, s>>>(p);
+  launch_pdl(slice_gemm_kernel<BN, S>, (unsigned)std::min(p.nitems, sm_count()), kGemmThreads, C::SMEM, s, p);
   VGB_LAUNCH_CHECK();
 }
 
@@ -350,8 +352,7 @@ void slice_gemm(const SliceMat &A, const SliceMat &B, int64_t M, int64_t N, int6
   if (bn == 64) launch_digits<64>(digits, p, s);
   else launch_digits<32>(digits, p, s);
   if (p.groups > 1) {
-    reduce_pairs_kernel<<<(unsigned)std::min<int64_t>(ceil_div(M * N, 256), 16LL * sm_count()), 256, 0, s>>>(
-        reinterpret_cast<const float2 *>(gpart.get()), M, N, p.groups, fe);
+    launch_pdl(reduce_pairs_kernel, (unsigned)std::min<int64_t>(ceil_div(M * N, 256), 16LL * sm_count()), 256, 0, s, reinterpret_cast<const float2 *>(gpart.get()), M, N, p.groups, fe);
     VGB_LAUNCH_CHECK();
   }
 }

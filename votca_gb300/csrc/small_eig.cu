@@ -211,6 +211,7 @@ __device__ void tri_apply_singles(const double *d, const double *e, const double
 }
 
 __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_constant__ SymEigGroup g) {
+  pdl_wait();
   const SymEigJob q = g.j[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t m = q.m, nw = q.nw;
@@ -685,7 +686,7 @@ void sym_eig_device(const SymEigJob *jobs, int64_t njobs, cudaStream_t s) {
       need = std::max(need, job_need);
     }
     g->smem_doubles = need;
-    sym_eig_kernel<<<g->n, kEigThreads, need * sizeof(double), s>>>(*g);
+    launch_pdl(sym_eig_kernel, g->n, kEigThreads, need * sizeof(double), s, *g);
     VGB_LAUNCH_CHECK();
   }
 }

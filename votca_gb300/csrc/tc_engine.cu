@@ -619,6 +619,7 @@ namespace {
 // along P.
 __global__ void transpose_split_cc_kernel(const double *__restrict__ Mcc, int64_t naux, int64_t ct,
                                           uint16_t *__restrict__ hi, uint16_t *__restrict__ lo, int64_t ldo) {
+  pdl_wait();
   __shared__ double tile[32][33];
   const int64_t q0 = (int64_t)blockIdx.x * 32, p0 = (int64_t)blockIdx.y * 32;
   const int64_t nq = ct * ct;
@@ -646,6 +647,7 @@ __global__ void transpose_split_cc_kernel(const double *__restrict__ Mcc, int64_
 // The diagonal is zeroed: the products add the exact FP64 diagonal of the whole operator
 // beside the dense part, so the largest entries are not rounded to bf16 hi/lo.
 __global__ void symmetrize_kernel(double *H, int64_t n) {
+  pdl_wait();
   const int64_t total = n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = t / n, j = t % n;
@@ -730,7 +732,7 @@ void MixedEngine::build_dense_grouped(const std::vector<BseOperator *> &ops, con
       sj.push_back(j1);
       // Bc[(c1, c)][P] = M(c1, c, P) = Mcc[P][c][c1]: a transpose, done through shared memory
       const dim3 grid((unsigned)ceil_div(op.ct * op.ct, 32), (unsigned)ceil_div(op.naux, 32));
-      transpose_split_cc_kernel<<<grid, dim3(32, 8), 0, s>>>(op.Mcc.get(), op.naux, op.ct, Bc.hi.get() + boff[q],
+      launch_pdl(transpose_split_cc_kernel, grid, dim3(32, 8), 0, s, op.Mcc.get(), op.naux, op.ct, Bc.hi.get() + boff[q],
                                                             Bc.lo.get() + boff[q], m.Kn);
       VGB_LAUNCH_CHECK();
     }
@@ -785,8 +787,7 @@ void MixedEngine::build_dense_grouped(const std::vector<BseOperator *> &ops, con
       const size_t q = t - a;
       if (c.cx == 0 && c.cd == 0)
         VGB_CUDA(cudaMemsetAsync(H.get() + hoff[q], 0, op.dim * op.dim * sizeof(double), s));
-      symmetrize_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(op.dim * op.dim, 256), 4096)),
-                          256, 0, s>>>(H.get() + hoff[q], op.dim);
+      launch_pdl(symmetrize_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(op.dim * op.dim, 256), 4096)), 256, 0, s, H.get() + hoff[q], op.dim);
       VGB_LAUNCH_CHECK();
       m.Kd = pad64(op.dim);
       m.Hdense.ensure(op.dim, m.Kd, s);

@@ -132,6 +132,7 @@ static_assert(sizeof(GroupSrc) <= 32000, "grouped GEMM parameters exceed the ker
 
 template <int BN, int BK, class Src>
 __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_constant__ Src src) {
+  pdl_wait();
   using C = Cfg<BN, BK>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -392,6 +393,7 @@ __device__ __forceinline__ void split_range(const double *__restrict__ x, int64_
 __global__ void split_kernel(const double *__restrict__ x, int64_t rows, int64_t cols,
                              const SplitMap m, uint16_t *__restrict__ hi, uint16_t *__restrict__ lo,
                              int64_t ldo) {
+  pdl_wait();
   split_range(x, rows, cols, m, hi, lo, ldo, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
               (int64_t)gridDim.x * blockDim.x);
 }
@@ -408,6 +410,7 @@ struct ReduceGroup {
 static_assert(sizeof(SplitGroup) <= 32000 && sizeof(ReduceGroup) <= 32000, "grouped job lists too large");
 
 __global__ void split_group_kernel(const __grid_constant__ SplitGroup g) {
+  pdl_wait();
   const SplitJob q = g.j[blockIdx.y];
   split_range(q.x, q.rows, q.cols, q.map, q.hi, q.lo, q.ldo,
               blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
@@ -440,6 +443,7 @@ __device__ __forceinline__ void reduce_range(const float *__restrict__ part, int
 
 __global__ void reduce_partials_kernel(const float *__restrict__ part, int64_t M, int64_t N,
                                        int ksplit, const TcEpilogue e) {
+  pdl_wait();
   reduce_range(part, M, N, ksplit, e, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
                (int64_t)gridDim.x * blockDim.x);
 }
@@ -554,6 +558,7 @@ __device__ __forceinline__ void digits(long long rem, int nsl, long long (&d)[kM
 template <class In, int VEC, int NSL>
 __global__ void slice_kernel(const In in, int64_t rows, int64_t cols, const SplitMap m, int nsl_rt, int64_t chunk,
                              uint16_t *__restrict__ out, int64_t ldo, int64_t plane) {
+  pdl_wait();
   const int nsl = NSL > 0 ? NSL : nsl_rt;
   const int lane = threadIdx.x & 31;
   const int64_t nchunks = (cols + chunk - 1) / chunk;
@@ -653,6 +658,7 @@ template <class In, int NSL>
 __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t rows, int64_t cols, const SplitMap m,
                                                         int64_t chunk, uint16_t *__restrict__ out, int64_t ldo,
                                                         int64_t plane) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t nchunks = (cols + chunk - 1) / chunk;
   const int64_t units = rows * nchunks;
@@ -752,6 +758,7 @@ template <int NG>
 __global__ void __launch_bounds__(256) slice_pairs_kernel(const float *__restrict__ x2, int64_t rows, int64_t cols,
                                                           const SplitMap m, int64_t chunk, uint16_t *__restrict__ out,
                                                           int64_t ldo, int64_t plane) {
+  pdl_wait();
   constexpr int S = kMaxDigits;
   const int lane = threadIdx.x & 31;
   const int64_t nchunks = (cols + chunk - 1) / chunk;
@@ -832,6 +839,7 @@ __global__ void __launch_bounds__(256) slice_pairs_kernel(const float *__restric
 }
 
 __global__ void reduce_group_kernel(const __grid_constant__ ReduceGroup g) {
+  pdl_wait();
   const ReduceJob q = g.j[blockIdx.y];
   reduce_range(q.part, q.M, q.N, q.ksplit, q.epi, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
                (int64_t)gridDim.x * blockDim.x);
@@ -846,7 +854,7 @@ void launch_src(const Src &src, int64_t ntiles, cudaStream_t s) {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   });
   const int64_t grid = std::min<int64_t>(ntiles, sm_count());
-  tc_gemm_kernel<BN, BK, Src><<<(unsigned)grid, kThreads, C::SMEM, s>>>(src);
+  launch_pdl(tc_gemm_kernel<BN, BK, Src>, (unsigned)grid, kThreads, C::SMEM, s, src);
   VGB_LAUNCH_CHECK();
 }
 
@@ -1031,7 +1039,7 @@ void split_f64_to_bf16(const double *x, int64_t rows, int64_t cols, const SplitM
                        uint16_t *lo, int64_t ldo, cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return;
   VGB_REQUIRE(m.rdiv >= 1, "split: bad row map");
-  split_kernel<<<grid_1d(rows * cols), 256, 0, s>>>(x, rows, cols, m, hi, lo, ldo);
+  launch_pdl(split_kernel, grid_1d(rows * cols), 256, 0, s, x, rows, cols, m, hi, lo, ldo);
   VGB_LAUNCH_CHECK();
 }
 
@@ -1057,7 +1065,7 @@ void split_grouped(const std::vector<SplitJob> &jobs, cudaStream_t s) {
       mx = std::max(mx, jobs[i].rows * jobs[i].cols);
     }
     if (g->n == 0) continue;
-    split_group_kernel<<<dim3(group_blocks(mx, g->n), (unsigned)g->n), 256, 0, s>>>(*g);
+    launch_pdl(split_group_kernel, dim3(group_blocks(mx, g->n), (unsigned)g->n), 256, 0, s, *g);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -1074,7 +1082,7 @@ void reduce_grouped(const std::vector<ReduceJob> &jobs, cudaStream_t s) {
       mx = std::max(mx, jobs[i].M * jobs[i].N);
     }
     if (g->n == 0) continue;
-    reduce_group_kernel<<<dim3(group_blocks(mx, g->n), (unsigned)g->n), 256, 0, s>>>(*g);
+    launch_pdl(reduce_group_kernel, dim3(group_blocks(mx, g->n), (unsigned)g->n), 256, 0, s, *g);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -1090,10 +1098,10 @@ void slice_f64(const double *x, int64_t rows, int64_t cols, const SplitMap &m, i
   const F64In in{reinterpret_cast<const unsigned long long *>(x)};
   if (m.cs == 1 && chunk % 4 == 0 && m.rs1 % 4 == 0 && m.rs2 % 4 == 0 && ldo % 4 == 0 && plane % 4 == 0 &&
       ((uintptr_t)x & 31) == 0 && ((uintptr_t)out & 7) == 0) {
-    if (nslices == 5) slice_run_kernel<F64In, 5><<<blocks, 256, 0, s>>>(in, rows, cols, m, chunk, out, ldo, plane);
-    else slice_kernel<F64In, 4, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    if (nslices == 5) launch_pdl(slice_run_kernel<F64In, 5>, blocks, 256, 0, s, in, rows, cols, m, chunk, out, ldo, plane);
+    else launch_pdl(slice_kernel<F64In, 4, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
   } else {
-    slice_kernel<F64In, 1, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    launch_pdl(slice_kernel<F64In, 1, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
   }
   VGB_LAUNCH_CHECK();
 }
@@ -1111,7 +1119,7 @@ void slice_pairs(const float *x2, int64_t rows, int64_t cols, const SplitMap &m,
       ((uintptr_t)x2 & 31) == 0 && ((uintptr_t)out & 7) == 0) {
     if (nslices == 5) {
       const int ng = (int)ceil_div(std::min(chunk, cols), 128);
-#define VGB_SLICE(NG) slice_pairs_kernel<NG><<<blocks, 256, 0, s>>>(x2, rows, cols, m, chunk, out, ldo, plane)
+#define VGB_SLICE(NG) launch_pdl(slice_pairs_kernel<NG>, blocks, 256, 0, s, x2, rows, cols, m, chunk, out, ldo, plane)
       switch (ng) {
         case 1: VGB_SLICE(1); break;
         case 2: VGB_SLICE(2); break;
@@ -1122,16 +1130,16 @@ void slice_pairs(const float *x2, int64_t rows, int64_t cols, const SplitMap &m,
         default: VGB_SLICE(8); break;
       }
 #undef VGB_SLICE
-    } else slice_kernel<PairIn, 4, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    } else launch_pdl(slice_kernel<PairIn, 4, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
   } else {
-    slice_kernel<PairIn, 1, 0><<<blocks, 256, 0, s>>>(in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    launch_pdl(slice_kernel<PairIn, 1, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
   }
   VGB_LAUNCH_CHECK();
 }
 
 void reduce_partials(const float *partial, int64_t M, int64_t N, int ksplit, const TcEpilogue &epi,
                      cudaStream_t s) {
-  reduce_partials_kernel<<<grid_1d(M * N), 256, 0, s>>>(partial, M, N, ksplit, epi);
+  launch_pdl(reduce_partials_kernel, grid_1d(M * N), 256, 0, s, partial, M, N, ksplit, epi);
   VGB_LAUNCH_CHECK();
 }
 
