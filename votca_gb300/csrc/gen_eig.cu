@@ -21,6 +21,7 @@
 //      solves a lane each, everything elementwise on the whole block.
 // The matrices stay in shared memory up to m = 97.  m = 44, 10 pairs: 11.4 ms before the lane-wise
 // divisions and scans and the parallel inverse iteration, 4.4 ms with them; the bits are the same.
+#include "fast_fp64.cuh"
 #include "small_eig.cuh"
 
 #include <algorithm>
@@ -86,32 +87,6 @@ __device__ double wsum(double v) {
 constexpr int kQrThreads = 128;
 __device__ __forceinline__ void qr_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kQrThreads) : "memory"); }
 
-// The float nearest below a double in FP32's range and back, in integers (a conversion is an FP64
-// instruction).
-__device__ __forceinline__ float to_float(double x) {
-  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
-  return __uint_as_float((h & 0x80000000u) | (((h & 0x7FFFFFFFu) - (896u << 20)) << 3) | (l >> 29));
-}
-__device__ __forceinline__ double to_double(float x) {  // normal x
-  const unsigned b = __float_as_uint(x);
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
-}
-// 1 / sqrt(x) for x within [1, 64) from the FP32 estimate f, and 1 / x: one step of third order
-// (Householder's iteration, e < 2^-20: y (1 + e/2 + 3 e^2 / 8) and y (1 + e + e^2)), six and three FP64
-// instructions for a square root of 700 and a division of 565 clocks.
-__device__ __forceinline__ double fast_rsqrt(double x, float f) {
-  const double y = to_double(f);
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-__device__ __forceinline__ double fast_rcp(double x, float f) {
-  const double y = to_double(f);
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double with_sign(double a, double b) {  // |a| with b's sign bit
-  return __hiloint2double((__double2hiint(a) & 0x7FFFFFFF) | (__double2hiint(b) & (int)0x80000000), __double2loint(a));
-}
 __device__ __forceinline__ int max_exponent(double p, double q, double r) {
   return max((__double2hiint(p) >> 20) & 0x7FF, max((__double2hiint(q) >> 20) & 0x7FF, (__double2hiint(r) >> 20) & 0x7FF));
 }

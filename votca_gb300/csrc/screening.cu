@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "dgemm.cuh"
+#include "fast_fp64.cuh"
 #include "host_eig.hpp"
 
 namespace vgb {
@@ -68,21 +69,6 @@ __global__ void add_identity_kernel(double *A, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     A[i + n * i] += 1.0;
-}
-
-// 1 / sqrt(d) for d > 0: an FP32 estimate of the mantissa (exponent split off, any FP64 range) and
-// one step of Householder's third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2 < 2^-20:
-// five FP64 instructions instead of a square root and a division (1265 clocks of the pipe).
-__device__ __forceinline__ double rsqrt64(double d) {
-  const long long b = __double_as_longlong(d);
-  const int ex = (int)((b >> 52) & 0x7FF) - 1023;
-  if (ex == -1023) return 1.0 / sqrt(d);  // subnormal
-  const int h = ex >> 1;                  // d = m 4^h, m in [1, 4)
-  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | ((long long)(1023 + (ex & 1)) << 52));
-  const double y = (double)rsqrtf((float)m);
-  const double e = fma(-(m * y), y, 1.0);
-  const double r = fma(y * e, fma(0.375, e, 0.5), y);
-  return __longlong_as_double(__double_as_longlong(r) - ((long long)h << 52));
 }
 
 // Cholesky factor L and its inverse of the nb x nb (<= 64) diagonal block at A (lda), one CTA: the

@@ -1,6 +1,8 @@
 // Small dense symmetric eigenproblems on the device; the method is described in small_eig.cuh.
 #include "small_eig.cuh"
 
+#include "fast_fp64.cuh"
+
 #include <algorithm>
 #include <memory>
 #include <mutex>
@@ -92,6 +94,7 @@ __device__ int sturm_count(const float *d, const float *e2, int64_t m, float x, 
 // subdiagonal entry is larger than the pivot; U has two superdiagonals.  r0 holds 1/U_ii.  Both
 // cases share one division and one update (lanes of a warp take different cases).  ds: the
 // shifted diagonal d - sigma; may be r0 itself (an entry is read before it is written).
+template <bool FAST>
 __device__ void tri_lu(const double *ds, const double *__restrict__ e, int m, double tiny,
                        double *r0, double *__restrict__ u1, double *__restrict__ u2, double *__restrict__ l,
                        double *__restrict__ pv) {
@@ -102,7 +105,7 @@ __device__ void tri_lu(const double *ds, const double *__restrict__ e, int m, do
     const double bn = (i + 2 < m) ? e[i + 1] : 0.0, an1 = (i + 2 < m) ? ds[i + 2] : 0.0;
     const bool keep = abs_bits(da) >= abs_bits(c);
     if (keep && abs_bits(da) < tb) da = negative(da) ? -tiny : tiny;
-    const double r = 1.0 / (keep ? da : c);  // one division per row
+    const double r = FAST ? rcp64(keep ? da : c) : 1.0 / (keep ? da : c);  // one division per row
     const double li = (keep ? c : da) * r;
     r0[i] = r; l[i] = li;
     u1[i] = keep ? db : an;
@@ -153,12 +156,13 @@ __device__ void tri_solve(int m, const double *__restrict__ r0, const double *__
   }
 }
 
-__device__ double vnorm(const double *z, int64_t m) {
+__device__ double vdot(const double *z, int64_t m) {
   double s = 0.0;
 #pragma unroll 4
   for (int i = 0; i < m; ++i) s = fma(z[i], z[i], s);
-  return sqrt(s);
+  return s;
 }
+__device__ double vnorm(const double *z, int64_t m) { return sqrt(vdot(z, m)); }
 __device__ void vscale(double *z, int64_t m, double f) {
   for (int64_t i = 0; i < m; ++i) z[i] *= f;
 }
@@ -252,6 +256,8 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
   __syncthreads();
 
   // ---- 1. Householder tridiagonalisation ----
+  // fast (FP64 solves): square roots and divisions by rsqrt64 and rcp64, 781 to 753 us for the three
+  // problems of a ten-root solve; split-precision solves keep the divisions and their bits.
   // Scalars are computed by warp 0 alone and broadcast; the two divisions of a reflector share an
   // instruction; the four interleaved chains of a row of A v run in four threads.
   __shared__ double sc[4], scl[kEigThreads];
@@ -268,12 +274,19 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
       if (xn2 == 0.0) {
         if (lane == 0) { tau[k] = 0.0; e[k] = alpha; d[k] = A[k + ld * k]; sc[2] = 0.0; }
       } else {
-        const double beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-        // tau = (beta - alpha) / beta in lane 0, 1 / (alpha - beta) in lane 1
-        const double diff = lane == 0 ? beta - alpha : alpha - beta;
-        const double v = (lane == 0 ? diff : 1.0) / (lane == 0 ? beta : diff);
-        if (lane < 2) sc[lane] = v;
-        if (lane == 0) { tau[k] = v; e[k] = beta; d[k] = A[k + ld * k]; sc[2] = 1.0; }
+        // beta = -|(alpha, x)| sign(alpha), tau = (beta - alpha) / beta, 1 / (alpha - beta)
+        if (q.fast) {
+          const double n2 = alpha * alpha + xn2, rs = rsqrt64(n2);
+          const double beta = -with_sign(n2 * rs, alpha), diff = alpha - beta;
+          const double t = diff * with_sign(rs, alpha), r = rcp64(diff);
+          if (lane == 0) { sc[0] = t; sc[1] = r; tau[k] = t; e[k] = beta; d[k] = A[k + ld * k]; sc[2] = 1.0; }
+        } else {
+          const double beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
+          const double diff = lane == 0 ? beta - alpha : alpha - beta;
+          const double v = (lane == 0 ? diff : 1.0) / (lane == 0 ? beta : diff);
+          if (lane < 2) sc[lane] = v;
+          if (lane == 0) { tau[k] = v; e[k] = beta; d[k] = A[k + ld * k]; sc[2] = 1.0; }
+        }
       }
     }
     __syncthreads();
@@ -447,11 +460,15 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
         __syncthreads();
         shift_singles(d, m, cl, cb, ncl, scl, scratch);
         __syncthreads();
-        if (single) tri_lu(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
+        if (single) {
+          if (q.fast) tri_lu<true>(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
+          else tri_lu<false>(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
+        }
         for (int st = 0; st < 2; ++st) {
           if (single) {
             tri_solve((int)m, r0, u1, u2, l, pv, z);
-            scl[tid] = 1.0 / vnorm(z, m);
+            const double zz = vdot(z, m);
+            scl[tid] = q.fast ? rsqrt64(zz) : 1.0 / sqrt(zz);
           } else {
             scl[tid] = 1.0;
           }
@@ -482,7 +499,7 @@ __global__ void __launch_bounds__(kEigThreads, 2) sym_eig_kernel(const __grid_co
       double *z = Z + ldz * jj;
       start_vector(z, m, jj);
       for (int64_t i = 0; i < m; ++i) r0[i] = d[i] - (double)lam32[jj];
-      tri_lu(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
+      tri_lu<false>(r0, e, (int)m, tiny, r0, u1, u2, l, pv);
       for (int st = 0; st < 5; ++st) {
         tri_solve((int)m, r0, u1, u2, l, pv, z);
         for (int64_t kk = j0; kk < jj; ++kk) {  // earlier members of the cluster

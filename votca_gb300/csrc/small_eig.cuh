@@ -42,6 +42,7 @@ struct SymEigJob {
   double *work = nullptr;     // sym_eig_work_doubles(m, nw) doubles of device scratch
   int *info = nullptr;        // may be null; set nonzero when the job's sizes are invalid
   long long *clocks = nullptr;  // may be null; 5 SM clock readings at the phase boundaries
+  bool fast = false;          // reflectors and factors without divisions (last bits differ)
 };
 
 // Device scratch one job needs.
