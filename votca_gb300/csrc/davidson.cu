@@ -32,15 +32,18 @@ unsigned blocks_for(int64_t n, int threads = 256) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, threads), 16LL * 152));
 }
 
-// out[c] = sum of A[:, c] * B[:, c] (its root with take_sqrt): the sums of kRedChunks chunks of rows,
-// one per block, are added in chunk order by the column's last block.  arrived[c] counts the
-// column's blocks and is back at zero afterwards.
+// out[c] = sum of A[:, c] * B[:, c] (its root with take_sqrt): the sums of gridDim.x chunks of rows, one
+// per block, are added by the column's last block.  arrived[c] counts the column's blocks and is
+// back at zero afterwards.  fast (FP64 solves): chunks of 512 rows, added pairwise; otherwise
+// kRedChunks chunks, added in chunk order by one thread (64 dependent additions of 75 clocks; the
+// bits of split-precision solves).
 __global__ void coldot_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ B, int64_t ldb,
-                              int64_t n, double *__restrict__ partial, unsigned *arrived, int take_sqrt,
+                              int64_t n, double *__restrict__ partial, unsigned *arrived, int take_sqrt, int fast,
                               double *__restrict__ out) {
   pdl_wait();
   const int64_t c = blockIdx.y;
-  const int64_t chunk = ceil_div(n, kRedChunks);
+  const int chunks = (int)gridDim.x;
+  const int64_t chunk = ceil_div(n, chunks);
   const int64_t r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
   const double *a = A + c * lda, *b = B + c * ldb;
   double s = 0.0;
@@ -53,22 +56,28 @@ __global__ void coldot_kernel(const double *__restrict__ A, int64_t lda, const d
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    __stcg(partial + c * kRedChunks + blockIdx.x, red[0]);
-    __threadfence();
-    last = atomicInc(arrived + c, kRedChunks - 1) == kRedChunks - 1;
+  if (chunks > 1) {
+    if (threadIdx.x == 0) {
+      __stcg(partial + c * kRedChunks + blockIdx.x, red[0]);
+      __threadfence();
+      last = atomicInc(arrived + c, chunks - 1) == chunks - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    if (threadIdx.x < kRedChunks) {
+      __threadfence();
+      red[threadIdx.x] = threadIdx.x < chunks ? __ldcg(partial + c * kRedChunks + threadIdx.x) : 0.0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  if (!last) return;
-  if (threadIdx.x < kRedChunks) {
-    __threadfence();
-    red[threadIdx.x] = __ldcg(partial + c * kRedChunks + threadIdx.x);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32 && fast && chunks > 1) {
+    double t = red[threadIdx.x] + red[threadIdx.x + 32];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) out[c] = take_sqrt ? sqrt(t) : t;
+  } else if (threadIdx.x == 0) {
     double t = 0.0;
 #pragma unroll 8
-    for (int k = 0; k < kRedChunks; ++k) t += red[k];
+    for (int k = 0; k < chunks; ++k) t += red[k];
     out[c] = take_sqrt ? sqrt(t) : t;
   }
 }
@@ -307,9 +316,11 @@ struct Ctx {
       red_arrived.resize(ncols);
       VGB_CUDA(cudaMemsetAsync(red_arrived.get(), 0, ncols * sizeof(unsigned), s));
     }
-    dim3 grid(kRedChunks, (unsigned)ncols);
+    const bool fast = gemm_path == 0;
+    dim3 grid(fast ? (unsigned)std::max<int64_t>(1, std::min<int64_t>(kRedChunks, ceil_div(n, 512))) : kRedChunks,
+              (unsigned)ncols);
     launch_pdl(coldot_kernel, grid, 256, 0, s, A, lda, B ? B : A, B ? ldb : lda, n, red_partial.get(), red_arrived.get(),
-                                       sqrt_ ? 1 : 0, out);
+                                       sqrt_ ? 1 : 0, fast ? 1 : 0, out);
     VGB_LAUNCH_CHECK();
   }
   void scale_cols(double *A, int64_t lda, int64_t ncols, const double *norms) {
