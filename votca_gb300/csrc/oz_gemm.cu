@@ -420,8 +420,8 @@ __device__ __noinline__ void fma_tile(const GemmArgs &p, const Tile &tc, double 
 
 // Persistent kernel, one CTA per SM.  A stage holds the seven A planes (128 rows) and the seven B
 // planes (64 rows) of 32 K elements: every plane is loaded once for its 34 pair products, 48
-// bytes per clock and SM at the full MMA rate (a stage per pair group, as the slice mode of
-// tc_gemm.cu, loads 96).  One MMA multiplies A plane a with up to four stacked B planes
+// bytes per clock and SM at the full MMA rate (a stage per pair group would
+// load 96).  One MMA multiplies A plane a with up to four stacked B planes
 // b .. b + 3 into the adjacent accumulators of levels a + b .. a + b + 3: the TMEM column of a
 // product is its level, so the pairs of a level add up in the tensor core.  Levels 0..3 (H) are
 // issued before levels 4..7 (L) in every stage, and the epilogue drains H while the MMAs of L
