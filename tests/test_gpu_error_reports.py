@@ -1,0 +1,78 @@
+"""A bounded wait of the tensor-core FP64 products that gives up leaves a code in a page-locked slot of
+the workspace.  Every call that waits for its products must return it as BSE_ERR_TIMEOUT, and only
+that call.  The code is planted from the host here; no wait runs out."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import native
+from votca_gb300 import _lib
+from votca_gb300 import bse_operator as bo
+from votca_gb300.synthetic import Problem
+
+pytestmark = pytest.mark.gpu
+
+TIMEOUT = 4
+P = lambda a: a.ctypes.data_as(_lib.c_dp)
+I4 = ctypes.c_int32 * 4
+
+
+def _context(seed=5, v=4, c=20, naux=30, precision=bo.PRECISION_FP64):
+    p = Problem(v=v, c=c, naux=naux, nmo=v + c, seed=seed)
+    opt = bo.BSEOperator_Options(homo=v - 1, rpamin=0, qpmin=0, vmin=0, cmax=v + c - 1)
+    return bo.GpuBSEContext(p.w, bo.TCMatrix_gwbse(p.mmn), p.hqp, opt, precision=precision)
+
+
+def _plant(ctx, code=13):
+    native.load().shim_plant_error(ctx.handle, code)
+
+
+def _times_out(call):
+    with pytest.raises(_lib.BSEError) as e:
+        call()
+    assert e.value.code == TIMEOUT
+
+
+def _vectors(ctx, k, seed=1):
+    return np.asfortranarray(np.random.default_rng(seed).standard_normal((ctx.size, k)))
+
+
+@pytest.mark.parametrize("full", [False, True])
+def test_gradient(full):
+    ctx = _context()
+    X, Y, g = _vectors(ctx, 2), 0.1 * _vectors(ctx, 2, 2), np.ones(2)
+    gw = np.zeros(30)
+
+    def call():
+        if full:
+            _lib.check(ctx._L.bse_op_eig_gradient_full(ctx.handle, I4(1, 2, 1, 0), I4(0, 2, 0, 1), P(X), P(Y), ctx.size,
+                                                       2, P(g), None, None, P(gw)))
+        else:
+            _lib.check(ctx._L.bse_op_eig_gradient(ctx.handle, 1, 2, 1, 0, P(X), ctx.size, 2, P(g), None, None, P(gw)))
+
+    call()
+    _plant(ctx)
+    _times_out(call)
+    call()
+    ctx.close()
+
+
+def test_gradient_device():
+    import torch
+
+    ctx = _context()
+    X = torch.from_numpy(_vectors(ctx, 2).T.copy()).cuda()
+    gw = torch.zeros(30, dtype=torch.float64, device="cuda")
+    g = np.ones(2)
+
+    def call():
+        _lib.check(ctx._L.bse_op_eig_gradient_device(ctx.handle, I4(1, 2, 1, 0), None, X.data_ptr(), None, ctx.size, 2,
+                                                     P(g), None, None, None, None, None, gw.data_ptr(),
+                                                     torch.cuda.current_stream().cuda_stream))
+
+    call()
+    _plant(ctx)
+    _times_out(call)
+    call()
+    ctx.close()

@@ -402,6 +402,7 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
     }
   }
   VGB_CUDA(cudaStreamSynchronize(s));
+  check_errors(s);  // the products' bounded waits
 }
 
 }  // namespace vgb
