@@ -18,4 +18,6 @@ def load():
     subprocess.run([build.nvcc(), "-std=c++17", "-O1", "-shared", "-Xcompiler", "-fPIC",
                     os.path.join(HERE, "native_shim.cpp"), "-o", so, "-L" + d, "-lvotca_gb300",
                     "-Xlinker", "-rpath=" + d], check=True)
-    return ctypes.CDLL(so)
+    L = ctypes.CDLL(so)
+    L.shim_last_error.restype = ctypes.c_char_p
+    return L

@@ -76,3 +76,21 @@ def test_gradient_device():
     _times_out(call)
     call()
     ctx.close()
+
+
+def test_dense_screening_staging():
+    v, c, naux = 4, 20, 30
+    p = Problem(v=v, c=c, naux=naux, nmo=v + c, seed=5)
+    M = bo.TCMatrix_gwbse(p.mmn)
+    d = _lib.bse_mmn_desc(M.auxsize(), M.get_mmin(), M.get_mmax(), M.get_nmin(), M.get_nmax())
+    ptrs = (_lib.c_dp * M.msize())(*[ctypes.cast(M.data.ctypes.data + m * M.data.strides[0], _lib.c_dp)
+                                     for m in range(M.msize())])
+    W = np.asfortranarray(np.diag(p.w))
+    h = np.asfortranarray(p.hqp)
+    o = _lib.bse_options(v - 1, 0, 0, 0, v + c - 1)
+    L = native.load()
+    run = lambda code: L.shim_stage_dense_screening(ctypes.byref(d), ptrs, P(W), P(h), ctypes.c_int64(h.shape[0]),
+                                                    ctypes.byref(o), code)
+    assert run(0) == 0, L.shim_last_error()
+    assert run(13) == TIMEOUT
+    assert run(0) == 0

@@ -483,6 +483,7 @@ void BseOperator::stage(const bse_mmn_desc &desc, const double *const *slices, c
                                cudaMemcpyDeviceToDevice, s));
     }
     VGB_CUDA(cudaStreamSynchronize(s));
+    ws.check();
   }
   launch_pdl(dvv_from_gvv_kernel, grid_for(naux * vt), 256, 0, s, Gvv.get(), naux, vt, dvv.get());
   VGB_LAUNCH_CHECK();
