@@ -61,4 +61,15 @@ int shim_stage_dense_screening(const bse_mmn_desc *d, const double *const *slice
   });
 }
 
+// The same for an unrestricted operator with this Mmn in both spins, the code in its cross-spin products.
+int shim_stage_dense_screening_uks(const bse_mmn_desc *d, const double *const *slices, const double *w,
+                                   const double *hqp, int64_t nh, const bse_options *opt, int code) {
+  return on_stream([&](cudaStream_t s) {
+    vgb::UksOperator op;
+    *op.workspace().error_slot() = code;
+    const bse_uks_options o = {opt->homo, opt->homo, opt->rpamin, opt->qpmin, opt->vmin, opt->cmax};
+    op.stage(*d, slices, *d, slices, w, true, hqp, nh, nh, hqp, nh, nh, o, BSE_PRECISION_FP64, s);
+  });
+}
+
 }  // extern "C"

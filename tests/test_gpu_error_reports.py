@@ -78,7 +78,8 @@ def test_gradient_device():
     ctx.close()
 
 
-def test_dense_screening_staging():
+@pytest.mark.parametrize("name", ["shim_stage_dense_screening", "shim_stage_dense_screening_uks"])
+def test_dense_screening_staging(name):
     v, c, naux = 4, 20, 30
     p = Problem(v=v, c=c, naux=naux, nmo=v + c, seed=5)
     M = bo.TCMatrix_gwbse(p.mmn)
@@ -89,8 +90,8 @@ def test_dense_screening_staging():
     h = np.asfortranarray(p.hqp)
     o = _lib.bse_options(v - 1, 0, 0, 0, v + c - 1)
     L = native.load()
-    run = lambda code: L.shim_stage_dense_screening(ctypes.byref(d), ptrs, P(W), P(h), ctypes.c_int64(h.shape[0]),
-                                                    ctypes.byref(o), code)
+    run = lambda code: getattr(L, name)(ctypes.byref(d), ptrs, P(W), P(h), ctypes.c_int64(h.shape[0]), ctypes.byref(o),
+                                        code)
     assert run(0) == 0, L.shim_last_error()
     assert run(13) == TIMEOUT
     assert run(0) == 0

@@ -112,6 +112,7 @@ void UksOperator::stage(const bse_mmn_desc &desc_a, const double *const *slices_
       dgemm(g, s, &ws_);
       VGB_CUDA(cudaMemcpyAsync(Y->get(), tmp.get(), rc * naux * sizeof(double), cudaMemcpyDeviceToDevice, s));
       VGB_CUDA(cudaStreamSynchronize(s));
+      ws_.check();
     }
   }
 }

@@ -45,6 +45,7 @@ class UksOperator {
   void ham_matmul(const Coef &a, const Coef &b, const double *X, int64_t ldx, int64_t k, double *Y,
                   int64_t ldy, cudaStream_t s);
   void check_errors(cudaStream_t s);
+  GemmWorkspace &workspace() { return ws_; }  // of the cross-spin products
 
  private:
   DeviceBuffer<double> Z_, U_, hamA_, hamB_, hamX_;
