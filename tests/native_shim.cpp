@@ -3,6 +3,7 @@
 #include <string>
 
 #include "../votca_gb300/csrc/handle.cuh"
+#include "../votca_gb300/csrc/tc_engine.cuh"
 
 namespace {
 
@@ -49,6 +50,13 @@ const char *shim_last_error() { return g_error.c_str(); }
 void shim_plant_error(bse_handle *h, int code) {
   vgb::GemmWorkspace &ws = h->kind == 0 ? h->bse->ws : h->kind == 1 ? h->dense->ws : h->uks->alpha.ws;
   *ws.error_slot() = code;
+}
+
+// The same for the handle's split-precision engine.
+int shim_plant_engine_error(bse_handle *h, int code) {
+  return guarded([&] {
+    VGB_CUDA(cudaMemcpy(h->bse->mixed->error_flag(), &code, sizeof(int), cudaMemcpyHostToDevice));
+  });
 }
 
 // Staging with a dense screening after such a code.

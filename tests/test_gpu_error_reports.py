@@ -9,6 +9,7 @@ import pytest
 import native
 from votca_gb300 import _lib
 from votca_gb300 import bse_operator as bo
+from votca_gb300.davidson import DavidsonSolver
 from votca_gb300.synthetic import Problem
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +96,48 @@ def test_dense_screening_staging(name):
     assert run(0) == 0, L.shim_last_error()
     assert run(13) == TIMEOUT
     assert run(0) == 0
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_lockstep_batch(which):
+    """Every molecule's products, whichever place it has in the batch."""
+    ctxs = [_context(seed=s, c=c) for s, c in ((5, 20), (6, 31), (7, 12))]
+    ops = [bo.SingletOperator_TDA(x) for x in ctxs]
+
+    def call():
+        ds = DavidsonSolver()
+        ds.set_tolerance(1e-7)
+        return ds.solve_batch(ops, 2)
+
+    ref = call()[0]
+    _plant(ctxs[which])
+    _times_out(call)
+    np.testing.assert_array_equal(call()[0], ref)
+    for x in ctxs:
+        x.close()
+
+
+@pytest.mark.parametrize("which", ["dense", "factorised"])
+def test_lockstep_batch_engines(which):
+    """The grouped tensor-core products report into the first engine of their group, which need not be
+    the first molecule's: an FP64 molecule first, then one without a dense form (off-diagonal Hqp)
+    and one with it."""
+    p = Problem(v=4, c=18, naux=30, nmo=22, seed=6)
+    h = p.hqp.copy()
+    h[5, 6] = h[6, 5] = 1e-3
+    opt = bo.BSEOperator_Options(homo=3, rpamin=0, qpmin=0, vmin=0, cmax=21)
+    ctxs = [_context(seed=5), bo.GpuBSEContext(p.w, bo.TCMatrix_gwbse(p.mmn), h, opt, precision=bo.PRECISION_MIXED),
+            _context(seed=7, c=16, precision=bo.PRECISION_MIXED)]
+    ops = [bo.SingletOperator_TDA(x) for x in ctxs]
+
+    def call():
+        ds = DavidsonSolver()
+        ds.set_tolerance(1e-5)
+        return ds.solve_batch(ops, 2)
+
+    call()
+    native.load().shim_plant_engine_error(ctxs[2 if which == "dense" else 1].handle, 3)
+    _times_out(call)
+    call()
+    for x in ctxs:
+        x.close()

@@ -1039,7 +1039,20 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
       std::vector<int> hflags(2 * nm);
       VGB_CUDA(cudaMemcpyAsync(hflags.data(), flags.get(), 2 * nm * sizeof(int), cudaMemcpyDeviceToHost, s));
       VGB_CUDA(cudaStreamSynchronize(s));
-      act.front()->op->check_errors(s);  // grouped tensor-core stages report into the first engine
+      // Bounded waits that gave up: every operator's own FP64 products, the engines of operators that
+      // are applied one by one, and of the first dense and the first factorised operator, which the
+      // grouped stages report into.
+      bool seen[2] = {false, false};
+      for (Mol *M : act) {
+        BseOperator &op = *M->op;
+        const bool grouped = op.precision == BSE_PRECISION_MIXED && op.mixed;
+        if (grouped && seen[M->dense]) {
+          op.ws.check();
+          continue;
+        }
+        op.check_errors(s);
+        if (grouped) seen[M->dense] = true;
+      }
       for (size_t b = 0; b < nm; ++b) {
         if (hflags[b]) fail(BSE_ERR_NUMERICAL, "molecule " + std::to_string(b) + ": Linear dependencies in Gram-Schmidt.");
         if (hflags[nm + b]) fail(BSE_ERR_NUMERICAL, "molecule " + std::to_string(b) + ": Small hermitian eigenvalue problem failed.");

@@ -204,6 +204,8 @@ void MixedEngine::stage(BseOperator &op, cudaStream_t s, bool split_operands) {
   VGB_CUDA(cudaStreamSynchronize(s));
 }
 
+int *MixedEngine::error_flag() const { return impl_->err.get(); }
+
 void MixedEngine::check(cudaStream_t s) {
   int h = 0;
   VGB_CUDA(cudaMemcpyAsync(&h, impl_->err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -54,6 +54,7 @@ class MixedEngine {
   static void prepare_grouped(const std::vector<BseOperator *> &ops, int64_t kmax, cudaStream_t s);
   // Synchronise and raise if a kernel reported a bounded-wait timeout.
   void check(cudaStream_t s);
+  int *error_flag() const;  // device int that such a kernel sets
 
  private:
   struct Impl;
