@@ -141,3 +141,21 @@ def test_lockstep_batch_engines(which):
     call()
     for x in ctxs:
         x.close()
+
+
+def test_dense_forms_are_not_kept_after_an_error():
+    """The dense forms of a batch are built on its first solve, with the smallest operator's engine."""
+    ctxs = [_context(seed=5, c=24, precision=bo.PRECISION_MIXED), _context(seed=7, c=16, precision=bo.PRECISION_MIXED)]
+    ops = [bo.SingletOperator_TDA(x) for x in ctxs]
+
+    def call():
+        ds = DavidsonSolver()
+        ds.set_tolerance(1e-5)
+        return ds.solve_batch(ops, 2)
+
+    native.load().shim_plant_engine_error(ctxs[1].handle, 3)
+    _times_out(call)
+    evals, info, _ = call()
+    assert all(i == "Success" for i in info)
+    for x in ctxs:
+        x.close()

@@ -805,7 +805,7 @@ void MixedEngine::build_dense_grouped(const std::vector<BseOperator *> &ops, con
       hj.push_back(j);
     }
     split_grouped(hj, s);
-    VGB_CUDA(cudaStreamSynchronize(s));  // the slice temporaries are freed next
+    todo[0]->mixed->check(s);  // synchronises: the slice temporaries are freed next
     for (size_t t = a; t < b; ++t) {
       Impl &m = *todo[t]->mixed->impl_;
       m.dense_ready = true;
