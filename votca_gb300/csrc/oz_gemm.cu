@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
       for (int j = 0; j < EC; ++j) h1[j] = l1[j] = h2[j] = l2[j] = 0.f;
       for (int i = 0; i < n; ++i) {
         if ((i + 1) % HB == 0 || i + 1 == n) {
-          if (!mbar_wait(&accf[0], ph, abort_flag, p.err, 14)) goto epi_done;
+          if (!mbar_wait_warp(&accf[0], ph, abort_flag, p.err, 14)) goto epi_done;
           ph ^= 1;
           fence_after();
           add_level(h1, l1, tl);
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
           if (lane == 0) mbar_arrive(&acce[0]);
         }
         if ((i + 1) % LB == 0 || i + 1 == n) {
-          if (!mbar_wait(&accf[1], pl, abort_flag, p.err, 17)) goto epi_done;
+          if (!mbar_wait_warp(&accf[1], pl, abort_flag, p.err, 17)) goto epi_done;
           pl ^= 1;
           fence_after();
           add_low(l2, tl + 448);
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
           if (lane == 0) mbar_arrive(&acce[1]);
         }
       }
-      if (!mbar_wait(&tabf[it & 1], (it >> 1) & 1, abort_flag, p.err, 19)) goto epi_done;
+      if (!mbar_wait_warp(&tabf[it & 1], (it >> 1) & 1, abort_flag, p.err, 19)) goto epi_done;
       const TileTab &tb = tabs[it & 1];
       const int64_t ro = tb.row[q * 32 + lane];
       if (ro >= 0) {

@@ -231,14 +231,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
       for (int i = 0; i < it.n_kb; ++i) {
         dr.step(p.run);
         if (!dr.last) continue;
-        if (!mbar_wait(&accf[hb], ph, abort_flag, p.err, 4)) goto epi_done;
+        if (!mbar_wait_warp(&accf[hb], ph, abort_flag, p.err, 4)) goto epi_done;
         fence_after();
         add_levels<BN>(C::H, kh, kl, tl + (uint32_t)(hb ? C::H1 : 0));
         fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&acce[hb]);
         if constexpr (C::L > 0) {
-          if (!mbar_wait(&accf[2], pl, abort_flag, p.err, 7)) goto epi_done;
+          if (!mbar_wait_warp(&accf[2], pl, abort_flag, p.err, 7)) goto epi_done;
           pl ^= 1;
           fence_after();
           add_levels<BN>(C::L, kh, kl, tl + (uint32_t)C::HW);

@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       // partial offset: the K split (F32 partials); none with kacc
       const int64_t rbase = ix.q * e.ro1 + ix.r * e.ro2 + tc.b * e.bo + (p.kacc ? 0 : tc.s * e.so);
       for (int64_t u = 0; u < len; ++u, ++tc.s) {
-      if (!mbar_wait(&accf[buf], aphase, abort_flag, err, 4)) goto epi_done;
+      if (!mbar_wait_warp(&accf[buf], aphase, abort_flag, err, 4)) goto epi_done;
       fence_after();
       if constexpr (BN <= 64) {
         if (p.kacc) {

@@ -58,6 +58,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     }
   }
 }
+// The same for a warp that goes on together: TMEM loads need all of its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err,
+                                               int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint64_t *bar,
                                             int x, int y) {
   asm volatile(
