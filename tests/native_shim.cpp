@@ -1,8 +1,9 @@
 // C entries into the C++ core for tests that the C ABI does not reach: error codes planted on the host
-// in place of a device wait that gave up.
+// in place of a device wait that gave up, and single FP64 products.
 #include <string>
 
 #include "../votca_gb300/csrc/handle.cuh"
+#include "../votca_gb300/csrc/oz_gemm.cuh"
 #include "../votca_gb300/csrc/tc_engine.cuh"
 
 namespace {
@@ -39,6 +40,19 @@ int on_stream(F &&f) {
     cudaStreamDestroy(s);
   });
 }
+
+template <class T>
+struct Dev : vgb::DeviceBuffer<T> {
+  cudaStream_t s;
+  Dev(const T *h, int64_t n, cudaStream_t s_) : vgb::DeviceBuffer<T>((size_t)n), s(s_) {
+    if (h) VGB_CUDA(cudaMemcpyAsync(this->get(), h, n * sizeof(T), cudaMemcpyHostToDevice, s));
+    else VGB_CUDA(cudaMemsetAsync(this->get(), 0, n * sizeof(T), s));
+  }
+  void read(T *h, int64_t n) {
+    VGB_CUDA(cudaMemcpyAsync(h, this->get(), n * sizeof(T), cudaMemcpyDeviceToHost, s));
+    VGB_CUDA(cudaStreamSynchronize(s));
+  }
+};
 
 }  // namespace
 
@@ -77,6 +91,27 @@ int shim_stage_dense_screening_uks(const bse_mmn_desc *d, const double *const *s
     *op.workspace().error_slot() = code;
     const bse_uks_options o = {opt->homo, opt->homo, opt->rpamin, opt->qpmin, opt->vmin, opt->cmax};
     op.stage(*d, slices, *d, slices, w, true, hqp, nh, nh, hqp, nh, nh, o, BSE_PRECISION_FP64, s);
+  });
+}
+
+// A strided batched product on the tensor-core path; d: M, N, K, nb1, nb2, a_rs, a_cs, a_b1, a_b2,
+// b_rs, b_cs, b_b1, b_b2, c_rs, c_cs, c_b1, c_b2; wait_us: the limit of its waits; *taken: whether that
+// path took it.
+int shim_oz_dgemm(const int64_t *v, const double *A, int64_t na, const double *B, int64_t nb, double *C, int64_t nc,
+                  double alpha, double beta, int wait_us, int *taken) {
+  return on_stream([&](cudaStream_t s) {
+    Dev<double> a(A, na, s), b(B, nb, s), c(C, nc, s);
+    vgb::GemmWorkspace ws;
+    ws.wait_us = wait_us;
+    vgb::GemmDesc d;
+    d.M = v[0]; d.N = v[1]; d.K = v[2]; d.nb1 = v[3]; d.nb2 = v[4];
+    d.A = a.get(); d.a_rs = v[5]; d.a_cs = v[6]; d.a_b1 = v[7]; d.a_b2 = v[8];
+    d.B = b.get(); d.b_rs = v[9]; d.b_cs = v[10]; d.b_b1 = v[11]; d.b_b2 = v[12];
+    d.C = c.get(); d.c_rs = v[13]; d.c_cs = v[14]; d.c_b1 = v[15]; d.c_b2 = v[16];
+    d.alpha = alpha; d.beta = beta;
+    *taken = vgb::oz_dgemm(d, s, &ws) ? 1 : 0;
+    c.read(C, nc);
+    ws.check();
   });
 }
 

@@ -159,3 +159,27 @@ def test_dense_forms_are_not_kept_after_an_error():
     assert all(i == "Success" for i in info)
     for x in ctxs:
         x.close()
+
+
+@pytest.mark.parametrize("M,N,K", [(640, 64, 512), (2000, 130, 230), (300, 40, 4000)])
+def test_wait_limit(M, N, K):
+    """Waits that give up at once, with loads and MMAs in flight: an error, and the next product is right."""
+    L = native.load()
+    rng = np.random.default_rng(M)
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    v = np.array([M, N, K, 1, 1, K, 1, 0, 0, N, 1, 0, 0, N, 1, 0, 0], dtype=np.int64)
+
+    def run(us):
+        C, taken = np.zeros((M, N)), ctypes.c_int()
+        n = lambda a: ctypes.c_int64(a.size)
+        rc = L.shim_oz_dgemm(P(v.view(np.float64)), P(A), n(A), P(B), n(B), P(C), n(C), ctypes.c_double(1.0),
+                             ctypes.c_double(0.0), us, ctypes.byref(taken))
+        assert taken.value == 1
+        return rc, C
+
+    assert run(0)[0] == TIMEOUT
+    rc, C = run(2000000)
+    assert rc == 0
+    bound = K * 2.0**-53 * np.abs(A).max(axis=1)[:, None] * np.abs(B).max(axis=0)[None, :]
+    ref = A.astype(np.longdouble) @ B.astype(np.longdouble)
+    assert np.all(np.abs(C - ref) <= bound + 2.0**-52 * np.abs(ref))

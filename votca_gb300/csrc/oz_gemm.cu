@@ -273,6 +273,7 @@ struct GemmArgs {
   double alpha, beta;
   int alpha_exp, alpha_pow2; // alpha = +-2^alpha_exp
   int accumulate;            // beta != 0 (an FP64 comparison costs what an FMA does)
+  int wait_us;               // limit of the waits
   int plain;                 // neither alpha (a power of two) nor beta costs FP64 work per element
   int *err;
 };
@@ -448,8 +449,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
   uint64_t *acce = accf + 2;        // drained
   uint64_t *tabf = acce + 2;        // table of a tile ready / read, two deep
   uint64_t *tabe = tabf + 2;
-  uint32_t *tmem_slot = (uint32_t *)(tabe + 2);
-  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  TcControl *ctl = (TcControl *)(tabe + 2);
+  volatile int *abort_flag = &ctl->abort;
   TileTab *tabs = reinterpret_cast<TileTab *>(smem + STAGES * STAGE_BYTES + 256);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (threadIdx.x == 0) {
@@ -463,18 +464,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
       mbar_init(&tabf[i], 32 * kTab);
       mbar_init(&tabe[i], kEpi);
     }
-    *abort_flag = 0;
+    ctl->init(p.wait_us);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem)),
                  "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = ctl->tmem;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -495,11 +496,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
-      for (int i = 0; i < STAGES; ++i) {  // every stage consumed before the CTA leaves
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 15)) break;
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
-      }
-    tma_done:;
+      for (int j = 0; j < STAGES; ++j)  // every stage consumed before the CTA leaves
+        if (!mbar_wait(&empty[j], j < stage ? phase : phase ^ 1, abort_flag, p.err, 15)) break;
+    tma_done:
+      drain_loads(full, STAGES, stage, phase);  // passes at once unless a wait gave up
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -551,7 +551,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
-    mma_done:;
+    mma_done:
+      drain_mmas(&ctl->mma_done);  // the epilogue may have given up before the last of them
     }
   } else if (warp >= 2 + kEpi) {
     // ---- output offsets and exponents of every tile, ahead of its epilogue ----
@@ -732,6 +733,7 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   p.splits = q.splits;
   p.flag = ip;
   p.err = ws->error_slot();
+  p.wait_us = ws->wait_us;
   p.c_split = 0;
   if (q.splits > 1) {  // FP64 partials [batch][split][column][row]
     p.C = partial;

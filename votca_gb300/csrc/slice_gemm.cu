@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
   uint64_t *empty = full + C::STAGES;
   uint64_t *accf = empty + C::STAGES;  // [0], [1]: H buffers complete, [2]: L
   uint64_t *acce = accf + 3;           // drained
-  uint32_t *tmem_slot = (uint32_t *)(acce + 3);
-  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  TcControl *ctl = (TcControl *)(acce + 3);
+  volatile int *abort_flag = &ctl->abort;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::STAGES; ++i) {
@@ -137,18 +137,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
       mbar_init(&accf[i], 1);
       mbar_init(&acce[i], kEpi);
     }
-    *abort_flag = 0;
+    ctl->init(kWaitUs);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem)),
                  "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = ctl->tmem;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -169,11 +169,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
           if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
         }
       }
-      for (int i = 0; i < C::STAGES; ++i) {  // every stage consumed before the CTA leaves
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 5)) break;
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-      }
-    tma_done:;
+      for (int j = 0; j < C::STAGES; ++j)  // every stage consumed before the CTA leaves
+        if (!mbar_wait(&empty[j], j < stage ? phase : phase ^ 1, abort_flag, p.err, 5)) break;
+    tma_done:
+      drain_loads(full, C::STAGES, stage, phase);  // passes at once unless a wait gave up
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -211,7 +210,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
           if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
         }
       }
-    mma_done:;
+    mma_done:
+      drain_mmas(&ctl->mma_done);  // the epilogue may have given up before the last of them
     }
   } else {
     const int q = warp % 4, part = (warp - 2) / 4;

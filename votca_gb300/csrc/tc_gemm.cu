@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
   uint64_t *empty = full + C::STAGES;
   uint64_t *accf = empty + C::STAGES;
   uint64_t *acce = accf + C::NBUF;
-  uint32_t *tmem_slot = (uint32_t *)(acce + C::NBUF);
-  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  TcControl *ctl = (TcControl *)(acce + C::NBUF);
+  volatile int *abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (threadIdx.x == 0) {
@@ -153,19 +153,19 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       mbar_init(&accf[i], 1);
       mbar_init(&acce[i], kEpiWarps);  // one arrive per epilogue warp  // one arrive per epilogue warp
     }
-    *abort_flag = 0;
+    ctl->init(kWaitUs);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
+                     smem_u32(&ctl->tmem)),
                  "r"((uint32_t)C::TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = ctl->tmem;
   int *const err = src.err();
   const int64_t nitems = src.total();  // item R: jobs li * len + u, u < len (see item_len)
 
@@ -200,12 +200,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
           }
         }
       }
-      // drain: wait until the MMA warp has consumed every stage issued (bounded)
-      for (int i = 0; i < C::STAGES; ++i) {
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, err, 5)) break;
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-      }
-    producer_done:;
+      for (int j = 0; j < C::STAGES; ++j)  // every stage consumed before the CTA leaves
+        if (!mbar_wait(&empty[j], j < stage ? phase : phase ^ 1, abort_flag, err, 5)) break;
+    producer_done:
+      drain_loads(full, C::STAGES, stage, phase);  // passes at once unless a wait gave up
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -257,7 +255,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
           if (++buf == C::NBUF) { buf = 0; aphase ^= 1; }
         }
       }
-    mma_done:;
+    mma_done:
+      drain_mmas(&ctl->mma_done);  // the epilogue may have given up before the last of them
     }
   } else {
     // ---------------- epilogue warps ----------------

@@ -10,7 +10,7 @@
 
 namespace vgb {
 
-constexpr unsigned long long kWaitNs = 2000000000ull;  // bounded waits: 2 s
+constexpr int kWaitUs = 2000000;  // bounded waits: 2 s
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -41,16 +41,28 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after kWaitNs or when another role aborted.
+// What follows the barriers of a kernel in shared memory.
+struct alignas(8) TcControl {
+  uint32_t tmem;            // base of the TMEM allocation
+  int abort, wait_us;       // set when a wait gave up; the limit of the waits
+  uint64_t mma_done;        // barrier of drain_mmas
+  __device__ void init(int limit_us) {
+    abort = 0;
+    wait_us = limit_us;
+    mbar_init(&mma_done, 1);
+  }
+};
+static_assert(sizeof(TcControl) == 24, "abort and wait_us are read as an array of two");
+// Bounded wait: gives up after abort_flag[1] microseconds (at once for 0) or when another role aborted.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
                                           int *err, int code) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = now_ns();
+  const uint64_t t0 = now_ns(), limit = 1000ull * (uint64_t)abort_flag[1];
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255) == 0) {
+    if ((it & 255) == 0 || limit == 0) {
       if (*abort_flag) return false;
-      if (now_ns() - t0 > kWaitNs) {
+      if (now_ns() - t0 > limit || limit == 0) {
         *abort_flag = 1;
         atomicExch(err, code);
         return false;
@@ -62,6 +74,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err,
                                                int code) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code));
+}
+// A role's wait for what it has in flight itself, before the CTA may leave: not cut short by an abort.
+__device__ __forceinline__ void mbar_wait_own(uint64_t *bar, uint32_t parity) {
+  const uint64_t t0 = now_ns();
+  while (!mbar_try_wait(bar, parity) && now_ns() - t0 <= 1000ull * kWaitUs) {}
+}
+// The loads of a ring of stages, of which `stage` is the next to fill in the round with parity phase (a
+// barrier that was never filled passes).
+__device__ __forceinline__ void drain_loads(uint64_t *full, int stages, int stage, uint32_t phase) {
+  for (int j = 0; j < stages; ++j) mbar_wait_own(&full[j], j < stage ? phase : phase ^ 1);
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint64_t *bar,
                                             int x, int y) {
@@ -100,6 +122,11 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
           smem_u32(bar))
       : "memory");
+}
+// The MMAs that this thread has issued; bar: of its own, unused before.
+__device__ __forceinline__ void drain_mmas(uint64_t *bar) {
+  mma_commit(bar);
+  mbar_wait_own(bar, 0);
 }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
