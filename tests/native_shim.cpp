@@ -115,4 +115,17 @@ int shim_oz_dgemm(const int64_t *v, const double *A, int64_t na, const double *B
   });
 }
 
+// A product whose digit planes no GPU can hold: nothing is launched, *keep: bytes left in the workspace.
+int shim_oz_no_room(int *taken, int64_t *keep) {
+  return on_stream([&](cudaStream_t s) {
+    vgb::GemmWorkspace ws;
+    ws.plane_budget = 1LL << 50;
+    vgb::GemmDesc d;  // planes of A: 2^26 x 512 x 14 bytes
+    d.M = 1LL << 26; d.N = 64; d.K = 512;
+    d.a_colmajor(nullptr, d.M, false).b_colmajor(nullptr, d.K, false).c_colmajor(nullptr, d.M);
+    *taken = vgb::oz_dgemm(d, s, &ws) ? 1 : 0;
+    *keep = (int64_t)(ws.oz_a.bytes() + ws.oz_b.bytes() + ws.oz_int.bytes() + ws.partial.bytes());
+  });
+}
+
 }  // extern "C"

@@ -22,6 +22,7 @@ struct GemmWorkspace {
   DeviceBuffer<uint16_t> oz_a, oz_b;
   DeviceBuffer<int> oz_int;
   DeviceBuffer<unsigned> arrived;  // finished splits per tile, zero between products
+  int64_t plane_budget = 3LL << 29;  // bytes of digit planes per operand and launch
   int wait_us = 2000000;           // after which a wait inside a product gives up
   GemmWorkspace() = default;
   GemmWorkspace(const GemmWorkspace &) = delete;

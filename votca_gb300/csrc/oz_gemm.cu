@@ -682,13 +682,11 @@ __global__ void oz_reduce_kernel(const double *__restrict__ part, int64_t M, int
 
 // ---------------- host ----------------
 
-constexpr int64_t kPlaneBudget = 3LL << 29;  // bytes of digit planes per operand and launch
-
 }  // namespace
 
 bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   OzPlan q;
-  if (!ws || !oz_plan(d, sm_count(), kPlaneBudget, q) || !q.faster) return false;
+  if (!ws || !oz_plan(d, sm_count(), ws->plane_budget, q) || !q.faster) return false;
   const int nruns = (int)ceil_div(q.Kp, RUN);
   const int64_t nseg = ceil_div(q.Kp, SEG);
   const bool two = nseg > 1;  // exponents before digits
@@ -705,7 +703,10 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
     }
   } catch (const Error &e) {
     if (e.code != BSE_ERR_OUT_OF_MEMORY) throw;
-    cudaGetLastError();  // no room for the planes: the FMA kernel needs none
+    cudaGetLastError();  // no room for the planes: the FMA kernel needs none, and its caller the memory
+    ws->oz_int.release();
+    ws->oz_a.release();
+    ws->oz_b.release();
     return false;
   }
   static std::once_flag attr;
