@@ -96,12 +96,13 @@ int shim_stage_dense_screening_uks(const bse_mmn_desc *d, const double *const *s
 
 // A strided batched product on the tensor-core path; d: M, N, K, nb1, nb2, a_rs, a_cs, a_b1, a_b2,
 // b_rs, b_cs, b_b1, b_b2, c_rs, c_cs, c_b1, c_b2; wait_us: the limit of its waits; *taken: whether that
-// path took it.
+// path took it; *keep: bytes the workspace holds afterwards.
 int shim_oz_dgemm(const int64_t *v, const double *A, int64_t na, const double *B, int64_t nb, double *C, int64_t nc,
-                  double alpha, double beta, int wait_us, int *taken) {
+                  double alpha, double beta, int64_t budget, int wait_us, int *taken, int64_t *keep) {
   return on_stream([&](cudaStream_t s) {
     Dev<double> a(A, na, s), b(B, nb, s), c(C, nc, s);
     vgb::GemmWorkspace ws;
+    ws.plane_budget = budget;
     ws.wait_us = wait_us;
     vgb::GemmDesc d;
     d.M = v[0]; d.N = v[1]; d.K = v[2]; d.nb1 = v[3]; d.nb2 = v[4];
@@ -112,6 +113,7 @@ int shim_oz_dgemm(const int64_t *v, const double *A, int64_t na, const double *B
     *taken = vgb::oz_dgemm(d, s, &ws) ? 1 : 0;
     c.read(C, nc);
     ws.check();
+    *keep = (int64_t)(ws.oz_a.bytes() + ws.oz_b.bytes() + ws.oz_int.bytes());
   });
 }
 

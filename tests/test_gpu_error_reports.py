@@ -170,10 +170,11 @@ def test_wait_limit(M, N, K):
     v = np.array([M, N, K, 1, 1, K, 1, 0, 0, N, 1, 0, 0, N, 1, 0, 0], dtype=np.int64)
 
     def run(us):
-        C, taken = np.zeros((M, N)), ctypes.c_int()
+        C, taken, keep = np.zeros((M, N)), ctypes.c_int(), ctypes.c_int64()
         n = lambda a: ctypes.c_int64(a.size)
         rc = L.shim_oz_dgemm(P(v.view(np.float64)), P(A), n(A), P(B), n(B), P(C), n(C), ctypes.c_double(1.0),
-                             ctypes.c_double(0.0), us, ctypes.byref(taken))
+                             ctypes.c_double(0.0), ctypes.c_int64(1 << 30), us, ctypes.byref(taken),
+                             ctypes.byref(keep))
         assert taken.value == 1
         return rc, C
 

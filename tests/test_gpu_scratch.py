@@ -1,11 +1,27 @@
-"""Scratch of the tensor-core FP64 products: what stays allocated after a call."""
+"""Scratch of the tensor-core FP64 products: what stays allocated after a call, and products cut into
+chunks of rows and of batches."""
 import ctypes
 
+import numpy as np
 import pytest
 
 import native
 
 pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def _product(v, A, B, C, alpha=1.0, beta=0.0, budget=3 << 29):
+    L = native.load()
+    taken, keep = ctypes.c_int(), ctypes.c_int64()
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    n = lambda a: ctypes.c_int64(a.size)
+    v = np.array(v, dtype=np.int64)
+    assert L.shim_oz_dgemm(p(v), p(A), n(A), p(B), n(B), p(C), n(C), ctypes.c_double(alpha), ctypes.c_double(beta),
+                           ctypes.c_int64(budget), 2000000, ctypes.byref(taken),
+                           ctypes.byref(keep)) == 0, L.shim_last_error()
+    return taken.value, keep.value
 
 
 def test_no_room_for_the_planes():
@@ -14,3 +30,38 @@ def test_no_room_for_the_planes():
     taken, keep = ctypes.c_int(1), ctypes.c_int64(-1)
     assert L.shim_oz_no_room(ctypes.byref(taken), ctypes.byref(keep)) == 0, L.shim_last_error()
     assert (taken.value, keep.value) == (0, 0)
+
+
+def test_large_planes_are_given_back():
+    """20480 x 1024 times 1024 x 64: 294 MB of planes; a workspace keeps no more than 128 MB."""
+    M, N, K = 20480, 64, 1024
+    rng = np.random.default_rng(2)
+    A, B, C = rng.standard_normal(M * K), rng.standard_normal(K * N), np.zeros(M * N)
+    taken, keep = _product([M, N, K, 1, 1, 1, M, 0, 0, 1, K, 0, 0, 1, M, 0, 0], A, B, C)
+    assert taken == 1 and keep <= 128 * MB
+    rows = rng.integers(0, M, 16)
+    ref = A.reshape(K, M)[:, rows].T.astype(np.longdouble) @ B.reshape(N, K).T.astype(np.longdouble)
+    a, b = np.abs(A.reshape(K, M)[:, rows].T), np.abs(B.reshape(N, K).T)
+    bound = K * 2.0**-53 * a.max(axis=1)[:, None] * b.max(axis=0)[None, :]
+    assert np.all(np.abs(C.reshape(N, M)[:, rows].T - ref) <= bound + 2.0**-52 * np.abs(ref))
+
+
+# bytes of planes per row: 14 Kp; budgets of a few row tiles or batches, K of one and of several
+# exponent segments (256) and runs (1024)
+@pytest.mark.parametrize("K", [224, 257, 1100])
+@pytest.mark.parametrize("M,N,batch,rows", [(1000, 70, 1, 300), (1300, 65, 1, 128), (260, 130, 7, 600), (300, 257, 5, 310)])
+def test_chunks(M, N, batch, rows, K):
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((batch, M, K)), rng.standard_normal((batch, K, N))
+    A *= 2.0 ** rng.integers(-30, 30, (batch, M, 1))  # every row its own exponent, also in reused tables
+    C = rng.standard_normal((batch, M, N))
+    C0 = C.copy()
+    budget = rows * 14 * ((K + 31) // 32 * 32)
+    ab, bb = (M * K, K * N) if batch > 1 else (0, 0)
+    # a product this small stays with the FMA kernel unless the plan finds it faster: both are checked
+    taken, _ = _product([M, N, K, batch, 1, K, 1, ab, 0, N, 1, bb, 0, N, 1, M * N, 0], A, B, C, -2.0, 0.5, budget)
+    if not taken:
+        pytest.skip("left to the FMA kernel")
+    ref = -2.0 * (A.astype(np.longdouble) @ B.astype(np.longdouble)) + 0.5 * C0
+    bound = 2.0 * K * 2.0**-53 * np.abs(A).max(axis=2)[:, :, None] * np.abs(B).max(axis=1)[:, None, :]
+    assert np.all(np.abs(C - ref) <= bound + 2.0**-51 * (np.abs(ref) + np.abs(C0)))

@@ -15,7 +15,7 @@
 
 namespace vgb {
 
-// Scratch owned by the caller (split-K partials; digit planes, exponents and the error slot of
+// Scratch owned by the caller (split-K partials; small digit planes, exponents and the error slot of
 // the tensor-core path).  Grows on demand.
 struct GemmWorkspace {
   DeviceBuffer<double> partial;

@@ -682,6 +682,31 @@ __global__ void oz_reduce_kernel(const double *__restrict__ part, int64_t M, int
 
 // ---------------- host ----------------
 
+// Digit planes of one operand: the workspace's, or beyond what it keeps a block of the stream-ordered
+// pool that goes back on the stream after the product.  They are 14 bytes an element, up to several
+// GB, and a handle that kept them would take that from the next one's staging.
+constexpr int64_t kPlaneKeep = 64LL << 20;
+struct Planes {
+  cudaStream_t s;
+  DeviceBuffer<uint16_t> own;
+  uint16_t *p = nullptr;
+  explicit Planes(cudaStream_t stream) : s(stream ? stream : cudaStreamLegacy) {}
+  void take(DeviceBuffer<uint16_t> &kept, int64_t elems) {
+    if (elems * (int64_t)sizeof(uint16_t) <= kPlaneKeep) {
+      kept.resize((size_t)elems);
+      p = kept.get();
+    } else {
+      AllocStreamScope scope(s);
+      own.resize((size_t)elems);
+      p = own.get();
+    }
+  }
+  ~Planes() {
+    AllocStreamScope scope(s);
+    own.release();
+  }
+};
+
 }  // namespace
 
 bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
@@ -693,10 +718,11 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   const int64_t rows_a = q.m_chunk * q.tb_chunk, rows_b = q.N * q.tb_chunk;
   const int64_t ni = 64 + rows_a + rows_b;  // [flag | row exponents of A | of B], then run exponents
   double *partial = nullptr;
+  Planes pa(stream), pb(stream);
   try {
     ws->oz_int.resize((size_t)(ni + (two ? (rows_a + rows_b) * nruns : 0)));
-    ws->oz_a.resize((size_t)(rows_a * q.Kp * S));
-    ws->oz_b.resize((size_t)(rows_b * q.Kp * S));
+    pa.take(ws->oz_a, rows_a * q.Kp * S);
+    pb.take(ws->oz_b, rows_b * q.Kp * S);
     if (q.splits > 1) {
       ws->partial.resize((size_t)(q.nbatch * q.splits * q.M * q.N));
       partial = ws->partial.get();
@@ -721,8 +747,8 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   A.K = B.K = d.K;
   A.Kp = B.Kp = q.Kp;
   A.nruns = B.nruns = nruns;
-  A.planes = ws->oz_a.get();
-  B.planes = ws->oz_b.get();
+  A.planes = pa.p;
+  B.planes = pb.p;
   int *ip = ws->oz_int.get();
   A.erow = ip + 64;
   B.erow = A.erow + rows_a;
