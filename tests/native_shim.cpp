@@ -1,5 +1,5 @@
 // C entries into the C++ core for tests that the C ABI does not reach: error codes planted on the host
-// in place of a device wait that gave up, and single FP64 products.
+// in place of a device wait that gave up, single FP64 products, and the memory pools.
 #include <string>
 
 #include "../votca_gb300/csrc/handle.cuh"
@@ -127,6 +127,18 @@ int shim_oz_no_room(int *taken, int64_t *keep) {
     d.a_colmajor(nullptr, d.M, false).b_colmajor(nullptr, d.K, false).c_colmajor(nullptr, d.M);
     *taken = vgb::oz_dgemm(d, s, &ws) ? 1 : 0;
     *keep = (int64_t)(ws.oz_a.bytes() + ws.oz_b.bytes() + ws.oz_int.bytes() + ws.partial.bytes());
+  });
+}
+
+// The default memory pool: reserved bytes, and its release threshold.
+int shim_pool_state(uint64_t *reserved, uint64_t *threshold) {
+  return guarded([&] {
+    int dev = 0;
+    cudaMemPool_t p;
+    VGB_CUDA(cudaGetDevice(&dev));
+    VGB_CUDA(cudaDeviceGetDefaultMemPool(&p, dev));
+    VGB_CUDA(cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, reserved));
+    VGB_CUDA(cudaMemPoolGetAttribute(p, cudaMemPoolAttrReleaseThreshold, threshold));
   });
 }
 

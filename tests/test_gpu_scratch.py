@@ -24,12 +24,21 @@ def _product(v, A, B, C, alpha=1.0, beta=0.0, budget=3 << 29):
     return taken.value, keep.value
 
 
+def _pool():
+    r, t = ctypes.c_uint64(), ctypes.c_uint64()
+    assert native.load().shim_pool_state(ctypes.byref(r), ctypes.byref(t)) == 0
+    return r.value, t.value
+
+
 def test_no_room_for_the_planes():
-    """The FMA kernel takes over: nothing of the other path may stay allocated beside it."""
+    """The FMA kernel takes over: nothing of the other path may stay allocated beside it, nor what the
+    pool reserved for the attempt."""
     L = native.load()
+    before = _pool()[0]
     taken, keep = ctypes.c_int(1), ctypes.c_int64(-1)
     assert L.shim_oz_no_room(ctypes.byref(taken), ctypes.byref(keep)) == 0, L.shim_last_error()
     assert (taken.value, keep.value) == (0, 0)
+    assert _pool()[0] <= before + 1024 * MB
 
 
 def test_large_planes_are_given_back():

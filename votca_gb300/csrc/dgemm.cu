@@ -253,20 +253,22 @@ void keep_pool_blocks() {
 }  // namespace
 
 void *device_alloc(size_t bytes, cudaStream_t &used) {
-  void *p = nullptr;
   used = alloc_stream();
-  if (used) {
+  auto get = [&](void **p) {
+    if (!used) return cudaMalloc(p, bytes);
     keep_pool_blocks();
-    VGB_CUDA(cudaMallocAsync(&p, bytes, used));
-  } else {
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation) {  // the pool's unused blocks may be what is missing
-      cudaGetLastError();
-      trim_pool();
-      e = cudaMalloc(&p, bytes);
-    }
-    VGB_CUDA(e);
+    return cudaMallocAsync(p, bytes, used);
+  };
+  void *p = nullptr;
+  cudaError_t e = get(&p);
+  for (int again = 1; e == cudaErrorMemoryAllocation && again >= 0; --again) {
+    // the pool's unused blocks may be what is missing, and what it reserved for the attempt that failed
+    // (it can be all of the GPU's memory) would be missing elsewhere
+    cudaGetLastError();
+    trim_pool();
+    if (again) e = get(&p);
   }
+  VGB_CUDA(e);
   return p;
 }
 

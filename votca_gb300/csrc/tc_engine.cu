@@ -692,7 +692,7 @@ void MixedEngine::build_dense_grouped(const std::vector<BseOperator *> &ops, con
     for (BseOperator *op : todo) bytes += op->dim * pad64(op->dim) * 4 + 4096;
     void *p = nullptr;
     if (cudaMallocAsync(&p, (size_t)bytes, s) == cudaSuccess) VGB_CUDA(cudaFreeAsync(p, s));
-    else cudaGetLastError();  // no headroom for one block: allocated piece by piece
+    else cudaGetLastError(), trim_pool();  // no headroom for one block: allocated piece by piece
   }
   size_t a = 0;
   while (a < todo.size()) {
@@ -1030,7 +1030,7 @@ void MixedEngine::prepare_grouped(const std::vector<BseOperator *> &ops, int64_t
   if (alloc_stream()) {
     void *p = nullptr;
     if (cudaMallocAsync(&p, (size_t)bytes, s) == cudaSuccess) VGB_CUDA(cudaFreeAsync(p, s));
-    else cudaGetLastError();  // no headroom for one block: the buffers are allocated one by one
+    else cudaGetLastError(), trim_pool();  // no headroom for one block: the buffers are allocated one by one
   }
   for (Need &q : need) {
     if ((int64_t)q.m->Xs.hi.count < q.xs) q.m->Xs.ensure(q.xs / q.m->Kc, q.m->Kc, s);
