@@ -142,4 +142,19 @@ int shim_pool_state(uint64_t *reserved, uint64_t *threshold) {
   });
 }
 
+// What a handle keeps (used) and has given back to the pool (unused).
+static vgb::DeviceBuffer<char> *g_used = nullptr;
+int shim_pool_hold(int64_t used, int64_t unused) {
+  return on_stream([&](cudaStream_t) {
+    g_used = new vgb::DeviceBuffer<char>((size_t)used);
+    vgb::DeviceBuffer<char> tmp((size_t)unused);
+  });
+}
+int shim_pool_release() {
+  return on_stream([&](cudaStream_t) {
+    delete g_used;
+    g_used = nullptr;
+  });
+}
+
 }  // extern "C"

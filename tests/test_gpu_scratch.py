@@ -1,11 +1,15 @@
-"""Scratch of the tensor-core FP64 products: what stays allocated after a call, and products cut into
-chunks of rows and of batches."""
+"""Scratch of the tensor-core FP64 products and of calls without a handle: what stays allocated after
+a call, and products cut into chunks of rows and of batches."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 
 import native
+from votca_gb300 import screening
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +78,32 @@ def test_chunks(M, N, batch, rows, K):
     ref = -2.0 * (A.astype(np.longdouble) @ B.astype(np.longdouble)) + 0.5 * C0
     bound = 2.0 * K * 2.0**-53 * np.abs(A).max(axis=2)[:, :, None] * np.abs(B).max(axis=1)[:, None, :]
     assert np.all(np.abs(C - ref) <= bound + 2.0**-51 * (np.abs(ref) + np.abs(C0)))
+
+
+def test_calls_without_a_handle_leave_the_handles_pool_alone():
+    L = native.load()
+    assert L.shim_pool_hold(ctypes.c_int64(1280 * MB), ctypes.c_int64(512 * MB)) == 0
+    before = _pool()
+    assert before[0] >= 1792 * MB
+    a = np.eye(96) * 2.0
+    np.testing.assert_allclose(screening.cholesky_inverse(a), 0.5 * np.eye(96), rtol=1e-15)
+    after = _pool()
+    assert L.shim_pool_release() == 0
+    assert after == before
+
+
+def test_calls_without_a_handle_leave_the_default_threshold():
+    """In a process of its own, without any handle."""
+    code = """
+import ctypes, numpy as np, native
+from votca_gb300 import screening
+screening.cholesky_inverse(np.eye(300) * 2.0)
+r, t = ctypes.c_uint64(), ctypes.c_uint64()
+assert native.load().shim_pool_state(ctypes.byref(r), ctypes.byref(t)) == 0
+print("pool", r.value, t.value)
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split()[-3:] == ["pool", "0", "0"], r.stdout

@@ -44,27 +44,28 @@ vgb::Coef coef(int32_t a, int32_t b, int32_t c, int32_t d) {
 
 void require_handle(const bse_handle *h) { VGB_REQUIRE(h != nullptr, "null handle"); }
 
-// The stream of a call without a handle.  Its buffers come from the device's stream-ordered pool (a
+// The stream of a call without a handle.  Its buffers come from a stream-ordered pool of such calls (a
 // cudaMalloc and cudaFree pair each cost 0.15 to 0.2 ms: the dielectric matrix and its inverse at
-// Naux 1000 take 4.4 ms from the pool, 6.1 ms without it).  At most kPoolKeep of the pool stays reserved
-// afterwards, until a handle is destroyed or a plain allocation runs out; the lockstep batch keeps the
-// pool as the handles' own calls do (keep_all).
-constexpr size_t kPoolKeep = 1ull << 30;
+// Naux 1000 take 4.1 ms from the pool, 6.1 ms without it).  The pool is bounded (kScratchKeep) and apart
+// from the default one, whose blocks and settings belong to the handles and the application; the
+// lockstep batch works on handles and uses the default pool as their own calls do.
 struct TmpStream {
   cudaStream_t s = nullptr;
-  bool keep_all;
+  cudaMemPool_t saved_pool = vgb::alloc_pool();
   std::unique_ptr<vgb::AllocStreamScope> scope;
-  explicit TmpStream(bool keep = false) : keep_all(keep) {
+  explicit TmpStream(bool on_handles = false) {
+    const cudaMemPool_t pool = on_handles ? nullptr : vgb::scratch_pool();
     VGB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     scope.reset(new vgb::AllocStreamScope(s));
+    vgb::alloc_pool() = pool;
   }
   ~TmpStream() {
     scope.reset();
+    vgb::alloc_pool() = saved_pool;
     if (s) {
-      cudaStreamSynchronize(s);
+      cudaStreamSynchronize(s);  // the pool gives back what it holds beyond its bound
       cudaStreamDestroy(s);
     }
-    if (!keep_all) vgb::trim_pool(kPoolKeep);
   }
 };
 

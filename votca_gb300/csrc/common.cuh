@@ -45,9 +45,16 @@ struct AllocStreamScope {
   explicit AllocStreamScope(cudaStream_t s) : saved(alloc_stream()) { alloc_stream() = s; }
   ~AllocStreamScope() { alloc_stream() = saved; }
 };
+// The pool of such allocations on the calling thread; null: the device's default pool, in which the
+// handles keep their freed blocks.
+cudaMemPool_t &alloc_pool();
+// The pool of calls without a handle, one per device: at most kScratchKeep of it stays reserved between
+// them, until trim_pool.
+constexpr uint64_t kScratchKeep = 1ull << 30;
+cudaMemPool_t scratch_pool();
 void *device_alloc(size_t bytes, cudaStream_t &used);
 void device_free(void *p, cudaStream_t used);
-void trim_pool(size_t keep = 0);  // return unused stream-ordered blocks to the driver, down to keep bytes
+void trim_pool();  // return the unused blocks of both pools to the driver
 
 // Owning device buffer.
 template <typename T>

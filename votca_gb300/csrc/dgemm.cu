@@ -252,17 +252,47 @@ void keep_pool_blocks() {
 }
 }  // namespace
 
+cudaMemPool_t &alloc_pool() {
+  static thread_local cudaMemPool_t p = nullptr;
+  return p;
+}
+
+namespace {
+std::mutex g_scratch_mu;
+cudaMemPool_t g_scratch[64] = {};
+}  // namespace
+
+cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  VGB_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  if (!g_scratch[dev]) {
+    cudaMemPoolProps pp = {};
+    pp.allocType = cudaMemAllocationTypePinned;
+    pp.location.type = cudaMemLocationTypeDevice;
+    pp.location.id = dev;
+    cudaMemPool_t pool;
+    VGB_CUDA(cudaMemPoolCreate(&pool, &pp));
+    uint64_t keep = kScratchKeep;
+    VGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    g_scratch[dev] = pool;
+  }
+  return g_scratch[dev];
+}
+
 void *device_alloc(size_t bytes, cudaStream_t &used) {
   used = alloc_stream();
   auto get = [&](void **p) {
     if (!used) return cudaMalloc(p, bytes);
+    if (cudaMemPool_t pool = alloc_pool()) return cudaMallocFromPoolAsync(p, bytes, pool, used);
     keep_pool_blocks();
     return cudaMallocAsync(p, bytes, used);
   };
   void *p = nullptr;
   cudaError_t e = get(&p);
   for (int again = 1; e == cudaErrorMemoryAllocation && again >= 0; --again) {
-    // the pool's unused blocks may be what is missing, and what it reserved for the attempt that failed
+    // the pools' unused blocks may be what is missing, and what was reserved for the attempt that failed
     // (it can be all of the GPU's memory) would be missing elsewhere
     cudaGetLastError();
     trim_pool();
@@ -287,11 +317,13 @@ void device_free(void *p, cudaStream_t used) {
   }
 }
 
-void trim_pool(size_t keep) {
+void trim_pool() {
   int dev = 0;
   cudaMemPool_t pool;
-  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
-    cudaMemPoolTrimTo(pool, keep);
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  if (dev < 64 && g_scratch[dev]) cudaMemPoolTrimTo(g_scratch[dev], 0);
 }
 
 int sm_count() {
