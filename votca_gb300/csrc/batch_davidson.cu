@@ -661,8 +661,8 @@ void run_gs(const std::vector<GsJob> &jobs, cudaStream_t s) {
     launch_jobs(jobs, gs_kernel<false>, kGsCluster, true, s, kGsThreads);
     return;
   }
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice attr;
+  attr.run(current_device(), [] {
     VGB_CUDA(cudaFuncSetAttribute(gs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGsStaged));
   });
   std::unique_ptr<Group<GsJob>> g(new Group<GsJob>());

@@ -10,6 +10,7 @@
 #include <utility>
 
 #include "../../include/votca_gb300_bse.h"
+#include "per_device.hpp"
 
 namespace vgb {
 
@@ -97,6 +98,11 @@ struct DeviceBuffer {
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+inline int current_device() {
+  int dev = 0;
+  VGB_CUDA(cudaGetDevice(&dev));
+  return dev;
+}
 // Number of SMs of the current device (152 on GB300).
 int sm_count();
 

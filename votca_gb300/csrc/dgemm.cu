@@ -240,11 +240,11 @@ namespace {
 // the driver at every synchronisation (the Davidson loop synchronises once per
 // iteration); bse_op_destroy trims the pool.
 void keep_pool_blocks() {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    int dev = 0;
+  static PerDevice once;
+  const int dev = current_device();
+  once.run(dev, [&] {
     cudaMemPool_t pool;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
       uint64_t thr = UINT64_MAX;
       cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }

@@ -3,7 +3,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "oz_plan.hpp"
 #include "tc_ptx.cuh"
@@ -735,8 +734,8 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
     ws->oz_b.release();
     return false;
   }
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice attr;
+  attr.run(current_device(), [] {
     VGB_CUDA(cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     VGB_CUDA(cudaFuncSetAttribute(oz_slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SLICE_SMEM));
   });

@@ -1,7 +1,6 @@
 // Slice products: FP64-accurate GEMM from 7-bit digit planes on the tensor cores (slice_gemm.cuh).
 #include "slice_gemm.cuh"
 
-#include <mutex>
 
 #include "slice_plan.hpp"
 #include "tc_epilogue.cuh"
@@ -289,8 +288,8 @@ __global__ void reduce_pairs_kernel(const float2 *__restrict__ part, int64_t M, 
 template <int BN, int S>
 void launch(const Args &p, cudaStream_t s) {
   using C = Cfg<BN, S>;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice attr;
+  attr.run(current_device(), [] {
     VGB_CUDA(cudaFuncSetAttribute(slice_gemm_kernel<BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   });
   launch_pdl(slice_gemm_kernel<BN, S>, (unsigned)std::min(p.nitems, sm_count()), kGemmThreads, C::SMEM, s, p);

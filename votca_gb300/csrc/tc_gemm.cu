@@ -907,8 +907,8 @@ __global__ void reduce_group_kernel(const __grid_constant__ ReduceGroup g) {
 template <int BN, int BK, class Src>
 void launch_src(const Src &src, int64_t ntiles, cudaStream_t s) {
   using C = Cfg<BN, BK>;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice attr;
+  attr.run(current_device(), [] {
     VGB_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<BN, BK, Src>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
   });
