@@ -335,7 +335,7 @@ constexpr int kGsThreads = 128;
 // constant.  The reduction folds the LC sums together, exchanging half of them at each distance: 9
 // additions for 8 sums instead of 40, the same pairs of lanes added in each.
 template <int LC>
-__device__ __forceinline__ void gs_dots(const double *__restrict__ M, const double *qj, int64_t n, int64_t r0,
+__device__ __forceinline__ void gs_dots(const double *M, const double *qj, int64_t n, int64_t r0,
                                         int64_t r1, double *red) {
   double acc[8];
 #pragma unroll
@@ -374,7 +374,7 @@ __device__ __forceinline__ void gs_dots(const double *__restrict__ M, const doub
 
 // NR rows of q less their part in the range columns of M, and the squares of the result.
 template <int NR>
-__device__ __forceinline__ void gs_update(const double *__restrict__ M, const double *h, int range, int64_t n,
+__device__ __forceinline__ void gs_update(const double *M, const double *h, int range, int64_t n,
                                           double *qi, int64_t i, double &nacc) {
   double s[NR];
 #pragma unroll

@@ -77,9 +77,9 @@ __global__ void dvv_from_gvv_kernel(const double *Gvv, int64_t naux, int64_t vt,
   }
 }
 
-__global__ void hqp_diag_kernel(double cqp, const double *__restrict__ Hcc,
-                                const double *__restrict__ Hvv, int64_t vt, int64_t ct,
-                                const double *__restrict__ X, int64_t ldx, int64_t k,
+__global__ void hqp_diag_kernel(double cqp, const double *Hcc,
+                                const double *Hvv, int64_t vt, int64_t ct,
+                                const double *X, int64_t ldx, int64_t k,
                                 double *__restrict__ Y, int64_t ldy, int accumulate) {
   pdl_wait();
   const int64_t dim = vt * ct, total = dim * k;
@@ -243,7 +243,7 @@ __global__ void diagonal_group_kernel(const __grid_constant__ DiagGroup g) {
   diagonal_range(a, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
-__global__ void ham_combine_kernel(const double *__restrict__ TA, const double *__restrict__ TB,
+__global__ void ham_combine_kernel(const double *TA, const double *TB,
                                    int64_t dim, int64_t k, double *__restrict__ Y, int64_t ldy) {
   pdl_wait();
   const int64_t total = dim * k;

@@ -135,7 +135,9 @@ void aux_pseudo_inv_sqrt_gwbse(int64_t n, const double *S, int64_t lds, const do
 #ifdef __CUDACC__
 // Programmatic dependent launch: a kernel launched by launch_pdl is set up while the kernel before it
 // in the stream still runs, and waits here, first of all, until that one has completed and its
-// writes are visible.  Only kernels that begin with pdl_wait are launched this way.  A chain of
+// writes are visible.  Only kernels that begin with pdl_wait are launched this way, and they read with
+// plain loads: the read-only path (__ldg, or a parameter that is const and __restrict__) asks for
+// data that stays as it is from the start of the kernel, which lies before the wait.  A chain of
 // small dependent kernels: 4.1 us a kernel launched normally, 1.4 us this way.  No kernel lets its
 // successor start before its own end (griddepcontrol.launch_dependents): the chain is no faster
 // with it, and blocks that wait beside a large product slow it (Hd products of 10 vectors, v32 c256

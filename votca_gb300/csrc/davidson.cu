@@ -37,7 +37,7 @@ unsigned blocks_for(int64_t n, int threads = 256) {
 // back at zero afterwards.  fast (FP64 solves): chunks of 512 rows, added pairwise; otherwise
 // kRedChunks chunks, added in chunk order by one thread (64 dependent additions of 75 clocks; the
 // bits of split-precision solves).
-__global__ void coldot_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ B, int64_t ldb,
+__global__ void coldot_kernel(const double *A, int64_t lda, const double *B, int64_t ldb,
                               int64_t n, double *__restrict__ partial, unsigned *arrived, int take_sqrt, int fast,
                               double *__restrict__ out) {
   pdl_wait();
@@ -90,8 +90,8 @@ __global__ void set_unit_columns_kernel(double *V, int64_t ldv, const int64_t *r
 }
 
 // res[:, j] -= lam[j] * q[:, j]
-__global__ void residual_kernel(double *__restrict__ res, const double *__restrict__ q, int64_t n,
-                                int64_t ncols, const double *__restrict__ lam) {
+__global__ void residual_kernel(double *__restrict__ res, const double *q, int64_t n,
+                                int64_t ncols, const double *lam) {
   pdl_wait();
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -104,9 +104,9 @@ __global__ void residual_kernel(double *__restrict__ res, const double *__restri
 // out[:, kk] = -r_j / (D - lambda_j) for the listed roots (DPR, davidsonsolver.cc:416-422);
 // with olsen != 0 also dq[:, kk] = -q_j / (D - lambda_j).  clean != 0 zeroes
 // non-finite entries (computeCorrectionVector, :411-413).
-__global__ void dpr_kernel(double *__restrict__ out, int64_t ldo, const double *__restrict__ res,
-                           const double *__restrict__ q, int64_t n, const double *__restrict__ D,
-                           const int64_t *__restrict__ cols, const double *__restrict__ lams,
+__global__ void dpr_kernel(double *__restrict__ out, int64_t ldo, const double *res,
+                           const double *q, int64_t n, const double *D,
+                           const int64_t *cols, const double *lams,
                            int64_t count, int clean, double *__restrict__ dq) {
   pdl_wait();
   const int64_t total = n * count;
@@ -125,9 +125,9 @@ __global__ void dpr_kernel(double *__restrict__ out, int64_t ldo, const double *
 
 // Olsen: delta += (num/denom) q_j, then non-finite -> 0 (davidsonsolver.cc:424-436)
 __global__ void olsen_finish_kernel(double *__restrict__ out, int64_t ldo,
-                                    const double *__restrict__ q, int64_t n,
-                                    const int64_t *__restrict__ cols, const double *__restrict__ num,
-                                    const double *__restrict__ den, int64_t count) {
+                                    const double *q, int64_t n,
+                                    const int64_t *cols, const double *num,
+                                    const double *den, int64_t count) {
   pdl_wait();
   const int64_t total = n * count;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -143,7 +143,7 @@ __global__ void olsen_finish_kernel(double *__restrict__ out, int64_t ldo,
 
 // A[:, c] /= norm[c] where norm[c] > 0 (Eigen's normalize leaves zero columns alone)
 __global__ void scale_columns_kernel(double *A, int64_t lda, int64_t n, int64_t ncols,
-                                     const double *__restrict__ norm) {
+                                     const double *norm) {
   pdl_wait();
   const int64_t total = n * ncols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -227,7 +227,7 @@ __device__ bool gs_grid_barrier(unsigned *count, volatile unsigned *gen, unsigne
 
 __global__ void __launch_bounds__(kGsThreads)
     gs_columns_kernel(double *Q, int64_t n, int64_t nstart, int64_t ncols, int check,
-                      const double *__restrict__ norms0, double *partial, double *npartial,
+                      const double *norms0, double *partial, double *npartial,
                       unsigned *bar_count, unsigned *bar_gen, int *flag, int *err) {
   const unsigned nb = gridDim.x;
   const int64_t rows_per = ceil_div(n, (int64_t)nb);

@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(THREADS)
   x = quot_rem(batch, d.nb2);
   const int64_t b1 = x.q, b2 = x.r;
 
-  const double *__restrict__ A = d.A + b1 * d.a_b1 + b2 * d.a_b2;
-  const double *__restrict__ B = d.B + b1 * d.b_b1 + b2 * d.b_b2;
+  const double *A = d.A + b1 * d.a_b1 + b2 * d.a_b2;
+  const double *B = d.B + b1 * d.b_b1 + b2 * d.b_b2;
 
   const int64_t m0 = mtile * TM, n0 = ntile * TN;
   const int64_t kbeg = s * g.kchunk;

@@ -56,9 +56,9 @@ double *noalloc_scratch() {
   return g_noalloc_ptr[dev];
 }
 
-__global__ void na_hqp_diag_kernel(double cqp, const double *__restrict__ Hcc,
-                                   const double *__restrict__ Hvv, int64_t vt, int64_t ct,
-                                   const double *__restrict__ X, int64_t ldx, int64_t k,
+__global__ void na_hqp_diag_kernel(double cqp, const double *Hcc,
+                                   const double *Hvv, int64_t vt, int64_t ct,
+                                   const double *X, int64_t ldx, int64_t k,
                                    double *__restrict__ Y, int64_t ldy) {
   pdl_wait();
   const int64_t dim = vt * ct, total = dim * k;

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant_
       unsigned long long x[32];
       const unsigned long long *src = base + o.map.at(o.r0 + rb + (in ? r : 0)) + (k0 + k) * o.ks;
 #pragma unroll
-      for (int v = 0; v < 32; ++v, src += o.ks) x[v] = in && k + v < kn ? __ldg(src) : 0ull;
+      for (int v = 0; v < 32; ++v, src += o.ks) x[v] = in && k + v < kn ? *src : 0ull;
       __syncthreads();  // the previous unit's shared values are read
       if (phase & 1) {
         unsigned long long mx = 0;
@@ -216,13 +216,13 @@ __global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant_
         if (in && ((uintptr_t)src & 15) == 0 && k + 8 <= kn) {
 #pragma unroll
           for (int v = 0; v < 8; v += 2) {
-            const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(src + v));
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(src + v);
             x[v] = a.x;
             x[v + 1] = a.y;
           }
         } else {
 #pragma unroll
-          for (int v = 0; v < 8; ++v) x[v] = in && k + v < kn ? __ldg(src + v) : 0ull;
+          for (int v = 0; v < 8; ++v) x[v] = in && k + v < kn ? src[v] : 0ull;
         }
       }
       int e = 0, rel = 0;
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
 }
 
 // C (+)= alpha * sum over the K splits of the FP64 partials, in split order; M fastest.
-__global__ void oz_reduce_kernel(const double *__restrict__ part, int64_t M, int64_t N, int64_t nbt, int splits,
+__global__ void oz_reduce_kernel(const double *part, int64_t M, int64_t N, int64_t nbt, int splits,
                                  const OzMap crow, const OzMap ccol, const OzMap cbatch, double *__restrict__ C,
                                  double alpha, double beta) {
   pdl_wait();

@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
 }
 
 // Y = epi(sum over the groups' float pairs), part[g][n][i]: a float-pair sum in group order.
-__global__ void reduce_pairs_kernel(const float2 *__restrict__ part, int64_t M, int64_t N, int groups,
+__global__ void reduce_pairs_kernel(const float2 *part, int64_t M, int64_t N, int groups,
                                     const TcEpilogue e) {
   pdl_wait();
   const int64_t total = M * N;

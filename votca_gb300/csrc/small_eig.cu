@@ -95,7 +95,7 @@ __device__ int sturm_count(const float *d, const float *e2, int64_t m, float x, 
 // cases share one division and one update (lanes of a warp take different cases).  ds: the
 // shifted diagonal d - sigma; may be r0 itself (an entry is read before it is written).
 template <bool FAST>
-__device__ void tri_lu(const double *ds, const double *__restrict__ e, int m, double tiny,
+__device__ void tri_lu(const double *ds, const double *e, int m, double tiny,
                        double *r0, double *__restrict__ u1, double *__restrict__ u2, double *__restrict__ l,
                        double *__restrict__ pv) {
   double da = ds[0], db = m > 1 ? e[0] : 0.0;
@@ -122,9 +122,9 @@ __device__ void tri_lu(const double *ds, const double *__restrict__ e, int m, do
 }
 
 // z <- (T - sigma)^-1 z with the factors of tri_lu
-__device__ void tri_solve(int m, const double *__restrict__ r0, const double *__restrict__ u1,
-                          const double *__restrict__ u2, const double *__restrict__ l,
-                          const double *__restrict__ pv, double *__restrict__ z) {
+__device__ void tri_solve(int m, const double *r0, const double *u1,
+                          const double *u2, const double *l,
+                          const double *pv, double *__restrict__ z) {
   double a = z[0];
 #pragma unroll 4
   for (int i = 0; i + 1 < m; ++i) {

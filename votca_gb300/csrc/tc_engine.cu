@@ -619,7 +619,7 @@ namespace {
 // Bc[(c1, c)][P] = split(M(c1, c, P)) from Mcc[P][c][c1] (= the [P][q] matrix, q = c ct + c1):
 // a 32 x 32 tiled transpose through shared memory, so that reads run along q and writes
 // along P.
-__global__ void transpose_split_cc_kernel(const double *__restrict__ Mcc, int64_t naux, int64_t ct,
+__global__ void transpose_split_cc_kernel(const double *Mcc, int64_t naux, int64_t ct,
                                           uint16_t *__restrict__ hi, uint16_t *__restrict__ lo, int64_t ldo) {
   pdl_wait();
   __shared__ double tile[32][33];

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
 
 // ---------------- helpers ----------------
 
-__device__ __forceinline__ void split_range(const double *__restrict__ x, int64_t rows, int64_t cols,
+__device__ __forceinline__ void split_range(const double *x, int64_t rows, int64_t cols,
                                             const SplitMap &m, uint16_t *__restrict__ hi,
                                             uint16_t *__restrict__ lo, int64_t ldo, int64_t t0,
                                             int64_t step) {
@@ -389,7 +389,7 @@ __device__ __forceinline__ void split_range(const double *__restrict__ x, int64_
   }
 }
 
-__global__ void split_kernel(const double *__restrict__ x, int64_t rows, int64_t cols,
+__global__ void split_kernel(const double *x, int64_t rows, int64_t cols,
                              const SplitMap m, uint16_t *__restrict__ hi, uint16_t *__restrict__ lo,
                              int64_t ldo) {
   pdl_wait();
@@ -467,10 +467,10 @@ struct SplitMem {  // more: read again in each pass
   static constexpr int kMax = 1 << 30, kUnroll = 8;
   const unsigned *p;
   int64_t stride;
-  __device__ __forceinline__ unsigned operator()(int s) const { return __ldg(p + s * stride); }
+  __device__ __forceinline__ unsigned operator()(int s) const { return __ldcg(p + s * stride); }
 };
 
-__device__ __forceinline__ void reduce_range(const float *__restrict__ part, int64_t M, int64_t N,
+__device__ __forceinline__ void reduce_range(const float *part, int64_t M, int64_t N,
                                              int ksplit, const TcEpilogue &e, int64_t t0, int64_t step) {
   const int64_t total = M * N;
   for (int64_t t = t0; t < total; t += step) {
@@ -482,7 +482,7 @@ __device__ __forceinline__ void reduce_range(const float *__restrict__ part, int
     if (ksplit <= kSplitRegs) {
       SplitRegs r;
 #pragma unroll
-      for (int s = 0; s < kSplitRegs; ++s) r.w[s] = s < ksplit ? __ldg(p + s * total) : 0u;
+      for (int s = 0; s < kSplitRegs; ++s) r.w[s] = s < ksplit ? __ldcg(p + s * total) : 0u;
       acc = sum_splits(ksplit, r);
     } else {
       acc = sum_splits(ksplit, SplitMem{p, total});
@@ -500,7 +500,7 @@ __device__ __forceinline__ void reduce_range(const float *__restrict__ part, int
   }
 }
 
-__global__ void reduce_partials_kernel(const float *__restrict__ part, int64_t M, int64_t N,
+__global__ void reduce_partials_kernel(const float *part, int64_t M, int64_t N,
                                        int ksplit, const TcEpilogue e) {
   pdl_wait();
   reduce_range(part, M, N, ksplit, e, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
@@ -541,19 +541,19 @@ __device__ __forceinline__ long long fixed_point_f32(unsigned bits, int e, int B
 struct F64In {
   const unsigned long long *p;
   __device__ __forceinline__ unsigned long long abs_bits(int64_t i) const {
-    return __ldg(p + i) & 0x7FFFFFFFFFFFFFFFull;
+    return p[i] & 0x7FFFFFFFFFFFFFFFull;
   }
   // frexp exponent of a maximum (abs_bits): mx < 2^e; subnormal maxima as 2^-1022
   __device__ __forceinline__ static int exponent(unsigned long long mx) {
     return mx == 0 ? 0 : max((int)(mx >> 52), 1) - 1022;
   }
   __device__ __forceinline__ long long fixed(int64_t i, int e, int B) const {
-    return fixed_point(__ldg(p + i), e, B);
+    return fixed_point(p[i], e, B);
   }
   // four consecutive elements (32-byte aligned): raw words, |x| bits, fixed point of a word
   __device__ __forceinline__ void load4(int64_t i, unsigned long long (&w)[4]) const {
-    const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(p + i));
-    const ulonglong2 b = __ldg(reinterpret_cast<const ulonglong2 *>(p + i) + 1);
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(p + i);
+    const ulonglong2 b = reinterpret_cast<const ulonglong2 *>(p + i)[1];
     w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
   }
   __device__ __forceinline__ static unsigned long long abs_word(unsigned long long w) {
@@ -566,17 +566,17 @@ struct F64In {
 struct PairIn {
   const unsigned long long *p;  // float2 elements
   __device__ __forceinline__ unsigned long long abs_bits(int64_t i) const {
-    return (unsigned long long)((unsigned)__ldg(p + i) & 0x7FFFFFFFu);  // |hi|; hi holds the sum
+    return (unsigned long long)((unsigned)p[i] & 0x7FFFFFFFu);  // |hi|; hi holds the sum
   }
   __device__ __forceinline__ static int exponent(unsigned long long mx) {
     return mx == 0 ? 0 : max((int)(mx >> 23), 1) - 126;
   }
   __device__ __forceinline__ long long fixed(int64_t i, int e, int B) const {
-    return fixed_word(__ldg(p + i), e, B);
+    return fixed_word(p[i], e, B);
   }
   __device__ __forceinline__ void load4(int64_t i, unsigned long long (&w)[4]) const {
-    const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(p + i));
-    const ulonglong2 b = __ldg(reinterpret_cast<const ulonglong2 *>(p + i) + 1);
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(p + i);
+    const ulonglong2 b = reinterpret_cast<const ulonglong2 *>(p + i)[1];
     w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
   }
   __device__ __forceinline__ static unsigned long long abs_word(unsigned long long w) {
@@ -642,7 +642,7 @@ __global__ void slice_kernel(const In in, int64_t rows, int64_t cols, const Spli
           }
         } else {
           for (int64_t cc = c; cc < c1; ++cc) {
-            const unsigned long long a = In::abs_word(__ldg(in.p + base + cc));
+            const unsigned long long a = In::abs_word(in.p[base + cc]);
             mx = a > mx ? a : mx;
           }
         }
@@ -669,7 +669,7 @@ __global__ void slice_kernel(const In in, int64_t rows, int64_t cols, const Spli
         } else {
 #pragma unroll
           for (int v = 0; v < 4; ++v)
-            if (v < nv) w[v] = __ldg(in.p + base + c + v);
+            if (v < nv) w[v] = in.p[base + c + v];
         }
         long long d[4][kMaxDigits];
 #pragma unroll
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t row
       } else if (c < c1) {
 #pragma unroll
         for (int v = 0; v < 3; ++v)
-          if (c + v < c1) w[g][v] = __ldg(in.p + base + c + v);
+          if (c + v < c1) w[g][v] = in.p[base + c + v];
       }
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(256) slice_run_kernel(const In in, int64_t row
 // 668 us with 32-bit ones, 428 us; 9000 x 40000 in runs of 320: 2090 us with the registers of 1024
 // columns, 946 us.
 template <int NG>
-__global__ void __launch_bounds__(256) slice_pairs_kernel(const float *__restrict__ x2, int64_t rows, int64_t cols,
+__global__ void __launch_bounds__(256) slice_pairs_kernel(const float *x2, int64_t rows, int64_t cols,
                                                           const SplitMap m, int64_t chunk, uint16_t *__restrict__ out,
                                                           int64_t ldo, int64_t plane) {
   pdl_wait();
@@ -834,14 +834,14 @@ __global__ void __launch_bounds__(256) slice_pairs_kernel(const float *__restric
       const int64_t c = c0 + 128 * g + 4 * lane;
       float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
       if (c + 4 <= c1) {
-        a = __ldg(src + c / 2);
-        b = __ldg(src + c / 2 + 1);
+        a = src[c / 2];
+        b = src[c / 2 + 1];
       } else if (c < c1) {
         const float2 *p = reinterpret_cast<const float2 *>(src) + c;
-        const float2 y0 = __ldg(p);
+        const float2 y0 = *p;
         a.x = y0.x; a.y = y0.y;
-        if (c + 1 < c1) { const float2 y = __ldg(p + 1); a.z = y.x; a.w = y.y; }
-        if (c + 2 < c1) { const float2 y = __ldg(p + 2); b.x = y.x; b.y = y.y; }
+        if (c + 1 < c1) { const float2 y = p[1]; a.z = y.x; a.w = y.y; }
+        if (c + 2 < c1) { const float2 y = p[2]; b.x = y.x; b.y = y.y; }
       }
       h[g][0] = make_float2(a.x, a.z); l[g][0] = make_float2(a.y, a.w);
       h[g][1] = make_float2(b.x, b.z); l[g][1] = make_float2(b.y, b.w);
