@@ -1,7 +1,9 @@
 // C entries into the C++ core for tests that the C ABI does not reach: error codes planted on the host
-// in place of a device wait that gave up, single FP64 products, and the memory pools.
+// in place of a device wait that gave up, single FP64 products, the memory pools, and the small dense
+// solvers in both of their forms.
 #include <string>
 
+#include "../votca_gb300/csrc/davidson.cuh"
 #include "../votca_gb300/csrc/handle.cuh"
 #include "../votca_gb300/csrc/oz_gemm.cuh"
 #include "../votca_gb300/csrc/tc_engine.cuh"
@@ -154,6 +156,20 @@ int shim_pool_release() {
   return on_stream([&](cudaStream_t) {
     delete g_used;
     g_used = nullptr;
+  });
+}
+
+// Cholesky QR of a Gram matrix.
+int shim_cholqr(const double *G, int nb, const double *norms0, int check, int fast, double *Rinv, int *ok, int *flag) {
+  return on_stream([&](cudaStream_t s) {
+    Dev<double> g(G, nb * nb, s), n0(norms0, nb, s), r(nullptr, nb * nb, s);
+    Dev<int> o(nullptr, 2, s);
+    vgb::cholqr(g.get(), nb, r.get(), n0.get(), check != 0, o.get(), o.get() + 1, fast != 0, s);
+    int h[2];
+    o.read(h, 2);
+    r.read(Rinv, nb * nb);
+    *ok = h[0];
+    *flag = h[1];
   });
 }
 

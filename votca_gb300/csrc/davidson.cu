@@ -451,7 +451,8 @@ __global__ void __launch_bounds__(256) cholqr_fast_kernel(const double *G, int n
     } else if (warp == 1) {  // the tests, on other quarters of the SM
       if (lane == 0 && !(d > 1e-10 * g0[k])) bad = 1;
     } else if (warp == 2 && chk && k > 0) {
-      if (lane == 0 && sqrt(d) <= 1e-12 * n0[k]) *flag = 1;
+      // only a pivot that passes the other test: the Gram-Schmidt that takes over judges the others
+      if (lane == 0 && d > 1e-10 * g0[k] && sqrt(d) <= 1e-12 * n0[k]) *flag = 1;
     }
     __syncthreads();
     if (bad) break;
@@ -473,6 +474,16 @@ __global__ void __launch_bounds__(256) cholqr_fast_kernel(const double *G, int n
   }
   if (tid == 0) *ok = 1;
 }
+
+}  // namespace
+
+void cholqr(const double *G, int nb, double *Rinv, const double *norms0, bool check, int *ok, int *flag, bool fast,
+            cudaStream_t s) {
+  launch_pdl(fast ? cholqr_fast_kernel : cholqr_kernel, 1, 256, 0, s, G, nb, Rinv, norms0, check ? 1 : 0, ok, flag);
+  VGB_LAUNCH_CHECK();
+}
+
+namespace {
 
 // DavidsonSolver::gramschmidt on columns [nstart, ncols) of Q (ld n).
 void gramschmidt(Ctx &x, double *Q, int64_t nstart, int64_t ncols, DeviceBuffer<double> &work,
@@ -501,9 +512,7 @@ void gramschmidt(Ctx &x, double *Q, int64_t nstart, int64_t ncols, DeviceBuffer<
       double *G = x.gs_part.get(), *Ri = G + nupdate * nupdate, *T = Ri + nupdate * nupdate;
       x.gs_err.resize(2);
       x.gemm_tn(Q + nstart * n, n, nupdate, Q + nstart * n, n, nupdate, G, nupdate, 1.0, 0.0);
-      launch_pdl(x.gemm_path == 0 ? cholqr_fast_kernel : cholqr_kernel, 1, 256, 0, x.s, G, (int)nupdate, Ri, norms0, pass == 1 ? 1 : 0, x.gs_err.get() + 1,
-                                        flag.get());
-      VGB_LAUNCH_CHECK();
+      cholqr(G, (int)nupdate, Ri, norms0, pass == 1, x.gs_err.get() + 1, flag.get(), x.gemm_path == 0, x.s);
       int ok = 0;
       VGB_CUDA(cudaMemcpyAsync(&ok, x.gs_err.get() + 1, sizeof(int), cudaMemcpyDeviceToHost, x.s));
       VGB_CUDA(cudaStreamSynchronize(x.s));

@@ -25,4 +25,10 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
                     const double *host_guess, int64_t guess_cols, double *evecs_dev,
                     DavidsonOutput &out, cudaStream_t s);
 
+// R^-1 (nb x nb, upper triangular, nb <= 64) of the Cholesky factor R of a block's Gram matrix G, on the
+// device.  *ok = 0 (and no R^-1) when a pivot is too small a part of its diagonal; check: *flag = 1
+// when a column lost all of its norms0 to the ones before it.  fast: without divisions.
+void cholqr(const double *G, int nb, double *Rinv, const double *norms0, bool check, int *ok, int *flag, bool fast,
+            cudaStream_t s);
+
 }  // namespace vgb
