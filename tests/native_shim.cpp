@@ -6,6 +6,7 @@
 #include "../votca_gb300/csrc/davidson.cuh"
 #include "../votca_gb300/csrc/handle.cuh"
 #include "../votca_gb300/csrc/oz_gemm.cuh"
+#include "../votca_gb300/csrc/small_eig.cuh"
 #include "../votca_gb300/csrc/tc_engine.cuh"
 
 namespace {
@@ -170,6 +171,43 @@ int shim_cholqr(const double *G, int nb, const double *norms0, int check, int fa
     r.read(Rinv, nb * nb);
     *ok = h[0];
     *flag = h[1];
+  });
+}
+
+// One symmetric eigenproblem (m x m, nw lowest pairs).
+int shim_sym_eig(const double *T, int64_t m, int64_t nw, int fast, double *lam, double *U) {
+  return on_stream([&](cudaStream_t s) {
+    Dev<double> t(T, m * m, s), l(nullptr, nw, s), u(nullptr, m * nw, s), w(nullptr, vgb::sym_eig_work_doubles(m, nw), s);
+    Dev<int> info(nullptr, 1, s);
+    vgb::SymEigJob j;
+    j.T = t.get(); j.ldt = m; j.m = m; j.nw = nw; j.U = u.get(); j.ldu = m; j.lam = l.get();
+    j.work = w.get(); j.info = info.get(); j.fast = fast != 0;
+    vgb::sym_eig_device(&j, 1, s);
+    int st = 0;
+    info.read(&st, 1);
+    if (st) vgb::fail(BSE_ERR_NUMERICAL, "sym_eig");
+    l.read(lam, nw);
+    u.read(U, m * nw);
+  });
+}
+
+// One harmonic-Ritz problem.
+int shim_gen_eig(const double *T, const double *B, int64_t m, int64_t nw, int fast, double *lam, double *U,
+                 int *selected) {
+  return on_stream([&](cudaStream_t s) {
+    Dev<double> t(T, m * m, s), b(B, m * m, s), l(nullptr, nw, s), u(nullptr, m * nw, s),
+        w(nullptr, vgb::gen_eig_work_doubles(m, nw), s);
+    Dev<int> info(nullptr, 2, s);
+    vgb::GenEigJob j;
+    j.T = t.get(); j.B = b.get(); j.ldt = m; j.m = m; j.nw = nw; j.U = u.get(); j.ldu = m; j.lam = l.get();
+    j.work = w.get(); j.info = info.get(); j.fast = fast != 0;
+    vgb::gen_eig_device(&j, 1, s);
+    int st[2];
+    info.read(st, 2);
+    if (st[0]) vgb::fail(BSE_ERR_NUMERICAL, "gen_eig " + std::to_string(st[0]));
+    *selected = st[1];
+    l.read(lam, nw);
+    u.read(U, m * nw);
   });
 }
 

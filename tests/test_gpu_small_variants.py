@@ -1,15 +1,87 @@
 """The small dense solvers of the Davidson iteration in both of their forms (with divisions: split-precision
-solves; without: FP64 solves) at the edges of their layouts, through the same checks: the Cholesky QR."""
+solves, lockstep batches and the solvers' own entry points; without: FP64 solves) at the edges of their
+layouts, through the same checks: the symmetric eigensolver, the harmonic-Ritz solver and the Cholesky QR."""
 import ctypes
 
 import numpy as np
 import pytest
 
 import native
+from votca_gb300 import _lib
 
 pytestmark = pytest.mark.gpu
 
 p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+i64 = ctypes.c_int64
+
+
+def _sym(T, nw, fast):
+    L = native.load()
+    m = T.shape[0]
+    lam, U = np.zeros(nw), np.zeros((m, nw), order="F")
+    assert L.shim_sym_eig(p(T), i64(m), i64(nw), fast, p(lam), p(U)) == 0, L.shim_last_error()
+    return lam, U
+
+
+def _gen(T, B, nw, fast):
+    L = native.load()
+    m = T.shape[0]
+    lam, U, sel = np.zeros(nw), np.zeros((m, nw), order="F"), ctypes.c_int()
+    assert L.shim_gen_eig(p(T), p(B), i64(m), i64(nw), fast, p(lam), p(U), ctypes.byref(sel)) == 0, L.shim_last_error()
+    return lam, U, sel.value
+
+
+# tolerances as in test_gpu_sym_eig_sizes.py and test_gpu_harmonic_ritz_sizes.py
+@pytest.mark.parametrize("fast", [0, 1])
+@pytest.mark.parametrize("m,nw", [(1, 1), (2, 2), (3, 1), (32, 8), (33, 9), (37, 37), (64, 20), (65, 20), (86, 86), (257, 3)])
+def test_symmetric(m, nw, fast):
+    rng = np.random.default_rng(m + nw)
+    d = np.linspace(5.0, 30.0, m)
+    Q = np.linalg.qr(rng.standard_normal((m, m)))[0]
+    T = (Q * d) @ Q.T
+    T = np.asfortranarray(0.5 * (T + T.T))
+    lam, U = _sym(T, nw, fast)
+    tol = 30.0 * m * 2.0**-49
+    assert np.abs(lam - d[:nw]).max() < tol
+    assert np.abs(T @ U - U * lam).max() < tol
+    assert np.abs(U.T @ U - np.eye(nw)).max() < max(1.0, (m - 1) / 25.0) * tol
+
+
+@pytest.mark.parametrize("fast", [0, 1])
+@pytest.mark.parametrize("m,nw", [(1, 1), (2, 2), (31, 31), (60, 33), (97, 4), (98, 4), (128, 40), (129, 3)])
+def test_pencil(m, nw, fast):
+    rng = np.random.default_rng(m)
+    d = np.linspace(1.0, 3.0, m)
+    Q = np.linalg.qr(rng.standard_normal((m, m)))[0]
+    T = (Q * d) @ Q.T
+    T = np.asfortranarray(0.5 * (T + T.T))
+    B = np.asfortranarray(T @ T)
+    lam, U, sel = _gen(T, B, nw, fast)
+    assert sel == nw
+    np.testing.assert_allclose(lam, d[:nw], rtol=0, atol=1e-10)
+    assert np.abs(T @ U - U * lam).max() < 1e-10
+
+
+def test_entry_points_divide():
+    """bse_small_sym_eig and bse_small_gen_eig: the variants with divisions, to the last bit."""
+    L = _lib.load()
+    rng = np.random.default_rng(5)
+    m, nw = 40, 12
+    T = rng.standard_normal((m, m))
+    T = np.asfortranarray(T + T.T)
+    one = lambda x: np.array([x], dtype=np.int64).ctypes.data_as(ctypes.POINTER(i64))
+    dp = lambda a: a.ctypes.data_as(_lib.c_dp)
+    lam, U = np.zeros(nw), np.zeros((m, nw), order="F")
+    _lib.check(L.bse_small_sym_eig(1, one(m), one(nw), dp(T), dp(lam), dp(U), None))
+    ref = _sym(T, nw, 0)
+    np.testing.assert_array_equal(lam, ref[0])
+    np.testing.assert_array_equal(U, ref[1])
+    B = np.asfortranarray(T @ T + 40 * np.eye(m))
+    sel = i64()
+    _lib.check(L.bse_small_gen_eig(m, nw, dp(T), dp(B), dp(lam), dp(U), ctypes.byref(sel)))
+    ref = _gen(T, B, nw, 0)
+    np.testing.assert_array_equal(lam, ref[0])
+    np.testing.assert_array_equal(U, ref[1])
 
 
 def _cholqr(G, n0, fast):

@@ -671,7 +671,6 @@ int bse_small_sym_eig(int64_t njobs, const int64_t *m, const int64_t *nw, const 
       vgb::SymEigJob &j = jobs[i];
       j.T = dT.get() + ot; j.ldt = m[i]; j.m = m[i]; j.nw = nw[i];
       j.U = dU.get() + ou; j.ldu = m[i]; j.lam = dl.get() + ol; j.work = dw.get() + ow; j.info = dinfo.get() + i;
-      j.fast = true;
       if (phase_cycles) j.clocks = dclk.get() + 5 * i;
       ot += m[i] * m[i]; ol += nw[i]; ou += m[i] * nw[i]; ow += vgb::sym_eig_work_doubles(m[i], nw[i]);
     }

@@ -68,7 +68,7 @@ struct GenEigJob {
   int *info = nullptr;   // two ints: [0] 0 ok, 1 invalid sizes, 2 B singular or B^-1 T not finite,
                          // 3 QR iteration without convergence, 4 a complex eigenvalue without
                          // partner (its index in [1]); on success [1] = pairs selected
-  bool fast = true;      // reflectors of the QR iteration without divisions (last bits differ)
+  bool fast = false;     // reflectors of the QR iteration without divisions (last bits differ)
 };
 constexpr int64_t kGenEigMaxM = 1024;
 int64_t gen_eig_work_doubles(int64_t m, int64_t nw);
