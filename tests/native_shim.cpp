@@ -1,11 +1,12 @@
 // C entries into the C++ core for tests that the C ABI does not reach: error codes planted on the host
 // in place of a device wait that gave up, single FP64 products, the memory pools, and the small dense
-// solvers in both of their forms.
+// solvers in both of their forms, and single slice products.
 #include <string>
 
 #include "../votca_gb300/csrc/davidson.cuh"
 #include "../votca_gb300/csrc/handle.cuh"
 #include "../votca_gb300/csrc/oz_gemm.cuh"
+#include "../votca_gb300/csrc/slice_gemm.cuh"
 #include "../votca_gb300/csrc/small_eig.cuh"
 #include "../votca_gb300/csrc/tc_engine.cuh"
 
@@ -208,6 +209,29 @@ int shim_gen_eig(const double *T, const double *B, int64_t m, int64_t nw, int fa
     *selected = st[1];
     l.read(lam, nw);
     u.read(U, m * nw);
+  });
+}
+
+// C (M x N, column-major) = A B^T for A (M x K) and B (N x K), rows contiguous, as one slice product.
+int shim_slice_gemm(const double *A, const double *B, int64_t M, int64_t N, int64_t K, int64_t chain, double *C) {
+  return on_stream([&](cudaStream_t s) {
+    constexpr int S = 5;
+    Dev<double> a(A, M * K, s), b(B, N * K, s), c(nullptr, M * N, s);
+    Dev<uint16_t> pa(nullptr, S * M * K, s), pb(nullptr, S * N * K, s);
+    Dev<int> err(nullptr, 1, s);
+    vgb::SplitMap m;
+    m.rdiv = 1; m.rs1 = K; m.rs2 = 0; m.cs = 1; m.rlim = 1;
+    vgb::slice_f64(a.get(), M, K, m, S, chain, pa.get(), K, M * K, s);
+    vgb::slice_f64(b.get(), N, K, m, S, chain, pb.get(), K, N * K, s);
+    vgb::TcEpilogue e;
+    e.kind = vgb::TcEpilogue::AXPBY_F64;
+    e.rd = M; e.ro2 = 1; e.rlim = M;
+    e.cd = N; e.co2 = M; e.clim = N;
+    e.out_f64 = c.get(); e.alpha = 1.0; e.beta = 0.0;
+    vgb::DeviceBuffer<double> gpart;
+    vgb::slice_gemm(vgb::SliceMat{pa.get(), K, M, 0}, vgb::SliceMat{pb.get(), K, N, 0}, M, N, K, chain, S, e, gpart,
+                    err.get(), s);
+    c.read(C, M * N);
   });
 }
 

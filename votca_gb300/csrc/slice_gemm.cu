@@ -262,25 +262,36 @@ __global__ void __launch_bounds__(kGemmThreads, 1) slice_gemm_kernel(const __gri
   }
 }
 
-// Y = epi(sum over the groups' float pairs), part[g][n][i]: a float-pair sum in group order.
-__global__ void reduce_pairs_kernel(const float2 *part, int64_t M, int64_t N, int groups,
-                                    const TcEpilogue e) {
+// FP64 sum of element t over the groups' float pairs, the high and the low parts each exactly where
+// sum_splits can; N >= groups.
+template <int N>
+__device__ __forceinline__ double sum_pairs(const float2 *part, int64_t total, int groups) {
+  SplitRegs<N> h, l;
+#pragma unroll
+  for (int g = 0; g < N; ++g) {
+    const float2 x = g < groups ? __ldcg(part + g * total) : make_float2(0.f, 0.f);
+    h.w[g] = __float_as_uint(x.x);
+    l.w[g] = __float_as_uint(x.y);
+  }
+  return sum_splits(groups, h) + sum_splits(groups, l);
+}
+
+// Y = epi(sum over the groups' float pairs), part[g][n][i].
+__global__ void reduce_pairs_kernel(const float2 *part, int64_t M, int64_t N, int groups, const TcEpilogue e) {
   pdl_wait();
   const int64_t total = M * N;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const QuotRem tx = quot_rem(t, M);
     const QuotRem ix = quot_rem(tx.r, e.rd), nx = quot_rem(tx.q, e.cd);
     if (ix.r >= e.rlim || nx.r >= e.clim) continue;
-    float h = 0.f, l = 0.f;
-#pragma unroll 4
-    for (int g = 0; g < groups; ++g) {
-      const float2 x = part[g * total + t];
-      const float s = h + x.x, bb = s - h;
-      l += (h - (s - bb)) + (x.x - bb) + x.y;
-      h = s;
-    }
+    const unsigned *p = reinterpret_cast<const unsigned *>(part + t);
+    double sum;
+    if (groups <= 4) sum = sum_pairs<4>(part + t, total, groups);
+    else if (groups <= 8) sum = sum_pairs<8>(part + t, total, groups);
+    else if (groups <= 16) sum = sum_pairs<16>(part + t, total, groups);
+    else sum = sum_splits(groups, SplitMem{p, 2 * total}) + sum_splits(groups, SplitMem{p + 1, 2 * total});
     double *y = e.out_f64 + ix.q * e.ro1 + ix.r * e.ro2 + nx.q * e.co1 + nx.r * e.co2;
-    const double r = e.alpha * ((double)h + (double)l);
+    const double r = e.alpha * sum;
     *y = (e.beta == 0.0) ? r : fma(e.beta, *y, r);
   }
 }

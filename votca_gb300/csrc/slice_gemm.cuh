@@ -18,8 +18,8 @@ struct SliceMat {
 // PAIR_F32: the sum as float pairs).  chain: the K elements of one digit scale in both operands, at
 // most 1024, dividing K.  A digit level a + b accumulates in the tensor core for at most 512 K
 // elements of one run: level 4 sums at most 512 (2 2^13 + 3 2^12) < 2^24 units, the others less, so
-// the sums are exact; runs and levels are added as float pairs (about 48 bits).  gpart: scratch for
-// the partial sums of tiles whose runs are shared by several CTAs.  err: device int, set when a
+// the sums are exact; the runs and levels of a CTA are added as float pairs (about 48 bits), the
+// sums of CTAs that share a tile's runs in FP64.  gpart: scratch for those.  err: device int, set when a
 // bounded wait gives up.
 void slice_gemm(const SliceMat &A, const SliceMat &B, int64_t M, int64_t N, int64_t K, int64_t chain, int digits,
                 const TcEpilogue &fe, DeviceBuffer<double> &gpart, int *err, cudaStream_t s);
