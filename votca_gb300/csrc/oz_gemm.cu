@@ -36,6 +36,8 @@ constexpr int kGemmThreads = 64 + 32 * (kEpi + kTab);  // warp 0: TMA, warp 1: M
 constexpr int BITS = 8 * S - 1;              // digit window: |x| < 2^e -> |m| <= 2^BITS
 constexpr int BIAS = 50;                     // operand digits carry 2^(BIAS - row exponent)
 constexpr int ZERO_RUN = -100000;            // exponent of a run of zeros
+constexpr int kOpposed = 12;                 // bits that opposed gradings along K may have
+constexpr int TOP = 127 + BIAS - 1;          // exponent of a row's largest first digits (64 .. 127)
 constexpr int E_MAX = 900;                   // larger or smaller exponents take the FMA path
 static_assert(LV * BN <= 512 && SMEM_BYTES <= 232448, "tile exceeds the SM");
 
@@ -48,6 +50,7 @@ struct Operand {
   int *erow = nullptr;         // exponent of the row's largest element (per row)
   int *erun = nullptr;         // per (row, run), only for rows of several segments
   int nruns = 1;
+  int *prof = nullptr;         // per K element: the largest first digit of any row, as bf16 bits
 };
 
 // ---------------- digits ----------------
@@ -90,12 +93,16 @@ __device__ __forceinline__ void digits2(unsigned long long x0, unsigned long lon
   }
 }
 
-// Eight consecutive K elements into the planes (16 bytes each).
+// Eight consecutive K elements into the planes (16 bytes each); top: the largest magnitudes of their first
+// digits so far, two bf16 to a word.
 __device__ __forceinline__ void store8(const unsigned long long *x, int e, const float (&sc)[S], const float (&cc)[S],
-                                       uint16_t *out, int64_t plane) {
+                                       uint16_t *out, int64_t plane, uint32_t (&top)[4]) {
   uint32_t d[4][S];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) digits2(x[2 * v], x[2 * v + 1], e, sc, cc, d[v]);
+  for (int v = 0; v < 4; ++v) {
+    digits2(x[2 * v], x[2 * v + 1], e, sc, cc, d[v]);
+    top[v] = __vmaxu2(top[v], d[v][0] & 0x7FFF7FFFu);
+  }
 #pragma unroll
   for (int t = 0; t < S; ++t, out += plane)
     *reinterpret_cast<uint4 *>(out) = make_uint4(d[0][t], d[1][t], d[2][t], d[3][t]);
@@ -136,6 +143,8 @@ __global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant_
   extern __shared__ __align__(16) unsigned long long tile[];
   __shared__ unsigned long long red[256];
   __shared__ int s_e[256];
+  __shared__ uint4 s_top[2][8][SEG / 8];  // first digits per warp, two units deep
+  int pair = 0;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr unsigned long long kAbs = ~(1ull << 63);  // |x| as integers: of a double it is an FP64 instruction
   for (int u0 = blockIdx.x; u0 < units; u0 += gridDim.x) {  // 32-bit divisions: 64-bit ones use the FP64 pipe
@@ -166,6 +175,9 @@ __global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant_
       }
     };
     const bool turned = o.ks != 1;
+    uint32_t top[4] = {0, 0, 0, 0};
+    // read ahead: most units find nothing larger, and need no atomic on a line that all of them share
+    const int known = phase != 1 && tid < kn ? __ldcg(o.prof + k0 + tid) : 0;
     if (turned) {  // lanes along the rows: loads, maxima, tile
       const int r = (warp / nwk) * 32 + lane, k = (warp % nwk) * 32;
       const bool in = r < nrow && k < kp;
@@ -248,9 +260,23 @@ __global__ void __launch_bounds__(256, 2) oz_slice_kernel(const __grid_constant_
       if (in) {
         float sc[S], cc[S];
         digit_scales(rel, sc, cc);
-        store8(x, e, sc, cc, o.planes + row * o.Kp + k0 + k, plane);
+        store8(x, e, sc, cc, o.planes + row * o.Kp + k0 + k, plane, top);
       }
     }
+    if (phase == 1) continue;
+    for (int w = lpr; w < 32; w *= 2) {  // lanes of other rows
+#pragma unroll
+      for (int v = 0; v < 4; ++v) top[v] = __vmaxu2(top[v], __shfl_xor_sync(0xffffffffu, top[v], w));
+    }
+    if (lane < lpr) s_top[pair][warp][lane] = make_uint4(top[0], top[1], top[2], top[3]);
+    __syncthreads();
+    if (tid < kn) {
+      unsigned t = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) t = max(t, (unsigned)reinterpret_cast<const uint16_t *>(s_top[pair][w])[tid]);
+      if ((int)t > max(known, 0)) atomicMax(o.prof + k0 + tid, (int)t);
+    }
+    pair ^= 1;
   }
 }
 
@@ -265,6 +291,7 @@ struct GemmArgs {
   int64_t m_first, b_first;  // first C row and batch of this launch (chunks)
   int mt, nt, ntiles;
   const int *erow_a, *erow_b, *flag;
+  const int *prof_a, *prof_b;
   Operand A, B;              // sources, for the FMA path
   OzMap crow, ccol, cbatch;  // C offsets of tile rows, columns and batches
   int64_t c_split;           // C offset between K splits (partials)
@@ -451,6 +478,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
   TcControl *ctl = (TcControl *)(tabe + 2);
   volatile int *abort_flag = &ctl->abort;
   TileTab *tabs = reinterpret_cast<TileTab *>(smem + STAGES * STAGE_BYTES + 256);
+  __shared__ int s_meet[3];  // A has elements, B has, some meet
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
@@ -464,6 +492,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
       mbar_init(&tabe[i], kEpi);
     }
     ctl->init(p.wait_us);
+    s_meet[0] = s_meet[1] = s_meet[2] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -557,6 +586,27 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
     // ---- output offsets and exponents of every tile, ahead of its epilogue ----
     const int i = threadIdx.x - 64 - 32 * kEpi;  // 0 .. 63
     static_assert(32 * kTab == BN && 2 * BN == BM, "two rows and one column per table thread");
+    // Operands graded in opposite directions along K: with their rows scaled to one, no two first digits
+    // meet in a product above 2^-kOpposed, and the digits, cut 2^-56 below the largest element of a
+    // row, are too few for the whole result.  The same on every CTA.
+    {
+      int any_a = 0, any_b = 0;
+      bool meet = false;  // as a rule among the first K elements
+      for (int64_t k0 = 0; k0 < p.K && !__any_sync(0xffffffffu, meet); k0 += 4 * 32 * kTab)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t k = k0 + u * 32 * kTab + i;
+          const int a = k < p.K ? max(__ldcg(p.prof_a + k), 0) >> 7 : 0;
+          const int b = k < p.K ? max(__ldcg(p.prof_b + k), 0) >> 7 : 0;
+          any_a |= a;
+          any_b |= b;
+          meet |= a && b && a + b >= 2 * TOP - kOpposed;
+        }
+      if (any_a) s_meet[0] = 1;
+      if (any_b) s_meet[1] = 1;
+      if (meet) s_meet[2] = 1;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kTab) : "memory");
+    }
     int it = 0;
     for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x, ++it) {
       const Tile tc = tile_of(p, R);
@@ -616,7 +666,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
       if (!mbar_wait_warp(&tabf[it & 1], (it >> 1) & 1, abort_flag, p.err, 19)) goto epi_done;
       const TileTab &tb = tabs[it & 1];
       const int64_t ro = tb.row[q * 32 + lane];
-      if (ro >= 0) {
+      const bool opposed = s_meet[0] && s_meet[1] && !s_meet[2];  // written before the first table
+      if (ro >= 0 && !opposed) {
         double *crow = p.C + ro;
         const int ea = tb.ea[q * 32 + lane];
         if (p.plain) {
@@ -658,6 +709,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   }
+  if (s_meet[0] && s_meet[1] && !s_meet[2])
+    for (int R = blockIdx.x; R < p.ntiles; R += gridDim.x)
+      fma_tile(p, tile_of(p, R), reinterpret_cast<double *>(smem));
 }
 
 // C (+)= alpha * sum over the K splits of the FP64 partials, in split order; M fastest.
@@ -715,7 +769,8 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   const int64_t nseg = ceil_div(q.Kp, SEG);
   const bool two = nseg > 1;  // exponents before digits
   const int64_t rows_a = q.m_chunk * q.tb_chunk, rows_b = q.N * q.tb_chunk;
-  const int64_t ni = 64 + rows_a + rows_b;  // [flag | row exponents of A | of B], then run exponents
+  // [flag | row exponents of A | of B | K profiles of A | of B], then run exponents
+  const int64_t ni = 64 + rows_a + rows_b + 2 * q.Kp;
   double *partial = nullptr;
   Planes pa(stream), pb(stream);
   try {
@@ -751,7 +806,9 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   int *ip = ws->oz_int.get();
   A.erow = ip + 64;
   B.erow = A.erow + rows_a;
-  A.erun = B.erow + rows_b;
+  A.prof = B.erow + rows_b;
+  B.prof = A.prof + q.Kp;
+  A.erun = B.prof + q.Kp;
   B.erun = A.erun + rows_a * nruns;
   p.K = d.K;
   p.nkb = q.nkb;
@@ -815,6 +872,8 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
       p.b_plane = (int)B.rows;
       p.erow_a = A.erow;
       p.erow_b = B.erow;
+      p.prof_a = A.prof;
+      p.prof_b = B.prof;
       p.mt = (int)ceil_div(p.M, BM);
       p.nt = (int)ceil_div(p.N, BN);
       p.ntiles = (int)(p.mt * p.nt * tn * q.splits);
