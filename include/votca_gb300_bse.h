@@ -19,6 +19,11 @@
  * Threading: a handle may be used from one host thread at a time; every call
  * is synchronous on return (host-pointer calls) or stream-ordered on the
  * stream passed in (the *_device calls).
+ *
+ * Memory: freed blocks of handles stay in the device's default stream-ordered
+ * pool until a handle is destroyed or an allocation of this library fails; calls
+ * without a handle use a pool of their own, of which at most 1 GB stays
+ * reserved, until the same events.
  */
 #ifndef VOTCA_GB300_BSE_H
 #define VOTCA_GB300_BSE_H
@@ -40,16 +45,29 @@ typedef enum bse_status {
 } bse_status;
 
 typedef enum bse_precision {
-  BSE_PRECISION_FP64 = 0,   /* every product in FP64 (the plain drop-in) */
+  BSE_PRECISION_FP64 = 0,   /* every product in FP64 (the plain drop-in).  Small contractions are
+                               FMA chains; larger ones, by a rule on their sizes, exact products
+                               of base-256 digits on the tcgen05 tensor cores.  With K terms an
+                               element of A X is then off by at most
+                               K 2^-53 max|row of A| max|column of X|, and by less than the FMA
+                               chain in the 2-norm; the chain's own bound, K 2^-53 sum |a||x|, is
+                               not kept element by element: what lies more than 2^56 below the
+                               largest element of its row or column (within 1024 terms) does not
+                               count.  Operands graded in opposite directions along K by more
+                               than 12 bits run as FMA chains; for callers that need that bound
+                               for every element, bse_op_matmul_device_noalloc always does.
+                               The dense operator, the screening, three-centre and dipole
+                               entry points and the gradients use the same products. */
   BSE_PRECISION_MIXED = 1,  /* Hx/Hd/Hd2 contractions as BF16x3 split products on
                                tcgen05 tensor cores with FP32 accumulation;
                                Hqp and all Davidson algebra in FP64 */
   BSE_PRECISION_SLICED = 2  /* Hx/Hd/Hd2 contractions as Ozaki slice products on the
                                tcgen05 tensor cores: each FP64 operand cut into five 7-bit
                                digit planes (power-of-two scale per run of <= 1024 K
-                               elements), every pair of digit levels up to the fifth
-                               accumulated exactly in FP32 over one run, runs and pairs
-                               summed in FP64, intermediates kept in FP64; agrees with the
+                               elements), the pairs of the digit levels up to the fifth
+                               accumulated exactly in FP32 over at most 512 of them, levels and
+                               runs summed as float pairs (about 48 bits) and across CTAs in
+                               FP64, intermediates kept as float pairs; agrees with the
                                FP64 product to about 1e-11 of its scale */
 } bse_precision;
 
@@ -246,7 +264,9 @@ int bse_op_matmul(bse_handle *h, int32_t cqp, int32_t cx, int32_t cd,
                   double *Y, int64_t ldy);
 
 /* Same on device pointers, stream-ordered on `stream` (a cudaStream_t, NULL =
- * legacy default stream). */
+ * legacy default stream).  It returns before the product has run: a bounded wait of a
+ * tensor-core kernel that gives up (any precision) is reported as BSE_ERR_TIMEOUT by the next call
+ * on the handle that waits for its products, and the product is then not complete. */
 int bse_op_matmul_device(bse_handle *h, int32_t cqp, int32_t cx, int32_t cd,
                          int32_t cd2, const double *dX, int64_t ldx, int64_t k,
                          double *dY, int64_t ldy, void *stream);
