@@ -49,11 +49,11 @@ typedef enum bse_precision {
                                FMA chains; larger ones, by a rule on their sizes, exact products
                                of base-256 digits on the tcgen05 tensor cores.  With K terms an
                                element of A X is then off by at most
-                               K 2^-53 max|row of A| max|column of X|, and by less than the FMA
-                               chain in the 2-norm; the chain's own bound, K 2^-53 sum |a||x|, is
-                               not kept element by element: what lies more than 2^56 below the
-                               largest element of its row or column (within 1024 terms) does not
-                               count.  Operands graded in opposite directions along K by more
+                               K 2^-53 max|row of A| max|column of X|, and the result as a rule
+                               by less than that of FMA chains in the 2-norm; the chain's bound,
+                               K 2^-53 sum |a||x|, is not kept element by element: what lies
+                               more than 2^56 below the largest element of its row or column
+                               (within 1024 terms) does not count.  Operands graded in opposite directions along K by more
                                than 12 bits run as FMA chains; for callers that need that bound
                                for every element, bse_op_matmul_device_noalloc always does.
                                The dense operator, the screening, three-centre and dipole

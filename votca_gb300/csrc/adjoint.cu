@@ -152,7 +152,9 @@ void scatter_mmn_gradient(const BseOperator &op, const double *gMvc, const doubl
     a.m_v0 = op.m_v0; a.m_c0 = op.m_c0; a.n_v0 = op.n_v0; a.n_c0 = op.n_c0;
     a.out = buf.get();
     const int64_t total = a.cnt * slice;
-    launch_pdl(scatter_grad_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 16LL * 152)), 256, 0, s, a);
+    launch_pdl(scatter_grad_kernel,
+               (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(total, 256), 16LL * 152)), 256, 0, s,
+               a);
     VGB_LAUNCH_CHECK();
     VGB_CUDA(cudaMemcpyAsync(host_out + m0 * slice, buf.get(), total * sizeof(double),
                              cudaMemcpyDeviceToHost, s));
@@ -178,7 +180,8 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
   VGB_CUDA(cudaMemcpyAsync(g.get(), g_host, nr * sizeof(double), cudaMemcpyHostToDevice, s));
   const std::vector<double> gh(g_host, g_host + nr);
   if (gH && c.cqp != 0) {
-    launch_pdl(hqp_grad_kernel, gfor((vt + ct) * (vt + ct)), 256, 0, s, X, ldx, nr, g.get(), vt, ct, c.cqp, gH);
+    launch_pdl(hqp_grad_kernel, gfor((vt + ct) * (vt + ct)), 256, 0, s, X, ldx, nr, g.get(), vt, ct, c.cqp,
+               gH);
     VGB_LAUNCH_CHECK();
   }
   if (gMvc && c.cx != 0) {
@@ -243,8 +246,8 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
     }
     if (gMvv) {
       if (!dense_screening) {
-        launch_pdl(scale_batches_kernel, gfor(naux * vt * vt), 256, 0, s, Q.get(), Wscr.get(), naux, vt * vt, -cd, gMvv,
-                                                                   1);
+        launch_pdl(scale_batches_kernel, gfor(naux * vt * vt), 256, 0, s, Q.get(), Wscr.get(), naux, vt * vt,
+                   -cd, gMvv, 1);
         VGB_LAUNCH_CHECK();
       } else {
         GemmDesc d;  // gMvv[Q][e] += -cd sum_P W[P][Q] Q[P][e]
@@ -258,8 +261,8 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
     }
     if (gW) {
       if (!dense_screening) {
-        launch_pdl(dot_per_batch_kernel, (unsigned)std::min<int64_t>(naux, 4096), 256, 0, s, Q.get(), Mvv.get(), naux,
-                                                                                  vt * vt, -cd, gW);
+        launch_pdl(dot_per_batch_kernel, (unsigned)std::min<int64_t>(naux, 4096), 256, 0, s, Q.get(),
+                   Mvv.get(), naux, vt * vt, -cd, gW);
         VGB_LAUNCH_CHECK();
       } else {
         GemmDesc d;  // gW[P][Q] += -cd sum_e Q[P][e] Mvv[Q][e]   (column-major naux x naux)
@@ -362,8 +365,8 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
         a.nb1 = naux;
         dgemm(a, s, &ws);
         if (!dense_screening) {
-          launch_pdl(dot_per_batch_kernel, (unsigned)std::min<int64_t>(naux, 4096), 256, 0, s, T2.get(), T3.get(), naux,
-                                                                                    vv, alpha, gW);
+          launch_pdl(dot_per_batch_kernel, (unsigned)std::min<int64_t>(naux, 4096), 256, 0, s, T2.get(),
+                     T3.get(), naux, vv, alpha, gW);
           VGB_LAUNCH_CHECK();
         } else {
           // the product pairs a^Q with bw^Q = sum_P b^P W(P, Q):  dW(P, Q) += alpha <Yb^P, Za^Q>
@@ -379,7 +382,8 @@ void BseOperator::quad_gradient(const Coef &c, const double *X, int64_t ldx, int
       if (gMcv) {
         const double *Zw = T2.get();  // sum_Q W_QP Za^Q
         if (!dense_screening) {
-          launch_pdl(scale_batches_kernel, gfor(naux * vv), 256, 0, s, T2.get(), Wscr.get(), naux, vv, 1.0, T1.get(), 0);
+          launch_pdl(scale_batches_kernel, gfor(naux * vv), 256, 0, s, T2.get(), Wscr.get(), naux, vv, 1.0,
+                     T1.get(), 0);
           VGB_LAUNCH_CHECK();
           Zw = T1.get();
         } else {

@@ -656,7 +656,7 @@ constexpr int kGsStaged = 200 * 1024;
 void run_gs(const std::vector<GsJob> &jobs, cudaStream_t s) {
   int64_t bytes = 0;
   for (const GsJob &j : jobs)
-    bytes = std::max<int64_t>(bytes, ceil_div(j.n, (int64_t)kGsCluster) * (j.ncols - j.nstart) * (int64_t)sizeof(double));
+    bytes = std::max<int64_t>(bytes, ceil_div(j.n, (int64_t)kGsCluster) * (j.ncols - j.nstart) * 8);
   if (bytes > kGsStaged || (int64_t)jobs.size() * kGsCluster * (bytes + 4096) > (int64_t)sm_count() * kGsStaged) {
     launch_jobs(jobs, gs_kernel<false>, kGsCluster, true, s, kGsThreads);
     return;

@@ -523,8 +523,8 @@ void BseOperator::apply_hqp(double cqp, const double *X, int64_t ldx, int64_t k,
   timer.begin(STAGE_HQP, s);
   struct End { StageTimer &t; cudaStream_t s; ~End() { t.end(STAGE_HQP, s); } } end_{timer, s};
   if (hqp_diagonal) {
-    launch_pdl(hqp_diag_kernel, grid_for(dim * k), 256, 0, s, cqp, Hcc.get(), Hvv.get(), vt, ct, X, ldx, k,
-                                                      Y, ldy, accumulate ? 1 : 0);
+    launch_pdl(hqp_diag_kernel, grid_for(dim * k), 256, 0, s, cqp, Hcc.get(), Hvv.get(), vt, ct, X, ldx, k, Y,
+               ldy, accumulate ? 1 : 0);
     VGB_LAUNCH_CHECK();
     return;
   }
@@ -717,7 +717,8 @@ void BseOperator::diagonal(const Coef &c, double *D, cudaStream_t s) {
   a.vt = vt; a.ct = ct; a.naux = naux; a.dim = dim;
   a.Bvc = Bvc.get(); a.Mcv = Mcv.get(); a.dcc = dcc.get(); a.dvv = dvv.get();
   a.Hcc = Hcc.get(); a.Hvv = Hvv.get(); a.D = D;
-  launch_pdl(diagonal_kernel, (unsigned)std::min<int64_t>(ceil_div(dim, 32), 64LL * sm_count()), 32 * kDiagSlices, 0, s, a);
+  launch_pdl(diagonal_kernel, (unsigned)std::min<int64_t>(ceil_div(dim, 32), 64LL * sm_count()),
+             32 * kDiagSlices, 0, s, a);
   VGB_LAUNCH_CHECK();
 }
 

@@ -107,7 +107,9 @@ void eig_gradient_blocks(vgb::BseOperator &op, const vgb::Coef &a, const vgb::Co
     half[nr + k] = -0.5 * g[k];
   }
   vgb::DeviceBuffer<double> PM(2 * op.dim * nr);
-  vgb::launch_pdl(plus_minus_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(vgb::ceil_div(op.dim * nr, 256), 2432)), 256, 0, s, X, Y, ldx, op.dim, nr, PM.get(), PM.get() + op.dim * nr);
+  vgb::launch_pdl(plus_minus_kernel,
+                  (unsigned)std::max<int64_t>(1, std::min<int64_t>(vgb::ceil_div(op.dim * nr, 256), 2432)),
+                  256, 0, s, X, Y, ldx, op.dim, nr, PM.get(), PM.get() + op.dim * nr);
   VGB_LAUNCH_CHECK();
   op.quad_gradient(*b, PM.get(), op.dim, 2 * nr, half.data(), gvc, gcv, gvv, gcc, gh, gw, true, s);
 }

@@ -319,8 +319,8 @@ struct Ctx {
     const bool fast = gemm_path == 0;
     dim3 grid(fast ? (unsigned)std::max<int64_t>(1, std::min<int64_t>(kRedChunks, ceil_div(n, 512))) : kRedChunks,
               (unsigned)ncols);
-    launch_pdl(coldot_kernel, grid, 256, 0, s, A, lda, B ? B : A, B ? ldb : lda, n, red_partial.get(), red_arrived.get(),
-                                       sqrt_ ? 1 : 0, fast ? 1 : 0, out);
+    launch_pdl(coldot_kernel, grid, 256, 0, s, A, lda, B ? B : A, B ? ldb : lda, n, red_partial.get(),
+               red_arrived.get(), sqrt_ ? 1 : 0, fast ? 1 : 0, out);
     VGB_LAUNCH_CHECK();
   }
   void scale_cols(double *A, int64_t lda, int64_t ncols, const double *norms) {
@@ -479,7 +479,8 @@ __global__ void __launch_bounds__(256) cholqr_fast_kernel(const double *G, int n
 
 void cholqr(const double *G, int nb, double *Rinv, const double *norms0, bool check, int *ok, int *flag, bool fast,
             cudaStream_t s) {
-  launch_pdl(fast ? cholqr_fast_kernel : cholqr_kernel, 1, 256, 0, s, G, nb, Rinv, norms0, check ? 1 : 0, ok, flag);
+  launch_pdl(fast ? cholqr_fast_kernel : cholqr_kernel, 1, 256, 0, s, G, nb, Rinv, norms0, check ? 1 : 0, ok,
+             flag);
   VGB_LAUNCH_CHECK();
 }
 
@@ -752,16 +753,16 @@ bool fp64_polish(Ctx &x, TimedApply &apply, const double *Dd, const double *q0, 
     VGB_CUDA(cudaMemcpyAsync(lamu, upd_lam.data(), nupdate * sizeof(double), cudaMemcpyHostToDevice, s));
     double *Vnew = V.get() + m * n;
     const bool olsen = correction == 1;
-    launch_pdl(dpr_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, res.get(), q.get(), n, Dd, colsd.get(), lamu,
-                                                      nupdate, olsen ? 0 : 1, olsen ? dq : nullptr);
+    launch_pdl(dpr_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, res.get(), q.get(), n, Dd,
+               colsd.get(), lamu, nupdate, olsen ? 0 : 1, olsen ? dq : nullptr);
     VGB_LAUNCH_CHECK();
     if (olsen) {
       for (int64_t kk = 0; kk < nupdate; ++kk) {
         x.coldots(q.get() + upd[kk] * n, n, Vnew + kk * n, n, 1, numd + kk, false);
         x.coldots(q.get() + upd[kk] * n, n, dq + kk * n, n, 1, dend + kk, false);
       }
-      launch_pdl(olsen_finish_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, q.get(), n, colsd.get(), numd, dend,
-                                                                 nupdate);
+      launch_pdl(olsen_finish_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, q.get(), n, colsd.get(),
+                 numd, dend, nupdate);
       VGB_LAUNCH_CHECK();
     }
     work.resize(nupdate + 8);
@@ -1021,8 +1022,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
     double *Vnew = V.get() + ncols * n;
     const bool olsen = opt.correction == 1;
     launch_pdl(dpr_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, res.get(), q.get(), n, D.get(),
-                                                      colsd.get(), lamu, nupdate, olsen ? 0 : 1,
-                                                      olsen ? dq : nullptr);
+               colsd.get(), lamu, nupdate, olsen ? 0 : 1, olsen ? dq : nullptr);
     VGB_LAUNCH_CHECK();
     if (olsen) {
       // num_k = q_j . delta_k ; den_k = q_j . dpr(q_j)   (signs applied in the finish kernel)
@@ -1031,7 +1031,7 @@ void davidson_solve(DeviceOperator &A, int64_t neigen, const bse_davidson_option
         x.coldots(q.get() + upd[kk] * n, n, dq + kk * n, n, 1, dend + kk, false);
       }
       launch_pdl(olsen_finish_kernel, blocks_for(n * nupdate), 256, 0, s, Vnew, n, q.get(), n, colsd.get(),
-                                                                 numd, dend, nupdate);
+                 numd, dend, nupdate);
       VGB_LAUNCH_CHECK();
     }
     // w.normalized()

@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(THREADS)
   __threadfence();
   const int64_t mn = d.M * d.N;
   const int64_t gi = m0 + tid % TM, gn = n0 + tid / TM;  // lanes along the columns of the partials
-  if (gi < d.M && gn < d.N) add_splits(d, b1, b2, gi, gn, partial + batch * g.splits * mn + gi + gn * d.M, mn, g.splits);
+  if (gi < d.M && gn < d.N)
+    add_splits(d, b1, b2, gi, gn, partial + batch * g.splits * mn + gi + gn * d.M, mn, g.splits);
 }
 
 // The same for all outputs in a launch of its own, for callers without counters.
@@ -189,7 +190,7 @@ void launch_tile(const GemmDesc &d, const Grid &g, double *partial, unsigned *ar
   const int64_t blocks = g.mt * g.nt * g.nbatch * g.splits;
   VGB_REQUIRE(blocks < (1LL << 31), "dgemm: grid too large");
   launch_pdl(dgemm_kernel<TM, TN>, (unsigned)blocks, THREADS, 0, stream, d, g, partial, arrived,
-                                                                  d.a_rs == 1 ? 1 : 0, d.b_rs == 1 ? 1 : 0);
+             d.a_rs == 1 ? 1 : 0, d.b_rs == 1 ? 1 : 0);
   VGB_LAUNCH_CHECK();
 }
 
@@ -223,7 +224,8 @@ void launch(const GemmDesc &d, const FmaPlan &f, double *partial, GemmWorkspace 
   }
   if (f.splits > 1 && !arrived) {
     const int64_t total = d.M * d.N * g.nbatch;
-    launch_pdl(splitk_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256, 0, stream, d, g, partial);
+    launch_pdl(splitk_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 8 * sm_count()), 256,
+               0, stream, d, g, partial);
     VGB_LAUNCH_CHECK();
   }
 }
@@ -383,7 +385,8 @@ void dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws, int splitk
   if (splitk == 0 && oz_dgemm(d, stream, ws)) return;
   if (d.K == 0) {  // C = beta * C
     const int64_t total = d.M * d.N * nbatch;
-    launch_pdl(scale_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream, d, nbatch);
+    launch_pdl(scale_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream, d,
+               nbatch);
     VGB_LAUNCH_CHECK();
     return;
   }
@@ -403,7 +406,8 @@ void dgemm_prealloc(const GemmDesc &d, cudaStream_t stream, double *ws, int64_t 
   if (d.M == 0 || d.N == 0 || nbatch == 0) return;
   if (d.K == 0) {
     const int64_t total = d.M * d.N * nbatch;
-    launch_pdl(scale_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream, d, nbatch);
+    launch_pdl(scale_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 65535), 256, 0, stream, d,
+               nbatch);
     VGB_LAUNCH_CHECK();
     return;
   }

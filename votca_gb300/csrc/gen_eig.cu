@@ -88,7 +88,8 @@ constexpr int kQrThreads = 128;
 __device__ __forceinline__ void qr_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kQrThreads) : "memory"); }
 
 __device__ __forceinline__ int max_exponent(double p, double q, double r) {
-  return max((__double2hiint(p) >> 20) & 0x7FF, max((__double2hiint(q) >> 20) & 0x7FF, (__double2hiint(r) >> 20) & 0x7FF));
+  auto ex = [](double x) { return (__double2hiint(x) >> 20) & 0x7FF; };
+  return max(ex(p), max(ex(q), ex(r)));
 }
 // x 2^-sh for a normal result (else 0), in integers
 __device__ __forceinline__ double scale_down(double x, int sh) {
@@ -679,7 +680,8 @@ __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_const
   double *Uf = place((int64_t)nw * mm, vec);
   double *Hq = LU == gLU ? vec + nw * (2 * mm + 5 * (int64_t)m) : LU;
   double *piv = small ? small : gsmall, *wr = piv + m, *wi = wr + m, *colv = wi + m;
-  int *selv = small ? reinterpret_cast<int *>(small + 4 * m + 4 * (int64_t)m * nw) : reinterpret_cast<int *>(vec + nw * (2 * mm + 5 * (int64_t)m) + (int64_t)hl * m);
+  int *selv = reinterpret_cast<int *>(small ? small + 4 * m + 4 * (int64_t)m * nw
+                                            : vec + nw * (2 * mm + 5 * (int64_t)m) + (int64_t)hl * m);
   if (tid == 0) flag = 0;
   // ---- load ----
   double bm = 0.0;
@@ -917,7 +919,7 @@ __global__ void __launch_bounds__(kGenThreads) gen_eig_kernel(const __grid_const
   int *list = fast + nw;
   const bool can = small != nullptr && m <= kInvMaxM;
   for (int c = tid; c < nw; c += kGenThreads)
-    fast[c] = (can && c < ns && wi[selv[c]] == 0.0 && !close_to_prev(c) && !(c + 1 < ns && close_to_prev(c + 1))) ? 1 : 0;
+    fast[c] = can && c < ns && wi[selv[c]] == 0.0 && !close_to_prev(c) && !(c + 1 < ns && close_to_prev(c + 1));
   __syncthreads();
   if (tid == 0) {
     int n = 0;
@@ -1114,7 +1116,9 @@ void pencil_finish_device(const double *W, int64_t m, const double *nu, const do
   VGB_LAUNCH_CHECK();
 }
 
-int64_t gen_eig_work_doubles(int64_t m, int64_t nw) { return 3 * m * m + 5 * m + nw * (2 * m * m + 5 * m) + m * (m + 1) + 2 * nw + 64; }
+int64_t gen_eig_work_doubles(int64_t m, int64_t nw) {
+  return 3 * m * m + 5 * m + nw * (2 * m * m + 5 * m) + m * (m + 1) + 2 * nw + 64;
+}
 
 void gen_eig_device(const GenEigJob *jobs, int64_t njobs, cudaStream_t s) {
   if (njobs <= 0) return;

@@ -113,7 +113,7 @@ void matmul_noalloc(BseOperator &op, const Coef &c, const double *X, int64_t ldx
   if (c.cqp != 0) {
     if (op.hqp_diagonal) {
       launch_pdl(na_hqp_diag_kernel, na_grid(dim * k), 256, 0, s, c.cqp, op.Hcc.get(), op.Hvv.get(), vt, ct,
-                                                           X, ldx, k, Y, ldy);
+                 X, ldx, k, Y, ldy);
       VGB_LAUNCH_CHECK();
     } else {
       GemmDesc g;

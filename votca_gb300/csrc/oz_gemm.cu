@@ -128,7 +128,8 @@ __host__ __device__ __forceinline__ int slice_rows(int64_t Kp) {
 
 // Digit planes of slice_rows rows and a segment of K per block.  phase 3 (rows of one segment): the
 // row maxima, then the digits; longer rows: phase 1 takes the run and row exponents, phase 2 the
-// digits.  Every element is loaded once per phase.  The digits are made by a warp (part) per row,
+// digits and, for the check of opposed gradings, the largest first digit of every K element (3 % of the
+// kernel's time).  Every element is loaded once per phase.  The digits are made by a warp (part) per row,
 // eight elements per lane, so that the planes are written in whole lines; operands contiguous
 // along K are read that way, others (contiguous along the rows) with a lane per row, 32 elements
 // of it in flight, and turned in shared memory.  Bound: HBM (8 bytes read, 14 written per element)
@@ -388,8 +389,8 @@ __device__ __forceinline__ void store_c(const GemmArgs &p, double *c, double v) 
   *c = p.accumulate ? fma(p.beta, *c, v) : v;
 }
 
-// The tile by FP64 FMA, for operands with infinities, NaNs or exponents at the ends of the range:
-// the 64 x 64 register tiles of dgemm.cu on the CTA's first 256 threads.
+// The tile by FP64 FMA, for operands with infinities, NaNs or exponents at the ends of the range, and for
+// operands graded in opposite directions: the 64 x 64 register tiles of dgemm.cu on the CTA's first 256 threads.
 __device__ __noinline__ void fma_tile(const GemmArgs &p, const Tile &tc, double *smem) {
   constexpr int TK = 16, LD = 65;
   double *As = smem, *Bs = As + TK * LD;
@@ -860,7 +861,8 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
         launch_pdl(oz_slice_kernel, sg, 256, SLICE_SMEM, stream, A, B, (int)ua, (int)(ua + ub), 1, ip);
         VGB_LAUNCH_CHECK();
       }
-      launch_pdl(oz_slice_kernel, sg, 256, SLICE_SMEM, stream, A, B, (int)ua, (int)(ua + ub), two ? 2 : 3, ip);
+      launch_pdl(oz_slice_kernel, sg, 256, SLICE_SMEM, stream, A, B, (int)ua, (int)(ua + ub), two ? 2 : 3,
+                 ip);
       VGB_LAUNCH_CHECK();
       encode_kmajor(&p.map_a, A.planes, S * A.rows, q.Kp, q.Kp, BM, BK);
       encode_kmajor(&p.map_b, B.planes, S * B.rows, q.Kp, q.Kp, BN, BK);
@@ -879,12 +881,14 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
       p.ntiles = (int)(p.mt * p.nt * tn * q.splits);
       p.m_first = m0;
       p.b_first = t0;
-      launch_pdl(oz_gemm_kernel, (unsigned)std::min(p.ntiles, sm_count()), kGemmThreads, SMEM_BYTES, stream, p);
+      launch_pdl(oz_gemm_kernel, (unsigned)std::min(p.ntiles, sm_count()), kGemmThreads, SMEM_BYTES, stream,
+                 p);
       VGB_LAUNCH_CHECK();
     }
   if (q.splits > 1) {
     const int64_t total = q.nbatch * q.M * q.N;
-    launch_pdl(oz_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 8LL * sm_count()), 256, 0, stream, partial, q.M, q.N, q.nbatch, q.splits, q.crow, q.ccol, q.cbatch, d.C, d.alpha, d.beta);
+    launch_pdl(oz_reduce_kernel, (unsigned)std::min<int64_t>(ceil_div(total, 256), 8LL * sm_count()), 256, 0,
+               stream, partial, q.M, q.N, q.nbatch, q.splits, q.crow, q.ccol, q.cbatch, d.C, d.alpha, d.beta);
     VGB_LAUNCH_CHECK();
   }
   return true;

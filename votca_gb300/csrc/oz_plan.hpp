@@ -113,7 +113,7 @@ inline bool oz_plan(const GemmDesc &d, int sms, int64_t plane_budget, OzPlan &q)
   q.Kp = oz_ceil(d.K, kOzStageK) * kOzStageK;
   if (q.Kp >= (1LL << 31) || q.M >= (1LL << 27) || q.N >= (1LL << 27)) return false;
   const int64_t tiles = oz_ceil(q.M, kOzTileM) * oz_ceil(q.N, kOzTileN) * q.nbatch;
-  if (tiles >= (1LL << 24)) return false;  // tile indices (times at most 152 splits) in 32 bits
+  if (tiles >= (1LL << 24)) return false;  // tile indices (times at most 64 splits) in 32 bits
   q.nkb = (int)(q.Kp / kOzStageK);
   // chunks: equal shares of the batches, or of the row tiles of A, within the budget of planes
   const int64_t plane_row = (int64_t)kOzDigits * q.Kp * 2;

@@ -177,9 +177,12 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
     }
     const int64_t rows = cnt * n_unocc;
     // Mmn_[m].bottomRows(n_unocc), as the reference reads it
-    launch_pdl(rpa_chi_kernel, g1d(rows), 256, 0, s, dE.get(), cnt, m0, n_unocc, lumo - rpamin, wr, wi, eta, chi.get());
+    launch_pdl(rpa_chi_kernel, g1d(rows), 256, 0, s, dE.get(), cnt, m0, n_unocc, lumo - rpamin, wr, wi, eta,
+               chi.get());
     VGB_LAUNCH_CHECK();
-    launch_pdl(rpa_weights_kernel, (unsigned)std::min<int64_t>(cnt * naux, 64LL * sm_count()), 128, 0, s, raw.get(), n_unocc, naux, nsize, nsize - n_unocc, chi.get(), B.get(), Bw.get(), rows, cnt * naux);
+    launch_pdl(rpa_weights_kernel, (unsigned)std::min<int64_t>(cnt * naux, 64LL * sm_count()), 128, 0, s,
+               raw.get(), n_unocc, naux, nsize, nsize - n_unocc, chi.get(), B.get(), Bw.get(), rows,
+               cnt * naux);
     VGB_LAUNCH_CHECK();
     GemmDesc g;  // eps (+)= B^T Bw
     g.M = naux; g.N = naux; g.K = rows;
@@ -210,7 +213,7 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
   for (int64_t j = 0; j < n; j += NB) {
     const int nb = (int)std::min<int64_t>(NB, n - j);
     launch_pdl(chol_block_kernel, 1, 256, 0, s, A.get() + j + n * j, n, nb, L.get() + j + n * j, n,
-                                                 Y.get() + j + n * j, n, info.get(), j);
+               Y.get() + j + n * j, n, info.get(), j);
     VGB_LAUNCH_CHECK();
     const int64_t rest = n - j - nb;
     if (rest > 0) {

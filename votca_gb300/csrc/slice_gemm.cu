@@ -362,7 +362,8 @@ void slice_gemm(const SliceMat &A, const SliceMat &B, int64_t M, int64_t N, int6
   if (bn == 64) launch_digits<64>(digits, p, s);
   else launch_digits<32>(digits, p, s);
   if (p.groups > 1) {
-    launch_pdl(reduce_pairs_kernel, (unsigned)std::min<int64_t>(ceil_div(M * N, 256), 16LL * sm_count()), 256, 0, s, reinterpret_cast<const float2 *>(gpart.get()), M, N, p.groups, fe);
+    launch_pdl(reduce_pairs_kernel, (unsigned)std::min<int64_t>(ceil_div(M * N, 256), 16LL * sm_count()), 256,
+               0, s, reinterpret_cast<const float2 *>(gpart.get()), M, N, p.groups, fe);
     VGB_LAUNCH_CHECK();
   }
 }

@@ -10,7 +10,8 @@
 //      matrix fits (else in the job's global scratch): per column one reflector
 //      H = I - tau v v^T (v_0 = 1), p = tau A v, w = p - (tau/2)(p.v) v, A -= v w^T + w v^T.
 //   2. The wanted (lowest nw) eigenvalues of the tridiagonal matrix by bisection on the Sturm
-//      count in FP32, one thread per eigenvalue (FP32 runs at 64x the FP64 rate of GB300).
+//      count in FP32 (64x the FP64 rate of GB300), on groups of 7, 3 or 1 threads per
+//      eigenvalue that count at the points of its next 3, 2 or 1 steps at once.
 //   3. Eigenvectors by inverse iteration in FP64 with the tridiagonal LU with partial
 //      pivoting: two steps at the FP32 shift, then the FP64 Rayleigh quotient as the shift
 //      and two more steps (Rayleigh quotient iteration).  Eigenvalues closer than 1e-5 of the

@@ -734,8 +734,8 @@ void MixedEngine::build_dense_grouped(const std::vector<BseOperator *> &ops, con
       sj.push_back(j1);
       // Bc[(c1, c)][P] = M(c1, c, P) = Mcc[P][c][c1]: a transpose, done through shared memory
       const dim3 grid((unsigned)ceil_div(op.ct * op.ct, 32), (unsigned)ceil_div(op.naux, 32));
-      launch_pdl(transpose_split_cc_kernel, grid, dim3(32, 8), 0, s, op.Mcc.get(), op.naux, op.ct, Bc.hi.get() + boff[q],
-                                                            Bc.lo.get() + boff[q], m.Kn);
+      launch_pdl(transpose_split_cc_kernel, grid, dim3(32, 8), 0, s, op.Mcc.get(), op.naux, op.ct,
+                 Bc.hi.get() + boff[q], Bc.lo.get() + boff[q], m.Kn);
       VGB_LAUNCH_CHECK();
     }
     split_grouped(sj, s);
@@ -789,7 +789,9 @@ void MixedEngine::build_dense_grouped(const std::vector<BseOperator *> &ops, con
       const size_t q = t - a;
       if (c.cx == 0 && c.cd == 0)
         VGB_CUDA(cudaMemsetAsync(H.get() + hoff[q], 0, op.dim * op.dim * sizeof(double), s));
-      launch_pdl(symmetrize_kernel, (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(op.dim * op.dim, 256), 4096)), 256, 0, s, H.get() + hoff[q], op.dim);
+      launch_pdl(symmetrize_kernel,
+                 (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(op.dim * op.dim, 256), 4096)), 256,
+                 0, s, H.get() + hoff[q], op.dim);
       VGB_LAUNCH_CHECK();
       m.Kd = pad64(op.dim);
       m.Hdense.ensure(op.dim, m.Kd, s);

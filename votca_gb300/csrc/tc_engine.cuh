@@ -25,7 +25,8 @@ class MixedEngine {
   // (slice_f64): every operand cut into 7-bit digit planes with power-of-two scales per run of
   // at most 1024 K elements, the pairs of a digit level accumulated exactly in FP32 over at most
   // 512 of them, levels and runs summed as float pairs (in FP64 across CTAs), the intermediates kept as
-  // float pairs and sliced again.  With five digits the result agrees with the FP64 product to about 1e-11 of its scale.
+  // float pairs and sliced again.  With five digits the result agrees with the FP64 product to about
+  // 1e-11 of its scale.
   void apply_sliced(BseOperator &op, const Coef &c, const double *X, int64_t ldx, int64_t k, double *Y,
                     int64_t ldy, bool accumulate, cudaStream_t s);
   // FP64-accurate GEMM of FP64 operands on the tensor cores (the slice products of

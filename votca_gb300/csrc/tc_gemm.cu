@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     }
     for (int i = 0; i < C::NBUF; ++i) {
       mbar_init(&accf[i], 1);
-      mbar_init(&acce[i], kEpiWarps);  // one arrive per epilogue warp  // one arrive per epilogue warp
+      mbar_init(&acce[i], kEpiWarps);  // one arrive per epilogue warp
     }
     ctl->init(kWaitUs);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1102,10 +1102,13 @@ void slice_f64(const double *x, int64_t rows, int64_t cols, const SplitMap &m, i
   const F64In in{reinterpret_cast<const unsigned long long *>(x)};
   if (m.cs == 1 && chunk % 4 == 0 && m.rs1 % 4 == 0 && m.rs2 % 4 == 0 && ldo % 4 == 0 && plane % 4 == 0 &&
       ((uintptr_t)x & 31) == 0 && ((uintptr_t)out & 7) == 0) {
-    if (nslices == 5) launch_pdl(slice_run_kernel<F64In, 5>, blocks, 256, 0, s, in, rows, cols, m, chunk, out, ldo, plane);
-    else launch_pdl(slice_kernel<F64In, 4, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    if (nslices == 5) launch_pdl(slice_run_kernel<F64In, 5>, blocks, 256, 0, s, in, rows, cols, m, chunk, out,
+                                 ldo, plane);
+    else launch_pdl(slice_kernel<F64In, 4, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo,
+                    plane);
   } else {
-    launch_pdl(slice_kernel<F64In, 1, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    launch_pdl(slice_kernel<F64In, 1, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo,
+               plane);
   }
   VGB_LAUNCH_CHECK();
 }
@@ -1134,9 +1137,11 @@ void slice_pairs(const float *x2, int64_t rows, int64_t cols, const SplitMap &m,
         default: VGB_SLICE(8); break;
       }
 #undef VGB_SLICE
-    } else launch_pdl(slice_kernel<PairIn, 4, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    } else launch_pdl(slice_kernel<PairIn, 4, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out,
+                      ldo, plane);
   } else {
-    launch_pdl(slice_kernel<PairIn, 1, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo, plane);
+    launch_pdl(slice_kernel<PairIn, 1, 0>, blocks, 256, 0, s, in, rows, cols, m, nslices, chunk, out, ldo,
+               plane);
   }
   VGB_LAUNCH_CHECK();
 }
