@@ -235,4 +235,9 @@ int shim_slice_gemm(const double *A, const double *B, int64_t M, int64_t N, int6
   });
 }
 
+// A^-1 of a positive definite matrix with the factor in place of A's lower triangle.
+int shim_cholesky_inverse_in_place(int64_t n, const double *A, double *inv) {
+  return on_stream([&](cudaStream_t s) { vgb::cholesky_inverse(n, A, n, inv, n, s, true); });
+}
+
 }  // extern "C"

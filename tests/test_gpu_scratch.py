@@ -107,3 +107,19 @@ print("pool", r.value, t.value)
     r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split()[-3:] == ["pool", "0", "0"], r.stdout
+
+
+# n below, at and above the blocks (64) and their pairs, with a short last pair
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 190, 257, 449, 640])
+def test_cholesky_inverse_in_place(n):
+    """Without room for a third matrix, what the call took before the factor had one of its own."""
+    rng = np.random.default_rng(n)
+    B = rng.standard_normal((n, n + 20))
+    A = np.asfortranarray(B @ B.T / n + np.eye(n))
+    W = np.zeros((n, n), order="F")
+    L = native.load()
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    assert L.shim_cholesky_inverse_in_place(ctypes.c_int64(n), p(A), p(W)) == 0, L.shim_last_error()
+    # n eps |W| |A| |W| for the factorisation and the products each, |A| < 8, |W| <= 1
+    assert np.abs(W - np.linalg.inv(A)).max() < 16 * 8 * n * 2.0**-53
+    np.testing.assert_allclose(W, screening.cholesky_inverse(A), rtol=0, atol=16 * 8 * n * 2.0**-53)

@@ -199,10 +199,22 @@ void rpa_epsilon(const bse_mmn_desc &desc, const double *const *slices, const do
 }
 
 void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_host, int64_t ldi,
-                      cudaStream_t s) {
+                      cudaStream_t s, bool in_place) {
   VGB_REQUIRE(n >= 1 && lda >= n && ldi >= n, "cholesky_inverse: bad size");
-  // L beside A (the panel product then needs no copy), Y = L^-1
-  DeviceBuffer<double> A(n * n), L(n * n), Y(n * n), T((n / 2 + NB) * (n / 2 + NB) + n * NB);
+  // Y = L^-1; L beside A, so that the panel product needs no copy, or where there is no room for a third
+  // matrix in place of A's lower triangle, through a panel
+  DeviceBuffer<double> A(n * n), Y(n * n), Lbeside, panel;
+  if (!in_place) {
+    try {
+      Lbeside.resize((size_t)(n * n));
+    } catch (const Error &e) {
+      if (e.code != BSE_ERR_OUT_OF_MEMORY) throw;
+      cudaGetLastError();
+      in_place = true;
+    }
+  }
+  if (in_place) panel.resize((size_t)(n * NB));
+  double *const L = in_place ? A.get() : Lbeside.get();
   DeviceBuffer<int> info(1);
   GemmWorkspace ws;
   VGB_CUDA(cudaMemcpy2DAsync(A.get(), n * sizeof(double), a_host, lda * sizeof(double),
@@ -212,19 +224,23 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
   // right-looking blocked Cholesky: A = L L^T (lower), the diagonal blocks' inverses into Y
   for (int64_t j = 0; j < n; j += NB) {
     const int nb = (int)std::min<int64_t>(NB, n - j);
-    launch_pdl(chol_block_kernel, 1, 256, 0, s, A.get() + j + n * j, n, nb, L.get() + j + n * j, n,
+    launch_pdl(chol_block_kernel, 1, 256, 0, s, A.get() + j + n * j, n, nb, L + j + n * j, n,
                Y.get() + j + n * j, n, info.get(), j);
     VGB_LAUNCH_CHECK();
     const int64_t rest = n - j - nb;
     if (rest > 0) {
-      double *L21 = L.get() + (j + nb) + n * j;
+      double *A21 = A.get() + (j + nb) + n * j, *L21 = in_place ? panel.get() : L + (j + nb) + n * j;
+      const int64_t ld = in_place ? rest : n;
       GemmDesc t;  // L21 = A21 L11^-T
       t.M = rest; t.N = nb; t.K = nb;
-      t.a_colmajor(A.get() + (j + nb) + n * j, n, false).b_colmajor(Y.get() + j + n * j, n, true).c_colmajor(L21, n);
+      t.a_colmajor(A21, n, false).b_colmajor(Y.get() + j + n * j, n, true).c_colmajor(L21, ld);
       dgemm(t, s, &ws);
+      if (in_place)
+        VGB_CUDA(cudaMemcpy2DAsync(A21, n * sizeof(double), L21, ld * sizeof(double), rest * sizeof(double), nb,
+                                   cudaMemcpyDeviceToDevice, s));
       GemmDesc u;  // A22 -= L21 L21^T
       u.M = rest; u.N = rest; u.K = nb;
-      u.a_colmajor(L21, n, false).b_colmajor(L21, n, true).c_colmajor(A.get() + (j + nb) + n * (j + nb), n);
+      u.a_colmajor(L21, ld, false).b_colmajor(L21, ld, true).c_colmajor(A.get() + (j + nb) + n * (j + nb), n);
       u.alpha = -1.0; u.beta = 1.0;
       dgemm(u, s, &ws);
     }
@@ -237,7 +253,8 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
                                 std::to_string(hinfo) + ")");
   // Y = L^-1 by doubling: of [L11 0; L21 L22] with the inverses of both diagonal blocks of h rows,
   // Y21 = -Y22 (L21 Y11), all pairs of a level at once: 2 log2(n / 64) launches of large products
-  // in place of 5 small ones per block row.
+  // in place of 5 small ones per block row.  T lies in A, which is free beside L; with L in place in the
+  // upper triangle, transposed.
   for (int64_t h = NB; h < n; h *= 2) {
     const int64_t full = n / (2 * h);  // pairs of two whole blocks
     const int64_t i0 = full * 2 * h, last = n - i0 - h;  // a last pair whose second block is short
@@ -245,17 +262,20 @@ void cholesky_inverse(int64_t n, const double *a_host, int64_t lda, double *inv_
       const int64_t np = r == 0 ? full : (last > 0 ? 1 : 0), h2 = r == 0 ? h : last, o = r == 0 ? 0 : i0;
       if (np == 0) continue;
       const int64_t step = 2 * h * (n + 1);
+      double *T = A.get() + (in_place ? o + n * (o + h) : o + h + n * o);
+      const int64_t t_rs = in_place ? n : 1, t_cs = in_place ? 1 : n;
       GemmDesc t;  // T = L21 Y11
       t.M = h2; t.N = h; t.K = h;
-      t.a_colmajor(L.get() + o + h + n * o, n, false).b_colmajor(Y.get() + o + n * o, n, false).c_colmajor(T.get(), h2);
-      t.nb1 = np; t.a_b1 = step; t.b_b1 = step; t.c_b1 = h * h2;
+      t.a_colmajor(L + o + h + n * o, n, false).b_colmajor(Y.get() + o + n * o, n, false);
+      t.C = T; t.c_rs = t_rs; t.c_cs = t_cs;
+      t.nb1 = np; t.a_b1 = step; t.b_b1 = step; t.c_b1 = step;
       dgemm(t, s, &ws);
       GemmDesc u;  // Y21 = -Y22 T
       u.M = h2; u.N = h; u.K = h2;
-      u.a_colmajor(Y.get() + (o + h) * (n + 1), n, false).b_colmajor(T.get(), h2, false)
-          .c_colmajor(Y.get() + o + h + n * o, n);
+      u.a_colmajor(Y.get() + (o + h) * (n + 1), n, false).c_colmajor(Y.get() + o + h + n * o, n);
+      u.B = T; u.b_rs = t_rs; u.b_cs = t_cs;
       u.alpha = -1.0;
-      u.nb1 = np; u.a_b1 = step; u.b_b1 = h * h2; u.c_b1 = step;
+      u.nb1 = np; u.a_b1 = step; u.b_b1 = step; u.c_b1 = step;
       dgemm(u, s, &ws);
     }
   }
