@@ -53,9 +53,10 @@ typedef enum bse_precision {
                                by less than that of FMA chains in the 2-norm; the chain's bound,
                                K 2^-53 sum |a||x|, is not kept element by element: what lies
                                more than 2^56 below the largest element of its row or column
-                               (within 1024 terms) does not count.  Operands graded in opposite directions along K by more
-                               than 12 bits run as FMA chains; for callers that need that bound
-                               for every element, bse_op_matmul_device_noalloc always does.
+                               (within 1024 terms) does not count.  Operands graded in
+                               opposite directions along K by more than 12 bits run as FMA
+                               chains; for callers that need their bound for every element,
+                               bse_op_matmul_device_noalloc always does.
                                The dense operator, the screening, three-centre and dipole
                                entry points and the gradients use the same products. */
   BSE_PRECISION_MIXED = 1,  /* Hx/Hd/Hd2 contractions as BF16x3 split products on
