@@ -21,8 +21,8 @@
 // meet in a product above 2^-12, the tiles run as FMA.
 //
 // Measured on a GB300, FMA kernel against this one (L2 flushed between runs): 4096^3 110 ms and
-// 2.80 ms (49 TFLOP/s of FP64 results), the Hd stage 1 of eight vectors of v64 c512 and 256
-// auxiliary functions 55.1 and 1.72 ms, its stage 2 (K = 32768) 13.8 and 1.17 ms, 1000^3 1.71 and
+// 2.82 ms (49 TFLOP/s of FP64 results), the Hd stage 1 of eight vectors of v64 c512 and 256
+// auxiliary functions 55.1 and 1.76 ms, its stage 2 (K = 32768) 13.8 and 1.17 ms, 1000^3 1.71 and
 // 0.08 ms.
 #pragma once
 
