@@ -59,24 +59,26 @@ def test_large_planes_are_given_back():
     assert np.all(np.abs(C.reshape(N, M)[:, rows].T - ref) <= bound + 2.0**-52 * np.abs(ref))
 
 
-# bytes of planes per row: 14 Kp; budgets of a few row tiles or batches, K of one and of several
-# exponent segments (256) and runs (1024)
+# bytes of planes per row: 14 Kp; budgets of some row tiles (of the longer side, which the plan makes the
+# rows) and of one and two batches; K of one and of several exponent segments (256), runs (1024)
+# and K splits
 @pytest.mark.parametrize("K", [224, 257, 1100])
-@pytest.mark.parametrize("M,N,batch,rows", [(1000, 70, 1, 300), (1300, 65, 1, 128), (260, 130, 7, 600), (300, 257, 5, 310)])
+@pytest.mark.parametrize("M,N,batch,rows", [(130, 2600, 1, 900), (300, 2100, 1, 700), (260, 130, 7, 600), (300, 257, 5, 310)])
 def test_chunks(M, N, batch, rows, K):
     rng = np.random.default_rng(M + N + K)
     A, B = rng.standard_normal((batch, M, K)), rng.standard_normal((batch, K, N))
-    A *= 2.0 ** rng.integers(-30, 30, (batch, M, 1))  # every row its own exponent, also in reused tables
+    # every row and column its own exponent, also in reused tables
+    A *= 2.0 ** rng.integers(-30, 30, (batch, M, 1))
+    B *= 2.0 ** rng.integers(-30, 30, (batch, 1, N))
     C = rng.standard_normal((batch, M, N))
     C0 = C.copy()
     budget = rows * 14 * ((K + 31) // 32 * 32)
     ab, bb = (M * K, K * N) if batch > 1 else (0, 0)
-    # a product this small stays with the FMA kernel unless the plan finds it faster: both are checked
     taken, _ = _product([M, N, K, batch, 1, K, 1, ab, 0, N, 1, bb, 0, N, 1, M * N, 0], A, B, C, -2.0, 0.5, budget)
-    if not taken:
-        pytest.skip("left to the FMA kernel")
-    ref = -2.0 * (A.astype(np.longdouble) @ B.astype(np.longdouble)) + 0.5 * C0
-    bound = 2.0 * K * 2.0**-53 * np.abs(A).max(axis=2)[:, :, None] * np.abs(B).max(axis=1)[:, None, :]
+    assert taken == 1
+    ref = -2.0 * (A @ B) + 0.5 * C0  # itself a chain of K terms
+    bound = 2.0 * K * 2.0**-53 * (np.abs(A).max(axis=2)[:, :, None] * np.abs(B).max(axis=1)[:, None, :]
+                                  + np.abs(A) @ np.abs(B))
     assert np.all(np.abs(C - ref) <= bound + 2.0**-51 * (np.abs(ref) + np.abs(C0)))
 
 
