@@ -98,9 +98,9 @@ def test_dense_screening_staging(name):
     assert run(0) == 0
 
 
-@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("which", [[0], [1], [2], [0, 1, 2]])
 def test_lockstep_batch(which):
-    """Every molecule's products, whichever place it has in the batch."""
+    """Every molecule's products, whichever place it has in the batch, and of several none is left over."""
     ctxs = [_context(seed=s, c=c) for s, c in ((5, 20), (6, 31), (7, 12))]
     ops = [bo.SingletOperator_TDA(x) for x in ctxs]
 
@@ -110,7 +110,8 @@ def test_lockstep_batch(which):
         return ds.solve_batch(ops, 2)
 
     ref = call()[0]
-    _plant(ctxs[which])
+    for w in which:
+        _plant(ctxs[w])
     _times_out(call)
     np.testing.assert_array_equal(call()[0], ref)
     for x in ctxs:
@@ -184,3 +185,16 @@ def test_wait_limit(M, N, K):
     bound = K * 2.0**-53 * np.abs(A).max(axis=1)[:, None] * np.abs(B).max(axis=0)[None, :]
     ref = A.astype(np.longdouble) @ B.astype(np.longdouble)
     assert np.all(np.abs(C - ref) <= bound + 2.0**-52 * np.abs(ref))
+
+
+def test_workspace_and_engine_at_once():
+    """A split-precision handle with a code in its workspace and one in its engine: one call reports both."""
+    ctx = _context(precision=bo.PRECISION_MIXED)
+    op = bo.SingletOperator_TDA(ctx)
+    X = _vectors(ctx, 3)
+    ref = op.matmul(X)
+    _plant(ctx)
+    native.load().shim_plant_engine_error(ctx.handle, 3)
+    _times_out(lambda: op.matmul(X))
+    np.testing.assert_array_equal(op.matmul(X), ref)
+    ctx.close()

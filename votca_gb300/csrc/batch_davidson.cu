@@ -1043,16 +1043,18 @@ void davidson_solve_batch(const std::vector<BseOperator *> &ops, const Coef &coe
       // are applied one by one, and of the first dense and the first factorised operator, which the
       // grouped stages report into.
       bool seen[2] = {false, false};
+      FirstError gave_up;
       for (Mol *M : act) {
         BseOperator &op = *M->op;
         const bool grouped = op.precision == BSE_PRECISION_MIXED && op.mixed;
         if (grouped && seen[M->dense]) {
-          op.ws.check();
+          gave_up.run([&] { op.ws.check(); });
           continue;
         }
-        op.check_errors(s);
+        gave_up.run([&] { op.check_errors(s); });
         if (grouped) seen[M->dense] = true;
       }
+      gave_up.raise();
       for (size_t b = 0; b < nm; ++b) {
         if (hflags[b]) fail(BSE_ERR_NUMERICAL, "molecule " + std::to_string(b) + ": Linear dependencies in Gram-Schmidt.");
         if (hflags[nm + b]) fail(BSE_ERR_NUMERICAL, "molecule " + std::to_string(b) + ": Small hermitian eigenvalue problem failed.");

@@ -706,8 +706,10 @@ void matmul_grouped(const Coef &c, const std::vector<GroupedItem> &items, cudaSt
 }
 
 void BseOperator::check_errors(cudaStream_t s) {
-  ws.check();
-  if (mixed) mixed->check(s);
+  FirstError e;
+  e.run([&] { ws.check(); });
+  if (mixed) e.run([&] { mixed->check(s); });
+  e.raise();
 }
 
 void BseOperator::diagonal(const Coef &c, double *D, cudaStream_t s) {

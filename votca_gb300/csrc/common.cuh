@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <exception>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -21,6 +22,23 @@ struct Error : std::runtime_error {
 };
 
 [[noreturn]] inline void fail(int code, const std::string &msg) { throw Error(code, msg); }
+
+// Several checks of which each takes back what it reports: all of them run, and the first error is raised,
+// so that none is left for a later call.
+struct FirstError {
+  std::exception_ptr first;
+  template <class F>
+  void run(F &&f) {
+    try {
+      f();
+    } catch (...) {
+      if (!first) first = std::current_exception();
+    }
+  }
+  void raise() const {
+    if (first) std::rethrow_exception(first);
+  }
+};
 
 inline void cuda_check(cudaError_t e, const char *what, const char *file, int line) {
   if (e != cudaSuccess) {

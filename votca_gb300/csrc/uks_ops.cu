@@ -215,9 +215,11 @@ void UksOperator::ham_matmul(const Coef &a, const Coef &b, const double *X, int6
 }
 
 void UksOperator::check_errors(cudaStream_t s) {
-  ws_.check();
-  if (alpha.dim > 0) alpha.check_errors(s);
-  if (beta.dim > 0) beta.check_errors(s);
+  FirstError e;
+  e.run([&] { ws_.check(); });
+  if (alpha.dim > 0) e.run([&] { alpha.check_errors(s); });
+  if (beta.dim > 0) e.run([&] { beta.check_errors(s); });
+  e.raise();
 }
 
 }  // namespace vgb
