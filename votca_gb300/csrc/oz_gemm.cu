@@ -292,7 +292,8 @@ struct GemmArgs {
   int64_t m_first, b_first;  // first C row and batch of this launch (chunks)
   int mt, nt, ntiles;
   const int *erow_a, *erow_b, *flag;
-  const int *prof_a, *prof_b;
+  const int *prof_a, *prof_b;  // 4 nprof each
+  int nprof;
   Operand A, B;              // sources, for the FMA path
   OzMap crow, ccol, cbatch;  // C offsets of tile rows, columns and batches
   int64_t c_split;           // C offset between K splits (partials)
@@ -592,17 +593,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1) oz_gemm_kernel(const __grid_c
     // row, are too few for the whole result.  The same on every CTA.
     {
       int any_a = 0, any_b = 0;
-      bool meet = false;  // as a rule among the first K elements
-      for (int64_t k0 = 0; k0 < p.K && !__any_sync(0xffffffffu, meet); k0 += 4 * 32 * kTab)
+      bool meet = false;  // as a rule among the first K elements; unit vectors may have theirs last
+      const int4 *qa = reinterpret_cast<const int4 *>(p.prof_a), *qb = reinterpret_cast<const int4 *>(p.prof_b);
+      auto one = [&](int a, int b) {
+        a = max(a, 0) >> 7;
+        b = max(b, 0) >> 7;
+        any_a |= a;
+        any_b |= b;
+        meet |= a && b && a + b >= 2 * TOP - kOpposed;
+      };
+      for (int k0 = 0; k0 < p.nprof && !__any_sync(0xffffffffu, meet); k0 += 4 * 32 * kTab) {
+        int4 a[4], b[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int64_t k = k0 + u * 32 * kTab + i;
-          const int a = k < p.K ? max(__ldcg(p.prof_a + k), 0) >> 7 : 0;
-          const int b = k < p.K ? max(__ldcg(p.prof_b + k), 0) >> 7 : 0;
-          any_a |= a;
-          any_b |= b;
-          meet |= a && b && a + b >= 2 * TOP - kOpposed;
+          const int k = k0 + u * 32 * kTab + i;
+          a[u] = k < p.nprof ? __ldcg(qa + k) : make_int4(0, 0, 0, 0);
+          b[u] = k < p.nprof ? __ldcg(qb + k) : make_int4(0, 0, 0, 0);
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          one(a[u].x, b[u].x);
+          one(a[u].y, b[u].y);
+          one(a[u].z, b[u].z);
+          one(a[u].w, b[u].w);
+        }
+      }
       if (any_a) s_meet[0] = 1;
       if (any_b) s_meet[1] = 1;
       if (meet) s_meet[2] = 1;
@@ -770,8 +785,8 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   const int64_t nseg = ceil_div(q.Kp, SEG);
   const bool two = nseg > 1;  // exponents before digits
   const int64_t rows_a = q.m_chunk * q.tb_chunk, rows_b = q.N * q.tb_chunk;
-  // [flag | row exponents of A | of B | K profiles of A | of B], then run exponents
-  const int64_t ni = 64 + rows_a + rows_b + 2 * q.Kp;
+  // [flag | K profiles of A | of B (16-byte aligned) | row exponents of A | of B], then run exponents
+  const int64_t ni = 64 + 2 * q.Kp + rows_a + rows_b;
   double *partial = nullptr;
   Planes pa(stream), pb(stream);
   try {
@@ -805,11 +820,11 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
   A.planes = pa.p;
   B.planes = pb.p;
   int *ip = ws->oz_int.get();
-  A.erow = ip + 64;
-  B.erow = A.erow + rows_a;
-  A.prof = B.erow + rows_b;
+  A.prof = ip + 64;
   B.prof = A.prof + q.Kp;
-  A.erun = B.prof + q.Kp;
+  A.erow = B.prof + q.Kp;
+  B.erow = A.erow + rows_a;
+  A.erun = B.erow + rows_b;
   B.erun = A.erun + rows_a * nruns;
   p.K = d.K;
   p.nkb = q.nkb;
@@ -876,6 +891,7 @@ bool oz_dgemm(const GemmDesc &d, cudaStream_t stream, GemmWorkspace *ws) {
       p.erow_b = B.erow;
       p.prof_a = A.prof;
       p.prof_b = B.prof;
+      p.nprof = (int)(q.Kp / 4);
       p.mt = (int)ceil_div(p.M, BM);
       p.nt = (int)ceil_div(p.N, BN);
       p.ntiles = (int)(p.mt * p.nt * tn * q.splits);
